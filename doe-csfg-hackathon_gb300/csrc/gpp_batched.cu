@@ -71,11 +71,12 @@ batched_reduce_kernel(const ReduceJob *jobs, const int *seg_prefix, int njobs) {
 }
 
 // Persistent FP64 kernel over a list of tiles.
-template <int RN, int RG, int NWC>
+// NWC frequencies per unoccupied-band tile, NWCF per occupied-band tile.
+template <int RN, int RG, int NWC, int NWCF>
 __global__ void __launch_bounds__(kThreads)
 batched_fp64_kernel(const Problem *probs, const Partials *parts, const BatchItem *items,
                     int n_items, int *head) {
-    constexpr int KN = RN * RG * NWC * 2, KF = RG * NWC * 4;
+    constexpr int KN = RN * RG * NWC * 2, KF = RG * NWCF * 4;
     constexpr int K = KN > KF ? KN : KF;
     __shared__ double red[(kThreads / 32) * K];
     __shared__ double S[K];
@@ -91,11 +92,11 @@ batched_fp64_kernel(const Problem *probs, const Partials *parts, const BatchItem
         const Partials part = parts[bi.state];
         if (bi.kind == 0) {
             if (p.semantics == kSemKerSeq)
-                flag_fp64_tile<RG, NWC, kThreads, kSemKerSeq>(p, part, bi.row_tile, bi.band_tile,
-                                                              bi.iw_chunk, bi.tile, red, S);
+                flag_fp64_tile<RG, NWCF, 1, kThreads, kSemKerSeq>(
+                    p, part, bi.row_tile, bi.band_tile, bi.iw_chunk, (p.ng + RG - 1) / RG, red, S);
             else
-                flag_fp64_tile<RG, NWC, kThreads, kSemComplexSeq>(
-                    p, part, bi.row_tile, bi.band_tile, bi.iw_chunk, bi.tile, red, S);
+                flag_fp64_tile<RG, NWCF, 1, kThreads, kSemComplexSeq>(
+                    p, part, bi.row_tile, bi.band_tile, bi.iw_chunk, (p.ng + RG - 1) / RG, red, S);
         } else {
             noflag_fp64_tile<RN, RG, NWC, kThreads>(p, part, p.nv, p.nb, bi.row_tile,
                                                     bi.band_tile, bi.iw_chunk, bi.tile, red, S);
@@ -108,7 +109,7 @@ batched_fp64_kernel(const Problem *probs, const Partials *parts, const BatchItem
 // register-heavy) and unoccupied-band tiles (shared-memory pipeline) run as
 // two launches so each keeps its own occupancy.
 template <int NWC, int FRG>
-__global__ void __launch_bounds__(kThreads, NWC <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, 3)
 batched_flag_mixed_kernel(const Problem *probs, const Partials *parts, const SplitPlanes *splits,
                           const BatchItem *items, int n_items, int *head) {
     constexpr int KF = FRG * NWC * 4;
@@ -257,6 +258,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     const bool mixed = precision == GPP_PRECISION_MIXED;
     const int nwc = nw <= 4 ? nw : 8;
     const int nchunk = (nw + nwc - 1) / nwc;
+    const int nwcf = flag_nwc(nw), nchunk_f = (nw + nwcf - 1) / nwcf;
 
     // Tile geometry shared by the planner and the kernels.
     Problem p0{};
@@ -356,11 +358,12 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
             const Problem &p = b->probs[i];
             const StateGeom &s = g[i];
             const double tile_cost = (double)p.nc;
-            for (int c = 0; c < nchunk; ++c) {
+            for (int c = 0; c < nchunk_f; ++c)
                 for (int band = 0; band < (s.tiles_f ? p.nv : 0); ++band)
                     for (int r = 0; r < s.rows_f; ++r)
                         flag.push_back({tile_cost * (mixed ? 1.5 : 1.25),
                                         BatchItem{i, 0, r, band, c, (int)(band * s.rows_f + r)}});
+            for (int c = 0; c < nchunk; ++c) {
                 const long long bt = s.tiles_n ? s.tiles_n / s.rows_n : 0;
                 for (long long t = 0; t < bt; ++t)
                     for (int r = 0; r < s.rows_n; ++r)
@@ -480,10 +483,10 @@ gpp_status upload_tables(gpp_batch *b, int *fault_word) {
     return GPP_OK;
 }
 
-// Launch configuration of the persistent kernels for a frequency chunk NWC:
-// dynamic shared memory (opted in here, outside any stream capture) and the
+// Launch configuration of the persistent kernels for frequency chunks NWC
+// (unoccupied bands) and NWCF (occupied bands): dynamic shared memory (opted in here, outside any stream capture) and the
 // resident grid sizes.
-template <int NWC>
+template <int NWC, int NWCF = NWC>
 cudaError_t prepare_persistent(gpp_batch *b) {
     if (b->precision == GPP_PRECISION_MIXED) {
         constexpr int RG = 2;  // one row pair of the split planes
@@ -505,16 +508,16 @@ cudaError_t prepare_persistent(gpp_batch *b) {
             if (e != cudaSuccess) return e;
             b->grid = resident_blocks(kern, b->smem);
         }
-        b->grid_flag = resident_blocks(batched_flag_mixed_kernel<NWC, 2>, 0);
+        b->grid_flag = resident_blocks(batched_flag_mixed_kernel<NWCF, 2>, 0);
     } else {
         constexpr int RN = NWC <= 4 ? 4 : 2;
         b->smem = 0;
-        b->grid = b->grid_flag = resident_blocks(batched_fp64_kernel<RN, 2, NWC>, 0);
+        b->grid = b->grid_flag = resident_blocks(batched_fp64_kernel<RN, 2, NWC, NWCF>, 0);
     }
     return cudaGetLastError();
 }
 
-template <int NWC>
+template <int NWC, int NWCF = NWC>
 cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
     const auto &w = b->waves[wave];
     int *heads = b->d_heads + 2 * wave;
@@ -523,7 +526,7 @@ cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
         constexpr int RG = 2;  // one row pair of the split planes
         const int nf = w.i_mid - w.i0, nu = w.i1 - w.i_mid;
         if (nf > 0) {
-            batched_flag_mixed_kernel<NWC, 2><<<std::min(nf, b->grid_flag), kThreads, 0, s>>>(
+            batched_flag_mixed_kernel<NWCF, 2><<<std::min(nf, b->grid_flag), kThreads, 0, s>>>(
                 b->d_probs, b->d_parts, b->d_splits, b->d_items + w.i0, nf, heads);
             e = cudaGetLastError();
         }
@@ -547,7 +550,7 @@ cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
         constexpr int RN = NWC <= 4 ? 4 : 2;
         const int n = w.i1 - w.i0;
         if (n > 0) {
-            batched_fp64_kernel<RN, 2, NWC><<<std::min(n, b->grid), kThreads, 0, s>>>(
+            batched_fp64_kernel<RN, 2, NWC, NWCF><<<std::min(n, b->grid), kThreads, 0, s>>>(
                 b->d_probs, b->d_parts, b->d_items + w.i0, n, heads);
             e = cudaGetLastError();
         }
@@ -561,7 +564,7 @@ cudaError_t prepare(gpp_batch *b) {
         case 2: return prepare_persistent<2>(b);
         case 3: return prepare_persistent<3>(b);
         case 4: return prepare_persistent<4>(b);
-        default: return prepare_persistent<8>(b);
+        default: return flag_nwc(b->nw) == 3 ? prepare_persistent<8, 3>(b) : prepare_persistent<8, 4>(b);
     }
 }
 
@@ -588,7 +591,10 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
             case 2: e = launch_persistent<2>(b, (int)wv, s); break;
             case 3: e = launch_persistent<3>(b, (int)wv, s); break;
             case 4: e = launch_persistent<4>(b, (int)wv, s); break;
-            default: e = launch_persistent<8>(b, (int)wv, s); break;
+            default:
+                e = flag_nwc(b->nw) == 3 ? launch_persistent<8, 3>(b, (int)wv, s)
+                                         : launch_persistent<8, 4>(b, (int)wv, s);
+                break;
         }
         launches += 2;
     }

@@ -43,39 +43,31 @@ noflag_fp64_kernel(Problem p, Partials part, int band_begin, int band_end, int r
                                            red, S);
 }
 
-template <int RG, int NWC, int THREADS, int SEM>
-__global__ void __launch_bounds__(THREADS)
-flag_fp64_kernel(Problem p, Partials part, int row_tile0, int row_tiles) {
-    constexpr int K = RG * NWC * 4;
-    __shared__ double red[(THREADS / 32) * K];
-    __shared__ double S[K];
-    const int row_tile = row_tile0 + blockIdx.x;
-    flag_fp64_tile<RG, NWC, THREADS, SEM>(p, part, row_tile, blockIdx.y, blockIdx.z,
-                                          (long long)blockIdx.y * row_tiles + row_tile, red, S);
-}
-
-// Band-independent frequencies: blockIdx.y covers NB occupied bands and
-// blockIdx.z a frequency chunk, blockIdx.x one of `count` row tiles from
-// row_tile0.  With `next` set, a persistent grid instead: each block takes
-// (row tile, band group, chunk) items from the counter until none is left,
+// Occupied bands: blockIdx.x is one of `count` row tiles from row_tile0,
+// blockIdx.y a group of NB bands (NB > 1: band-independent frequencies) and
+// blockIdx.z a frequency chunk (the grid's z strides over the chunks).
+// With `next` set, a persistent grid instead: each block takes (row tile,
+// band group, chunk) items from the counter until none is left,
 // so blocks that share an SM take fewer; every item is computed and written
 // as in the one-tile grid, so the bits do not depend on the grid.
 template <int RG, int NWC, int NB, int THREADS, int SEM>
 __global__ void __launch_bounds__(THREADS)
-flag_fp64_multi_kernel(Problem p, Partials part, int row_tile0, int count, int row_tiles,
-                       int *next) {
+flag_fp64_kernel(Problem p, Partials part, int row_tile0, int count, int row_tiles, int *next) {
     constexpr int K = NB * RG * NWC * 4;
     __shared__ double red[(THREADS / 32) * K];
     __shared__ double S[K];
     __shared__ int item;
+    const int chunks = (p.nw + NWC - 1) / NWC;
     if (!next) {
-        flag_fp64_multi_tile<RG, NWC, NB, THREADS, SEM>(p, part, row_tile0 + blockIdx.x,
-                                                        blockIdx.y * NB, blockIdx.z, row_tiles,
-                                                        red, S);
+        for (int z = blockIdx.z; z < chunks; z += gridDim.z) {
+            flag_fp64_tile<RG, NWC, NB, THREADS, SEM>(p, part, row_tile0 + blockIdx.x,
+                                                      blockIdx.y * NB, z, row_tiles, red, S);
+            __syncthreads();  // S read by the epilogue before the next chunk
+        }
         return;
     }
     const int groups = (p.nv + NB - 1) / NB;
-    const long long items = (long long)count * groups * ((p.nw + NWC - 1) / NWC);
+    const long long items = (long long)count * groups * chunks;
     for (;;) {
         if (threadIdx.x == 0) item = atomicAdd(next, 1);
         __syncthreads();
@@ -83,9 +75,8 @@ flag_fp64_multi_kernel(Problem p, Partials part, int row_tile0, int count, int r
         if (it >= items) break;
         const int t = (int)(it % count);
         const long long rest = it / count;
-        flag_fp64_multi_tile<RG, NWC, NB, THREADS, SEM>(p, part, row_tile0 + t,
-                                                        (int)(rest % groups) * NB,
-                                                        (int)(rest / groups), row_tiles, red, S);
+        flag_fp64_tile<RG, NWC, NB, THREADS, SEM>(p, part, row_tile0 + t, (int)(rest % groups) * NB,
+                                                  (int)(rest / groups), row_tiles, red, S);
         __syncthreads();  // S read by the epilogue, `item` by every thread, before reuse
     }
 }
@@ -166,13 +157,15 @@ bool flag_multi_enabled() {
 }
 
 template <int RG, int NWC, int NB, int THREADS>
-cudaError_t launch_flag_multi_t(const Problem &p, const Partials &part, RowTiles r, int row_tiles,
-                                int blocks_per_sm, int *next, cudaStream_t s) {
+cudaError_t launch_flag_nb(const Problem &p, const Partials &part, RowTiles r, int row_tiles,
+                           int blocks_per_sm, int *next, cudaStream_t s) {
     const int count = r.end - r.begin;
-    dim3 grid(count, ceil_div(p.nv, NB), ceil_div(p.nw, NWC));
+    const int chunks = ceil_div(p.nw, NWC);
+    dim3 grid(count, ceil_div(p.nv, NB), std::min(chunks, 65535));
     // The counter is a 32-bit int: past 2^30 items the one-tile grid instead.
-    const long long items = (long long)count * grid.y * grid.z;
-    const int per_sm = next && items < (1ll << 30) ? flag_blocks_per_sm(blocks_per_sm) : 0;
+    const long long items = (long long)count * grid.y * chunks;
+    const int per_sm =
+        NB > 1 && next && items < (1ll << 30) ? flag_blocks_per_sm(blocks_per_sm) : 0;
     if (per_sm > 0) {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
@@ -184,12 +177,12 @@ cudaError_t launch_flag_multi_t(const Problem &p, const Partials &part, RowTiles
         next = nullptr;
     }
     if (p.semantics == kSemKerSeq) {
-        prefer_max_shared(flag_fp64_multi_kernel<RG, NWC, NB, THREADS, kSemKerSeq>);
-        flag_fp64_multi_kernel<RG, NWC, NB, THREADS, kSemKerSeq><<<grid, THREADS, 0, s>>>(
+        prefer_max_shared(flag_fp64_kernel<RG, NWC, NB, THREADS, kSemKerSeq>);
+        flag_fp64_kernel<RG, NWC, NB, THREADS, kSemKerSeq><<<grid, THREADS, 0, s>>>(
             p, part, r.begin, count, row_tiles, next);
     } else {
-        prefer_max_shared(flag_fp64_multi_kernel<RG, NWC, NB, THREADS, kSemComplexSeq>);
-        flag_fp64_multi_kernel<RG, NWC, NB, THREADS, kSemComplexSeq><<<grid, THREADS, 0, s>>>(
+        prefer_max_shared(flag_fp64_kernel<RG, NWC, NB, THREADS, kSemComplexSeq>);
+        flag_fp64_kernel<RG, NWC, NB, THREADS, kSemComplexSeq><<<grid, THREADS, 0, s>>>(
             p, part, r.begin, count, row_tiles, next);
     }
     count_launch();
@@ -202,23 +195,9 @@ cudaError_t launch_flag_t(const Problem &p, const Partials &part, RowTiles rt, i
     const int row_tiles = ceil_div(p.ng, RG);
     const RowTiles r = rt.clip(row_tiles);
     if (r.end <= r.begin) return cudaSuccess;
-    if constexpr (NWC <= 4) {  // two bands of 8 frequencies would spill
-        if (p.wx_stride == 0 && p.nv >= 2 && flag_multi_enabled())
-            return launch_flag_multi_t<RG, NWC, 2, THREADS>(p, part, r, row_tiles, blocks_per_sm,
-                                                            next, s);
-    }
-    dim3 grid(r.end - r.begin, p.nv, ceil_div(p.nw, NWC));
-    if (p.semantics == kSemKerSeq) {
-        prefer_max_shared(flag_fp64_kernel<RG, NWC, THREADS, kSemKerSeq>);
-        flag_fp64_kernel<RG, NWC, THREADS, kSemKerSeq><<<grid, THREADS, 0, s>>>(p, part, r.begin,
-                                                                                row_tiles);
-    } else {
-        prefer_max_shared(flag_fp64_kernel<RG, NWC, THREADS, kSemComplexSeq>);
-        flag_fp64_kernel<RG, NWC, THREADS, kSemComplexSeq><<<grid, THREADS, 0, s>>>(
-            p, part, r.begin, row_tiles);
-    }
-    count_launch();
-    return cudaGetLastError();
+    if (p.wx_stride == 0 && p.nv >= 2 && flag_multi_enabled())
+        return launch_flag_nb<RG, NWC, 2, THREADS>(p, part, r, row_tiles, blocks_per_sm, next, s);
+    return launch_flag_nb<RG, NWC, 1, THREADS>(p, part, r, row_tiles, 0, nullptr, s);
 }
 
 }  // namespace
@@ -237,7 +216,7 @@ TileShape fp64_noflag_shape(const Problem &p) {
     return nwc <= 4 ? TileShape{4, 2, nwc, 128} : TileShape{2, 2, nwc, 128};
 }
 
-TileShape flag_shape(const Problem &p) { return TileShape{1, 2, nwc_for(p.nw), 128}; }
+TileShape flag_shape(const Problem &p) { return TileShape{1, 2, flag_nwc(p.nw), 128}; }
 
 cudaError_t launch_noflag_fp64(const Problem &p, const Partials &part, int b0, int b1,
                                cudaStream_t s, RowTiles rt) {
@@ -254,12 +233,11 @@ cudaError_t launch_noflag_fp64(const Problem &p, const Partials &part, int b0, i
 cudaError_t launch_flag_fp64(const Problem &p, const Partials &part, cudaStream_t s, RowTiles rt,
                              int blocks_per_sm, int *next) {
     if (p.nv <= 0 || p.ng == 0) return cudaSuccess;
-    switch (nwc_for(p.nw)) {
+    switch (flag_nwc(p.nw)) {
         case 1: return launch_flag_t<2, 1, 128>(p, part, rt, blocks_per_sm, next, s);
         case 2: return launch_flag_t<2, 2, 128>(p, part, rt, blocks_per_sm, next, s);
         case 3: return launch_flag_t<2, 3, 128>(p, part, rt, blocks_per_sm, next, s);
-        case 4: return launch_flag_t<2, 4, 128>(p, part, rt, blocks_per_sm, next, s);
-        default: return launch_flag_t<2, 8, 128>(p, part, rt, blocks_per_sm, next, s);
+        default: return launch_flag_t<2, 4, 128>(p, part, rt, blocks_per_sm, next, s);
     }
 }
 

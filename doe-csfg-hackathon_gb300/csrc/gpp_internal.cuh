@@ -105,20 +105,8 @@ __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
     return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
                         __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
-__device__ __forceinline__ double2 cmul_conj_b_rn(double2 a, double2 b) {  // a * conj(b)
-    return make_double2(__fma_rn(a.x, b.x, __dmul_rn(a.y, b.y)),
-                        __fma_rn(a.y, b.x, -__dmul_rn(a.x, b.y)));
-}
 __device__ __forceinline__ double2 cscale_rn(double2 a, double s) {
     return make_double2(__dmul_rn(a.x, s), __dmul_rn(a.y, s));
-}
-__device__ __forceinline__ double abs2_rn(double2 a) {
-    return __fma_rn(a.x, a.x, __dmul_rn(a.y, a.y));
-}
-// acc + a*b in two FMAs per component.
-__device__ __forceinline__ double2 cmul_acc_rn(double2 acc, double2 a, double2 b) {
-    return make_double2(__fma_rn(a.x, b.x, __fma_rn(-a.y, b.y, acc.x)),
-                        __fma_rn(a.x, b.y, __fma_rn(a.y, b.x, acc.y)));
 }
 
 // FP64 reciprocal: hardware seed (rcp.approx.ftz.f64, issued to the

@@ -36,6 +36,13 @@ struct RowTiles {
     }
 };
 
+// Frequencies per occupied-band tile: at most 4 (8 would put two complex sums
+// per row and frequency past the register file), or 3 where that leaves fewer
+// empty places in the last chunk.
+__host__ __device__ constexpr int flag_nwc(int nw) {
+    return nw <= 4 ? nw : (nw + 2) / 3 * 3 < (nw + 3) / 4 * 4 ? 3 : 4;
+}
+
 // Unoccupied bands [band_begin, band_end), FP64.  Writes one ach partial per
 // (row tile, band tile) block and, when part.n1 is set, per-band partials.
 cudaError_t launch_noflag_fp64(const Problem &p, const Partials &part, int band_begin,

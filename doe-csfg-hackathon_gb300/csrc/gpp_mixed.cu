@@ -26,6 +26,8 @@
 // Work decomposition: a block owns one row pair x 4 bands x NWC frequencies,
 // threads stride over ig, and a grouped tile order keeps GROUP row tiles
 // resident in L2 while all band tiles stream past them.
+#include <algorithm>
+
 #include "gpp_kernels.h"
 #include "gpp_tiles_mixed.cuh"
 
@@ -283,27 +285,29 @@ cudaError_t launch_split(const Problem &p, void *split_ws, int b0, int b1, cudaS
     return e;
 }
 
-// Three resident blocks (at most 168 registers) for up to 4 frequencies:
-// the occupied-band kernel is latency-bound, and the third block beat the
-// compiler's 222-register choice by 15% (4 blocks spilled and lost).
+// Three resident blocks (at most 168 registers).
 template <int RG, int NWC, int THREADS, int SEM>
-__global__ void __launch_bounds__(THREADS, NWC <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(THREADS, 3)
 flag_mixed_kernel(Problem p, Partials part, SplitPlanes s, int row_tile0, int count,
                   int row_tiles, int *next) {
     constexpr int K = RG * NWC * 4;
     __shared__ double red[(THREADS / 32) * K];
     __shared__ double S[K];
     __shared__ int item;
+    const int chunks = (p.nw + NWC - 1) / NWC;
     if (!next) {
         const int row_tile = row_tile0 + blockIdx.x;
-        flag_mixed_tile<RG, NWC, THREADS, SEM>(p, part, s, row_tile, blockIdx.y, blockIdx.z,
-                                               (long long)blockIdx.y * row_tiles + row_tile, red,
-                                               S);
+        for (int z = blockIdx.z; z < chunks; z += gridDim.z) {
+            flag_mixed_tile<RG, NWC, THREADS, SEM>(p, part, s, row_tile, blockIdx.y, z,
+                                                   (long long)blockIdx.y * row_tiles + row_tile,
+                                                   red, S);
+            __syncthreads();  // S read by the epilogue before the next chunk
+        }
         return;
     }
     // Persistent grid beside the tensor-core GEMM: (row tile, band, chunk)
     // items from the counter, each computed and written as in the grid above.
-    const long long items = (long long)count * p.nv * ((p.nw + NWC - 1) / NWC);
+    const long long items = (long long)count * p.nv * chunks;
     for (;;) {
         if (threadIdx.x == 0) item = atomicAdd(next, 1);
         __syncthreads();
@@ -325,9 +329,10 @@ cudaError_t launch_flag_mixed_t(const Problem &p, const Partials &part, const Sp
     const RowTiles r = rt.clip(row_tiles);
     if (r.end <= r.begin) return cudaSuccess;
     const int count = r.end - r.begin;
-    dim3 grid(count, p.nv, ceil_div(p.nw, NWC));
+    const int chunks = ceil_div(p.nw, NWC);
+    dim3 grid(count, p.nv, std::min(chunks, 65535));
     // The counter is a 32-bit int: past 2^30 items the one-tile grid instead.
-    const long long items = (long long)count * grid.y * grid.z;
+    const long long items = (long long)count * grid.y * chunks;
     const int per_sm = next && items < (1ll << 30) ? flag_blocks_per_sm(blocks_per_sm) : 0;
     if (per_sm > 0) {
         int dev = 0, sms = 0;
@@ -382,12 +387,11 @@ cudaError_t launch_flag_mixed(const Problem &p, const Partials &part, void *spli
                               cudaStream_t st, RowTiles rt, int blocks_per_sm, int *next) {
     if (p.nv <= 0 || p.ng == 0) return cudaSuccess;
     const SplitPlanes s = planes(p, split_ws);
-    switch (nwc_for(p.nw)) {
+    switch (flag_nwc(p.nw)) {
         case 1: return launch_flag_mixed_t<1>(p, part, s, rt, blocks_per_sm, next, st);
         case 2: return launch_flag_mixed_t<2>(p, part, s, rt, blocks_per_sm, next, st);
         case 3: return launch_flag_mixed_t<3>(p, part, s, rt, blocks_per_sm, next, st);
-        case 4: return launch_flag_mixed_t<4>(p, part, s, rt, blocks_per_sm, next, st);
-        default: return launch_flag_mixed_t<8>(p, part, s, rt, blocks_per_sm, next, st);
+        default: return launch_flag_mixed_t<4>(p, part, s, rt, blocks_per_sm, next, st);
     }
 }
 

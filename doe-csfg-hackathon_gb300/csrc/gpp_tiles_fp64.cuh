@@ -162,135 +162,143 @@ __device__ __forceinline__ void flag_epilogue(const Problem &p, const Partials &
     }
 }
 
-// Per (row, column) factors of the occupied-band solver: wtilde^2 and
-// Omega2 = wtilde^2 I_eps (gppComplex_seq.cpp:346-350).
-__device__ __forceinline__ void flag_row_terms(double2 wt, double2 ie, double2 &wt2,
-                                               double2 &om2) {
-    wt2 = make_double2(__fma_rn(wt.x, wt.x, -__dmul_rn(wt.y, wt.y)),
-                       __dmul_rn(__dmul_rn(2.0, wt.x), wt.y));
-    om2 = cmul_rn(wt2, ie);
+// a > t and a < t for a, t >= 0 (t finite), on the bits: the order of the bit
+// patterns is that of the values, and NaN (any sign) compares false as it
+// does in FP64.  Integer compares keep the tests off the FP64 pipe.
+__device__ __forceinline__ bool pos_gt(double a, double t) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+    return u > (unsigned long long)__double_as_longlong(t) && u <= 0x7FF0000000000000ull;
+}
+__device__ __forceinline__ bool pos_lt(double a, double t) {
+    return (unsigned long long)__double_as_longlong(a) <
+           (unsigned long long)__double_as_longlong(t);
+}
+
+// What an occupied-band tile keeps per frequency (uniform over the block):
+// c = wx^2, and how the branch-A sum of aqsn Omega2 is formed.  Away from
+// small wx nearly every term is branch A and `most` is set: the tile sums
+// aqsn Omega2 once for all frequencies, over the columns with
+// |wtilde|^2 <= flag_bound (none of which any frequency's cutoff takes), and
+// each frequency adds or takes off only the terms where its own set differs.
+// What is taken off lies near the frequency (|wtilde| about |wx|), so the
+// difference loses nothing; with a small wx the 1/wx^2 scale would enlarge
+// its rounding, and those frequencies add their terms one by one.
+struct FlagFreq {
+    double wx, c;
+    bool most, cut;
+};
+// x with its sign bit flipped where `neg` is set (no FP64 instruction).
+__device__ __forceinline__ double flip(double x, bool neg) {
+    return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+template <int SEM>
+__device__ __forceinline__ FlagFreq flag_freq(double wx) {
+    FlagFreq f;
+    f.wx = wx;
+    f.c = __dmul_rn(wx, wx);
+    f.cut = SEM == kSemComplexSeq && wx < 0.0;
+    f.most = fabs(wx) >= 1.0 && fabs(wx) < 1e60;
+    return f;
+}
+constexpr double kFlagNoBound = 1.7976931348623157e308;  // the largest double
+// The smallest |wtilde|^2 at which a frequency's branch-A cutoff starts.
+__device__ __forceinline__ double flag_bound(double bound, const FlagFreq &f) {
+    const double t = __dmul_rn(4.0, f.c);
+    return f.cut && t < bound ? t : bound;
+}
+// 1/wx^2 of branch A as the reference forms it (wx^2 / pow(wx^2, 2),
+// gppComplex_seq.cpp:38-41) times the sum y; no terms give 0 whatever wx is.
+__device__ __forceinline__ double flag_ssx_scale(double c, double y) {
+    return y == 0.0 ? 0.0 : __dmul_rn(y, c / (c * c));
 }
 
 // ssxt_scht_solver (gppComplex_seq.cpp:16-63) for one (row, column,
-// frequency): sch and ssx before the aqsn factor.  cwr = 1/wx^2 for branch A.
-// Every rounding is explicit (the _rn helpers), so the one-band and the
-// band-pair tiles produce the same bits.
-template <int SEM>
-__device__ __forceinline__ void flag_solve(double wx, double cwr, double2 wt, double2 wt2,
-                                           double2 om2, double2 ie, double2 &sch_out,
-                                           double2 &ssx_out) {
-    const double2 wd = make_double2(__dsub_rn(wx, wt.x), -wt.y);
-    const double wdr = abs2_rn(wd);
-    const double rden = rcp_fp64(wdr);
-    const double2 delw = cscale_rn(cmul_conj_b_rn(wt, wd), rden);
-    const double delwr = abs2_rn(delw);
-    double2 sch = make_double2(0.0, 0.0), ssx = make_double2(0.0, 0.0);
-    if (wdr > kLimitTwo && delwr < kLimitOne) {
-        sch = cmul_rn(delw, ie);
-        ssx = cscale_rn(om2, cwr);
-    } else if (delwr > kTo1) {
-        const double2 cden =
-            cscale_rn(cmul_rn(wt2, make_double2(__dadd_rn(0.5, delw.x), delw.y)), 4.0);
-        const double r2 = rcp_fp64(abs2_rn(cden));
-        ssx = cmul_rn(cmul_conj_b_rn(make_double2(-om2.x, -om2.y), cden), cscale_rn(delw, r2));
-    }
-    // |ssx| > sexcut |I_eps| compared on squares (sexcut^2 = 16 is exact).
-    if (SEM == kSemComplexSeq && wx < 0.0 && abs2_rn(ssx) > __dmul_rn(16.0, abs2_rn(ie)))
-        ssx = make_double2(0.0, 0.0);
-    sch_out = sch;
-    ssx_out = ssx;
-}
-
-// One occupied-band term, accumulated as aqsn*sch and aqsn*ssx (the
-// conj(aqsm) factor of matngmatmgp is applied in the epilogue).
-template <int SEM>
-__device__ __forceinline__ void flag_term(double wx, double cwr, double2 wt, double2 wt2,
-                                          double2 om2, double2 ie, double2 a, double2 &acc_s,
-                                          double2 &acc_x) {
-    double2 sch, ssx;
-    flag_solve<SEM>(wx, cwr, wt, wt2, om2, ie, sch, ssx);
-    acc_s = cmul_acc_rn(acc_s, a, sch);
-    acc_x = cmul_acc_rn(acc_x, a, ssx);
-}
-
-// One occupied-band tile in FP64: rows row_tile*RG.., one band, frequencies
-// iw_chunk*NWC..; `tile` indexes this launch's segment of block partials.
-// red/S are shared scratch of (THREADS/32)*K and K doubles, K = RG*NWC*4.
-template <int RG, int NWC, int THREADS, int SEM>
-__device__ __forceinline__ void flag_fp64_tile(const Problem &p, const Partials &part,
-                                               int row_tile, int band, int iw_chunk,
-                                               long long tile, double *red, double *S) {
-    constexpr int K = RG * NWC * 4;
-    const int row0 = row_tile * RG;
-    const int iw0 = iw_chunk * NWC;
-    const int nc = p.nc;
-
-    const double2 *wrow[RG];
-    const double2 *erow[RG];
+// frequency) and NB bands, accumulated as acc_s += aqsn sch and
+// y += wx^2 aqsn ssx (the conj(aqsm) factor of matngmatmgp and 1/wx^2 are
+// applied to the sums).  In exact arithmetic, with Q = wtilde I_eps and
+// A = aqsn Q:
+//   branch A (|wdiff|^2 > limittwo, |delw|^2 = |wtilde|^2 / |wdiff|^2 < limitone):
+//     aqsn sch = A conj(wdiff) / |wdiff|^2,  wx^2 aqsn ssx = aqsn Omega2 = A wtilde;
+//   branch B (|delw|^2 > to1): sch = 0 and, as Omega2 = wtilde^2 I_eps and
+//     cden = 4 wtilde^2 (0.5 + delw), ssx = -Omega2 delw / cden
+//     = -Q / (2 (wx + wtilde));
+//   the cutoff |ssx| > 4 |I_eps| is |wtilde|^2 > 4 wx^2 in branch A and
+//     |wtilde|^2 > 64 |wx + wtilde|^2 in branch B.
+// Bound by the FP64 pipe: 28 instructions per (row, column, frequency) of two
+// bands (6 shared, 4 per band, the rest per column; ncu), where evaluating
+// delw, Omega2, cden and the products as the reference does took 66.  819 x
+// 16384, two bands, 3 frequencies: 2.3 ms, the pipe 87% busy.  Every rounding
+// is explicit, so a band gives the same bits alone and beside another one.
+// in_all: whether the sum over all columns holds this one.
+template <int NB>
+__device__ __forceinline__ void flag_term(const FlagFreq &f, bool in_all, double2 wt, double wti2,
+                                          double awt2, const double2 (&A)[NB], const double2 (&Aw)[NB],
+                                          const double2 (&B)[NB], double2 (&acc_s)[NB],
+                                          double2 (&y)[NB]) {
+    const double wr = __dsub_rn(f.wx, wt.x);  // Re(wdiff); Im(wdiff) = -Im(wtilde)
+    const double rden = rcp_fp64(__fma_rn(wr, wr, wti2));
+    const double delwr = __dmul_rn(awt2, rden);
+    const bool in_a = pos_gt(__fma_rn(wr, wr, wti2), kLimitTwo) && pos_lt(delwr, kLimitOne);
+    if (in_a) {
 #pragma unroll
-    for (int g = 0; g < RG; ++g) {
-        const int r = min(row0 + g, p.ng - 1);
-        wrow[g] = p.wt + (size_t)r * nc;
-        erow[g] = p.ieps + (size_t)r * nc;
-    }
-    const double2 *nrow = p.aqsn + (size_t)band * nc;
-    double wx[NWC], cwr[NWC];
-#pragma unroll
-    for (int w = 0; w < NWC; ++w) {
-        wx[w] = __ldg(p.wx + (size_t)band * p.wx_stride + min(iw0 + w, p.nw - 1));
-        const double c = wx[w] * wx[w];
-        cwr[w] = c / (c * c);  // wx^2 / pow(wx^2, 2), once per (band, iw)
-    }
-
-    double2 acc_s[RG][NWC], acc_x[RG][NWC];
-#pragma unroll
-    for (int g = 0; g < RG; ++g)
-#pragma unroll
-        for (int w = 0; w < NWC; ++w) {
-            acc_s[g][w] = make_double2(0.0, 0.0);
-            acc_x[g][w] = make_double2(0.0, 0.0);
-        }
-
-    for (int ig = threadIdx.x; ig < nc; ig += THREADS) {
-        const double2 a = __ldg(nrow + ig);
-#pragma unroll
-        for (int g = 0; g < RG; ++g) {
-            const double2 wt = __ldg(wrow[g] + ig);
-            const double2 ie = __ldg(erow[g] + ig);
-            double2 wt2, om2;
-            flag_row_terms(wt, ie, wt2, om2);
-#pragma unroll
-            for (int w = 0; w < NWC; ++w)
-                flag_term<SEM>(wx[w], cwr[w], wt, wt2, om2, ie, a, acc_s[g][w], acc_x[g][w]);
+        for (int b = 0; b < NB; ++b) {
+            acc_s[b].x = __fma_rn(rden, __fma_rn(A[b].x, wr, -Aw[b].y), acc_s[b].x);
+            acc_s[b].y = __fma_rn(rden, __fma_rn(A[b].y, wr, Aw[b].x), acc_s[b].y);
         }
     }
-
-    double v[K];
+    const bool inc = in_a && !(f.cut && pos_gt(awt2, __dmul_rn(4.0, f.c)));
+    const bool base = f.most && in_all;
+    if (inc != base) {  // a branch-A term to add, or one to take off the sum over all columns
 #pragma unroll
-    for (int g = 0; g < RG; ++g)
-#pragma unroll
-        for (int w = 0; w < NWC; ++w) {
-            const int k = (g * NWC + w) * 4;
-            v[k] = acc_s[g][w].x;
-            v[k + 1] = acc_s[g][w].y;
-            v[k + 2] = acc_x[g][w].x;
-            v[k + 3] = acc_x[g][w].y;
+        for (int b = 0; b < NB; ++b) {
+            y[b].x = __dadd_rn(y[b].x, flip(B[b].x, base));
+            y[b].y = __dadd_rn(y[b].y, flip(B[b].y, base));
         }
-    block_reduce<K, THREADS>(v, red, S);
-    flag_epilogue<RG, NWC>(p, part, S, row0, band, iw0, tile, row_tile);
+    }
+    if (!in_a && pos_gt(delwr, kTo1)) {
+        const double sr = __dadd_rn(f.wx, wt.x);  // wx + wtilde = (sr, Im(wtilde))
+        const double rs = rcp_fp64(__fma_rn(sr, sr, wti2));
+        if (!(f.cut && pos_gt(__dmul_rn(awt2, rs), 64.0))) {
+            const double m = __dmul_rn(__dmul_rn(-0.5, f.c), rs);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                y[b].x = __fma_rn(m, __fma_rn(A[b].x, sr, Aw[b].y), y[b].x);
+                y[b].y = __fma_rn(m, __fma_rn(A[b].y, sr, -Aw[b].x), y[b].y);
+            }
+        }
+    }
 }
 
-// Occupied bands with band-independent frequencies (wx_stride == 0): the
-// solver's sch / ssx depend on (row, column, frequency) only, so one tile
-// evaluates them once for NB bands [band0, band0 + NB) and accumulates
-// aqsn * sch, aqsn * ssx per band.  Per band the operations, their order and
-// the reduction tree are those of flag_fp64_tile: the same bits, with 1/NB
-// of the solver work.  Bands past nv (a ragged last group) are computed on a
-// clamped band and not written.
+// The products of one (row, column) that its frequencies share: A = aqsn Q,
+// Aw = A Im(wtilde) and B = A wtilde = aqsn Omega2; wti2 = Im(wtilde)^2 and
+// awt2 = |wtilde|^2.
+template <int NB>
+__device__ __forceinline__ void flag_products(double2 wt, double2 ie, const double2 (&a)[NB],
+                                              double &wti2, double &awt2, double2 (&A)[NB],
+                                              double2 (&Aw)[NB], double2 (&B)[NB]) {
+    const double2 Q = cmul_rn(wt, ie);
+    wti2 = __dmul_rn(wt.y, wt.y);
+    awt2 = __fma_rn(wt.x, wt.x, wti2);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        A[b] = cmul_rn(a[b], Q);
+        Aw[b] = cscale_rn(A[b], wt.y);
+        B[b] = make_double2(__fma_rn(A[b].x, wt.x, -Aw[b].y), __fma_rn(A[b].y, wt.x, Aw[b].x));
+    }
+}
+
+// One occupied-band tile in FP64: rows row_tile*RG.., bands [band0,
+// band0 + NB), frequencies iw_chunk*NWC..; red/S are shared scratch of
+// (THREADS/32)*K and K doubles, K = NB*RG*NWC*4.  NB > 1 is for
+// band-independent frequencies (wx_stride == 0): |wdiff|^2, its reciprocal
+// and the branch are formed once for all NB bands; per band the operations,
+// their order and the reduction tree are those of NB = 1, and so the bits.
+// Bands past nv (a ragged last group) are computed on a clamped band and not
+// written.
 template <int RG, int NWC, int NB, int THREADS, int SEM>
-__device__ __forceinline__ void flag_fp64_multi_tile(const Problem &p, const Partials &part,
-                                                     int row_tile, int band0, int iw_chunk,
-                                                     int row_tiles, double *red, double *S) {
+__device__ __forceinline__ void flag_fp64_tile(const Problem &p, const Partials &part,
+                                               int row_tile, int band0, int iw_chunk,
+                                               int row_tiles, double *red, double *S) {
     constexpr int KB = RG * NWC * 4, K = NB * KB;
     const int row0 = row_tile * RG;
     const int iw0 = iw_chunk * NWC;
@@ -307,24 +315,26 @@ __device__ __forceinline__ void flag_fp64_multi_tile(const Problem &p, const Par
     const double2 *nrow[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) nrow[b] = p.aqsn + (size_t)min(band0 + b, p.nv - 1) * nc;
-    double wx[NWC], cwr[NWC];
+    FlagFreq f[NWC];
+    double bound = kFlagNoBound;
+    bool any_most = false;
 #pragma unroll
     for (int w = 0; w < NWC; ++w) {
-        wx[w] = __ldg(p.wx + min(iw0 + w, p.nw - 1));  // the same for every band
-        const double c = wx[w] * wx[w];
-        cwr[w] = c / (c * c);
+        f[w] = flag_freq<SEM>(__ldg(p.wx + (size_t)band0 * p.wx_stride + min(iw0 + w, p.nw - 1)));
+        bound = flag_bound(bound, f[w]);
+        any_most |= f[w].most;
     }
 
-    double2 acc_s[NB][RG][NWC], acc_x[NB][RG][NWC];
+    double2 acc_s[RG][NWC][NB], y[RG][NWC][NB], all[RG][NB];
 #pragma unroll
-    for (int b = 0; b < NB; ++b)
+    for (int g = 0; g < RG; ++g)
 #pragma unroll
-        for (int g = 0; g < RG; ++g)
+        for (int b = 0; b < NB; ++b) {
+            all[g][b] = make_double2(0.0, 0.0);
 #pragma unroll
-            for (int w = 0; w < NWC; ++w) {
-                acc_s[b][g][w] = make_double2(0.0, 0.0);
-                acc_x[b][g][w] = make_double2(0.0, 0.0);
-            }
+            for (int w = 0; w < NWC; ++w)
+                acc_s[g][w][b] = y[g][w][b] = make_double2(0.0, 0.0);
+        }
 
     for (int ig = threadIdx.x; ig < nc; ig += THREADS) {
         double2 a[NB];
@@ -334,18 +344,21 @@ __device__ __forceinline__ void flag_fp64_multi_tile(const Problem &p, const Par
         for (int g = 0; g < RG; ++g) {
             const double2 wt = __ldg(wrow[g] + ig);
             const double2 ie = __ldg(erow[g] + ig);
-            double2 wt2, om2;
-            flag_row_terms(wt, ie, wt2, om2);
+            double2 A[NB], Aw[NB], B[NB];
+            double wti2, awt2;
+            flag_products<NB>(wt, ie, a, wti2, awt2, A, Aw, B);
+            // Inf and NaN compare above the bound.
+            const bool in_all = (unsigned long long)__double_as_longlong(awt2) <=
+                                (unsigned long long)__double_as_longlong(bound);
+            if (any_most && in_all) {
 #pragma unroll
-            for (int w = 0; w < NWC; ++w) {
-                double2 sch, ssx;
-                flag_solve<SEM>(wx[w], cwr[w], wt, wt2, om2, ie, sch, ssx);
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    acc_s[b][g][w] = cmul_acc_rn(acc_s[b][g][w], a[b], sch);
-                    acc_x[b][g][w] = cmul_acc_rn(acc_x[b][g][w], a[b], ssx);
-                }
+                for (int b = 0; b < NB; ++b)
+                    all[g][b] = make_double2(__dadd_rn(all[g][b].x, B[b].x),
+                                             __dadd_rn(all[g][b].y, B[b].y));
             }
+#pragma unroll
+            for (int w = 0; w < NWC; ++w)
+                flag_term<NB>(f[w], in_all, wt, wti2, awt2, A, Aw, B, acc_s[g][w], y[g][w]);
         }
     }
 
@@ -357,10 +370,13 @@ __device__ __forceinline__ void flag_fp64_multi_tile(const Problem &p, const Par
 #pragma unroll
             for (int w = 0; w < NWC; ++w) {
                 const int k = b * KB + (g * NWC + w) * 4;
-                v[k] = acc_s[b][g][w].x;
-                v[k + 1] = acc_s[b][g][w].y;
-                v[k + 2] = acc_x[b][g][w].x;
-                v[k + 3] = acc_x[b][g][w].y;
+                double2 t = y[g][w][b];
+                if (f[w].most)
+                    t = make_double2(__dadd_rn(t.x, all[g][b].x), __dadd_rn(t.y, all[g][b].y));
+                v[k] = acc_s[g][w][b].x;
+                v[k + 1] = acc_s[g][w][b].y;
+                v[k + 2] = flag_ssx_scale(f[w].c, t.x);
+                v[k + 3] = flag_ssx_scale(f[w].c, t.y);
             }
     block_reduce<K, THREADS>(v, red, S);
 #pragma unroll

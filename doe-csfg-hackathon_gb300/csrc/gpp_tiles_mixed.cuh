@@ -442,46 +442,58 @@ __device__ __forceinline__ bool df_gt(df a, df t) {
 constexpr float kLim2H = (float)kLimitTwo, kLim2L = (float)(kLimitTwo - (double)kLim2H);
 constexpr float kLim1H = (float)kLimitOne, kLim1L = (float)(kLimitOne - (double)kLim1H);
 constexpr float kTo1H = (float)kTo1, kTo1L = (float)(kTo1 - (double)kTo1H);
-__device__ __forceinline__ df df_abs2(df re, df im) { return df_add(df_sqr(re), df_sqr(im)); }
-// (a.re + i a.im) * (b.re + i b.im) in df.
-__device__ __forceinline__ void df_cmul(df ar, df ai, df br, df bi, df &cr, df &ci) {
-    cr = df_sub(df_mul(ar, br), df_mul(ai, bi));
-    ci = df_add(df_mul(ar, bi), df_mul(ai, br));
+
+// a with the lanes whose flag is not set replaced by 0.
+__device__ __forceinline__ float2 f2mask(float2 a, bool x, bool y) {
+    return f2(x ? a.x : 0.f, y ? a.y : 0.f);
 }
-__device__ __forceinline__ df df_scale(df a, float k) { return {fmul(a.h, k), fmul(a.l, k)}; }
+__device__ __forceinline__ df2 df2_mask(const df2 &a, bool x, bool y) {
+    return {f2mask(a.h, x, y), f2mask(a.l, x, y)};
+}
 
 // An occupied-band term near the pole, in FP64 from the original inputs,
-// split to float-float: aqsn*sch (sr, si) and aqsn*ssx (xr, xi).  Out of line:
-// inlined, its FP64 code took registers from the float-float term loop.
+// split to float-float: aqsn*sch (sr, si) and its wx^2 aqsn*ssx, less its
+// share of the sum over all columns (xr, xi).  Out of line: inlined, its FP64
+// code took registers from the float-float term loop.
 struct FlagPole {
     df sr, si, xr, xi;
 };
 template <int SEM>
 static __device__ __noinline__ FlagPole flag_pole(const Problem &p, int row, int band, int ig,
-                                                  double wx, double cwr) {
+                                                  int iw, bool in_all) {
     const size_t nc = (size_t)p.nc;
+    const FlagFreq f = flag_freq<SEM>(__ldg(p.wx + (size_t)band * p.wx_stride + iw));
     const double2 wt = __ldg(p.wt + (size_t)row * nc + ig);
     const double2 ie = __ldg(p.ieps + (size_t)row * nc + ig);
-    const double2 a = __ldg(p.aqsn + (size_t)band * nc + ig);
-    double2 wt2, om2;
-    flag_row_terms(wt, ie, wt2, om2);
-    double2 s64 = make_double2(0.0, 0.0), x64 = make_double2(0.0, 0.0);
-    flag_term<SEM>(wx, cwr, wt, wt2, om2, ie, a, s64, x64);
-    return {split(s64.x), split(s64.y), split(x64.x), split(x64.y)};
+    const double2 a[1] = {__ldg(p.aqsn + (size_t)band * nc + ig)};
+    double wti2, awt2;
+    double2 A[1], Aw[1], B[1], s[1] = {make_double2(0.0, 0.0)}, y[1] = {make_double2(0.0, 0.0)};
+    flag_products<1>(wt, ie, a, wti2, awt2, A, Aw, B);
+    flag_term<1>(f, in_all, wt, wti2, awt2, A, Aw, B, s, y);
+    return {split(s[0].x), split(s[0].y), split(y[0].x), split(y[0].y)};
 }
 
-// One occupied-band tile in mixed precision: rows row_tile*RG.., one band,
+// One frequency of the mixed occupied-band tile, in float-float: the FlagFreq
+// of the FP64 tile, the high part above which |wdiff|^2 is clearly in branch
+// A and clear of the pole, and the |wtilde|^2 the cutoff starts at.
+struct FlagFreqM {
+    df wx, c4;     // wx, 4 wx^2 (the cutoff of branch A)
+    float clear;   // max(limittwo, (1e-3 wx)^2) with a margin above rounding
+    float keep;    // |wtilde|^2 clearly below the cutoff (or no cutoff)
+    bool most, cut;
+};
+
+// One occupied-band tile in mixed precision: the row pair row_tile, one band,
 // frequencies iw_chunk*NWC..; reads the float-float split planes (bands
-// [0, nvband) must have been split too).  Per term, on df values:
-//   wdiff, |wdiff|^2, rden = 1/|wdiff|^2, delwr = |delw|^2 = |wtilde|^2 rden;
-//   branch A (|wdiff|^2 > limittwo, delwr < limitone):
-//     aqsn*sch = A conj(wdiff) rden with A = aqsn Q,  aqsn*ssx = (aqsn Omega2) / wx^2
-//     (the 1/wx^2 factor is applied to the ig sum, in FP64);
-//   branch B (delwr > to1): sch = 0, ssx = -Omega2 conj(cden) delw / |cden|^2,
-//     cden = 4 wtilde^2 (0.5 + delw);
-//   cutoff |ssx|^2 |wtilde|^2 > 16 |Q|^2 (= |ssx| > 4 |I_eps|) when wx < 0
-//   under COMPLEX_SEQ semantics.
-// Terms within 1e-3 |wx| of the pole are computed in FP64 from the inputs.
+// [0, nvband) must have been split too).  The algebra is flag_term's, on df2
+// values whose lanes are the pair's two rows, as in mixed_column.  A term
+// whose two lanes are both clearly (beyond rounding) in branch A, uncut and
+// away from the pole takes one straight-line path of packed instructions;
+// any other term works out each lane's branch (df_gt: exact near the
+// thresholds) and zeroes the lanes a branch does not take.  Terms within
+// 1e-3 |wx| of the pole are computed in FP64 from the inputs.
+// Bound by the FP32 FMA pipe on the straight-line path (~78 packed
+// instructions per frequency of a row pair and ~96 per column).
 template <int RG, int NWC, int THREADS, int SEM>
 __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials &part,
                                                 const SplitPlanes &s, int row_tile, int band,
@@ -492,124 +504,167 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
     const int row0 = row_tile * RG;
     const int iw0 = iw_chunk * NWC;
     const int nc = p.nc;
-    const df kLim2 = {kLim2H, kLim2L}, kLim1 = {kLim1H, kLim1L}, kT1 = {kTo1H, kTo1L};
 
     const float4 *rp = s.rows + (size_t)row_tile * 4 * nc;  // this row pair's planes
     const float4 *bp = s.band + (size_t)band * nc;
-    df wx[NWC], cwr2[NWC];
-    double wx64[NWC], cwr[NWC];
-    float thr[NWC];
-    bool cut_on[NWC];  // the ssx cutoff applies (COMPLEX_SEQ, wx < 0); no FP64 test per term
+    const double *wxp = p.wx + (size_t)band * p.wx_stride;
+    FlagFreqM f[NWC];
+    double bound64 = kFlagNoBound;
+    bool any_most = false;
 #pragma unroll
     for (int w = 0; w < NWC; ++w) {
-        wx64[w] = __ldg(p.wx + (size_t)band * p.wx_stride + min(iw0 + w, p.nw - 1));
-        wx[w] = split(wx64[w]);
-        const double c = wx64[w] * wx64[w];
-        cwr[w] = c / (c * c);  // wx^2 / pow(wx^2, 2) (gppComplex_seq.cpp:38-41)
-        cwr2[w] = split(cwr[w] * cwr[w]);
-        thr[w] = 1e-6f * wx[w].h * wx[w].h;
-        cut_on[w] = SEM == kSemComplexSeq && wx64[w] < 0.0;
+        const FlagFreq d = flag_freq<SEM>(__ldg(wxp + min(iw0 + w, p.nw - 1)));
+        f[w].wx = split(d.wx);
+        f[w].c4 = split(4.0 * d.c);
+        f[w].clear = fmaxf(1.00002f * kLim2H, 1e-6f * f[w].wx.h * f[w].wx.h);
+        f[w].keep = d.cut ? 0.99998f * f[w].c4.h : __int_as_float(0x7F800000);
+        f[w].most = d.most;
+        f[w].cut = d.cut;
+        bound64 = flag_bound(bound64, d);
+        any_most |= d.most;
     }
-    // Accumulators: aqsn*sch, sum of aqsn*Omega2 over branch-A terms (times
-    // 1/wx^2 later), aqsn*ssx of branch-B and pole terms.
-    df as_r[RG][NWC], as_i[RG][NWC], xa_r[RG][NWC], xa_i[RG][NWC], xb_r[RG][NWC], xb_i[RG][NWC];
+    const float bound = (float)fmin(bound64, 3e38);
+    const df2 z = {f2(0.f, 0.f), f2(0.f, 0.f)};
+    // Lanes: the two rows.  aqsn*sch, wx^2 aqsn*ssx (less the sum over all
+    // columns where f.most), and aqsn*Omega2 over all columns.
+    df2 as_r[NWC], as_i[NWC], y_r[NWC], y_i[NWC], all_r = z, all_i = z;
 #pragma unroll
-    for (int g = 0; g < RG; ++g)
-#pragma unroll
-        for (int w = 0; w < NWC; ++w) {
-            as_r[g][w] = as_i[g][w] = xa_r[g][w] = xa_i[g][w] = xb_r[g][w] = xb_i[g][w] =
-                df{0.f, 0.f};
-        }
+    for (int w = 0; w < NWC; ++w) as_r[w] = as_i[w] = y_r[w] = y_i[w] = z;
 
     for (int ig = threadIdx.x; ig < nc; ig += THREADS) {
         const float4 av = __ldg(bp + ig);
-        const df ar = {av.x, av.y}, ai = {av.z, av.w};
-        const float4 pwr = __ldg(rp + ig), pwi = __ldg(rp + nc + ig);
-        const float4 pqr = __ldg(rp + 2 * nc + ig), pqi = __ldg(rp + 3 * nc + ig);
+        const float4 vr = __ldg(rp + ig), vi = __ldg(rp + nc + ig);
+        const float4 vqr = __ldg(rp + 2 * nc + ig), vqi = __ldg(rp + 3 * nc + ig);
+        const df2 ar = df2_bcast(df{av.x, av.y}), ai = df2_bcast(df{av.z, av.w});
+        const df2 wtr = {f2(vr.x, vr.y), f2(vr.z, vr.w)}, wti = {f2(vi.x, vi.y), f2(vi.z, vi.w)};
+        const df2 qr = {f2(vqr.x, vqr.y), f2(vqr.z, vqr.w)};
+        const df2 qi = {f2(vqi.x, vqi.y), f2(vqi.z, vqi.w)};
+        const df2 wti2 = df2_sqr(wti);
+        const df2 awt2 = df2_add(df2_sqr(wtr), wti2);                  // |wtilde|^2
+        const df2 Ar = df2_sub(df2_mul(ar, qr), df2_mul(ai, qi));      // A = aqsn Q
+        const df2 Ai = df2_add(df2_mul(ar, qi), df2_mul(ai, qr));
+        const df2 Ai_wti = df2_mul(Ai, wti), Ar_wti = df2_mul(Ar, wti);
+        const df2 Br = df2_sub(df2_mul(Ar, wtr), Ai_wti);              // aqsn Omega2 = A wtilde
+        const df2 Bi = df2_add(df2_mul(Ai, wtr), Ar_wti);
+        // The lanes the sum over all columns holds (not Inf or NaN).
+        const bool in0 = awt2.h.x <= bound, in1 = awt2.h.y <= bound;
+        if (any_most) {
+            const bool both = in0 && in1;
+            all_r = df2_add(all_r, both ? Br : df2_mask(Br, in0, in1));
+            all_i = df2_add(all_i, both ? Bi : df2_mask(Bi, in0, in1));
+        }
 #pragma unroll
-        for (int g = 0; g < RG; ++g) {
-            const df wtr = pair_lane(pwr, g), wti = pair_lane(pwi, g);
-            const df qr = pair_lane(pqr, g), qi = pair_lane(pqi, g);
-            const df wti2 = df_sqr(wti);
-            const df awt2 = df_add(df_sqr(wtr), wti2);                         // |wtilde|^2
-            df w2r, w2i;                                                          // wtilde^2
-            df_cmul(wtr, wti, wtr, wti, w2r, w2i);
-            df omr, omi;                                                          // Omega2 = wtilde Q
-            df_cmul(wtr, wti, qr, qi, omr, omi);
-            const df cut_rhs = df_scale(df_abs2(qr, qi), 16.f);                  // 16 |Q|^2
-            const df om_wt = df_mul(df_abs2(omr, omi), awt2);                   // |Omega2|^2 |wtilde|^2
-            df Ar, Ai, Br, Bi;
-            df_cmul(ar, ai, qr, qi, Ar, Ai);                                      // aqsn Q
-            df_cmul(ar, ai, omr, omi, Br, Bi);                                    // aqsn Omega2
-            const df Ai_wti = df_mul(Ai, wti), Ar_wti = df_mul(Ar, wti);
+        for (int w = 0; w < NWC; ++w) {
+            const df2 wr = df2_norm(df2_sub(df2_bcast(f[w].wx), wtr));  // Re(wdiff); Im = -wti
+            const df2 d = df2_add(df2_sqr(wr), wti2);                    // |wdiff|^2
+            float2 r0, rc;                                               // 1/d = r0 (1 + rc)
+            df2_rcp_parts(d, r0, rc);
+            const df2 delwr = df2_mul_rcp(awt2, r0, rc);                 // |delw|^2
+            const float lim1 = 0.99998f * kLim1H;
+            const bool clear = d.h.x > f[w].clear && d.h.y > f[w].clear && delwr.h.x < lim1 &&
+                               delwr.h.y < lim1 && awt2.h.x < f[w].keep && awt2.h.y < f[w].keep;
+            if (clear) {
+                const df2 tr = df2_mul_rcp(df2_sub(df2_mul(Ar, wr), Ai_wti), r0, rc);
+                const df2 ti = df2_mul_rcp(df2_add(df2_mul(Ai, wr), Ar_wti), r0, rc);
+                as_r[w] = df2_add(as_r[w], tr);
+                as_i[w] = df2_add(as_i[w], ti);
+                if (!f[w].most) {
+                    y_r[w] = df2_add(y_r[w], Br);
+                    y_i[w] = df2_add(y_i[w], Bi);
+                } else if (!in0 || !in1) {
+                    y_r[w] = df2_add(y_r[w], df2_mask(Br, !in0, !in1));
+                    y_i[w] = df2_add(y_i[w], df2_mask(Bi, !in0, !in1));
+                }
+                continue;
+            }
+            // Some lane is near a threshold, cut, in branch B or at the pole.
+            const float thr = 1e-6f * f[w].wx.h * f[w].wx.h;
+            bool pole[2], in_a[2], inc[2], in_b[2];
 #pragma unroll
-            for (int w = 0; w < NWC; ++w) {
-                const df wr = df_norm(df_sub(wx[w], wtr));   // Re(wdiff); Im(wdiff) = -wti
-                const df d = df_add(df_sqr(wr), wti2);       // |wdiff|^2
-                if (d.h < thr[w]) {
-                    // Near the pole: the whole term in FP64 from the inputs.
-                    const FlagPole t = flag_pole<SEM>(p, min(row0 + g, p.ng - 1), band, ig,
-                                                      wx64[w], cwr[w]);
-                    as_r[g][w] = df_add(as_r[g][w], t.sr);
-                    as_i[g][w] = df_add(as_i[g][w], t.si);
-                    xb_r[g][w] = df_add(xb_r[g][w], t.xr);
-                    xb_i[g][w] = df_add(xb_i[g][w], t.xi);
-                    continue;
-                }
-                const df rden = df_rcp(d);
-                const df delwr = df_mul(awt2, rden);
-                if (df_gt(d, kLim2) && df_gt(kLim1, delwr)) {
-                    // Branch A: aqsn*sch = A conj(wdiff) rden; aqsn*ssx = B / wx^2.
-                    const df tre = df_mul(df_sub(df_mul(Ar, wr), Ai_wti), rden);
-                    const df tim = df_mul(df_add(df_mul(Ai, wr), Ar_wti), rden);
-                    as_r[g][w] = df_add(as_r[g][w], tre);
-                    as_i[g][w] = df_add(as_i[g][w], tim);
-                    const bool cut = cut_on[w] && df_gt(df_mul(om_wt, cwr2[w]), cut_rhs);
-                    if (!cut) {
-                        xa_r[g][w] = df_add(xa_r[g][w], Br);
-                        xa_i[g][w] = df_add(xa_i[g][w], Bi);
+            for (int g = 0; g < 2; ++g) {
+                const df dg = df2_lane(d, g), wg = df2_lane(delwr, g);
+                pole[g] = dg.h < thr;
+                in_a[g] = !pole[g] && df_gt(dg, df{kLim2H, kLim2L}) && df_gt(df{kLim1H, kLim1L}, wg);
+                inc[g] = in_a[g] && !(f[w].cut && df_gt(df2_lane(awt2, g), f[w].c4));
+                in_b[g] = !pole[g] && !in_a[g] && df_gt(wg, df{kTo1H, kTo1L});
+            }
+            if (in_a[0] || in_a[1]) {
+                const float2 r0a = f2mask(r0, in_a[0], in_a[1]), rca = f2mask(rc, in_a[0], in_a[1]);
+                as_r[w] = df2_add(as_r[w], df2_mul_rcp(df2_mask(df2_sub(df2_mul(Ar, wr), Ai_wti), in_a[0], in_a[1]), r0a, rca));
+                as_i[w] = df2_add(as_i[w], df2_mul_rcp(df2_mask(df2_add(df2_mul(Ai, wr), Ar_wti), in_a[0], in_a[1]), r0a, rca));
+            }
+            // Add the branch-A lanes the sum over all columns lacks, take off
+            // the ones it should not hold (a pole lane's share comes from
+            // flag_pole).
+            const bool base[2] = {f[w].most && in0, f[w].most && in1};
+            const bool m0 = inc[0] != base[0] && !pole[0], m1 = inc[1] != base[1] && !pole[1];
+            if (m0 || m1) {
+                df2 xr = df2_mask(Br, m0, m1), xi = df2_mask(Bi, m0, m1);
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+                    if (base[g]) {
+                        const df r = df2_lane(xr, g), i = df2_lane(xi, g);
+                        df2_set_lane(xr, g, df{-r.h, -r.l});
+                        df2_set_lane(xi, g, df{-i.h, -i.l});
                     }
-                } else if (df_gt(delwr, kT1)) {
-                    // Branch B.  delw = wtilde conj(wdiff) rden, conj(wdiff) = (wr, wti).
-                    df dr, di;
-                    df_cmul(wtr, wti, wr, wti, dr, di);
-                    dr = df_mul(dr, rden);
-                    di = df_mul(di, rden);
-                    df cr, ci;                                   // cden = 4 wtilde^2 (0.5 + delw)
-                    df_cmul(w2r, w2i, df_add(dr, df{0.5f, 0.f}), di, cr, ci);
-                    cr = df_scale(cr, 4.f);
-                    ci = df_scale(ci, 4.f);
-                    const df r2 = df_rcp(df_norm(df_abs2(cr, ci)));
-                    df tr, ti;                                   // -Omega2 conj(cden)
-                    df_cmul(omr, omi, cr, df{-ci.h, -ci.l}, tr, ti);
-                    df sr, si;                                   // ssx = -(...) (delw r2)
-                    df_cmul(tr, ti, df_mul(dr, r2), df_mul(di, r2), sr, si);
-                    sr = df{-sr.h, -sr.l};
-                    si = df{-si.h, -si.l};
-                    const bool cut =
-                        cut_on[w] && df_gt(df_mul(df_abs2(sr, si), awt2), cut_rhs);
-                    if (!cut) {
-                        df pr, pi;
-                        df_cmul(ar, ai, sr, si, pr, pi);
-                        xb_r[g][w] = df_add(xb_r[g][w], pr);
-                        xb_i[g][w] = df_add(xb_i[g][w], pi);
-                    }
+                y_r[w] = df2_add(y_r[w], xr);
+                y_i[w] = df2_add(y_i[w], xi);
+            }
+            if (in_b[0] || in_b[1]) {
+                // wx^2 aqsn ssx = -(wx^2 / 2) A conj(wx + wtilde) / |wx + wtilde|^2
+                const df2 sr = df2_norm(df2_add(df2_bcast(f[w].wx), wtr));
+                const df2 sd = df2_add(df2_sqr(sr), wti2);
+                float2 s0, sc;
+                df2_rcp_parts(sd, s0, sc);
+                if (f[w].cut) {
+                    const df2 q = df2_mul_rcp(awt2, s0, sc);
+                    in_b[0] = in_b[0] && !df_gt(df2_lane(q, 0), df{64.f, 0.f});
+                    in_b[1] = in_b[1] && !df_gt(df2_lane(q, 1), df{64.f, 0.f});
                 }
+                s0 = f2mask(s0, in_b[0], in_b[1]);
+                sc = f2mask(sc, in_b[0], in_b[1]);
+                const df2 m = df2_bcast(df{fmul(-0.125f, f[w].c4.h), fmul(-0.125f, f[w].c4.l)});
+                const df2 tr = df2_mul_rcp(df2_mask(df2_add(df2_mul(Ar, sr), Ai_wti), in_b[0], in_b[1]), s0, sc);
+                const df2 ti = df2_mul_rcp(df2_mask(df2_sub(df2_mul(Ai, sr), Ar_wti), in_b[0], in_b[1]), s0, sc);
+                y_r[w] = df2_add(y_r[w], df2_mul(tr, m));
+                y_i[w] = df2_add(y_i[w], df2_mul(ti, m));
+            }
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                if (!pole[g]) continue;
+                const FlagPole t = flag_pole<SEM>(p, min(row0 + g, p.ng - 1), band, ig,
+                                                  min(iw0 + w, p.nw - 1), g == 0 ? in0 : in1);
+                df2 u = z;
+                df2_set_lane(u, g, t.sr);
+                as_r[w] = df2_add(as_r[w], u);
+                df2_set_lane(u, g, t.si);
+                as_i[w] = df2_add(as_i[w], u);
+                df2_set_lane(u, g, t.xr);
+                y_r[w] = df2_add(y_r[w], u);
+                df2_set_lane(u, g, t.xi);
+                y_i[w] = df2_add(y_i[w], u);
             }
         }
     }
 
     double v[K];
 #pragma unroll
-    for (int g = 0; g < RG; ++g)
+    for (int w = 0; w < NWC; ++w) {
+        const double wx = __ldg(wxp + min(iw0 + w, p.nw - 1));
 #pragma unroll
-        for (int w = 0; w < NWC; ++w) {
+        for (int g = 0; g < RG; ++g) {
             const int k = (g * NWC + w) * 4;
-            v[k] = to_double(as_r[g][w]);
-            v[k + 1] = to_double(as_i[g][w]);
-            v[k + 2] = to_double(xa_r[g][w]) * cwr[w] + to_double(xb_r[g][w]);
-            v[k + 3] = to_double(xa_i[g][w]) * cwr[w] + to_double(xb_i[g][w]);
+            double tr = to_double(df2_lane(y_r[w], g)), ti = to_double(df2_lane(y_i[w], g));
+            if (f[w].most) {
+                tr += to_double(df2_lane(all_r, g));
+                ti += to_double(df2_lane(all_i, g));
+            }
+            v[k] = to_double(df2_lane(as_r[w], g));
+            v[k + 1] = to_double(df2_lane(as_i[w], g));
+            v[k + 2] = flag_ssx_scale(wx * wx, tr);
+            v[k + 3] = flag_ssx_scale(wx * wx, ti);
         }
+    }
     block_reduce<K, THREADS>(v, red, S);
     flag_epilogue<RG, NWC>(p, part, S, row0, band, iw0, tile, row_tile);
 }
