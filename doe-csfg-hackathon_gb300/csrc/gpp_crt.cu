@@ -1,0 +1,684 @@
+// gpp_crt.cu -- FP64-accurate complex GEMM on the tensor cores by residues
+// (Ozaki, Uchino and Imamura, "Ozaki Scheme II: a GEMM-oriented emulation of
+// floating-point matrix multiplication using an integer modular technique",
+// 2025).
+//
+//  * Over a chunk of at most 512 k values every operand value x of a row is
+//    written as x = N 2^(e - 53), e the row's largest exponent in the chunk
+//    and N a 53-bit integer;
+//  * the product sum of such integers is an integer X, |X| < P / 2, fixed by
+//    its residues modulo 15 pairwise coprime integers p <= 256 of product
+//    P = 2^117.78 (gpp_crt.cuh): 15 products of 8-bit integers, each exact in
+//    bf16 with FP32 accumulation, where cutting the operands into slices
+//    (gpp_ozaki.cu) takes 36 products of slice pairs;
+//  * complex products take the 3M form (P1 = sum xr yr, P2 = sum xi yi,
+//    P3 = sum (xr + xi)(yr + yi)); re = P1 - P2 and im = P3 - P1 - P2 are
+//    formed on the residues, exactly;
+//  * the combining pass turns the residues of re and im into 2^128 X / P and
+//    rounds X 2^(ex + ey - 106) to a double; chunks are added in FP64.
+//
+// So the only roundings are those of the operands (to 53 bits of the chunk's
+// largest value), of each chunk's result and of the sum over chunks: at the
+// production shape the band sums are off by 1e-15 where the slices' float-float
+// combination left 5e-15.
+//
+// GB300, 1638 x 32768 over 510 bands / 510 x 1638 over 32768 columns: prepare
+// 0.35 / 1.3 ms, products 2.04 / 2.45 ms (1.23 / 1.10 PFLOP/s), combine 1.0 /
+// 1.0 ms; the slices took 0.4 / 1.3, 4.6 / 5.4 and 1.3 / 1.4 ms.  The products
+// are bound by the bytes in flight: the 96 KB ring of Y blocks covers about
+// two thirds of the L2 latency at the rate the tensor cores take them.
+//
+// crt_gemm_kernel keeps the core-matrix operand layout and the bulk-copy /
+// tcgen05.mma / TMEM pipeline of gpp_ozaki.cu and makes each block
+// persistent: it walks (plane, row tile, column tile) steps with the whole
+// chunk of its X rows resident in shared memory (128 x 512, loaded once per
+// row tile) while Y's blocks stream through a ring.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstdint>
+#include <cstdlib>
+
+#include "gpp_crt.cuh"
+#include "gpp_crt.h"
+#include "gpp_kernels.h"
+#include "gpp_umma.cuh"
+
+namespace gpp {
+
+namespace {
+
+constexpr int kKcMax = 512;             // k values per chunk
+constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli
+constexpr int kTM = 128, kTN = 256;     // tcgen05.mma M (rows of X) x N (rows of Y)
+constexpr int kTK = 64;                 // k per operand block
+constexpr int kKSMax = kKcMax / kTK;    // operand blocks per chunk
+constexpr int kStages = 3;              // ring of Y blocks
+constexpr unsigned kBytesA = kTM * kTK * 2, kBytesB = kTN * kTK * 2;  // 16 KB, 32 KB
+constexpr size_t kSmem = (size_t)kKSMax * kBytesA + (size_t)kStages * kBytesB + 256;
+constexpr int kThreads = 320;  // warp 0 loads, warp 1 issues the MMAs, warps 2-9 drain TMEM
+constexpr int kTmemCols = 2 * kTN;
+constexpr unsigned kIdesc = umma_idesc(kTM, kTN);
+
+constexpr int kExpZero = -4000;        // exponent of an all-zero chunk of a row
+constexpr int kExpNonFinite = 1 << 20; // of one that holds an Inf or a NaN
+
+__constant__ CrtGroup c_group[kCrtGroups] = {GPP_CRT_GROUPS};
+__constant__ CrtMod c_mod[kCrtN] = {
+    crt_mod(256), crt_mod(255), crt_mod(253), crt_mod(251), crt_mod(247),
+    crt_mod(241), crt_mod(239), crt_mod(233), crt_mod(229), crt_mod(227),
+    crt_mod(223), crt_mod(217), crt_mod(211), crt_mod(199), crt_mod(197)};
+
+struct Geometry {
+    int M, N, K;
+    int Mp, Np;      // X's rows, and a pass's rows of Y, padded to the block tile
+    int nch, Kc;     // chunks, chunk length (multiple of kTK)
+    int cps, splits; // chunks per split, splits
+    int slab_chunks, slab_tiles;  // chunks and row tiles of X per pass
+};
+
+// The operand planes and product residues of one pass take about 4 GB each
+// at most (GPP_OZAKI_FOLD_MB overrides it, for tests): a larger product runs
+// in passes over rows of Y, chunks and row tiles of X.
+size_t pass_budget() {
+    const char *v = getenv("GPP_OZAKI_FOLD_MB");
+    const long long mb = v ? atoll(v) : 0;
+    return mb > 0 ? (size_t)mb << 20 : size_t(4) << 30;
+}
+
+size_t operand_bytes(const Geometry &g) {  // per chunk
+    return sizeof(__nv_bfloat16) * kPlanes * (size_t)g.Kc * (g.Mp + g.Np);
+}
+
+Geometry geometry(int M, int N, int K, int splits) {
+    Geometry g;
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.nch = std::max(1, ceil_div(K, kKcMax));
+    g.Kc = ceil_div(ceil_div(std::max(K, 1), g.nch), kTK) * kTK;
+    g.Mp = ceil_div(std::max(M, 1), kTM) * kTM;
+    const size_t y_rows = pass_budget() / (sizeof(__nv_bfloat16) * kPlanes * (size_t)g.Kc);
+    g.Np = std::min(ceil_div(std::max(N, 1), kTN), (int)std::max<size_t>(1, std::min<size_t>(y_rows / kTN, 1 << 22))) * kTN;
+    g.cps = ceil_div(g.nch, std::max(1, splits));
+    g.splits = ceil_div(g.nch, g.cps);
+    const size_t per_tile = (size_t)kPlanes * kTM * g.Np;  // residues of one row tile and chunk
+    const int tiles = g.Mp / kTM;
+    const size_t per_chunk = operand_bytes(g) + per_tile * tiles;
+    g.slab_chunks = (int)std::max<size_t>(1, std::min<size_t>(g.cps, pass_budget() / per_chunk));
+    g.slab_tiles = (int)std::max<size_t>(
+        1, std::min<size_t>(tiles, pass_budget() / (per_tile * g.slab_chunks)));
+    return g;
+}
+
+size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
+
+struct Buffers {
+    __nv_bfloat16 *sx, *sy;  // [kPlanes][rows][slab k], core-matrix blocks
+    int *ex, *ey;            // [slab chunks][rows]
+    unsigned char *res;      // [slab chunks][kPlanes][slab rows][Np]: residues + 128
+};
+
+size_t carve(const Geometry &g, void *ws, Buffers *b) {
+    char *w = static_cast<char *>(ws);
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        char *p = w + off;
+        off = align_up(off + n);
+        return p;
+    };
+    Buffers o;
+    const size_t plane = sizeof(__nv_bfloat16) * kPlanes * (size_t)g.slab_chunks * g.Kc;
+    o.sx = reinterpret_cast<__nv_bfloat16 *>(take(plane * g.Mp));
+    o.sy = reinterpret_cast<__nv_bfloat16 *>(take(plane * g.Np));
+    o.ex = reinterpret_cast<int *>(take(sizeof(int) * (size_t)g.slab_chunks * g.Mp));
+    o.ey = reinterpret_cast<int *>(take(sizeof(int) * (size_t)g.slab_chunks * g.Np));
+    o.res = reinterpret_cast<unsigned char *>(
+        take((size_t)g.slab_chunks * kPlanes * ((size_t)g.slab_tiles * kTM) * g.Np));
+    if (b) *b = o;
+    return off;
+}
+
+__device__ __forceinline__ double2 operand_at(const OzOperand &z, int l, int k) {
+    return __ldg(z.kfast ? z.z + (size_t)l * z.ld + k : z.z + (size_t)k * z.ld + l);
+}
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+// The e of frexp for the nonzero magnitude with bits b (b < 2^e).
+__device__ __forceinline__ int exp_of_bits(unsigned long long b) {
+    if (b == 0) return kExpZero;
+    const int E = (int)(b >> 52);
+    if (E == 0x7FF) return kExpNonFinite;  // the bit patterns of Inf and NaN are the largest
+    return E > 0 ? E - 1022 : (63 - __clzll((long long)b)) - 1073;
+}
+
+struct PrepOperand {
+    OzOperand z;
+    int Lp, R;           // padded rows, rows per operand block
+    __nv_bfloat16 *out;
+    int *E;
+};
+
+// Exponents and residue planes of chunks [c0, c0 + nc): blocks [0, x blocks)
+// serve X, the rest Y.  A block stages 8 rows x one chunk in shared memory
+// (each value read once, 128 contiguous bytes or more at a time), takes each
+// row's largest exponent, and writes the residues of (re, im, re + im) to
+// every modulus as bf16: a thread per 8 consecutive k of a row, so that a
+// plane gets whole 16-byte core-matrix rows and a warp 512 contiguous bytes.
+// Layout of a plane, in memory order: row tile (R rows), k step (kTK), row
+// group of 8, k-core of 8, row, k -- the no-swizzle K-major core-matrix layout
+// of tcgen05.mma, one contiguous block per (row tile, k step).
+// Bound by its writes (90 bytes per complex value) and the FP32 pipe.
+__global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOperand Y, int xblocks,
+                                                          int K, int Kc, int c0, int nc) {
+    extern __shared__ __align__(16) double2 stage[];  // [8][Kc + 1]
+    __shared__ unsigned long long red[8][8];
+    __shared__ int exps[8];
+    const bool isx = (int)blockIdx.x < xblocks;
+    const PrepOperand &o = isx ? X : Y;
+    const int b = isx ? blockIdx.x : blockIdx.x - xblocks;
+    const int groups = o.Lp / 8;
+    const int l0 = (b % groups) * 8, c = b / groups;
+    const int kb = (c0 + c) * Kc, kn = min(Kc, K - kb);
+    const int pitch = Kc + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const OzOperand z = o.z;
+
+    unsigned long long mx = 0;
+    if (z.kfast) {  // a warp per row
+        const int l = l0 + warp;
+#pragma unroll 4
+        for (int k = lane; k < Kc; k += 32) {
+            const double2 v =
+                l < z.L && k < kn ? operand_at(z, l, kb + k) : make_double2(0.0, 0.0);
+            stage[warp * pitch + k] = v;
+            mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
+        }
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+        if (lane == 0) exps[warp] = exp_of_bits(mx);
+        __syncthreads();
+    } else {  // lanes along the 8 rows, 4 k per warp
+        const int r = lane & 7, l = l0 + r;
+#pragma unroll 4
+        for (int k = warp * 4 + (lane >> 3); k < Kc; k += 32) {
+            const double2 v =
+                l < z.L && k < kn ? operand_at(z, l, kb + k) : make_double2(0.0, 0.0);
+            stage[r * pitch + k] = v;
+            mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
+        }
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        if (lane < 8) red[warp][lane] = mx;
+        __syncthreads();
+        if (threadIdx.x < 8) {
+#pragma unroll
+            for (int w = 1; w < 8; ++w) mx = max(mx, red[w][threadIdx.x]);
+            exps[threadIdx.x] = exp_of_bits(mx);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < 8) o.E[(size_t)c * o.Lp + l0 + threadIdx.x] = exps[threadIdx.x];
+
+    const int row = threadIdx.x & 7;
+    const int e = exps[row];
+    const int ksteps = nc * (Kc / kTK);
+    const size_t plane = (size_t)o.Lp * ksteps * kTK;
+    const size_t base = ((size_t)(l0 / o.R) * ksteps * (o.R / 8) + (size_t)(l0 % o.R) / 8) * 512 + row * 8;
+    for (int kg = threadIdx.x >> 3; kg < Kc / 8; kg += 32) {
+        float2 dr[4][4], di[4][4];  // [pair of k][digit]
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            float a[4], bb[4], cr[4], ci[4];
+            const double2 v0 = stage[row * pitch + kg * 8 + 2 * t];
+            const double2 v1 = stage[row * pitch + kg * 8 + 2 * t + 1];
+            crt_digits(oz_fixed_point(v0.x, e, kCrtBits), a);
+            crt_digits(oz_fixed_point(v1.x, e, kCrtBits), bb);
+            crt_digits(oz_fixed_point(v0.y, e, kCrtBits), cr);
+            crt_digits(oz_fixed_point(v1.y, e, kCrtBits), ci);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                dr[t][k] = f2(a[k], bb[k]);
+                di[t][k] = f2(cr[k], ci[k]);
+            }
+        }
+        const int ks = c * (Kc / kTK) + (kg >> 3);
+        __nv_bfloat16 *w = o.out + base + (size_t)ks * (o.R / 8) * 512 + (kg & 7) * 64;
+#pragma unroll 1
+        for (int i = 0; i < kCrtN; ++i) {
+            const CrtMod m = c_mod[i];
+            unsigned pr[4], pi[4], ps[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float2 rr = crt_residue2(dr[t], m), ri = crt_residue2(di[t], m);
+                const float2 rs = crt_reduce2(f2add(rr, ri), m.p, m.inv);
+                const __nv_bfloat162 hr = __floats2bfloat162_rn(rr.x, rr.y);
+                const __nv_bfloat162 hi = __floats2bfloat162_rn(ri.x, ri.y);
+                const __nv_bfloat162 hs = __floats2bfloat162_rn(rs.x, rs.y);
+                pr[t] = *reinterpret_cast<const unsigned *>(&hr);
+                pi[t] = *reinterpret_cast<const unsigned *>(&hi);
+                ps[t] = *reinterpret_cast<const unsigned *>(&hs);
+            }
+            *reinterpret_cast<uint4 *>(w + (size_t)i * plane) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
+            *reinterpret_cast<uint4 *>(w + (size_t)(kCrtN + i) * plane) =
+                make_uint4(pi[0], pi[1], pi[2], pi[3]);
+            *reinterpret_cast<uint4 *>(w + (size_t)(2 * kCrtN + i) * plane) =
+                make_uint4(ps[0], ps[1], ps[2], ps[3]);
+        }
+    }
+}
+
+// The steps of one block: planes q in groups of `gq`, the (plane, row tile,
+// column tile) steps of a group in order, each block a contiguous run of them
+// (rotated from group to group, so that the runs' rounding evens out).
+// Consecutive steps of a row tile share X's rows in shared memory, and the
+// blocks in flight work on a few planes, whose operands fit in L2.
+struct Walk {
+    int Q, MT, NT, gq, grid;
+    int g = 0;
+    long long t = 0, end = 0;
+    int q0 = 0, q = 0, mt = 0, nt = 0;
+    bool first = false;  // this step starts a row tile's run (X's rows change)
+    __device__ __forceinline__ bool open_group() {
+        for (; g * gq < Q; ++g) {
+            q0 = g * gq;
+            const long long steps = (long long)min(gq, Q - q0) * MT * NT;
+            const long long j = (long long)((blockIdx.x + (unsigned)g * 61u) % (unsigned)grid);
+            t = j * steps / grid;
+            end = (j + 1) * steps / grid;
+            if (t < end) return true;
+        }
+        return false;
+    }
+    __device__ __forceinline__ void decode() {
+        const int per = MT * NT;
+        q = q0 + (int)(t / per);
+        const int r = (int)(t % per);
+        mt = r / NT;
+        nt = r % NT;
+    }
+    __device__ __forceinline__ bool start() {
+        if (!open_group()) return false;
+        decode();
+        first = true;
+        return true;
+    }
+    // Whether the next step leaves this row tile's run.
+    __device__ __forceinline__ bool last() const { return t + 1 == end || nt + 1 == NT; }
+    __device__ __forceinline__ bool next() {
+        if (++t == end) {
+            ++g;
+            return start();
+        }
+        first = false;
+        if (++nt == NT) {
+            nt = 0;
+            first = true;
+            if (++mt == MT) {
+                mt = 0;
+                ++q;
+            }
+        }
+        return true;
+    }
+};
+
+// Residues of the products: plane q = c kPlanes + (3M plane, modulus) of the
+// pass's chunks, rows [128 mt0, + 128 MT) of X against every row of Y; the
+// byte stored is the symmetric residue + 128, at res[(q Ms + row) Np + col].
+// Warp 0 (one thread) loads: X's blocks of a row tile into kKSMax resident
+// slots, each as soon as the MMAs of the previous run's last step released
+// it, and Y's blocks through a three-stage ring, all by 1-D bulk copies onto
+// mbarriers; warp 1 (one thread) issues four K = 16 tcgen05.mma per block into
+// one of two TMEM accumulators; warps 2-9 drain a finished accumulator (a
+// warp's 32 lanes x 128 columns), reduce the exact FP32 sums modulo p on the
+// FP32 pipe and store bytes, 32 at a time per thread.  Every wait is bounded;
+// a block that gives up records kErrPipelineTimeout, lets its copies and MMAs
+// finish and frees its TMEM.
+__global__ void __launch_bounds__(kThreads, 1)
+crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restrict__ SY, int Mp,
+                int Np, int KS, int nc, int mt0, int MT, int gq, unsigned char *__restrict__ res,
+                int Ms, int *err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *sA = smem;
+    unsigned char *sB = smem + (size_t)kKSMax * kBytesA;
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(sB + (size_t)kStages * kBytesB);
+    unsigned long long *full = bars, *empty = full + kStages;
+    unsigned long long *afull = empty + kStages, *aempty = afull + kKSMax;
+    unsigned long long *accfull = aempty + kKSMax, *accempty = accfull + 2;
+    unsigned *tmem_slot = reinterpret_cast<unsigned *>(accempty + 2);
+    int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
+    __shared__ int issued_a, issued_b, waited_a, waited_b;
+    volatile int *abort = abort_flag;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ksteps = nc * KS;
+    Walk w;
+    w.Q = nc * kPlanes;
+    w.MT = MT;
+    w.NT = Np / kTN;
+    w.gq = gq;
+    w.grid = gridDim.x;
+
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            bar_init(&full[s], 1);
+            bar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < kKSMax; ++s) {
+            bar_init(&afull[s], 1);
+            bar_init(&aempty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            bar_init(&accfull[a], 1);
+            bar_init(&accempty[a], 256);
+        }
+        *abort_flag = 0;
+        issued_a = issued_b = waited_a = waited_b = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(tmem_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {  // producer
+            const size_t xplane = (size_t)Mp * ksteps * kTK, yplane = (size_t)Np * ksteps * kTK;
+            int run = -1, nb = 0;  // row-tile runs and Y blocks so far
+            bool ok = true;
+            for (bool more = w.start(); ok && more; more = w.next()) {
+                const int c = w.q / kPlanes, pl = w.q % kPlanes;
+                const __nv_bfloat16 *a = SX + pl * xplane +
+                                         ((size_t)(mt0 + w.mt) * ksteps + (size_t)c * KS) * (kTM * kTK);
+                const __nv_bfloat16 *b =
+                    SY + pl * yplane + ((size_t)w.nt * ksteps + (size_t)c * KS) * (kTN * kTK);
+                if (w.first) ++run;
+                for (int s = 0; s < KS; ++s) {
+                    if (w.first) {
+                        if (run > 0 && !bar_wait(&aempty[s], (run - 1) & 1, abort)) { ok = false; break; }
+                        bar_expect_tx(&afull[s], kBytesA);
+                        bulk_g2s(sA + (size_t)s * kBytesA, a + (size_t)s * (kTM * kTK), kBytesA, &afull[s]);
+                        ++issued_a;
+                    }
+                    const int st = nb % kStages;
+                    if (nb >= kStages && !bar_wait(&empty[st], (nb / kStages - 1) & 1, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    bar_expect_tx(&full[st], kBytesB);
+                    bulk_g2s(sB + (size_t)st * kBytesB, b + (size_t)s * (kTN * kTK), kBytesB, &full[st]);
+                    ++nb;
+                }
+            }
+            issued_b = nb;
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {  // MMA issuer
+            int run = -1, nb = 0, G = 0;
+            bool ok = true;
+            for (bool more = w.start(); ok && more; more = w.next(), ++G) {
+                if (w.first) ++run;
+                const bool last = w.last();
+                const int acc = G & 1;
+                if (G >= 2 && !bar_wait(&accempty[acc], ((G >> 1) - 1) & 1, abort)) break;
+                for (int s = 0; s < KS; ++s) {
+                    if (w.first) {
+                        if (!bar_wait(&afull[s], run & 1, abort)) { ok = false; break; }
+                        ++waited_a;
+                    }
+                    const int st = nb % kStages;
+                    if (!bar_wait(&full[st], (nb / kStages) & 1, abort)) { ok = false; break; }
+                    tc_fence_after();
+                    const unsigned sa = smem_addr(sA + (size_t)s * kBytesA);
+                    const unsigned sb = smem_addr(sB + (size_t)st * kBytesB);
+#pragma unroll
+                    for (int k16 = 0; k16 < kTK / 16; ++k16)
+                        umma_bf16(tmem + acc * kTN, umma_desc(sa + k16 * 256, 128, 1024),
+                                  umma_desc(sb + k16 * 256, 128, 1024), kIdesc,
+                                  !(s == 0 && k16 == 0));
+                    umma_commit(&empty[st]);
+                    if (last) umma_commit(&aempty[s]);
+                    ++nb;
+                }
+                if (ok) umma_commit(&accfull[acc]);
+            }
+            waited_b = nb;
+        }
+    } else {  // epilogue: TMEM lanes 32 (warp % 4) .., columns 128 ((warp - 2) / 4) ..
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        int G = 0;
+        for (bool more = w.start(); more; more = w.next(), ++G) {
+            const int acc = G & 1;
+            if (!bar_wait(&accfull[acc], (G >> 1) & 1, abort)) break;
+            tc_fence_after();
+            const CrtMod m = c_mod[(w.q % kPlanes) % kCrtN];
+            unsigned char *o = res + ((size_t)w.q * Ms + (size_t)w.mt * kTM + quarter * 32 + lane) * Np +
+                               (size_t)w.nt * kTN + half * 128;
+            const unsigned ta = tmem + ((unsigned)(quarter * 32) << 16) + acc * kTN + half * 128;
+#pragma unroll 1
+            for (int cc = 0; cc < 128; cc += 32) {
+                float v[32];
+                tmem_ld32(ta + cc, v);
+                unsigned word[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    // r + 128 (mod 256) in the low byte of r + 2^23 + 128's bits.
+                    const float2 off = f2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
+                    const float2 x = f2add(crt_reduce2(f2(v[4 * j], v[4 * j + 1]), m.p, m.inv), off);
+                    const float2 y = f2add(crt_reduce2(f2(v[4 * j + 2], v[4 * j + 3]), m.p, m.inv), off);
+                    const unsigned lo = __byte_perm(__float_as_uint(x.x), __float_as_uint(x.y), 0x0040);
+                    const unsigned hi = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
+                    word[j] = __byte_perm(lo, hi, 0x5410);
+                }
+                *reinterpret_cast<uint4 *>(o + cc) = make_uint4(word[0], word[1], word[2], word[3]);
+                *reinterpret_cast<uint4 *>(o + cc + 16) = make_uint4(word[4], word[5], word[6], word[7]);
+            }
+            tc_fence_before();
+            bar_arrive(&accempty[acc]);
+        }
+    }
+
+    __syncthreads();
+    if (*abort && tid == 0) {
+        atomicOr(err, kErrPipelineTimeout);
+        // Let the copies still in flight land and the issued MMAs finish.
+        auto settle = [&](unsigned long long *bar, unsigned parity) {
+            int spin = 0;
+            while (!bar_try_wait(bar, parity) && ++spin < kWaitLimit) {
+            }
+        };
+        for (int t = waited_b; t < issued_b; ++t)
+            settle(&full[t % kStages], (unsigned)((t / kStages) & 1));
+        for (int t = waited_a; t < issued_a; ++t)
+            settle(&afull[t % KS], (unsigned)((t / KS) & 1));
+        if (waited_b > 0)
+            settle(&empty[(waited_b - 1) % kStages], (unsigned)(((waited_b - 1) / kStages) & 1));
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
+// Out (= or +=) the pass's chunks: a thread per row and 4 consecutive
+// columns reads the 45 residue words of a chunk, forms the residues of re and
+// im for each column, their sum of fractions (integer multiply-adds) and
+// X 2^(ex + ey - 106), and adds it to the running FP64 result, chunk by chunk.
+// Bound by integer issue.
+__global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char *res, const int *EX,
+                                                             const int *EY, int row0, int rows,
+                                                             int Ms, int N, int Mp, int Np, int nc,
+                                                             int accumulate, double2 *Out,
+                                                             long long out_ld) {
+    const unsigned quads = (N + 3) / 4;
+    const long long n = (long long)rows * quads;
+    const size_t plane = (size_t)Ms * Np;
+    for (long long t = (long long)blockIdx.x * 128 + threadIdx.x; t < n;
+         t += (long long)gridDim.x * 128) {
+        int r, col0;
+        if (n < (1ll << 31)) {
+            r = (int)((unsigned)t / quads);
+            col0 = (int)((unsigned)t % quads) * 4;
+        } else {
+            r = (int)(t / quads);
+            col0 = (int)(t % quads) * 4;
+        }
+        double2 *out = Out + (long long)(row0 + r) * out_ld + col0;
+        double2 acc[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            acc[j] = accumulate && col0 + j < N ? out[j] : make_double2(0.0, 0.0);
+        for (int c = 0; c < nc; ++c) {
+            const unsigned char *f = res + (size_t)c * kPlanes * plane + (size_t)r * Np + col0;
+            unsigned u[kPlanes];
+#pragma unroll
+            for (int q = 0; q < kPlanes; ++q)
+                u[q] = __ldg(reinterpret_cast<const unsigned *>(f + q * plane));
+            const int ex = __ldg(EX + (size_t)c * Mp + row0 + r);
+            const int4 ey = __ldg(reinterpret_cast<const int4 *>(EY + (size_t)c * Np + col0));
+            // Not unrolled: the residue words take 45 registers, and one column's
+            // state at a time leaves room for five blocks per SM.
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+                CrtSum re, im;
+                const unsigned sel = 0x4440 + j;
+#pragma unroll
+                for (int k = 0; k < kCrtGroups; ++k) {
+                    int rr[2] = {0, 0}, ri[2] = {0, 0};
+#pragma unroll
+                    for (int h = 0; h < 2 && 2 * k + h < kCrtN; ++h) {
+                        const int i = 2 * k + h;
+                        const int a = __byte_perm(u[i], 0, sel);
+                        const int b = __byte_perm(u[kCrtN + i], 0, sel);
+                        rr[h] = a - b;                                      // r1 - r2
+                        ri[h] = (int)__byte_perm(u[2 * kCrtN + i], 0, sel) - a - b;  // r3 - r1 - r2 - 128
+                    }
+                    re.add<0>(rr[0], rr[1], c_group[k]);
+                    im.add<-128>(ri[0], ri[1], c_group[k]);
+                }
+                const int eyj = j == 0 ? ey.x : j == 1 ? ey.y : j == 2 ? ey.z : ey.w;
+                double2 v;
+                if (ex >= kExpNonFinite || eyj >= kExpNonFinite)
+                    v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
+                else
+                    v = make_double2(crt_value(re, ex + eyj - 2 * kCrtBits),
+                                     crt_value(im, ex + eyj - 2 * kCrtBits));
+                if (c == 0 && !accumulate && nc == 1) {
+                    if (col0 + j < N) out[j] = v;
+                    continue;
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+                    if (m == j) acc[m] = c == 0 && !accumulate ? v : cadd(acc[m], v);
+            }
+        }
+        if (nc == 1 && !accumulate) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (col0 + j < N) out[j] = acc[j];
+    }
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 132;
+}
+
+}  // namespace
+
+size_t crt_bytes(int M, int N, int K, int splits) {
+    return carve(geometry(M, N, K, splits), nullptr, nullptr);
+}
+
+int crt_splits(int K, int splits) { return geometry(1, 1, K, splits).splits; }
+
+cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int K, int splits,
+                      double2 *Out, long long out_ld, long long split_stride, void *ws, int *err,
+                      cudaStream_t s, cudaEvent_t after_slices) {
+    if (M <= 0 || N <= 0) return cudaSuccess;
+    const Geometry g = geometry(M, N, K, splits);
+    Buffers b;
+    carve(g, ws, &b);
+    const size_t prep_smem = sizeof(double2) * 8 * (g.Kc + 1);
+    static std::atomic<bool> configured[256] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (!configured[dev & 255].load(std::memory_order_acquire)) {
+        e = cudaFuncSetAttribute(crt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSmem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(crt_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(double2) * 8 * (kKcMax + 1)));
+        if (e != cudaSuccess) return e;
+        configured[dev & 255].store(true, std::memory_order_release);
+    }
+    const int sms = sm_count();
+    const int mtiles = g.Mp / kTM, Ms = g.slab_tiles * kTM, KS = g.Kc / kTK;
+    int launches = 0;
+    for (int z = 0; z < g.splits; ++z) {
+        const int zc0 = z * g.cps, zc1 = std::min(g.nch, zc0 + g.cps);
+        for (int c0 = zc0; c0 < zc1; c0 += g.slab_chunks) {
+            const int nc = std::min(g.slab_chunks, zc1 - c0);
+            for (int n0 = 0; n0 < N; n0 += g.Np) {
+                OzOperand Yn = Y;
+                Yn.z += (long long)n0 * (Y.kfast ? Y.ld : 1);
+                Yn.L = std::min(N - n0, g.Np);
+                const int Np = ceil_div(Yn.L, kTN) * kTN, ntiles = Np / kTN;
+                const PrepOperand px{X, g.Mp, kTM, b.sx, b.ex}, py{Yn, Np, kTN, b.sy, b.ey};
+                // X's planes serve every pass over rows of Y.
+                const int xblocks = n0 == 0 ? g.Mp / 8 * nc : 0, yblocks = Np / 8 * nc;
+                crt_prep_kernel<<<xblocks + yblocks, 256, prep_smem, s>>>(px, py, xblocks, K, g.Kc,
+                                                                          c0, nc);
+                ++launches;
+                if (after_slices && z == 0 && c0 == 0 && n0 == 0) {
+                    e = cudaEventRecord(after_slices, s);
+                    if (e != cudaSuccess) return e;
+                }
+                for (int mt0 = 0; mt0 < mtiles; mt0 += g.slab_tiles) {
+                    const int tiles = std::min(g.slab_tiles, mtiles - mt0);
+                    const int row0 = mt0 * kTM, rows = std::min(M - row0, tiles * kTM);
+                    const long long steps = (long long)nc * kPlanes * tiles * ntiles;
+                    const int grid = (int)std::min<long long>(sms, steps);
+                    // Planes in flight: enough that every block has a step, with
+                    // their operands within about 80 MB of L2.
+                    const size_t plane = sizeof(__nv_bfloat16) * (size_t)g.Kc * (g.Mp + Np);
+                    const int gq = std::max(ceil_div(grid, (long long)tiles * ntiles),
+                                            std::min(ceil_div(grid, tiles),
+                                                     (int)((size_t(80) << 20) / plane)));
+                    crt_gemm_kernel<<<grid, kThreads, kSmem, s>>>(b.sx, b.sy, g.Mp, Np, KS, nc, mt0,
+                                                                  tiles, gq, b.res, Ms, err);
+                    ++launches;
+                    if (rows > 0) {
+                        const long long want = ((long long)rows * ceil_div(Yn.L, 4) + 127) / 128;
+                        crt_combine_kernel<<<(int)std::min<long long>(want, (long long)sms * 32),
+                                             128, 0, s>>>(
+                            b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, c0 > zc0,
+                            Out + z * split_stride + n0, out_ld);
+                        ++launches;
+                    }
+                }
+            }
+        }
+    }
+    count_launch(launches);
+    return cudaGetLastError();
+}
+
+}  // namespace gpp

@@ -190,10 +190,10 @@ cudaError_t launch_zgemm3m(const double2 *X, long long xs, const double2 *Y, lon
 
 // k splits of the per-band GEMM (H = aqsn M_2^T sums over all ncouls
 // columns): on the FP64 pipe enough blocks for ~10 waves of two blocks per
-// SM; on the tensor cores (128 x 128 output tiles, so only 4 x 13 tiles at
-// the production shape) 32 splits make ~5 waves.
+// SM; on the tensor cores the products of the k chunks are separate work
+// already, and their sum is formed where they are combined.
 constexpr int kHSplits = 8;
-constexpr int kHSplitsTensor = 32;
+constexpr int kHSplitsTensor = 1;
 int h_splits() { return fp64_gemm_on_tensor_cores() ? kHSplitsTensor : kHSplits; }
 
 // c[k][r] for bands b0 + k (k < K) and rows [r0, r1); rows whose G' index

@@ -1,4 +1,5 @@
-// gpp_ozaki.cu -- FP64-class complex GEMM on the tensor cores.
+// gpp_ozaki.cu -- FP64-class complex GEMM on the tensor cores: ozaki_zgemm,
+// by residues (gpp_crt.cu) or by the slices described here.
 //
 // GB300 retires about 1.9 FP64 FMAs per clock per SM, so the band-sum GEMM
 // of the FP64 path (gpp_gemm.cu) is bound by the FP64 pipe.  Its tensor
@@ -44,9 +45,11 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "gpp_crt.h"
 #include "gpp_kernels.h"
 #include "gpp_ozaki.h"
 #include "gpp_ozaki_split.cuh"
+#include "gpp_umma.cuh"
 
 namespace gpp {
 
@@ -62,6 +65,7 @@ constexpr int kSlots = kGroups / 2;  // stored values per (plane, chunk): groups
 constexpr int kTM = 128, kTN = 256, kTK = 64, kTStages = 4;
 constexpr unsigned kStageA = kTM * kTK * 2, kStageB = kTN * kTK * 2;  // 16 KB, 32 KB
 constexpr size_t kTcSmem = (size_t)kTStages * (kStageA + kStageB) + 256;
+constexpr unsigned kIdesc = umma_idesc(kTM, kTN);
 constexpr int kTcThreads = 192;  // warp 0 loads, warp 1 issues the MMAs, warps 2-5 drain TMEM
 constexpr int kTmemCols = 2 * kTN;  // two accumulators of 256 FP32 columns
 
@@ -296,104 +300,6 @@ __global__ void __launch_bounds__(256, 2) oz_split_kernel(OzOperand z, int K, in
     }
 }
 
-// ---------------------------------------------------------------------------
-// tcgen05 / mbarrier primitives.
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void bar_init(unsigned long long *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
-                 : "memory");
-}
-__device__ __forceinline__ void bar_arrive(unsigned long long *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void bar_expect_tx(unsigned long long *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool bar_try_wait(unsigned long long *bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait for phase `parity`: gives up after kWaitLimit polls, or as soon
-// as another thread of the block raised *abort (and then raises it itself).
-__device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity,
-                                         volatile int *abort) {
-    for (int it = 0; it < kWaitLimit; ++it) {
-        if (bar_try_wait(bar, parity)) return true;
-        if ((it & 63) == 63 && *abort) return false;
-    }
-    *abort = 1;
-    return false;
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes,
-                                         unsigned long long *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-// Shared-memory matrix descriptor of tcgen05.mma for the no-swizzle K-major
-// layout: start address, LBO (bytes to the next core matrix along K), SBO
-// (bytes to the next 8-row group), the sm_100 descriptor version (bit 46).
-__device__ __forceinline__ unsigned long long umma_desc(unsigned saddr, unsigned lbo,
-                                                        unsigned sbo) {
-    return (unsigned long long)((saddr & 0x3FFFF) >> 4) |
-           ((unsigned long long)((lbo >> 4) & 0x3FFF) << 16) |
-           ((unsigned long long)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
-}
-// Instruction descriptor of tcgen05.mma kind::f16: D FP32 (bits 4-5 = 1), A and
-// B bf16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at
-// bits 24-28.
-constexpr unsigned kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(kTN >> 3) << 17) |
-                            ((unsigned)(kTM >> 4) << 24);
-__device__ __forceinline__ void umma_bf16(unsigned tmem, unsigned long long a, unsigned long long b,
-                                          unsigned accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned long long *bar) {
-    asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_addr(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// 32 consecutive FP32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld32(unsigned taddr, float (&v)[32]) {
-    unsigned r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-        "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-          "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-          "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-}
-
 // Step t of a block's sequence (plane g, chunk cl of the split, slice pair p,
 // k step ks fastest).
 struct TcStep {
@@ -510,7 +416,7 @@ oz_tc_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restri
 #pragma unroll
                 for (int k16 = 0; k16 < kTK / 16; ++k16)
                     umma_bf16(tmem + a * kTN, umma_desc(sa + k16 * 256, 128, 1024),
-                              umma_desc(sb + k16 * 256, 128, 1024), !(first && k16 == 0));
+                              umma_desc(sb + k16 * 256, 128, 1024), kIdesc, !(first && k16 == 0));
                 umma_commit(&empty[s]);
                 if (last) {
                     umma_commit(&accfull[a]);
@@ -751,7 +657,18 @@ int grid_for(long long n) {
 
 }  // namespace
 
+// The products take the residues of gpp_crt.cu: 45 real products instead of
+// 108 (measured, slices against residues: 4.5 and 2.2 ms for 1638 x 32768 over
+// 64 k, 0.30 and 0.03 ms for 40 x 800), and no size was found where slices
+// were faster.  GPP_TENSOR_GEMM=slices in the environment (read on every
+// call) runs the slices instead, an independent check on the residues.
+static bool use_residues() {
+    const char *v = getenv("GPP_TENSOR_GEMM");
+    return !(v && v[0] == 's');
+}
+
 size_t ozaki_bytes(int M, int N, int K, int splits) {
+    if (use_residues()) return crt_bytes(M, N, K, splits);
     const Geometry g = geometry(M, N, K, splits);
     return align_up(sizeof(__nv_bfloat16) * 3 * kS * (size_t)g.Mp * g.Kp) +
            align_up(sizeof(__nv_bfloat16) * 3 * kS * (size_t)g.Np * g.Kp) +
@@ -760,12 +677,16 @@ size_t ozaki_bytes(int M, int N, int K, int splits) {
            align_up(sizeof(int) * fold_elems(g));
 }
 
-int ozaki_splits(int K, int splits) { return geometry(1, 1, K, splits).splits; }
+int ozaki_splits(int K, int splits) {
+    return use_residues() ? crt_splits(K, splits) : geometry(1, 1, K, splits).splits;
+}
 
 cudaError_t ozaki_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int K, int splits,
                         double2 *Out, long long out_ld, long long split_stride, void *ws, int *err,
                         cudaStream_t s, cudaEvent_t after_slices) {
     if (M <= 0 || N <= 0) return cudaSuccess;
+    if (use_residues())
+        return crt_zgemm(X, Y, M, N, K, splits, Out, out_ld, split_stride, ws, err, s, after_slices);
     const Geometry g = geometry(M, N, K, splits);
     if (g.Mp / kTM > 65535 || g.Np / kTN > 65535 || g.splits > 65535)
         return cudaErrorInvalidConfiguration;

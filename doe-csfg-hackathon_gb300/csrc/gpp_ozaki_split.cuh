@@ -14,10 +14,12 @@ namespace gpp {
 
 constexpr int kOzSlices = 8;
 
-// round(x 2^(7 S - e)) for |x| < 2^e (ties away from zero), from the
-// double's bits with integer operations only: |result| < 2^(7 S) = 2^56, so
-// it is exact in 64-bit arithmetic and the left shift never overflows.
-__host__ __device__ __forceinline__ long long oz_fixed_point(double x, int e) {
+// round(x 2^(bits - e)) for |x| < 2^e (ties away from zero), from the
+// double's bits with integer operations only: |result| <= 2^bits, bits = 7 S =
+// 56 for the slices, so it is exact in 64-bit arithmetic and the left shift
+// never overflows.
+__host__ __device__ __forceinline__ long long oz_fixed_point(double x, int e,
+                                                             int bits = 7 * kOzSlices) {
     unsigned long long u;
 #ifdef __CUDA_ARCH__
     u = (unsigned long long)__double_as_longlong(x);
@@ -32,7 +34,7 @@ __host__ __device__ __forceinline__ long long oz_fixed_point(double x, int e) {
         m |= 1ull << 52;
         ex = E - 1075;
     }
-    const int sh = ex + 7 * kOzSlices - e;
+    const int sh = ex + bits - e;
     unsigned long long N;
     if (sh >= 0)
         N = m << sh;
