@@ -12,6 +12,7 @@
 #include <chrono>
 #include <cstdlib>
 
+#include "gpp_far.h"
 #include "gpp_gb300.h"
 #include "gpp_gemm.h"
 #include "gpp_gemm_mixed.h"
@@ -307,10 +308,23 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const size_t o_gemm = off; off = align_up(off + gemm_ws);
     const size_t o_gemm64 = off;
     off = align_up(off + (mixed && tensor ? gemm_bytes(p, nb1 - nb0, want_n1) : 0));
+    // Per-band frequencies away from wtilde through the series of gpp_far.cu
+    // (not while the autotuner times the per-term kernel's variants).
+    bool far = has_noflag && !gemm && t_force_variant < 0 && far_eligible(p, nb1 - nb0, mixed);
+    const size_t o_far = off;
     const size_t ws_bytes = off > 0 ? off : 256;
 
     void *ws = nullptr;
-    st = workspace_alloc(&ws, ws_bytes, s);
+    if (far) {
+        st = workspace_alloc(&ws, off + far_bytes(p, nb1 - nb0, mixed), s);
+        if (st == GPP_ERR_OUT_OF_MEMORY) {  // the per-term kernel needs much less
+            cudaGetLastError();
+            far = false;
+        } else if (st != GPP_OK) {
+            return st;
+        }
+    }
+    if (!far) st = workspace_alloc(&ws, ws_bytes, s);
     if (st != GPP_OK) return st;
     char *w = static_cast<char *>(ws);
 
@@ -324,10 +338,14 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     part.err = err;
 
     cudaError_t e = cudaSuccess;
-    if (want_n1 && (rows_f != rows_n) && has_flag && has_noflag) {
-        // Different row tilings: pad the shorter per-band segments with zeros.
+    if (want_n1 && (far || (rows_f != rows_n && has_flag && has_noflag))) {
+        // Different row tilings: pad the shorter per-band segments with zeros
+        // (the series writes one slot per band).
         e = cudaMemsetAsync(part.n1, 0, sizeof(double2) * (size_t)(n1_seg * p.nb), s);
     }
+    if (e == cudaSuccess && far)  // the series writes one unoccupied slot per frequency
+        e = cudaMemset2DAsync(part.ach + tiles_f, sizeof(double2) * (size_t)ach_seg, 0,
+                              sizeof(double2) * (size_t)tiles_n, (size_t)p.nw, s);
     if (e == cudaSuccess && mixed)  // float-float planes of every band the call touches
         e = launch_split_bands(p, w + o_split, has_flag ? fb0 : nb0, has_noflag ? nb1 : fb1, s);
     SideStream *side = nullptr;
@@ -399,9 +417,17 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
                     cudaFreeAsync(ws, s);
                     return st;
                 }
-            } else {
+            } else if (!far) {
                 e = mixed ? launch_mixed_noflag(p, part, w + o_split, nb0, nb1, s, variant, rt)
                           : launch_noflag_fp64(p, part, nb0, nb1, s, rt);
+            } else if (k == pc.n - 1) {  // every row is there
+                const int *active = nullptr;
+                e = far_unoccupied(p, part, w + o_far, mixed ? w + o_split : nullptr, nb0, nb1, s,
+                                   &active);
+                if (e == cudaSuccess)
+                    e = mixed ? launch_mixed_noflag(p, part, w + o_split, nb0, nb1, s, variant,
+                                                    RowTiles(), active)
+                              : launch_noflag_fp64(p, part, nb0, nb1, s, RowTiles(), active);
             }
             if (k == pc.n - 1 && t_timing && t_ev1) {
                 cudaEventRecord(t_ev1, s);

@@ -20,6 +20,7 @@
 #include <cstring>
 #include <vector>
 
+#include "gpp_far.h"
 #include "gpp_gb300.h"
 #include "gpp_kernels.h"
 #include "gpp_tiles_fp64.cuh"
@@ -196,6 +197,11 @@ struct gpp_batch {
     std::vector<Partials> parts;
     std::vector<SplitPlanes> splits;
     std::vector<BatchItem> items;
+    // States whose unoccupied bands take the series of gpp_far.cu: each runs
+    // as its own gpp_sigma call on the stream (the same bits as alone).
+    std::vector<char> direct;
+    std::vector<gpp_problem> direct_problems;
+    std::vector<gpp_outputs> direct_outs;
     struct Wave {
         int s0, s1;      // states [s0, s1)
         int i0, i_mid, i1;  // occupied items [i0, i_mid), unoccupied [i_mid, i1)
@@ -311,7 +317,13 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
         p.semantics = q.semantics;
         b->probs.push_back(p);
         StateGeom &s = g[i];
-        const bool hf = p.nv > 0 && p.ng > 0, hn = p.nb > p.nv && p.ng > 0;
+        const bool direct = p.ng > 0 && far_eligible(p, p.nb - p.nv, mixed);
+        b->direct.push_back(direct);
+        if (direct) {
+            b->direct_problems.push_back(q);
+            b->direct_outs.push_back(outs[i]);
+        }
+        const bool hf = !direct && p.nv > 0 && p.ng > 0, hn = !direct && p.nb > p.nv && p.ng > 0;
         s.rows_f = hf ? ceil_div(p.ng, fs.rg) : 0;
         s.rows_n = hn ? ceil_div(p.ng, ns.rg) : 0;
         s.tiles_f = hf ? s.rows_f * p.nv : 0;
@@ -320,10 +332,10 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
         s.n1_seg = std::max(s.rows_f, s.rows_n);
         s.off_ach = reserve(sizeof(double2) * (size_t)(s.ach_seg * nw));
         s.off_asx = reserve(sizeof(double2) * (size_t)(s.tiles_f * nw));
-        s.off_n1 = outs[i].acht_n1_loc && p.ng > 0 ? reserve(sizeof(double2) * (size_t)(s.n1_seg * p.nb)) : 0;
-        s.achs_blocks = outs[i].achstemp && p.ng > 0 ? achstemp_blocks(p) : 0;
+        s.off_n1 = !direct && outs[i].acht_n1_loc && p.ng > 0 ? reserve(sizeof(double2) * (size_t)(s.n1_seg * p.nb)) : 0;
+        s.achs_blocks = !direct && outs[i].achstemp && p.ng > 0 ? achstemp_blocks(p) : 0;
         s.off_achs = s.achs_blocks ? reserve(sizeof(double2) * s.achs_blocks) : 0;
-        s.split = mixed ? align256(mixed_split_bytes(p)) : 0;
+        s.split = mixed && !direct ? align256(mixed_split_bytes(p)) : 0;
     }
     // Waves (mixed): consecutive states whose split planes fit the budget.
     std::vector<std::pair<int, int>> wave_states;
@@ -390,6 +402,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     for (int i = 0; i < nstates; ++i) {
         const StateGeom &s = g[i];
         const Problem &p = b->probs[i];
+        if (b->direct[i]) continue;
         b->jobs.push_back({nullptr, s.ach_seg, (int)s.ach_seg, nw,
                            reinterpret_cast<double2 *>(outs[i].achtemp), 0});
         b->jobs.push_back({nullptr, s.tiles_f, (int)s.tiles_f, nw,
@@ -436,6 +449,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
         b->parts.push_back(part);
         if (part.n1 && s.rows_f != s.rows_n)  // shorter per-band segments are zero-padded
             b->n1_zero.push_back({part.n1, sizeof(double2) * (size_t)(s.n1_seg * b->probs[i].nb)});
+        if (b->direct[i]) continue;
         b->jobs[ji++].src = part.ach;
         b->jobs[ji++].src = part.asx;
         if (s.off_n1 || (outs[i].acht_n1_loc && b->probs[i].nb > 0)) {
@@ -451,7 +465,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     b->splits.resize(nstates);
     for (auto &w : b->waves)
         for (int i = w.s0; i < w.s1; ++i)
-            b->splits[i] = mixed ? split_planes_at(b->probs[i], b->d_split + w.split_off[i - w.s0])
+            b->splits[i] = mixed && !b->direct[i] ? split_planes_at(b->probs[i], b->d_split + w.split_off[i - w.s0])
                                  : SplitPlanes{};
     b->seg_prefix.push_back(0);
     for (auto &j : b->jobs) b->seg_prefix.push_back(b->seg_prefix.back() + j.nseg);
@@ -580,7 +594,7 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
         if (b->precision == GPP_PRECISION_MIXED)
             for (int i = w.s0; i < w.s1 && e == cudaSuccess; ++i) {
                 const Problem &p = b->probs[i];
-                if (p.nb > 0 && p.ng > 0) {
+                if (p.nb > 0 && p.ng > 0 && !b->direct[i]) {
                     e = launch_split(p, b->d_split + w.split_off[i - w.s0], 0, p.nb, s);
                     launches += 2;
                 }
@@ -612,6 +626,11 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
     }
     b->launches_per_run = launches;
     if (e != cudaSuccess) return set_error(GPP_ERR_CUDA, cudaGetErrorString(e));
+    for (size_t k = 0; k < b->direct_problems.size(); ++k) {
+        const gpp_status st = gpp_sigma(&b->direct_problems[k], &b->direct_outs[k],
+                                        reinterpret_cast<gpp_stream_t>(s));
+        if (st != GPP_OK) return st;
+    }
     return GPP_OK;
 }
 

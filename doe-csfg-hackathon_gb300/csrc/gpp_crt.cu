@@ -40,8 +40,8 @@
 #include <cstdint>
 #include <cstdlib>
 
-#include "gpp_crt.cuh"
 #include "gpp_crt.h"
+#include "gpp_crt_planes.cuh"
 #include "gpp_kernels.h"
 #include "gpp_umma.cuh"
 
@@ -50,7 +50,7 @@ namespace gpp {
 namespace {
 
 constexpr int kKcMax = 512;             // k values per chunk
-constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli
+constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli, at level 0
 constexpr int kTM = 128, kTN = 256;     // tcgen05.mma M (rows of X) x N (rows of Y)
 constexpr int kTK = 64;                 // k per operand block
 constexpr int kKSMax = kKcMax / kTK;    // operand blocks per chunk
@@ -61,14 +61,7 @@ constexpr int kThreads = 320;  // warp 0 loads, warp 1 issues the MMAs, warps 2-
 constexpr int kTmemCols = 2 * kTN;
 constexpr unsigned kIdesc = umma_idesc(kTM, kTN);
 
-constexpr int kExpZero = -4000;        // exponent of an all-zero chunk of a row
-constexpr int kExpNonFinite = 1 << 20; // of one that holds an Inf or a NaN
-
-__constant__ CrtGroup c_group[kCrtGroups] = {GPP_CRT_GROUPS};
-__constant__ CrtMod c_mod[kCrtN] = {
-    crt_mod(256), crt_mod(255), crt_mod(253), crt_mod(251), crt_mod(247),
-    crt_mod(241), crt_mod(239), crt_mod(233), crt_mod(229), crt_mod(227),
-    crt_mod(223), crt_mod(217), crt_mod(211), crt_mod(199), crt_mod(197)};
+__constant__ CrtGroup c_group[kCrtLevels][kCrtGroups] = {GPP_CRT_GROUPS};
 
 struct Geometry {
     int M, N, K;
@@ -146,13 +139,6 @@ __device__ __forceinline__ double2 operand_at(const OzOperand &z, int l, int k) 
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
 }
-// The e of frexp for the nonzero magnitude with bits b (b < 2^e).
-__device__ __forceinline__ int exp_of_bits(unsigned long long b) {
-    if (b == 0) return kExpZero;
-    const int E = (int)(b >> 52);
-    if (E == 0x7FF) return kExpNonFinite;  // the bit patterns of Inf and NaN are the largest
-    return E > 0 ? E - 1022 : (63 - __clzll((long long)b)) - 1073;
-}
 
 struct PrepOperand {
     OzOperand z;
@@ -172,7 +158,9 @@ struct PrepOperand {
 // of tcgen05.mma, one contiguous block per (row tile, k step).
 // Bound by its writes (90 bytes per complex value) and the FP32 pipe.
 __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOperand Y, int xblocks,
-                                                          int K, int Kc, int c0, int nc) {
+                                                          int K, int Kc, int c0, int nc, int nmod,
+                                                          int bits, const int *go) {
+    if (go && !*go) return;
     extern __shared__ __align__(16) double2 stage[];  // [8][Kc + 1]
     __shared__ unsigned long long red[8][8];
     __shared__ int exps[8];
@@ -198,7 +186,7 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
         }
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-        if (lane == 0) exps[warp] = exp_of_bits(mx);
+        if (lane == 0) exps[warp] = crt_exponent(mx);
         __syncthreads();
     } else {  // lanes along the 8 rows, 4 k per warp
         const int r = lane & 7, l = l0 + r;
@@ -216,7 +204,7 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
         if (threadIdx.x < 8) {
 #pragma unroll
             for (int w = 1; w < 8; ++w) mx = max(mx, red[w][threadIdx.x]);
-            exps[threadIdx.x] = exp_of_bits(mx);
+            exps[threadIdx.x] = crt_exponent(mx);
         }
         __syncthreads();
     }
@@ -234,10 +222,10 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
             float a[4], bb[4], cr[4], ci[4];
             const double2 v0 = stage[row * pitch + kg * 8 + 2 * t];
             const double2 v1 = stage[row * pitch + kg * 8 + 2 * t + 1];
-            crt_digits(oz_fixed_point(v0.x, e, kCrtBits), a);
-            crt_digits(oz_fixed_point(v1.x, e, kCrtBits), bb);
-            crt_digits(oz_fixed_point(v0.y, e, kCrtBits), cr);
-            crt_digits(oz_fixed_point(v1.y, e, kCrtBits), ci);
+            crt_digits(oz_fixed_point(v0.x, e, bits), a);
+            crt_digits(oz_fixed_point(v1.x, e, bits), bb);
+            crt_digits(oz_fixed_point(v0.y, e, bits), cr);
+            crt_digits(oz_fixed_point(v1.y, e, bits), ci);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 dr[t][k] = f2(a[k], bb[k]);
@@ -246,27 +234,7 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
         }
         const int ks = c * (Kc / kTK) + (kg >> 3);
         __nv_bfloat16 *w = o.out + base + (size_t)ks * (o.R / 8) * 512 + (kg & 7) * 64;
-#pragma unroll 1
-        for (int i = 0; i < kCrtN; ++i) {
-            const CrtMod m = c_mod[i];
-            unsigned pr[4], pi[4], ps[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const float2 rr = crt_residue2(dr[t], m), ri = crt_residue2(di[t], m);
-                const float2 rs = crt_reduce2(f2add(rr, ri), m.p, m.inv);
-                const __nv_bfloat162 hr = __floats2bfloat162_rn(rr.x, rr.y);
-                const __nv_bfloat162 hi = __floats2bfloat162_rn(ri.x, ri.y);
-                const __nv_bfloat162 hs = __floats2bfloat162_rn(rs.x, rs.y);
-                pr[t] = *reinterpret_cast<const unsigned *>(&hr);
-                pi[t] = *reinterpret_cast<const unsigned *>(&hi);
-                ps[t] = *reinterpret_cast<const unsigned *>(&hs);
-            }
-            *reinterpret_cast<uint4 *>(w + (size_t)i * plane) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
-            *reinterpret_cast<uint4 *>(w + (size_t)(kCrtN + i) * plane) =
-                make_uint4(pi[0], pi[1], pi[2], pi[3]);
-            *reinterpret_cast<uint4 *>(w + (size_t)(2 * kCrtN + i) * plane) =
-                make_uint4(ps[0], ps[1], ps[2], ps[3]);
-        }
+        crt_store_residues<4, 4>(dr, di, nmod, w, plane);
     }
 }
 
@@ -325,7 +293,7 @@ struct Walk {
     }
 };
 
-// Residues of the products: plane q = c kPlanes + (3M plane, modulus) of the
+// Residues of the products: plane q = c (3 nmod) + (3M plane, modulus) of the
 // pass's chunks, rows [128 mt0, + 128 MT) of X against every row of Y; the
 // byte stored is the symmetric residue + 128, at res[(q Ms + row) Np + col].
 // Warp 0 (one thread) loads: X's blocks of a row tile into kKSMax resident
@@ -340,7 +308,9 @@ struct Walk {
 __global__ void __launch_bounds__(kThreads, 1)
 crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restrict__ SY, int Mp,
                 int Np, int KS, int nc, int mt0, int MT, int gq, unsigned char *__restrict__ res,
-                int Ms, int *err) {
+                int Ms, int nmod, const int *go, int *err) {
+    if (go && !*go) return;
+    const int planes = 3 * nmod;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *sA = smem;
     unsigned char *sB = smem + (size_t)kKSMax * kBytesA;
@@ -356,7 +326,7 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ksteps = nc * KS;
     Walk w;
-    w.Q = nc * kPlanes;
+    w.Q = nc * planes;
     w.MT = MT;
     w.NT = Np / kTN;
     w.gq = gq;
@@ -397,7 +367,7 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
             int run = -1, nb = 0;  // row-tile runs and Y blocks so far
             bool ok = true;
             for (bool more = w.start(); ok && more; more = w.next()) {
-                const int c = w.q / kPlanes, pl = w.q % kPlanes;
+                const int c = w.q / planes, pl = w.q % planes;
                 const __nv_bfloat16 *a = SX + pl * xplane +
                                          ((size_t)(mt0 + w.mt) * ksteps + (size_t)c * KS) * (kTM * kTK);
                 const __nv_bfloat16 *b =
@@ -461,7 +431,7 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
             const int acc = G & 1;
             if (!bar_wait(&accfull[acc], (G >> 1) & 1, abort)) break;
             tc_fence_after();
-            const CrtMod m = c_mod[(w.q % kPlanes) % kCrtN];
+            const CrtMod m = c_crt_mod[(w.q % planes) % nmod];
             unsigned char *o = res + ((size_t)w.q * Ms + (size_t)w.mt * kTM + quarter * 32 + lane) * Np +
                                (size_t)w.nt * kTN + half * 128;
             const unsigned ta = tmem + ((unsigned)(quarter * 32) << 16) + acc * kTN + half * 128;
@@ -519,11 +489,14 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
 // im for each column, their sum of fractions (integer multiply-adds) and
 // X 2^(ex + ey - 106), and adds it to the running FP64 result, chunk by chunk.
 // Bound by integer issue.
+template <int L>
 __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char *res, const int *EX,
                                                              const int *EY, int row0, int rows,
                                                              int Ms, int N, int Mp, int Np, int nc,
                                                              int accumulate, double2 *Out,
-                                                             long long out_ld) {
+                                                             long long out_ld, const int *go) {
+    if (go && !*go) return;
+    constexpr int NM = kCrtLevel[L].n, PLANES = 3 * NM, GROUPS = (NM + 1) / 2;
     const unsigned quads = (N + 3) / 4;
     const long long n = (long long)rows * quads;
     const size_t plane = (size_t)Ms * Np;
@@ -543,10 +516,10 @@ __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char
         for (int j = 0; j < 4; ++j)
             acc[j] = accumulate && col0 + j < N ? out[j] : make_double2(0.0, 0.0);
         for (int c = 0; c < nc; ++c) {
-            const unsigned char *f = res + (size_t)c * kPlanes * plane + (size_t)r * Np + col0;
-            unsigned u[kPlanes];
+            const unsigned char *f = res + (size_t)c * PLANES * plane + (size_t)r * Np + col0;
+            unsigned u[PLANES];
 #pragma unroll
-            for (int q = 0; q < kPlanes; ++q)
+            for (int q = 0; q < PLANES; ++q)
                 u[q] = __ldg(reinterpret_cast<const unsigned *>(f + q * plane));
             const int ex = __ldg(EX + (size_t)c * Mp + row0 + r);
             const int4 ey = __ldg(reinterpret_cast<const int4 *>(EY + (size_t)c * Np + col0));
@@ -557,26 +530,26 @@ __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char
                 CrtSum re, im;
                 const unsigned sel = 0x4440 + j;
 #pragma unroll
-                for (int k = 0; k < kCrtGroups; ++k) {
+                for (int k = 0; k < GROUPS; ++k) {
                     int rr[2] = {0, 0}, ri[2] = {0, 0};
 #pragma unroll
-                    for (int h = 0; h < 2 && 2 * k + h < kCrtN; ++h) {
+                    for (int h = 0; h < 2 && 2 * k + h < NM; ++h) {
                         const int i = 2 * k + h;
                         const int a = __byte_perm(u[i], 0, sel);
-                        const int b = __byte_perm(u[kCrtN + i], 0, sel);
+                        const int b = __byte_perm(u[NM + i], 0, sel);
                         rr[h] = a - b;                                      // r1 - r2
-                        ri[h] = (int)__byte_perm(u[2 * kCrtN + i], 0, sel) - a - b;  // r3 - r1 - r2 - 128
+                        ri[h] = (int)__byte_perm(u[2 * NM + i], 0, sel) - a - b;  // r3 - r1 - r2 - 128
                     }
-                    re.add<0>(rr[0], rr[1], c_group[k]);
-                    im.add<-128>(ri[0], ri[1], c_group[k]);
+                    re.add<0>(rr[0], rr[1], c_group[L][k]);
+                    im.add<-128>(ri[0], ri[1], c_group[L][k]);
                 }
                 const int eyj = j == 0 ? ey.x : j == 1 ? ey.y : j == 2 ? ey.z : ey.w;
                 double2 v;
                 if (ex >= kExpNonFinite || eyj >= kExpNonFinite)
                     v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
                 else
-                    v = make_double2(crt_value(re, ex + eyj - 2 * kCrtBits),
-                                     crt_value(im, ex + eyj - 2 * kCrtBits));
+                    v = make_double2(crt_value<L>(re, ex + eyj - 2 * kCrtLevel[L].bits),
+                                     crt_value<L>(im, ex + eyj - 2 * kCrtLevel[L].bits));
                 if (c == 0 && !accumulate && nc == 1) {
                     if (col0 + j < N) out[j] = v;
                     continue;
@@ -600,7 +573,75 @@ int sm_count() {
     return sms > 0 ? sms : 132;
 }
 
+cudaError_t configure() {
+    static std::atomic<bool> configured[256] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || configured[dev & 255].load(std::memory_order_acquire)) return e;
+    e = cudaFuncSetAttribute(crt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(crt_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double2) * 8 * (kKcMax + 1)));
+    if (e == cudaSuccess) configured[dev & 255].store(true, std::memory_order_release);
+    return e;
+}
+
+void launch_prep(const PrepOperand &px, const PrepOperand &py, int xblocks, int yblocks, int K,
+                 int Kc, int c0, int nc, int level, const int *go, cudaStream_t s) {
+    crt_prep_kernel<<<xblocks + yblocks, 256, sizeof(double2) * 8 * (Kc + 1), s>>>(
+        px, py, xblocks, K, Kc, c0, nc, kCrtLevel[level].n, kCrtLevel[level].bits, go);
+}
+
 }  // namespace
+
+cudaError_t crt_rows(const OzOperand &X, int Mp, int K, int Kc, int c0, int nc, int level, void *sx,
+                     int *ex, const int *go, cudaStream_t s) {
+    cudaError_t e = configure();
+    if (e != cudaSuccess) return e;
+    const PrepOperand px{X, Mp, kTM, static_cast<__nv_bfloat16 *>(sx), ex};
+    launch_prep(px, px, Mp / 8 * nc, 0, K, Kc, c0, nc, level, go, s);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0,
+                         int tiles, int level, unsigned char *res, int Ms, const int *go, int *err,
+                         cudaStream_t s) {
+    cudaError_t e = configure();
+    if (e != cudaSuccess) return e;
+    const int nmod = kCrtLevel[level].n, ntiles = Np / kTN;
+    const int grid = (int)std::min<long long>(sm_count(), (long long)nc * 3 * nmod * tiles * ntiles);
+    // Planes in flight: enough that every block has a step, with their
+    // operands within about 80 MB of L2.
+    const size_t plane = sizeof(__nv_bfloat16) * (size_t)Kc * (Mp + Np);
+    const int gq = std::max(ceil_div(grid, (long long)tiles * ntiles),
+                            std::min(ceil_div(grid, tiles), (int)((size_t(80) << 20) / plane)));
+    crt_gemm_kernel<<<grid, kThreads, kSmem, s>>>(
+        static_cast<const __nv_bfloat16 *>(sx), static_cast<const __nv_bfloat16 *>(sy), Mp, Np,
+        Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, err);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t crt_combine(const unsigned char *res, const int *ex, const int *ey, int row0, int rows,
+                        int Ms, int N, int Mp, int Np, int nc, int level, bool accumulate,
+                        double2 *Out, long long out_ld, const int *go, cudaStream_t s) {
+    const long long want = ((long long)rows * ceil_div(N, 4) + 127) / 128;
+    const int grid = (int)std::min<long long>(want, (long long)sm_count() * 32);
+    auto launch = [&](auto kern) {
+        kern<<<grid, 128, 0, s>>>(res, ex, ey, row0, rows, Ms, N, Mp, Np, nc, accumulate, Out, out_ld,
+                                  go);
+    };
+    switch (level) {
+        case 0: launch(crt_combine_kernel<0>); break;
+        case 1: launch(crt_combine_kernel<1>); break;
+        case 2: launch(crt_combine_kernel<2>); break;
+        default: launch(crt_combine_kernel<3>); break;
+    }
+    count_launch();
+    return cudaGetLastError();
+}
 
 size_t crt_bytes(int M, int N, int K, int splits) {
     return carve(geometry(M, N, K, splits), nullptr, nullptr);
@@ -615,23 +656,9 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
     const Geometry g = geometry(M, N, K, splits);
     Buffers b;
     carve(g, ws, &b);
-    const size_t prep_smem = sizeof(double2) * 8 * (g.Kc + 1);
-    static std::atomic<bool> configured[256] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    cudaError_t e = configure();
     if (e != cudaSuccess) return e;
-    if (!configured[dev & 255].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(crt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(crt_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(double2) * 8 * (kKcMax + 1)));
-        if (e != cudaSuccess) return e;
-        configured[dev & 255].store(true, std::memory_order_release);
-    }
-    const int sms = sm_count();
-    const int mtiles = g.Mp / kTM, Ms = g.slab_tiles * kTM, KS = g.Kc / kTK;
-    int launches = 0;
+    const int mtiles = g.Mp / kTM, Ms = g.slab_tiles * kTM;
     for (int z = 0; z < g.splits; ++z) {
         const int zc0 = z * g.cps, zc1 = std::min(g.nch, zc0 + g.cps);
         for (int c0 = zc0; c0 < zc1; c0 += g.slab_chunks) {
@@ -640,13 +667,12 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                 OzOperand Yn = Y;
                 Yn.z += (long long)n0 * (Y.kfast ? Y.ld : 1);
                 Yn.L = std::min(N - n0, g.Np);
-                const int Np = ceil_div(Yn.L, kTN) * kTN, ntiles = Np / kTN;
+                const int Np = ceil_div(Yn.L, kTN) * kTN;
                 const PrepOperand px{X, g.Mp, kTM, b.sx, b.ex}, py{Yn, Np, kTN, b.sy, b.ey};
                 // X's planes serve every pass over rows of Y.
-                const int xblocks = n0 == 0 ? g.Mp / 8 * nc : 0, yblocks = Np / 8 * nc;
-                crt_prep_kernel<<<xblocks + yblocks, 256, prep_smem, s>>>(px, py, xblocks, K, g.Kc,
-                                                                          c0, nc);
-                ++launches;
+                launch_prep(px, py, n0 == 0 ? g.Mp / 8 * nc : 0, Np / 8 * nc, K, g.Kc, c0, nc, 0,
+                            nullptr, s);
+                count_launch();
                 if (after_slices && z == 0 && c0 == 0 && n0 == 0) {
                     e = cudaEventRecord(after_slices, s);
                     if (e != cudaSuccess) return e;
@@ -654,30 +680,16 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                 for (int mt0 = 0; mt0 < mtiles; mt0 += g.slab_tiles) {
                     const int tiles = std::min(g.slab_tiles, mtiles - mt0);
                     const int row0 = mt0 * kTM, rows = std::min(M - row0, tiles * kTM);
-                    const long long steps = (long long)nc * kPlanes * tiles * ntiles;
-                    const int grid = (int)std::min<long long>(sms, steps);
-                    // Planes in flight: enough that every block has a step, with
-                    // their operands within about 80 MB of L2.
-                    const size_t plane = sizeof(__nv_bfloat16) * (size_t)g.Kc * (g.Mp + Np);
-                    const int gq = std::max(ceil_div(grid, (long long)tiles * ntiles),
-                                            std::min(ceil_div(grid, tiles),
-                                                     (int)((size_t(80) << 20) / plane)));
-                    crt_gemm_kernel<<<grid, kThreads, kSmem, s>>>(b.sx, b.sy, g.Mp, Np, KS, nc, mt0,
-                                                                  tiles, gq, b.res, Ms, err);
-                    ++launches;
-                    if (rows > 0) {
-                        const long long want = ((long long)rows * ceil_div(Yn.L, 4) + 127) / 128;
-                        crt_combine_kernel<<<(int)std::min<long long>(want, (long long)sms * 32),
-                                             128, 0, s>>>(
-                            b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, c0 > zc0,
-                            Out + z * split_stride + n0, out_ld);
-                        ++launches;
-                    }
+                    e = crt_products(b.sx, b.sy, g.Mp, Np, g.Kc, nc, mt0, tiles, 0, b.res, Ms,
+                                     nullptr, err, s);
+                    if (e == cudaSuccess && rows > 0)
+                        e = crt_combine(b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, 0,
+                                        c0 > zc0, Out + z * split_stride + n0, out_ld, nullptr, s);
+                    if (e != cudaSuccess) return e;
                 }
             }
         }
     }
-    count_launch(launches);
     return cudaGetLastError();
 }
 

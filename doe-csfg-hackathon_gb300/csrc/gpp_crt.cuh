@@ -18,33 +18,55 @@ constexpr int kCrtN = 15;
 #define GPP_CRT_MODULI \
     256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197
 constexpr int kCrtModuli[kCrtN] = {GPP_CRT_MODULI};
-// Bits of the operands' fixed point: |N| <= 2^53, so a real or imaginary part
-// of a complex product sum over 512 k is at most 2 512 2^106 = 2^116 < P / 2.
-constexpr int kCrtBits = 53;
+// Levels of precision: the first n moduli with operands of `bits` bits,
+// 2 512 2^(2 bits) < P / 2 for the product P of the n.  Level 0 is FP64's.
+constexpr int kCrtLevels = 4;
+struct CrtLevel {
+    int n, bits;
+    unsigned long long pn;  // P = pn 2^pe, its top 64 bits rounded
+    int pe;
+    unsigned long long off_hi, off_lo;  // below
+};
+constexpr CrtLevel kCrtLevel[kCrtLevels] = {
+    {15, 53, 0xDC47122BAA0C0C41ull, 54, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFFFFFECC9200ull},
+    {12, 41, 0xDF6327787D5133B8ull, 31, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFB6A7F4B9E00ull},
+    {9, 30, 0xAA977B6D2077B785ull, 8, 0xFFFFFFFFFFFFFFFCull, 0xFFA9A1B5A960FA00ull},
+    {6, 18, 0xE06F178117000000ull, -16, 0xFFFFFFFFFDB7FD11ull, 0x05004945E2C6AA00ull}};
 
 // The residues of a pair of moduli (p, q) enter as t = r_p a + r_q b, with
 // a = w_p q mod p q, b = w_q p mod p q and w_p = (P / p)^-1 mod p: then
-// X / P = sum over the 8 groups of t / (p q) (mod 1) for X = r mod every
+// X / P = sum over the groups of t / (p q) (mod 1) for X = r mod every
 // modulus, formed with E = round(2^128 / (p q)), least significant word first.
+// A level's off is -512 sum (a + b) E mod 2^128: t is offset by 512 (a + b) to
+// be positive.
 constexpr int kCrtGroups = 8;
 struct CrtGroup {
     unsigned a, b, E[4];
 };
-#define GPP_CRT_GROUPS                                                                  \
-    {57375u, 35072u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}},            \
-        {47941u, 45793u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}},        \
-        {28920u, 247u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}},          \
-        {32620u, 19120u, {0x317BC258u, 0x9B9BA76Cu, 0xEDD3DBC1u, 0x00012D46u}},        \
-        {14755u, 14427u, {0xD9951FDCu, 0x220C9DF6u, 0x89404322u, 0x000142BEu}},        \
-        {20615u, 17840u, {0x4AF518C9u, 0x79C54F61u, 0x7F7279BAu, 0x00015AB3u}},        \
-        {9552u, 27008u, {0xC98E25D0u, 0xC687FEF9u, 0xEA710C29u, 0x00018F8Fu}},         \
-        {91u, 0u, {0x3FACD51Eu, 0x4F44DF83u, 0x725AF6E7u, 0x014CAB88u}}
-constexpr CrtGroup kCrtGroup[kCrtGroups] = {GPP_CRT_GROUPS};
-// -512 sum (a + b) E mod 2^128: t is offset by 512 (a + b) to be positive.
-constexpr unsigned long long kCrtOffHi = 0xFFFFFFFFFFFFFFFFull, kCrtOffLo = 0xFFFFFFFFFECC9200ull;
-// P = kCrtPn 2^54, its top 64 bits rounded.
-constexpr unsigned long long kCrtPn = 0xDC47122BAA0C0C41ull;
-constexpr int kCrtPe = 54;
+#define GPP_CRT_GROUPS \
+    {{57375u, 35072u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
+     {47941u, 45793u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
+     {28920u, 247u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}, \
+     {32620u, 19120u, {0x317BC258u, 0x9B9BA76Cu, 0xEDD3DBC1u, 0x00012D46u}}, \
+     {14755u, 14427u, {0xD9951FDCu, 0x220C9DF6u, 0x89404322u, 0x000142BEu}}, \
+     {20615u, 17840u, {0x4AF518C9u, 0x79C54F61u, 0x7F7279BAu, 0x00015AB3u}}, \
+     {9552u, 27008u, {0xC98E25D0u, 0xC687FEF9u, 0xEA710C29u, 0x00018F8Fu}}, \
+     {91u, 0u, {0x3FACD51Eu, 0x4F44DF83u, 0x725AF6E7u, 0x014CAB88u}}}, \
+    {{47175u, 54016u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
+     {31124u, 19228u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
+     {17352u, 57057u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}, \
+     {10485u, 18642u, {0x317BC258u, 0x9B9BA76Cu, 0xEDD3DBC1u, 0x00012D46u}}, \
+     {10215u, 49693u, {0xD9951FDCu, 0x220C9DF6u, 0x89404322u, 0x000142BEu}}, \
+     {2170u, 33227u, {0x4AF518C9u, 0x79C54F61u, 0x7F7279BAu, 0x00015AB3u}}}, \
+    {{19635u, 61952u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
+     {29869u, 55913u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
+     {25546u, 56810u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}, \
+     {38212u, 34894u, {0x317BC258u, 0x9B9BA76Cu, 0xEDD3DBC1u, 0x00012D46u}}, \
+     {161u, 0u, {0xEF3B3FB8u, 0x313011E2u, 0xB3FB8744u, 0x011E2EF3u}}}, \
+    {{42585u, 37376u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
+     {13303u, 61479u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
+     {49646u, 45448u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}}
+constexpr CrtGroup kCrtGroup[kCrtLevels][kCrtGroups] = {GPP_CRT_GROUPS};
 
 // 1.5 2^23: a float of magnitude below 2^22 added to it is rounded to an
 // integer in the low mantissa bits.
@@ -76,6 +98,24 @@ __host__ __device__ __forceinline__ void crt_digits(long long N, float (&d)[4]) 
     for (int k = 0; k < 4; ++k) d[k] = small_int_to_float(v[k]);
 }
 
+// The same for |N| <= 2^bits, bits <= 41, in fewer digits: ND = 3 (the top one
+// up to 2^13) or, for bits <= 18, ND = 2.
+template <int ND>
+__host__ __device__ __forceinline__ void crt_digits_n(long long N, float (&d)[ND]) {
+    if constexpr (ND == 4) {
+        crt_digits(N, d);
+    } else if constexpr (ND == 3) {
+        const long long M = N + 8192ll * (1 + (1ll << 14));
+        d[0] = small_int_to_float((int)(M & 16383) - 8192);
+        d[1] = small_int_to_float((int)((M >> 14) & 16383) - 8192);
+        d[2] = small_int_to_float((int)(M >> 28));
+    } else {
+        const int M = (int)N + 8192;
+        d[0] = small_int_to_float((M & 16383) - 8192);
+        d[1] = small_int_to_float(M >> 14);
+    }
+}
+
 // v - p rint(v / p) on both lanes for integers |v| <= 2^23: the quotient is
 // rounded once, from the product by a 1 / p whose relative error is at most
 // 2^-25, so it is off by under 1 / (2 p) before rounding and the result is
@@ -87,9 +127,12 @@ __host__ __device__ __forceinline__ float2 crt_reduce2(float2 v, float p, float 
 }
 
 // Symmetric residues mod m.p of two values with the digits d (lanes).
-__host__ __device__ __forceinline__ float2 crt_residue2(const float2 (&d)[4], const CrtMod &m) {
-    const float2 v = f2fma(d[3], f2(m.c3, m.c3),
-                           f2fma(d[2], f2(m.c2, m.c2), f2fma(d[1], f2(m.c1, m.c1), d[0])));
+template <int ND>
+__host__ __device__ __forceinline__ float2 crt_residue2(const float2 (&d)[ND], const CrtMod &m) {
+    float2 v = d[0];
+    if constexpr (ND > 1) v = f2fma(d[1], f2(m.c1, m.c1), v);
+    if constexpr (ND > 2) v = f2fma(d[2], f2(m.c2, m.c2), v);
+    if constexpr (ND > 3) v = f2fma(d[3], f2(m.c3, m.c3), v);
     return crt_reduce2(v, m.p, m.inv);
 }
 
@@ -136,7 +179,8 @@ __device__ __noinline__
 #else
 inline
 #endif
-double crt_value_small(bool neg, unsigned w2, unsigned w1, unsigned w0, int e) {
+double crt_value_small(bool neg, unsigned w2, unsigned w1, unsigned w0, unsigned long long pn,
+                       int e) {
     unsigned long long hi = ((unsigned long long)w2 << 32) | w1, lo = (unsigned long long)w0 << 32;
     int n = 32;
     if (w2 == 0 && w1 == 0 && w0 < 71000000u) return 0.0;  // what a zero's rounding can leave
@@ -146,47 +190,50 @@ double crt_value_small(bool neg, unsigned w2, unsigned w1, unsigned w0, int e) {
         ++n;
     }
 #ifdef __CUDA_ARCH__
-    const unsigned long long h = __umul64hi(hi, kCrtPn);
+    const unsigned long long h = __umul64hi(hi, pn);
 #else
-    const unsigned long long h = (unsigned long long)(((unsigned __int128)hi * kCrtPn) >> 64);
+    const unsigned long long h = (unsigned long long)(((unsigned __int128)hi * pn) >> 64);
 #endif
-    return crt_assemble(neg, h, kCrtPe - n + e);
+    return crt_assemble(neg, h, e - n);
 }
 
 // X 2^e as a double, X the integer of magnitude below P / 2 with the given
-// residues: the sum is 2^128 X / P (mod 2^128) to within 2^26.1 (the rounding
+// residues at level L (bounds for level 0, where they matter most): the sum is 2^128 X / P (mod 2^128) to within 2^26.1 (the rounding
 // of the E), X to within 2^17 (a sum of that size is taken as 0) where the
 // largest products are 2^106; the top 64 bits of the fraction times P, rounded
 // to nearest.  Integer operations only, but for results outside the normal
 // range.
+template <int L>
 __host__ __device__ __forceinline__ double crt_value(const CrtSum &s, int e) {
-    const unsigned long long l0 = s.a0 + kCrtOffLo;
+    constexpr unsigned long long pn = kCrtLevel[L].pn, off_hi = kCrtLevel[L].off_hi,
+                                 off_lo = kCrtLevel[L].off_lo;
+    e += kCrtLevel[L].pe;
+    const unsigned long long l0 = s.a0 + off_lo;
     const unsigned long long c0 = l0 < s.a0 ? 1 : 0;
     const unsigned w0 = (unsigned)l0;
     unsigned long long l1 = (l0 >> 32) + (unsigned)s.a1;
     const unsigned w1 = (unsigned)l1;
-    unsigned long long l2 = (l1 >> 32) + (s.a1 >> 32) + s.a2 + c0 + kCrtOffHi;
+    unsigned long long l2 = (l1 >> 32) + (s.a1 >> 32) + s.a2 + c0 + off_hi;
     const unsigned w2 = (unsigned)l2;
-    // s.a2 and the carries stay below 2^63, and kCrtOffHi is -1: the upper
-    // words of the sum wrap as the 128-bit sum does.
+    // The upper words wrap as the 128-bit sum does.
     const unsigned w3 = (unsigned)(l2 >> 32) + s.a3;
     const bool neg = (int)w3 < 0;
     const unsigned x = neg ? 0xFFFFFFFFu : 0u;  // one's complement: off by one unit of 2^-128
     const unsigned v3 = w3 ^ x, v2 = w2 ^ x, v1 = w1 ^ x, v0 = w0 ^ x;
-    if (v3 == 0) return crt_value_small(neg, v2, v1, v0, e);
+    if (v3 == 0) return crt_value_small(neg, v2, v1, v0, pn, e);
 #ifdef __CUDA_ARCH__
     const int z = __clz((int)v3);
     const unsigned long long hi =
         ((unsigned long long)__funnelshift_l(v2, v3, z) << 32) | __funnelshift_l(v1, v2, z);
-    const unsigned long long h = __umul64hi(hi, kCrtPn);
+    const unsigned long long h = __umul64hi(hi, pn);
 #else
     const int z = __builtin_clz(v3);
     const unsigned long long up = ((unsigned long long)v3 << 32) | v2;
     const unsigned long long hi = z ? (up << z) | (v1 >> (32 - z)) : up;
-    const unsigned long long h = (unsigned long long)(((unsigned __int128)hi * kCrtPn) >> 64);
+    const unsigned long long h = (unsigned long long)(((unsigned __int128)hi * pn) >> 64);
 #endif
-    // |X| = hi 2^(64 - z) kCrtPn 2^kCrtPe / 2^128 = h 2^(kCrtPe - z)
-    return crt_assemble(neg, h, kCrtPe - z + e);
+    // |X| = hi 2^(64 - z) pn 2^pe / 2^128 = h 2^(pe - z)
+    return crt_assemble(neg, h, e - z);
 }
 
 }  // namespace gpp

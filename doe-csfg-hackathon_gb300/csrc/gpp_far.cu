@@ -1,0 +1,993 @@
+// gpp_far.cu -- unoccupied bands with per-band frequencies: the terms whose
+// frequency lies away from wtilde through a series, as products on the tensor
+// cores.
+//
+// An unoccupied term is c aqsn Q / (wx - wtilde).  The plasmon-pole
+// frequencies wtilde of a state lie in a band (a box of the complex plane,
+// centre z0, half width h after a margin), while wx = E - E_n1 runs over the
+// whole spectrum, so for most (band, frequency) pairs wx is well outside the
+// box, and there, with u = (wx - z0) / h, z = (wtilde - z0) / h and
+// r = u + sign(u) sqrt(u^2 - 1),
+//
+//   1 / (u - z) = (1 + 2 sum_{k >= 1} T_k(z) r^-k) / (r - u)
+//
+// (the generating function of the Chebyshev polynomials).  The sum over
+// columns of a pair is then
+//
+//   sum_ig aqsn Q / (wx - wtilde) = sum_k b_k(wx) H_k,  H_k[n1][r] = sum_ig aqsn[n1][ig] P_k[r][ig],
+//
+// P_k = Q T_k(z): one complex product per k that every frequency of every band
+// shares, instead of a division per (band, row, column, frequency).  |T_k| is
+// at most rho^k on the box (rho: its Bernstein ellipse); a pair is `far` when
+// |r| >= R rho, so the terms fall off by R and K = bits / log2 R of them reach
+// the working precision.  The products run as residues (gpp_crt.cu), each k at
+// the level of precision that R^-k leaves of the total's.
+//
+// What the series does not cover is computed term by term:
+//  * near pairs (|r| < R rho, or a wx that is not finite): over every column,
+//    in the call's precision;
+//  * the columns whose wtilde lies outside the box (a few strays, such as
+//    wtilde next to another band's frequency), for the far pairs, in FP64.
+//
+// The box is chosen on the device from a histogram of Re(wtilde) against the
+// histogram of wx, by the cost of what it leaves over; where no box pays, or
+// too many columns or pairs are left over, the plan is inactive, every kernel
+// here returns at once and the per-term kernel runs instead.  No host
+// synchronisation; nothing depends on the order in which blocks run.
+//
+// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 27 ms now (near
+// pairs 17, products 4.1, terms 2, combine 2); mixed, 128 bands x 819 x 16384 x
+// 32: 120 ms per term, 39 now (near 25, terms 7, products 4.3).
+#include <algorithm>
+#include <cmath>
+
+#include "gpp_crt.h"
+#include "gpp_crt_planes.cuh"
+#include "gpp_far.h"
+#include "gpp_tiles_fp64.cuh"
+
+namespace gpp {
+
+struct FarPlan {
+    int active;
+    int n_near;
+    long long n_out;
+    int lo, hi;          // the box's bins of Re(wtilde)
+    double x0, inv_w;    // bin = floor((x - x0) inv_w)
+    double im_max;       // |Im(wtilde)| of a column in the box is at most this
+    double z0, inv_h, h;
+    double dfar;         // |wx - z0| of a far pair is at least this
+    double log2_rho;
+    unsigned long long count[512];
+    unsigned im[512];    // bits of the largest |Im| (float, rounded up) in each bin
+};
+
+namespace {
+
+constexpr int kBins = 512;
+constexpr int kNearTile = 4;  // entries per block of the FP64 near kernel
+
+struct Sizes {
+    int bands, ng, nc, nw;
+    bool mixed;
+    double R;
+    int K;               // terms of the series
+    int Mp, ngp, nch, Kc;
+    int gm, slab;        // series terms and chunks per pass
+    int cap_near;
+    long long cap_out, seg_len;
+    int segs;
+    long long pairs;
+    double c0;           // cost of the series, in per-term pairs
+};
+
+constexpr size_t kPassBytes = size_t(8) << 30;
+int level_of(const Sizes &z, int k) {
+    const double need = (z.mixed ? 49.0 : 53.0) - k * std::log2(z.R);
+    int l = 0;
+    while (l + 1 < kCrtLevels && kCrtLevel[l + 1].bits >= need) ++l;
+    return l;
+}
+
+Sizes sizes(const Problem &p, int bands, bool mixed) {
+    Sizes z;
+    z.bands = bands;
+    z.ng = p.ng;
+    z.nc = p.nc;
+    z.nw = p.nw;
+    z.mixed = mixed;
+    z.R = mixed ? 3.0 : 2.5;
+    z.K = (int)std::ceil((mixed ? 50.0 : 55.0) / std::log2(z.R));
+    z.Mp = ceil_div(bands, kCrtRowsX) * kCrtRowsX;
+    z.ngp = ceil_div(p.ng, 8) * 8;
+    z.nch = std::max(1, ceil_div(p.nc, kCrtChunk));
+    z.Kc = ceil_div(ceil_div(p.nc, z.nch), kCrtBlockK) * kCrtBlockK;
+    const size_t per = (size_t)3 * kCrtN * z.ngp * (2 * (size_t)z.Kc + z.Mp);  // a term's, per chunk
+    z.gm = (int)std::min<size_t>(z.K, std::max<size_t>(4, kPassBytes / (per * z.nch)));
+    z.slab = (int)std::min<size_t>(z.nch, std::max<size_t>(1, kPassBytes / (per * z.gm)));
+    z.pairs = (long long)bands * p.nw;
+    z.cap_near = (int)std::min<long long>(z.pairs / 2 + 1, 1 << 26);
+    z.cap_out = (long long)p.ng * p.nc / 32 + 1;
+    z.seg_len = std::max<long long>(2048, (z.cap_out + 511) / 512);
+    z.segs = (int)((z.cap_out + z.seg_len - 1) / z.seg_len);
+    // Per cell: a per-term pair takes 20 ps (FP64) or 2.6 ps (mixed); a term of
+    // the series 14 ps for its planes and 0.07 ps per padded band.
+    z.c0 = z.K * (14.0 + 0.07 * z.Mp) / (mixed ? 2.6 : 20.0);
+    return z;
+}
+
+size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
+
+struct Buffers {
+    FarPlan *plan;
+    int4 *near;
+    int *rows;         // [ng + 1]: strays before each row
+    int2 *out;         // (row, column)
+    double2 *C;        // [bands][ng]
+    double2 *S1;       // [bands][K]
+    double2 *near_part, *near_val, *out_part;
+    double2 *state;    // P_(k-1), P_k between passes
+    int *E0, *EX, *EY;
+    __nv_bfloat16 *sx, *sy;
+    unsigned char *res;
+    double2 *H;        // [bands][gm ngp]
+};
+
+size_t carve(const Sizes &z, void *ws, Buffers *b) {
+    char *w = static_cast<char *>(ws);
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        char *q = w + off;
+        off = align_up(off + n);
+        return q;
+    };
+    Buffers o;
+    const size_t rt = (size_t)(z.ng + 1) / 2;
+    const int Np = ceil_div((long long)z.gm * z.ngp, kCrtRowsY) * kCrtRowsY;
+    o.plan = reinterpret_cast<FarPlan *>(take(sizeof(FarPlan)));
+    o.near = reinterpret_cast<int4 *>(take(sizeof(int4) * (size_t)z.cap_near));
+    o.rows = reinterpret_cast<int *>(take(sizeof(int) * ((size_t)z.ng + 1)));
+    o.out = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)z.cap_out));
+    o.C = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.ng));
+    o.S1 = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.K));
+    o.near_part = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near * rt));
+    o.near_val = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near));
+    o.out_part = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.segs * z.pairs));
+    o.state = reinterpret_cast<double2 *>(
+        take(sizeof(double2) * 2 * (size_t)z.nch * z.ngp * z.Kc));
+    o.E0 = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.ngp));
+    o.EX = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.Mp));
+    o.EY = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.slab * Np));
+    o.sx = reinterpret_cast<__nv_bfloat16 *>(
+        take(sizeof(__nv_bfloat16) * 3 * kCrtN * (size_t)z.Mp * z.nch * z.Kc));
+    o.sy = reinterpret_cast<__nv_bfloat16 *>(
+        take(sizeof(__nv_bfloat16) * 3 * kCrtN * (size_t)Np * z.slab * z.Kc));
+    o.res = reinterpret_cast<unsigned char *>(take((size_t)z.slab * 3 * kCrtN * z.Mp * Np));
+    o.H = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.gm * z.ngp));
+    if (b) *b = o;
+    return off;
+}
+
+__device__ __forceinline__ bool is_finite(double x) {
+    return (__double2hiint(x) & 0x7FF00000) != 0x7FF00000;
+}
+// The bin of Re(wtilde), or -1 for a value outside the bins, an imaginary
+// part above the cap or one that is not finite.
+__device__ __forceinline__ int bin_of(const FarPlan &f, double2 wt) {
+    if (!is_finite(wt.x) || !(fabs(wt.y) <= f.im_max)) return -1;
+    const double t = (wt.x - f.x0) * f.inv_w;
+    return t >= 0.0 && t < (double)kBins ? (int)t : -1;
+}
+__device__ __forceinline__ bool in_box(const FarPlan &f, double2 wt) {
+    const int b = bin_of(f, wt);
+    return b >= f.lo && b <= f.hi;
+}
+__device__ __forceinline__ bool is_far(const FarPlan &f, double wx) {
+    return is_finite(wx) && fabs(wx - f.z0) >= f.dfar;
+}
+
+// The bins: 512 over the range of the unoccupied bands' finite wx with a
+// margin, |Im(wtilde)| capped at 1/32 of it.
+__global__ void __launch_bounds__(1024) far_range_kernel(Problem p, int b0, int bands, FarPlan *f) {
+    __shared__ double lo[32], hi[32];
+    double a = 1.0 / 0.0, b = -1.0 / 0.0;
+    const long long n = (long long)bands * p.nw;
+    for (long long i = threadIdx.x; i < n; i += 1024) {
+        const double x = p.wx[(size_t)(b0 + i / p.nw) * p.wx_stride + i % p.nw];
+        if (is_finite(x)) {
+            a = fmin(a, x);
+            b = fmax(b, x);
+        }
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, s));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, s));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        lo[threadIdx.x >> 5] = a;
+        hi[threadIdx.x >> 5] = b;
+    }
+    for (int i = threadIdx.x; i < kBins; i += 1024) {
+        f->count[i] = 0;
+        f->im[i] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) {
+            a = fmin(a, lo[w]);
+            b = fmax(b, hi[w]);
+        }
+        f->active = f->n_near = 0;
+        f->n_out = 0;
+        const double margin = 0.02 * (b - a) + 1e-3 * fmax(fabs(a), fabs(b));
+        const double width = b - a + 2.0 * margin;
+        // No finite wx, all zero, or a range past what the bins can divide: no bins.
+        const bool ok = a <= b && width > 1e-100 && width < 1e100;
+        f->x0 = ok ? a - margin : 0.0;
+        f->inv_w = ok ? kBins / width : 0.0;
+        f->im_max = ok ? width / 32.0 : -1.0;
+    }
+}
+
+__global__ void __launch_bounds__(256) far_hist_kernel(Problem p, FarPlan *f) {
+    __shared__ unsigned cnt[kBins], im[kBins];
+    for (int i = threadIdx.x; i < kBins; i += 256) cnt[i] = im[i] = 0;
+    const double x0 = f->x0, inv_w = f->inv_w, cap = f->im_max;
+    __syncthreads();
+    const size_t n = (size_t)p.ng * p.nc;
+    FarPlan g;
+    g.x0 = x0;
+    g.inv_w = inv_w;
+    g.im_max = cap;
+#pragma unroll 4
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        const double2 wt = __ldg(p.wt + i);
+        const int b = bin_of(g, wt);
+        if (b >= 0) {
+            atomicAdd(&cnt[b], 1u);
+            const unsigned v = __float_as_uint(__double2float_ru(fabs(wt.y)));
+            if (v > im[b]) atomicMax(&im[b], v);  // a stale read only repeats the atomic
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kBins; i += 256) {
+        if (cnt[i]) atomicAdd(&f->count[i], (unsigned long long)cnt[i]);
+        if (im[i]) atomicMax(&f->im[i], im[i]);
+    }
+}
+
+// The box a .. b (bins lo .. hi, largest |Im| v): its half width after a
+// margin, and the log2 of its ellipse.
+struct Box {
+    float z0, h, rho;
+};
+__device__ __forceinline__ Box box_of(float a, float b, float v) {
+    Box q;
+    const float hw = 0.5f * (b - a);
+    q.z0 = 0.5f * (a + b);
+    q.h = fmaxf(hw + v, 1.02f * hw);
+    const float x = hw / q.h, y = v / q.h;
+    // Sum of the distances from the corner to the foci: the largest on the box.
+    const float s = 0.5f * (sqrtf((x - 1.f) * (x - 1.f) + y * y) + sqrtf((x + 1.f) * (x + 1.f) + y * y));
+    q.rho = s + sqrtf(fmaxf(s * s - 1.f, 0.f));
+    return q;
+}
+
+// One block: chooses the box and lists the near pairs in order.  The cost of
+// a box is what it leaves to the per-term kernels, in pairs over all columns:
+// its near pairs (times w_near), and the strays' share of the far ones (times
+// w_out).
+__global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int bands, FarPlan *f,
+                                                         int4 *near, int cap_near, long long cap_out,
+                                                         float R, float c0, float w_near,
+                                                         float w_out) {
+    __shared__ unsigned long long pre[kBins + 1];
+    __shared__ unsigned pairs_in[kBins];
+    __shared__ unsigned ppre[kBins + 1];
+    __shared__ float vb[kBins];
+    __shared__ unsigned long long best[kBins / 32];
+    __shared__ int scan[kBins / 32];
+    __shared__ int base, outside;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const long long n = (long long)bands * p.nw;
+    const long long cells = (long long)p.ng * p.nc;
+    if (t == 0) outside = 0;
+    pairs_in[t] = 0;
+    vb[t] = __uint_as_float(f->im[t]);
+    __syncthreads();
+    auto wx_at = [&](long long i) {
+        return p.wx[(size_t)(b0 + i / p.nw) * p.wx_stride + i % p.nw];
+    };
+    for (long long i = t; i < n; i += kBins) {
+        const int b = bin_of(*f, make_double2(wx_at(i), 0.0));
+        if (b >= 0)
+            atomicAdd(&pairs_in[b], 1u);
+        else
+            atomicAdd(&outside, 1);  // not finite: always near
+    }
+    __syncthreads();
+    if (t == 0) {
+        pre[0] = 0;
+        ppre[0] = 0;
+        for (int i = 0; i < kBins; ++i) {
+            pre[i + 1] = pre[i] + f->count[i];
+            ppre[i + 1] = ppre[i] + pairs_in[i];
+        }
+    }
+    __syncthreads();
+    const float w = (float)(1.0 / f->inv_w), total = (float)n, ncells = (float)cells;
+    unsigned long long mine = ~0ull;
+    if (pre[t + 1] > pre[t] && f->inv_w > 0.0) {
+        float v = 0.f;
+        for (int j = t; j < kBins; ++j) {
+            v = fmaxf(v, vb[j]);
+            if (pre[j + 1] == pre[j]) continue;
+            const long long out = cells - (long long)(pre[j + 1] - pre[t]);
+            if (out > cap_out) continue;
+            const Box q = box_of(t * w, (j + 1) * w, v);
+            const float r = R * q.rho, d = q.h * 0.5f * (r + 1.f / r);
+            const int i0 = max(0, min(kBins, (int)floorf((q.z0 - d) / w)));
+            const int i1 = max(0, min(kBins, (int)floorf((q.z0 + d) / w) + 1));
+            const float nr = (float)(ppre[i1] - ppre[i0]) + (float)outside;
+            const float cost = nr * w_near + (float)out / ncells * (total - nr) * w_out;
+            const unsigned long long key =
+                ((unsigned long long)__float_as_uint(fmaxf(cost, 0.f)) << 32) | (unsigned)(t * kBins + j);
+            if (key < mine) mine = key;
+        }
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) mine = min(mine, __shfl_xor_sync(0xffffffffu, mine, s));
+    if (lane == 0) best[warp] = mine;
+    __syncthreads();
+    __shared__ int go;
+    if (t == 0) {
+        for (int i = 1; i < kBins / 32; ++i) mine = min(mine, best[i]);
+        go = 0;
+        base = 0;
+        if (mine != ~0ull && __uint_as_float((unsigned)(mine >> 32)) + c0 < 0.9f * total) {
+            const int lo = (int)((unsigned)mine / kBins), hi = (int)((unsigned)mine % kBins);
+            float v = 0.f;
+            for (int j = lo; j <= hi; ++j) v = fmaxf(v, vb[j]);
+            const Box q = box_of(lo * w, (hi + 1) * w, v);
+            f->lo = lo;
+            f->hi = hi;
+            f->n_out = cells - (long long)(pre[hi + 1] - pre[lo]);
+            // In double, with margins above the float rounding of the choice.
+            const double a = f->x0 + lo / f->inv_w, b = f->x0 + (hi + 1) / f->inv_w;
+            f->z0 = 0.5 * (a + b);
+            f->h = fmax((double)q.h, 0.5 * (b - a));
+            f->inv_h = 1.0 / f->h;
+            const double rho = (double)q.rho * 1.00001, r = (double)R * rho;
+            f->log2_rho = log2(rho);
+            f->dfar = f->h * 0.5 * (r + 1.0 / r);
+            go = 1;
+        }
+    }
+    __syncthreads();
+    if (!go) return;
+    // Near pairs: counted first, then listed in order.
+    int c = 0;
+    for (long long i = t; i < n; i += kBins) c += !is_far(*f, wx_at(i));
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) scan[warp] = c;
+    __syncthreads();
+    if (t == 0) {
+        int s = 0;
+        for (int i = 0; i < kBins / 32; ++i) s += scan[i];
+        if (s > cap_near || s * w_near + c0 >= 0.95f * total) go = 0;
+    }
+    __syncthreads();
+    if (!go) return;
+    // An entry covers up to kNearFreq consecutive near frequencies of a band;
+    // the first pair of each such run of pairs writes it.  The longest entries
+    // come first, so that the warps of a block have equal work.
+    for (int want = kNearFreq; want >= 1; --want) {
+        for (long long i0 = 0; i0 < n; i0 += kBins) {
+            const long long i = i0 + t;
+            const int iw = (int)(i % p.nw);
+            int len = 0;
+            if (i < n && !is_far(*f, wx_at(i))) {
+                int before = 0;
+                while (before < iw && !is_far(*f, wx_at(i - before - 1))) ++before;
+                if (before % kNearFreq == 0)
+                    for (len = 1; len < kNearFreq && iw + len < p.nw && !is_far(*f, wx_at(i + len));) ++len;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, len == want);
+            if (lane == 0) scan[warp] = __popc(m);
+            __syncthreads();
+            int at = base + __popc(m & ((1u << lane) - 1));
+            for (int k = 0; k < warp; ++k) at += scan[k];
+            if (len == want) near[at] = make_int4(b0 + (int)(i / p.nw), iw, len, 0);
+            __syncthreads();
+            if (t == 0)
+                for (int k = 0; k < kBins / 32; ++k) base += scan[k];
+            __syncthreads();
+        }
+    }
+    if (t == 0) {
+        f->n_near = base;
+        f->active = 1;
+    }
+}
+
+// Strays per row, their offsets, and their (row, column) list in order.
+__global__ void __launch_bounds__(256) far_count_kernel(Problem p, const FarPlan *f, int *rows) {
+    if (!f->active || f->n_out == 0) return;
+    __shared__ int c[8];
+    const int r = blockIdx.x;
+    int n = 0;
+    for (int ig = threadIdx.x; ig < p.nc; ig += 256) n += !in_box(*f, __ldg(p.wt + (size_t)r * p.nc + ig));
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) c[threadIdx.x >> 5] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) n += c[w];
+        rows[r + 1] = n;
+    }
+}
+__global__ void __launch_bounds__(1024) far_scan_kernel(int ng, const FarPlan *f, int *rows) {
+    if (!f->active || f->n_out == 0) return;
+    __shared__ int part[1024];
+    const int per = (ng + 1023) / 1024, a = threadIdx.x * per, b = min(ng, a + per);
+    int s = 0;
+    for (int i = a; i < b; ++i) s += rows[i + 1];
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int acc = 0;
+        for (int i = 0; i < 1024; ++i) {
+            const int v = part[i];
+            part[i] = acc;
+            acc += v;
+        }
+        rows[0] = 0;
+    }
+    __syncthreads();
+    s = part[threadIdx.x];
+    for (int i = a; i < b; ++i) rows[i + 1] = s += rows[i + 1];
+}
+__global__ void __launch_bounds__(256) far_list_kernel(Problem p, const FarPlan *f, const int *rows,
+                                                       int2 *out) {
+    if (!f->active || f->n_out == 0) return;
+    __shared__ int c[8];
+    const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int at = rows[r];
+    if (rows[r + 1] == at) return;
+    for (int g0 = 0; g0 < p.nc; g0 += 256) {
+        const int ig = g0 + threadIdx.x;
+        const bool is = ig < p.nc && !in_box(*f, __ldg(p.wt + (size_t)r * p.nc + ig));
+        const unsigned m = __ballot_sync(0xffffffffu, is);
+        if (lane == 0) c[warp] = __popc(m);
+        __syncthreads();
+        int k = at + __popc(m & ((1u << lane) - 1));
+        int all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) k += c[w];
+            all += c[w];
+        }
+        if (is) out[k] = make_int2(r, ig);
+        at += all;
+        __syncthreads();
+    }
+}
+
+// c[k][r] = 0.5 vcoul conj(aqsm[b0 + k]) at row r's G' index (0 where that is
+// invalid; the fault is recorded).
+__global__ void __launch_bounds__(256) far_coeff_kernel(Problem p, int b0, int bands, double2 *C,
+                                                        const FarPlan *f, int *err) {
+    if (!f->active) return;
+    const long long n = (long long)bands * p.ng;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const int k = (int)(i / p.ng), r = (int)(i % p.ng);
+        const int igp = resolve_igp(p, r, err);
+        double2 c = make_double2(0.0, 0.0);
+        if (igp >= 0) {
+            const double2 m = __ldg(p.aqsm + (size_t)(b0 + k) * p.nc + igp);
+            c = cscale(make_double2(0.5 * m.x, -0.5 * m.y), __ldg(p.vcoul + igp));
+        }
+        C[i] = c;
+    }
+}
+
+// round(x 2^(bits - e)) for bits <= 30 on 32-bit words, |x| < 2^e and x normal
+// or zero (a subnormal, far below any chunk that matters, counts as zero).
+__device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
+    const unsigned hi = __double2hiint(x), lo = __double2loint(x);
+    const int E = (hi >> 20) & 0x7FF;
+    const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;  // 53-bit mantissa, x = m 2^(E - 1075)
+    // One bit more than the result, then rounded (ties away from zero).
+    const int sh = 1074 - E - bits + e;
+    unsigned n = 0;
+    if (sh < 32)
+        n = __funnelshift_r(lo, mh, sh);
+    else if (sh < 64)
+        n = mh >> (sh - 32);
+    if (E == 0) n = 0;
+    n = (n + 1) >> 1;
+    return (int)hi < 0 ? -(int)n : (int)n;
+}
+
+// Residue planes and exponents of P_k, k = k0 .. k0 + gm - 1, for 8 rows x one
+// chunk at level L: row r of term m is row m ngp + r of the product's Y
+// operand, in the core-matrix blocks of crt_prep_kernel.  A thread carries 4
+// consecutive columns of a row (half a core-matrix row; 8 would halve the
+// resident warps) through the recurrence P_(k+1) = 2 z P_k - P_(k-1) (P_-1 =
+// z Q starts it) and leaves P_(k-1), P_k for the next pass in `state`.  The
+// exponent of term k is that of the chunk's largest |re|, |im| of Q, raised by
+// the bound rho^k of |T_k| and 1.  Columns outside the box are zero.
+constexpr int kTermK = 4;  // columns per thread
+template <int L>
+__global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int c0,
+                                                           int nc, int Kc, int Np, int k0, int gm,
+                                                           int last, __nv_bfloat16 *out, int *EY,
+                                                           int *E0, double2 *state) {
+    constexpr int NMOD = kCrtLevel[L].n, BITS = kCrtLevel[L].bits, ND = BITS > 41 ? 4 : BITS > 18 ? 3 : 2;
+    if (!f->active) return;
+    __shared__ unsigned long long red[4][8];
+    __shared__ int exps[8];
+    const int groups = ngp / 8;
+    const int grp = blockIdx.x % groups, c = blockIdx.x / groups;
+    const int t = threadIdx.x, half = t & 1, row = (t >> 1) & 7, kg0 = t >> 4, r = grp * 8 + row;
+    const int kb = (c0 + c) * Kc, items = (Kc + 63) / 64;
+    const double2 *wrow = p.wt + (size_t)min(r, p.ng - 1) * p.nc;
+    const double2 *erow = p.ieps + (size_t)min(r, p.ng - 1) * p.nc;
+    const double z0 = f->z0, inv_h = f->inv_h;
+    auto at = [&](int ig, double2 &wt) {
+        if (r >= p.ng || ig >= p.nc) return false;
+        wt = __ldg(wrow + ig);
+        return in_box(*f, wt);
+    };
+    if (k0 == 0) {
+        unsigned long long mx = 0;
+        for (int i = 0; i < items; ++i) {
+#pragma unroll
+            for (int kk = 0; kk < kTermK; ++kk) {
+                double2 wt;
+                const int ig = kb + (kg0 + 8 * i) * 8 + half * kTermK + kk;
+                if (!at(ig, wt)) continue;
+                const double2 q = cmul(wt, __ldg(erow + ig));
+                const unsigned long long a = (unsigned long long)__double_as_longlong(q.x) & 0x7FFFFFFFFFFFFFFFull;
+                const unsigned long long b = (unsigned long long)__double_as_longlong(q.y) & 0x7FFFFFFFFFFFFFFFull;
+                mx = max(mx, max(a, b));
+            }
+        }
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        if ((t & 17) == 0) red[t >> 5][row] = mx;
+        __syncthreads();
+        if (t < 8) {
+            mx = red[0][t];
+            for (int w = 1; w < 4; ++w) mx = max(mx, red[w][t]);
+            exps[t] = crt_exponent(mx);
+            E0[(size_t)(c0 + c) * ngp + grp * 8 + t] = exps[t];
+        }
+    } else if (t < 8) {
+        exps[t] = E0[(size_t)(c0 + c) * ngp + grp * 8 + t];
+    }
+    __syncthreads();
+    const int e0 = exps[row];
+    const double log2_rho = f->log2_rho;
+    auto raise = [&](int k) { return k == 0 ? 0 : 1 + (int)ceil(k * log2_rho); };
+    if (half == 0)
+        for (int m = kg0; m < gm; m += 8) EY[(size_t)c * Np + (size_t)m * ngp + r] = e0 + raise(k0 + m);
+
+    const int ksteps = nc * (Kc / kCrtBlockK);
+    const size_t plane = (size_t)Np * ksteps * kCrtBlockK;
+    double2 *st = state + ((size_t)(c0 + c) * groups + grp) * (size_t)items * (2 * kTermK * 128);
+    for (int i = 0; i < items; ++i) {  // Kc is a multiple of 64: 8 k-cores per turn
+        const int kg = kg0 + 8 * i;
+        double2 cur[kTermK], prev[kTermK], z2[kTermK];
+#pragma unroll
+        for (int kk = 0; kk < kTermK; ++kk) {
+            const int ig = kb + kg * 8 + half * kTermK + kk;
+            double2 wt;
+            const bool in = at(ig, wt);
+            z2[kk] = in ? make_double2(2.0 * (wt.x - z0) * inv_h, 2.0 * wt.y * inv_h)
+                        : make_double2(0.0, 0.0);
+            if (k0 == 0) {
+                cur[kk] = in ? cmul(wt, __ldg(erow + ig)) : make_double2(0.0, 0.0);
+                const double2 d = cmul(cur[kk], z2[kk]);
+                prev[kk] = make_double2(0.5 * d.x, 0.5 * d.y);
+            } else {
+                prev[kk] = st[((size_t)(i * kTermK + kk) * 2) * 128 + t];
+                cur[kk] = st[((size_t)(i * kTermK + kk) * 2 + 1) * 128 + t];
+            }
+        }
+        const int ks = c * (Kc / kCrtBlockK) + i;
+#pragma unroll 1
+        for (int m = 0; m < gm; ++m) {
+            const int e = e0 + raise(k0 + m);
+            const int y = m * ngp + grp * 8;
+            __nv_bfloat16 *w = out + ((size_t)(y / kCrtRowsY) * ksteps + ks) * (kCrtRowsY * kCrtBlockK) +
+                               (size_t)((y % kCrtRowsY) / 8) * 512 + kg0 * 64 + row * 8 + half * kTermK;
+            float2 dr[kTermK / 2][ND], di[kTermK / 2][ND];
+            auto digits = [&](double x, float(&d)[ND]) {
+                if constexpr (BITS <= 30)
+                    crt_digits_n<ND>(fixed_point32(x, e, BITS), d);
+                else
+                    crt_digits_n<ND>(oz_fixed_point(x, e, BITS), d);
+            };
+#pragma unroll
+            for (int h = 0; h < kTermK / 2; ++h) {
+                float a[ND], b[ND], x[ND], v[ND];
+                digits(cur[2 * h].x, a);
+                digits(cur[2 * h + 1].x, b);
+                digits(cur[2 * h].y, x);
+                digits(cur[2 * h + 1].y, v);
+#pragma unroll
+                for (int k = 0; k < ND; ++k) {
+                    dr[h][k] = f2(a[k], b[k]);
+                    di[h][k] = f2(x[k], v[k]);
+                }
+            }
+            crt_store_residues<kTermK / 2, ND>(dr, di, NMOD, w, plane);
+#pragma unroll
+            for (int kk = 0; kk < kTermK; ++kk) {
+                const double2 n = make_double2(
+                    fma(z2[kk].x, cur[kk].x, fma(-z2[kk].y, cur[kk].y, -prev[kk].x)),
+                    fma(z2[kk].x, cur[kk].y, fma(z2[kk].y, cur[kk].x, -prev[kk].y)));
+                prev[kk] = cur[kk];
+                cur[kk] = n;
+            }
+        }
+        if (!last) {
+#pragma unroll
+            for (int kk = 0; kk < kTermK; ++kk) {
+                st[((size_t)(i * kTermK + kk) * 2) * 128 + t] = prev[kk];
+                st[((size_t)(i * kTermK + kk) * 2 + 1) * 128 + t] = cur[kk];
+            }
+        }
+    }
+}
+
+// S1[n][k0 + m] = sum_r c[n][r] H[n][m ngp + r].
+__global__ void __launch_bounds__(256) far_fold_kernel(const FarPlan *f, const double2 *C,
+                                                       const double2 *H, int ng, int ngp, int ld,
+                                                       int k0, int K, double2 *S1) {
+    if (!f->active) return;
+    __shared__ double red[16], S[2];
+    const int n = blockIdx.x, m = blockIdx.y;
+    double v[2] = {0.0, 0.0};
+    for (int r = threadIdx.x; r < ng; r += 256) {
+        const double2 x = cmul(C[(size_t)n * ng + r], H[(size_t)n * ld + (size_t)m * ngp + r]);
+        v[0] += x.x;
+        v[1] += x.y;
+    }
+    block_reduce<2, 256>(v, red, S);
+    if (threadIdx.x == 0) S1[(size_t)n * K + k0 + m] = make_double2(S[0], S[1]);
+}
+
+// Near pairs in FP64: a block takes a row pair x kNearTile entries, threads
+// striding over the columns as in noflag_fp64_tile; each entry's weighted sums
+// of the two rows go to partial[entry][frequency][row pair].
+__global__ void __launch_bounds__(128) far_near_fp64_kernel(Problem p, FarNear nr) {
+    constexpr int RN = kNearTile, NF = kNearFreq, K = RN * 2 * NF * 2;
+    __shared__ double red[4 * K], S[K];
+    if (!*nr.active) return;
+    const int count = *nr.count, tiles = (count + RN - 1) / RN, pairs = (p.ng + 1) / 2;
+    const int nc = p.nc;
+    constexpr int kRows = 16;  // row pairs in L2 while the entries stream past them
+    for (long long b = blockIdx.x; b < (long long)tiles * pairs; b += gridDim.x) {
+        const long long per = (long long)kRows * tiles;
+        const int g = (int)(b / per), in = (int)(b % per);
+        const int here = min(kRows, pairs - g * kRows);
+        const int rp = g * kRows + in % here, e0 = in / here * RN;
+        const double2 *wr_[2], *er_[2], *nrow[RN];
+        double wx[RN][NF];
+        int len[RN];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const size_t r = min(2 * rp + q, p.ng - 1);
+            wr_[q] = p.wt + r * nc;
+            er_[q] = p.ieps + r * nc;
+        }
+#pragma unroll
+        for (int n = 0; n < RN; ++n) {
+            const int4 e = nr.list[min(e0 + n, count - 1)];
+            nrow[n] = p.aqsn + (size_t)e.x * nc;
+            len[n] = e0 + n < count ? e.z : 0;
+#pragma unroll
+            for (int w = 0; w < NF; ++w)
+                wx[n][w] = __ldg(p.wx + (size_t)e.x * p.wx_stride + min(e.y + w, p.nw - 1));
+        }
+        double2 acc[RN][2][NF];
+#pragma unroll
+        for (int n = 0; n < RN; ++n)
+#pragma unroll
+            for (int w = 0; w < NF; ++w) acc[n][0][w] = acc[n][1][w] = make_double2(0.0, 0.0);
+        for (int ig = threadIdx.x; ig < nc; ig += 128) {
+            double2 Q[2], wt[2];
+            double wti2[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                wt[q] = __ldg(wr_[q] + ig);
+                Q[q] = cmul(wt[q], __ldg(er_[q] + ig));
+                wti2[q] = wt[q].y * wt[q].y;
+            }
+#pragma unroll
+            for (int n = 0; n < RN; ++n) {
+                const double2 a = __ldg(nrow[n] + ig);
+                double2 A[2], Aw[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    A[q] = cmul(a, Q[q]);
+                    Aw[q] = make_double2(A[q].x * wt[q].y, A[q].y * wt[q].y);
+                }
+#pragma unroll
+                for (int w = 0; w < NF; ++w) {
+                    if (w >= len[n]) break;  // the same for the whole block
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const double wr = wx[n][w] - wt[q].x;
+                        const double rr = rcp_fp64(fma(wr, wr, wti2[q]));
+                        acc[n][q][w].x = fma(rr, fma(A[q].x, wr, -Aw[q].y), acc[n][q][w].x);
+                        acc[n][q][w].y = fma(rr, fma(A[q].y, wr, Aw[q].x), acc[n][q][w].y);
+                    }
+                }
+            }
+        }
+        double v[K];
+#pragma unroll
+        for (int n = 0; n < RN; ++n)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int w = 0; w < NF; ++w) {
+                    v[((n * 2 + q) * NF + w) * 2] = acc[n][q][w].x;
+                    v[((n * 2 + q) * NF + w) * 2 + 1] = acc[n][q][w].y;
+                }
+        block_reduce<K, 128>(v, red, S);
+        near_epilogue<RN, NF>(p, nr, S, e0, count, rp);
+        __syncthreads();
+    }
+}
+
+// near_val[entry][frequency] = the sum over row pairs, a warp per sum.
+__global__ void __launch_bounds__(256) far_near_sum_kernel(FarNear nr, int pairs, double2 *val) {
+    if (!*nr.active) return;
+    const int lane = threadIdx.x & 31, count = *nr.count * kNearFreq;
+    for (int e = (blockIdx.x * 256 + threadIdx.x) >> 5; e < count; e += (gridDim.x * 256) >> 5) {
+        double x = 0.0, y = 0.0;
+        for (int r = lane; r < pairs; r += 32) {
+            const double2 v = nr.partial[(size_t)e * pairs + r];
+            x += v.x;
+            y += v.y;
+        }
+        x = warp_sum(x);
+        y = warp_sum(y);
+        if (lane == 0) val[e] = make_double2(x, y);
+    }
+}
+
+// The strays' terms of the far pairs, FP64: blockIdx.x a segment of the list,
+// blockIdx.y 4 bands, blockIdx.z up to 4 frequencies;
+// part[segment][pair] (0 for near pairs).
+constexpr int kOutBands = 4, kOutFreq = 4;
+__global__ void __launch_bounds__(128) far_out_kernel(Problem p, const FarPlan *f, const int2 *list,
+                                                      long long seg_len, int b0, int bands,
+                                                      const double2 *C, double2 *part) {
+    if (!f->active) return;
+    constexpr int K = kOutBands * kOutFreq * 2;
+    __shared__ double red[4 * K], S[K];
+    const long long a = blockIdx.x * seg_len, b = min((long long)f->n_out, a + seg_len);
+    if (a >= b) return;
+    const int n0 = blockIdx.y * kOutBands, w0 = blockIdx.z * kOutFreq;
+    const int nc = p.nc;
+    double wx[kOutBands][kOutFreq];
+    bool any = false;
+    unsigned far = 0;
+#pragma unroll
+    for (int n = 0; n < kOutBands; ++n)
+#pragma unroll
+        for (int w = 0; w < kOutFreq; ++w) {
+            const int band = b0 + min(n0 + n, bands - 1);
+            wx[n][w] = __ldg(p.wx + (size_t)band * p.wx_stride + min(w0 + w, p.nw - 1));
+            if (n0 + n < bands && w0 + w < p.nw && is_far(*f, wx[n][w])) far |= 1u << (n * kOutFreq + w);
+        }
+    any = far != 0;
+    double2 acc[kOutBands][kOutFreq];
+#pragma unroll
+    for (int n = 0; n < kOutBands; ++n)
+#pragma unroll
+        for (int w = 0; w < kOutFreq; ++w) acc[n][w] = make_double2(0.0, 0.0);
+    if (any)
+        for (long long i = a + threadIdx.x; i < b; i += 128) {
+            const int2 e = list[i];
+            const double2 wt = __ldg(p.wt + (size_t)e.x * nc + e.y);
+            const double2 Q = cmul(wt, __ldg(p.ieps + (size_t)e.x * nc + e.y));
+            const double wti2 = wt.y * wt.y;
+#pragma unroll
+            for (int n = 0; n < kOutBands; ++n) {
+                if (!((far >> (n * kOutFreq)) & ((1u << kOutFreq) - 1))) continue;
+                const int k = min(n0 + n, bands - 1);
+                const double2 A = cmul(cmul(__ldg(p.aqsn + (size_t)(b0 + k) * nc + e.y),
+                                            C[(size_t)k * p.ng + e.x]), Q);
+                const double ayw = A.y * wt.y, axw = A.x * wt.y;
+#pragma unroll
+                for (int w = 0; w < kOutFreq; ++w) {
+                    if (!((far >> (n * kOutFreq + w)) & 1)) continue;
+                    const double wr = wx[n][w] - wt.x;
+                    const double rr = rcp_fp64(fma(wr, wr, wti2));
+                    acc[n][w].x = fma(rr, fma(A.x, wr, -ayw), acc[n][w].x);
+                    acc[n][w].y = fma(rr, fma(A.y, wr, axw), acc[n][w].y);
+                }
+            }
+        }
+    double v[K];
+#pragma unroll
+    for (int n = 0; n < kOutBands; ++n)
+#pragma unroll
+        for (int w = 0; w < kOutFreq; ++w) {
+            v[(n * kOutFreq + w) * 2] = acc[n][w].x;
+            v[(n * kOutFreq + w) * 2 + 1] = acc[n][w].y;
+        }
+    block_reduce<K, 128>(v, red, S);
+    const int t = threadIdx.x, n = t / kOutFreq, w = t % kOutFreq;
+    if (t < kOutBands * kOutFreq && n0 + n < bands && w0 + w < p.nw)
+        part[(size_t)blockIdx.x * bands * p.nw + (size_t)(n0 + n) * p.nw + w0 + w] =
+            make_double2(S[t * 2], S[t * 2 + 1]);
+}
+
+// The series of a far pair from its band's sums S1.
+__device__ __forceinline__ double2 far_series(const FarPlan &f, double wx, const double2 *S1, int K) {
+    const double u = (wx - f.z0) * f.inv_h;
+    const double s = copysign(sqrt((u - 1.0) * (u + 1.0)), u);
+    const double q = 1.0 / (u + s);
+    double2 acc = make_double2(0.0, 0.0);
+    for (int k = K - 1; k >= 1; --k)  // Horner in 1 / r, smallest terms first
+        acc = make_double2(fma(acc.x, q, S1[k].x), fma(acc.y, q, S1[k].y));
+    const double g = f.inv_h / s;
+    return make_double2(g * fma(2.0 * q, acc.x, S1[0].x), g * fma(2.0 * q, acc.y, S1[0].y));
+}
+
+// Block iw < nw: that frequency's total over bands, near entries and strays;
+// block nw + n: band n's total at iw = 2.  Written into the first unoccupied
+// slot of the frequency, or the band's first row slot.
+__global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan *f, int b0, int bands,
+                                                        const int4 *near, const double2 *near_val,
+                                                        const double2 *out_part, long long seg_len,
+                                                        const double2 *S1, int K, Partials part) {
+    if (!f->active) return;
+    __shared__ double red[16], S[2];
+    const bool band = (int)blockIdx.x >= p.nw;
+    const int iw = band ? 2 : blockIdx.x;
+    const int n0 = band ? blockIdx.x - p.nw : 0, n1 = band ? n0 + 1 : bands;
+    const int segs = (int)((f->n_out + seg_len - 1) / seg_len);
+    double v[2] = {0.0, 0.0};
+    for (int n = n0 + (band ? 0 : (int)threadIdx.x); n < n1; n += 256) {
+        const double wx = p.wx[(size_t)(b0 + n) * p.wx_stride + iw];
+        if (!is_far(*f, wx)) continue;
+        if (!band || threadIdx.x == 0) {
+            const double2 x = far_series(*f, wx, S1 + (size_t)n * K, K);
+            v[0] += x.x;
+            v[1] += x.y;
+        }
+        for (int sg = band ? threadIdx.x : 0; sg < segs; sg += band ? 256 : 1) {
+            const double2 x = out_part[(size_t)sg * bands * p.nw + (size_t)n * p.nw + iw];
+            v[0] += x.x;
+            v[1] += x.y;
+        }
+    }
+    for (int e = threadIdx.x; e < f->n_near; e += 256) {
+        const int4 q = near[e];
+        const int w = iw - q.y;
+        if (w < 0 || w >= q.z || (band && q.x != b0 + n0)) continue;
+        v[0] += near_val[(size_t)e * kNearFreq + w].x;
+        v[1] += near_val[(size_t)e * kNearFreq + w].y;
+    }
+    block_reduce<2, 256>(v, red, S);
+    if (threadIdx.x == 0) {
+        if (band)
+            part.n1[(long long)(b0 + n0) * part.n1_seg] = make_double2(S[0], S[1]);
+        else
+            part.ach[(long long)iw * part.ach_seg + part.ach_tile0] = make_double2(S[0], S[1]);
+    }
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 132;
+}
+
+}  // namespace
+
+bool far_eligible(const Problem &p, int bands, bool mixed) {
+    if (p.wx_stride == 0 || bands < 32 || p.ng < 16 || p.nc < 512) return false;
+    const Sizes z = sizes(p, bands, mixed);
+    // The series and, say, a sixth of the pairs near must leave a gain, on a
+    // call long enough (3 ms of per-term work) for the fixed launches.
+    const double cells = (double)p.ng * p.nc;
+    const double per_pair = mixed ? 2.6e-12 : 20e-12;
+    return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > 3e-3 &&
+           z.pairs < (1 << 20) && cells < 2e9;
+}
+
+size_t far_bytes(const Problem &p, int bands, bool mixed) {
+    return carve(sizes(p, bands, mixed), nullptr, nullptr);
+}
+
+cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, void *split_ws, int b0,
+                           int b1, cudaStream_t s, const int **active) {
+    const int bands = b1 - b0;
+    const bool mixed = split_ws != nullptr;
+    const Sizes z = sizes(p, bands, mixed);
+    Buffers b;
+    carve(z, ws, &b);
+    const int *go = &b.plan->active;
+    *active = go;
+    const int sms = sm_count();
+    far_range_kernel<<<1, 1024, 0, s>>>(p, b0, bands, b.plan);
+    far_hist_kernel<<<sms * 4, 256, 0, s>>>(p, b.plan);
+    far_plan_kernel<<<1, kBins, 0, s>>>(p, b0, bands, b.plan, b.near, z.cap_near, z.cap_out, (float)z.R,
+                                        (float)z.c0, 1.4f, mixed ? 16.f : 2.f);
+    far_count_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows);
+    far_scan_kernel<<<1, 1024, 0, s>>>(p.ng, b.plan, b.rows);
+    far_list_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows, b.out);
+    far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
+    count_launch(7);
+    cudaError_t e = cudaGetLastError();
+
+    // The series, a pass per group of terms of one level and slab of chunks.
+    const OzOperand X{p.aqsn + (size_t)b0 * p.nc, p.nc, true, bands};
+    const size_t x_slab = (size_t)3 * kCrtN * z.Mp * z.slab * z.Kc;  // elements, at level 0
+    int level = -1;
+    for (int k0 = 0; k0 < z.K && e == cudaSuccess;) {
+        const int l = level_of(z, k0);
+        int gm = 1;
+        while (gm < z.gm && k0 + gm < z.K && level_of(z, k0 + gm) == l) ++gm;
+        const int rows = gm * z.ngp, Np = ceil_div(rows, kCrtRowsY) * kCrtRowsY;
+        for (int c0 = 0, q = 0; c0 < z.nch && e == cudaSuccess; c0 += z.slab, ++q) {
+            const int nc = std::min(z.slab, z.nch - c0);
+            __nv_bfloat16 *sx = b.sx + (size_t)q * x_slab;
+            int *ex = b.EX + (size_t)c0 * z.Mp;
+            if (l != level) e = crt_rows(X, z.Mp, p.nc, z.Kc, c0, nc, l, sx, ex, go, s);
+            if (e != cudaSuccess) break;
+            auto terms = [&](auto kern) {
+                kern<<<z.ngp / 8 * nc, 128, 0, s>>>(p, b.plan, z.ngp, c0, nc, z.Kc, Np, k0, gm,
+                                                    k0 + gm >= z.K, b.sy, b.EY, b.E0, b.state);
+            };
+            switch (l) {
+                case 0: terms(far_terms_kernel<0>); break;
+                case 1: terms(far_terms_kernel<1>); break;
+                case 2: terms(far_terms_kernel<2>); break;
+                default: terms(far_terms_kernel<3>); break;
+            }
+            count_launch();
+            e = crt_products(sx, b.sy, z.Mp, Np, z.Kc, nc, 0, z.Mp / kCrtRowsX, l, b.res, z.Mp, go,
+                             part.err, s);
+            if (e == cudaSuccess)
+                e = crt_combine(b.res, ex, b.EY, 0, bands, z.Mp, rows, z.Mp, Np, nc, l, c0 > 0, b.H,
+                                rows, go, s);
+        }
+        level = l;
+        if (e != cudaSuccess) break;
+        far_fold_kernel<<<dim3(bands, gm), 256, 0, s>>>(b.plan, b.C, b.H, p.ng, z.ngp, rows, k0, z.K,
+                                                        b.S1);
+        count_launch();
+        k0 += gm;
+    }
+    if (e != cudaSuccess) return e;
+
+    const FarNear nr{b.near, &b.plan->n_near, go, b.C, b0, b.near_part};
+    if (mixed) {
+        e = launch_near_mixed(p, part, split_ws, nr, z.cap_near, s);
+        if (e != cudaSuccess) return e;
+    } else {
+        far_near_fp64_kernel<<<sms * 4, 128, 0, s>>>(p, nr);
+        count_launch();
+    }
+    far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, (p.ng + 1) / 2, b.near_val);
+    far_out_kernel<<<dim3(z.segs, ceil_div(bands, kOutBands), ceil_div(p.nw, kOutFreq)), 128, 0, s>>>(
+        p, b.plan, b.out, z.seg_len, b0, bands, b.C, b.out_part);
+    far_final_kernel<<<p.nw + (part.n1 ? bands : 0), 256, 0, s>>>(p, b.plan, b0, bands, b.near,
+                                                                  b.near_val, b.out_part, z.seg_len,
+                                                                  b.S1, z.K, part);
+    count_launch(3);
+    return cudaGetLastError();
+}
+
+}  // namespace gpp

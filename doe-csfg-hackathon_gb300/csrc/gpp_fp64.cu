@@ -27,7 +27,8 @@ constexpr int kFp64Group = 16;
 template <int RN, int RG, int NWC, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 noflag_fp64_kernel(Problem p, Partials part, int band_begin, int band_end, int row_tile0,
-                   int rows_here, int row_tiles, int band_tiles) {
+                   int rows_here, int row_tiles, int band_tiles, const int *skip) {
+    if (skip && *skip) return;  // the series of gpp_far.cu covers the call
     constexpr int K = RN * RG * NWC * 2;
     __shared__ double red[(THREADS / 32) * K];
     __shared__ double S[K];
@@ -136,14 +137,14 @@ reduce_kernel(const double2 *src, long long stride, int len, ReduceOut out) {
 
 template <int RN, int RG, int NWC, int THREADS>
 cudaError_t launch_noflag_t(const Problem &p, const Partials &part, int b0, int b1, RowTiles rt,
-                            cudaStream_t s) {
+                            cudaStream_t s, const int *skip) {
     const int row_tiles = ceil_div(p.ng, RG);
     const RowTiles r = rt.clip(row_tiles);
     if (r.end <= r.begin) return cudaSuccess;
     const int band_tiles = ceil_div(b1 - b0, RN);
     dim3 grid((unsigned)((long long)(r.end - r.begin) * band_tiles), ceil_div(p.nw, NWC));
     noflag_fp64_kernel<RN, RG, NWC, THREADS><<<grid, THREADS, 0, s>>>(
-        p, part, b0, b1, r.begin, r.end - r.begin, row_tiles, band_tiles);
+        p, part, b0, b1, r.begin, r.end - r.begin, row_tiles, band_tiles, skip);
     count_launch();
     return cudaGetLastError();
 }
@@ -219,14 +220,14 @@ TileShape fp64_noflag_shape(const Problem &p) {
 TileShape flag_shape(const Problem &p) { return TileShape{1, 2, flag_nwc(p.nw), 128}; }
 
 cudaError_t launch_noflag_fp64(const Problem &p, const Partials &part, int b0, int b1,
-                               cudaStream_t s, RowTiles rt) {
+                               cudaStream_t s, RowTiles rt, const int *skip) {
     if (b1 <= b0 || p.ng == 0) return cudaSuccess;
     switch (nwc_for(p.nw)) {
-        case 1: return launch_noflag_t<4, 2, 1, 128>(p, part, b0, b1, rt, s);
-        case 2: return launch_noflag_t<4, 2, 2, 128>(p, part, b0, b1, rt, s);
-        case 3: return launch_noflag_t<4, 2, 3, 128>(p, part, b0, b1, rt, s);
-        case 4: return launch_noflag_t<4, 2, 4, 128>(p, part, b0, b1, rt, s);
-        default: return launch_noflag_t<2, 2, 8, 128>(p, part, b0, b1, rt, s);
+        case 1: return launch_noflag_t<4, 2, 1, 128>(p, part, b0, b1, rt, s, skip);
+        case 2: return launch_noflag_t<4, 2, 2, 128>(p, part, b0, b1, rt, s, skip);
+        case 3: return launch_noflag_t<4, 2, 3, 128>(p, part, b0, b1, rt, s, skip);
+        case 4: return launch_noflag_t<4, 2, 4, 128>(p, part, b0, b1, rt, s, skip);
+        default: return launch_noflag_t<2, 2, 8, 128>(p, part, b0, b1, rt, s, skip);
     }
 }
 

@@ -63,6 +63,20 @@ struct Partials {
     int *err;        // device fault word
 };
 
+// A list of entries -- a band and up to kNearFreq consecutive frequencies -- to
+// sum term by term over every column (the near pairs of gpp_far.cu): each
+// entry's weighted sums over a row pair go to partial[entry][frequency][row
+// pair].
+constexpr int kNearFreq = 3;
+struct FarNear {
+    const int4 *list;      // (band, first frequency, frequencies, 0)
+    const int *count;      // entries, on the device
+    const int *active;     // 0: nothing to do
+    const double2 *coeff;  // [bands][ng]: 0.5 vcoul conj(aqsm) at the row's G'
+    int b0;                // the band of coeff's first row
+    double2 *partial;
+};
+
 // Resolve the G' column index of local row my_igp exactly like the reference
 // (gppComplex_seq.cpp:342-344: values >= ncouls clamp to ncouls-1), then the
 // optional indinv remap.  Returns -1 (and raises a fault bit) for indices the
@@ -188,6 +202,21 @@ __device__ __forceinline__ void noflag_epilogue(const Problem &p, const Partials
         part.ach[(long long)(iw0 + w) * part.ach_seg + tile] = tot;
     else if (band0 + nlo < band_end)
         part.n1[(long long)(band0 + nlo) * part.n1_seg + row_tile] = tot;
+}
+
+// Epilogue of a near tile: S holds the ig sums of entry n (of the tile's NE
+// from e0), row q and frequency w as S[((n*2 + q)*NF + w)*2 + {0,1}]; a thread
+// per (entry, frequency) weights the two rows of pair rp and adds them.
+template <int NE, int NF>
+__device__ __forceinline__ void near_epilogue(const Problem &p, const FarNear &nr, const double *S,
+                                              int e0, int count, int rp) {
+    const int n = threadIdx.x / NF, w = threadIdx.x % NF, e = e0 + n;
+    if (n >= NE || e >= count) return;
+    const double2 *c = nr.coeff + (size_t)(nr.list[e].x - nr.b0) * p.ng;
+    const double *s = S + (n * 2 * NF + w) * 2;
+    double2 tot = cmul(c[2 * rp], make_double2(s[0], s[1]));
+    if (2 * rp + 1 < p.ng) tot = cadd(tot, cmul(c[2 * rp + 1], make_double2(s[NF * 2], s[NF * 2 + 1])));
+    nr.partial[((size_t)e * kNearFreq + w) * ((p.ng + 1) / 2) + rp] = tot;
 }
 
 }  // namespace gpp

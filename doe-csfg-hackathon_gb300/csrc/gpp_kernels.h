@@ -44,9 +44,11 @@ __host__ __device__ constexpr int flag_nwc(int nw) {
 }
 
 // Unoccupied bands [band_begin, band_end), FP64.  Writes one ach partial per
-// (row tile, band tile) block and, when part.n1 is set, per-band partials.
+// (row tile, band tile) block and, when part.n1 is set, per-band partials;
+// nothing where the device word `skip`, if given, is not 0.
 cudaError_t launch_noflag_fp64(const Problem &p, const Partials &part, int band_begin,
-                               int band_end, cudaStream_t s, RowTiles rows = RowTiles());
+                               int band_end, cudaStream_t s, RowTiles rows = RowTiles(),
+                               const int *skip = nullptr);
 // Occupied bands [0, nvband): full ssxt_scht_solver branch logic in FP64.
 // blocks_per_sm > 0 with a device counter `next` (band-independent
 // frequencies only): a persistent grid of that many blocks per SM taking row
@@ -89,7 +91,7 @@ bool mixed_variant_valid(int variant, int nw);
 // occupied one.
 cudaError_t launch_mixed_noflag(const Problem &p, const Partials &part, void *split_ws,
                                 int band_begin, int band_end, cudaStream_t s, int variant,
-                                RowTiles rows = RowTiles());
+                                RowTiles rows = RowTiles(), const int *skip = nullptr);
 // blocks_per_sm and next as for launch_flag_fp64.
 cudaError_t launch_flag_mixed(const Problem &p, const Partials &part, void *split_ws,
                               cudaStream_t s, RowTiles rows = RowTiles(), int blocks_per_sm = 0,

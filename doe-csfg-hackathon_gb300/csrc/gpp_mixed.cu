@@ -28,6 +28,7 @@
 // resident in L2 while all band tiles stream past them.
 #include <algorithm>
 
+#include "gpp_far.h"
 #include "gpp_kernels.h"
 #include "gpp_tiles_mixed.cuh"
 
@@ -111,7 +112,8 @@ __global__ void __launch_bounds__(256) split_bands_kernel(Problem p, SplitPlanes
 template <int RNW, int RG, int NWC, int NWARP, int KC, int NSTAGE, int SYNC, int GROUP, int MINB>
 __global__ void __launch_bounds__(NWARP * 32, MINB)
 mixed_noflag_kernel(Problem p, Partials part, SplitPlanes s, int band_begin, int band_end,
-                    int row_tile0, int rows_here, int row_tiles, int band_tiles) {
+                    int row_tile0, int rows_here, int row_tiles, int band_tiles, const int *skip) {
+    if (skip && *skip) return;  // the series of gpp_far.cu covers the call
     // Grouped tile order over this launch's row tiles [row_tile0, +rows_here):
     // GROUP consecutive row tiles share each band tile, so a group's row
     // planes stay in L2 while the band tiles stream past.
@@ -128,6 +130,7 @@ mixed_noflag_kernel(Problem p, Partials part, SplitPlanes s, int band_begin, int
 
 constexpr int kGroup = 16;
 constexpr int kWarps = 4;
+constexpr int kNearCols = 192;  // columns per pipeline chunk of the near kernel
 
 // Compiled variants of the mixed kernel (the autotuner picks one): the tile
 // shape -- `warps` warps per block, each owning `rnw` bands of the block's
@@ -170,7 +173,7 @@ bool variant_compiled(int v, int nwc) {
 
 template <int RNW, int RG, int NWC, int KC, int NSTAGE, int SYNC, int MINB = 0, int NWARP = kWarps>
 cudaError_t launch_mixed_t(const Problem &p, const Partials &part, const SplitPlanes &s, int b0,
-                           int b1, RowTiles rt, cudaStream_t st) {
+                           int b1, RowTiles rt, cudaStream_t st, const int *skip) {
     constexpr int BN = NWARP * RNW;
     const int row_tiles = ceil_div(p.ng, RG), band_tiles = ceil_div(b1 - b0, BN);
     const RowTiles r = rt.clip(row_tiles);
@@ -187,7 +190,7 @@ cudaError_t launch_mixed_t(const Problem &p, const Partials &part, const SplitPl
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)(r.end - r.begin) * band_tiles, ceil_div(p.nw, NWC));
     kern<<<grid, NWARP * 32, smem, st>>>(p, part, s, b0, b1, r.begin, r.end - r.begin, row_tiles,
-                                         band_tiles);
+                                         band_tiles, skip);
     count_launch();
     return cudaGetLastError();
 }
@@ -195,27 +198,27 @@ cudaError_t launch_mixed_t(const Problem &p, const Partials &part, const SplitPl
 template <int RG, int NWC>
 cudaError_t launch_mixed_variant(int v, const Problem &p, const Partials &part,
                                  const SplitPlanes &s, int b0, int b1, RowTiles rt,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, const int *skip) {
     switch (v) {
-        case 0: return launch_mixed_t<1, RG, NWC, 128, 2, kSyncBlock>(p, part, s, b0, b1, rt, st);
-        case 2: return launch_mixed_t<1, RG, NWC, 128, 2, kSyncRing>(p, part, s, b0, b1, rt, st);
-        case 3: return launch_mixed_t<1, RG, NWC, 64, 4, kSyncRing>(p, part, s, b0, b1, rt, st);
+        case 0: return launch_mixed_t<1, RG, NWC, 128, 2, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
+        case 2: return launch_mixed_t<1, RG, NWC, 128, 2, kSyncRing>(p, part, s, b0, b1, rt, st, skip);
+        case 3: return launch_mixed_t<1, RG, NWC, 64, 4, kSyncRing>(p, part, s, b0, b1, rt, st, skip);
         case 4:
-            return launch_mixed_t<1, RG, NWC, 128, 2, kSyncBlock, 5>(p, part, s, b0, b1, rt, st);
-        case 5: return launch_mixed_t<1, RG, NWC, 128, 3, kSyncRing>(p, part, s, b0, b1, rt, st);
-        case 6: return launch_mixed_t<1, RG, NWC, 192, 2, kSyncBlock>(p, part, s, b0, b1, rt, st);
-        case 7: return launch_mixed_t<1, RG, NWC, 256, 2, kSyncBlock>(p, part, s, b0, b1, rt, st);
+            return launch_mixed_t<1, RG, NWC, 128, 2, kSyncBlock, 5>(p, part, s, b0, b1, rt, st, skip);
+        case 5: return launch_mixed_t<1, RG, NWC, 128, 3, kSyncRing>(p, part, s, b0, b1, rt, st, skip);
+        case 6: return launch_mixed_t<1, RG, NWC, 192, 2, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
+        case 7: return launch_mixed_t<1, RG, NWC, 256, 2, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
         case 8:
-            return launch_mixed_t<1, RG, NWC, 192, 2, kSyncBlock, 0, 8>(p, part, s, b0, b1, rt, st);
+            return launch_mixed_t<1, RG, NWC, 192, 2, kSyncBlock, 0, 8>(p, part, s, b0, b1, rt, st, skip);
         case 9:
-            return launch_mixed_t<1, RG, NWC, 256, 2, kSyncBlock, 0, 8>(p, part, s, b0, b1, rt, st);
+            return launch_mixed_t<1, RG, NWC, 256, 2, kSyncBlock, 0, 8>(p, part, s, b0, b1, rt, st, skip);
         case 10:
             if constexpr (NWC <= 4)
-                return launch_mixed_t<2, RG, NWC, 192, 2, kSyncBlock, 3>(p, part, s, b0, b1, rt, st);
+                return launch_mixed_t<2, RG, NWC, 192, 2, kSyncBlock, 3>(p, part, s, b0, b1, rt, st, skip);
             else
                 return cudaErrorInvalidValue;
         default:
-            return launch_mixed_t<1, RG, NWC, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st);
+            return launch_mixed_t<1, RG, NWC, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
     }
 }
 
@@ -357,6 +360,42 @@ cudaError_t launch_flag_mixed_t(const Problem &p, const Partials &part, const Sp
     return cudaGetLastError();
 }
 
+// The near pairs of gpp_far.cu, a list entry per warp: persistent blocks of 4 warps
+// over (row pair, 4 entries) tiles, in groups of kGroup row pairs that stay in
+// L2 while the entries stream past them.
+__global__ void __launch_bounds__(kWarps * 32, 4)
+near_mixed_kernel(Problem p, Partials part, SplitPlanes s, FarNear near) {
+    if (!*near.active) return;
+    const int count = *near.count, tiles = (count + kWarps - 1) / kWarps, pairs = (p.ng + 1) / 2;
+    const long long per = (long long)kGroup * tiles;
+    bool reinit = false;
+    for (long long b = blockIdx.x; b < (long long)tiles * pairs; b += gridDim.x) {
+        const int g = (int)(b / per), in = (int)(b % per);
+        const int here = min(kGroup, pairs - g * kGroup);
+        if (!mixed_tile<1, 2, kNearFreq, kWarps, kNearCols, 2, kSyncBlock, true>(
+                p, part, s, 0, count, g * kGroup + in % here, in / here, 0, 0, reinit, &near))
+            return;  // abandoned after a bounded wait; the fault bit is set
+        reinit = true;
+        __syncthreads();
+    }
+}
+
+cudaError_t launch_near_mixed(const Problem &p, const Partials &part, void *split_ws,
+                              const FarNear &near, int cap, cudaStream_t st) {
+    const int smem = (int)sizeof(float4) * 2 * (4 + kWarps) * kNearCols;
+    cudaError_t e = cudaFuncSetAttribute(near_mixed_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long most = (long long)ceil_div(cap, kWarps) * ((p.ng + 1) / 2);
+    const int grid = (int)std::min<long long>(most, (long long)std::max(sms, 1) * 4);
+    near_mixed_kernel<<<grid, kWarps * 32, smem, st>>>(p, part, planes(p, split_ws), near);
+    count_launch();
+    return cudaGetLastError();
+}
+
 // Self-test of the bounded pipeline wait: one block waits on an mbarrier
 // that nothing arrives at, gives up after `polls` polls and records
 // kErrPipelineTimeout exactly as a tile does, then returns.
@@ -396,15 +435,16 @@ cudaError_t launch_flag_mixed(const Problem &p, const Partials &part, void *spli
 }
 
 cudaError_t launch_mixed_noflag(const Problem &p, const Partials &part, void *split_ws, int b0,
-                                int b1, cudaStream_t st, int variant, RowTiles rt) {
+                                int b1, cudaStream_t st, int variant, RowTiles rt,
+                                const int *skip) {
     if (b1 <= b0 || p.ng == 0) return cudaSuccess;
     const SplitPlanes s = planes(p, split_ws);
     switch (nwc_for(p.nw)) {
-        case 1: return launch_mixed_t<1, 2, 1, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st);
-        case 2: return launch_mixed_t<1, 2, 2, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st);
-        case 3: return launch_mixed_variant<2, 3>(variant, p, part, s, b0, b1, rt, st);
-        case 4: return launch_mixed_t<1, 2, 4, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st);
-        default: return launch_mixed_variant<2, 8>(variant, p, part, s, b0, b1, rt, st);
+        case 1: return launch_mixed_t<1, 2, 1, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
+        case 2: return launch_mixed_t<1, 2, 2, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
+        case 3: return launch_mixed_variant<2, 3>(variant, p, part, s, b0, b1, rt, st, skip);
+        case 4: return launch_mixed_t<1, 2, 4, 128, 3, kSyncBlock>(p, part, s, b0, b1, rt, st, skip);
+        default: return launch_mixed_variant<2, 8>(variant, p, part, s, b0, b1, rt, st, skip);
     }
 }
 

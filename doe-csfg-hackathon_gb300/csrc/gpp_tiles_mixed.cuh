@@ -166,13 +166,14 @@ static __device__ __noinline__ TermPair pole_pair(const Problem &p, df2 d, float
 // each step).  With CHECK, terms within 1e-3 |wx| of the pole are
 // recomputed in FP64 from the inputs; tiles call the CHECK = false form only
 // when no wtilde can come that near any of the warp's wx values.
-template <int RNW, int NWC, int KC, bool CHECK>
+// SOME: only the first `count` frequencies (the same for the whole warp).
+template <int RNW, int NWC, int KC, bool CHECK, bool SOME = false>
 __device__ __forceinline__ void mixed_column(const Problem &p, const float4 *st,
                                              const float4 *sb, int il, int ig, int row0,
                                              int bandw, int band_end, int iw0,
                                              const df (&wx)[RNW][NWC],
                                              const float (&pole_thr)[RNW][NWC],
-                                             df2 (&acc)[RNW][NWC][2]) {
+                                             df2 (&acc)[RNW][NWC][2], int count = NWC) {
     const float4 vr = st[il], vi = st[KC + il], vqr = st[2 * KC + il], vqi = st[3 * KC + il];
     const df2 wtr = {f2(vr.x, vr.y), f2(vr.z, vr.w)};
     const df2 wti = {f2(vi.x, vi.y), f2(vi.z, vi.w)};
@@ -190,6 +191,7 @@ __device__ __forceinline__ void mixed_column(const Problem &p, const float4 *st,
         const df2 Ar_wti = df2_mul(Ar, wti);
 #pragma unroll
         for (int w = 0; w < NWC; ++w) {
+            if (SOME && w >= count) break;
             const df2 wr = df2_norm(df2_sub(df2_bcast(wx[n][w]), wtr));  // Re(wdiff)
             const df2 d = df2_add(df2_sqr(wr), wti2);                     // |wdiff|^2
             float2 r0, rc;                              // 1/d = r0 (1 + rc)
@@ -236,11 +238,15 @@ enum : int { kSyncBlock = 0, kSyncRing = 1 };
 // launch's segment of block partials.  `reinit` must be set when the block
 // ran an earlier tile with the same barriers (persistent kernels).  Returns
 // false if the tile was abandoned after a bounded wait ran out.
-template <int RNW, int RG, int NWC, int NWARP, int KC, int NSTAGE, int SYNC>
+// LIST: the tile's bands are entries of `near` instead, one per warp (RNW = 1,
+// NWC = kNearFreq; band_begin = 0, band_end = the entry count).
+template <int RNW, int RG, int NWC, int NWARP, int KC, int NSTAGE, int SYNC, bool LIST = false>
 __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &part,
                                            const SplitPlanes &s, int band_begin, int band_end,
                                            int row_tile, int band_tile, int iw_chunk,
-                                           long long tile, bool reinit) {
+                                           long long tile, bool reinit,
+                                           const FarNear *near = nullptr) {
+    static_assert(!LIST || (RNW == 1 && NWC == kNearFreq), "a warp takes one list entry");
     constexpr int BN = NWARP * RNW;            // bands per block
     constexpr int K = BN * RG * NWC * 2;       // doubles in the block result
     constexpr int STAGE = (2 * RG + BN) * KC;  // float4 per stage
@@ -264,6 +270,19 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
     const int bandw = band0 + warp * RNW;
     const int nchunks = (nc + KC - 1) / KC;
     volatile int *abort = &abort_flag;
+    // The n-th band of the block, clamped to the last (or its list entry's).
+    auto band_at = [&](int n) {
+        const int b = min(band0 + n, band_end - 1);
+        if constexpr (LIST) return near->list[b].x;
+        return b;
+    };
+    // The warp's first frequency and how many it sums.
+    int iw_first = iw0, iw_count = NWC;
+    if constexpr (LIST) {
+        const int4 e = near->list[min(bandw, band_end - 1)];
+        iw_first = e.y;
+        iw_count = bandw < band_end ? e.z : 0;
+    }
 
     // Producer: copy chunk c into stage c % NSTAGE.
     auto issue = [&](int c) {
@@ -279,7 +298,7 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
         for (int k = 0; k < 4; ++k) bulk_copy_g2s(st + k * KC, s.rows + r + (size_t)k * nc, bytes, bar);
 #pragma unroll
         for (int n = 0; n < BN; ++n) {
-            const size_t b = (size_t)min(band0 + n, band_end - 1) * nc + k0;
+            const size_t b = (size_t)band_at(n) * nc + k0;
             bulk_copy_g2s(st + (2 * RG + n) * KC, s.band + b, bytes, bar);
         }
     };
@@ -309,15 +328,18 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
         s.masks + (size_t)row_tile * ((nc + kMaskCols - 1) / kMaskCols);
 #pragma unroll
     for (int n = 0; n < RNW; ++n) {
-        const int b = min(bandw + n, band_end - 1);
+        const int b = band_at(warp * RNW + n);
 #pragma unroll
         for (int w = 0; w < NWC; ++w) {
-            const float2 x = s.wx[(size_t)b * p.nw + min(iw0 + w, p.nw - 1)];
+            const float2 x = s.wx[(size_t)b * p.nw + min(iw_first + w, p.nw - 1)];
             wx[n][w] = {x.x, x.y};
             pole_thr[n][w] = 1e-6f * x.x * x.x;  // |wdiff|^2 < (1e-3 |wx|)^2
             pole_mask |= pole_buckets(x.x);
         }
     }
+    // What the columns' pole terms read: the warp's first band and frequency.
+    const int pole_band = LIST ? band_at(warp) : bandw;
+    const int pole_end = LIST ? pole_band + 1 : band_end;
     df2 acc[RNW][NWC][2];  // lanes: the two rows
 #pragma unroll
     for (int n = 0; n < RNW; ++n)
@@ -358,13 +380,15 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
             if (chunk_mask & pole_mask) {
 #pragma unroll kColUnroll
                 for (int il = lane; il < cnt; il += 32)
-                    mixed_column<RNW, NWC, KC, true>(p, st, sb, il, k0 + il, row0, bandw,
-                                                     band_end, iw0, wx, pole_thr, acc);
+                    mixed_column<RNW, NWC, KC, true, LIST>(p, st, sb, il, k0 + il, row0,
+                                                           pole_band, pole_end, iw_first, wx,
+                                                           pole_thr, acc, iw_count);
             } else {
 #pragma unroll kColUnroll
                 for (int il = lane; il < cnt; il += 32)
-                    mixed_column<RNW, NWC, KC, false>(p, st, sb, il, k0 + il, row0, bandw,
-                                                      band_end, iw0, wx, pole_thr, acc);
+                    mixed_column<RNW, NWC, KC, false, LIST>(p, st, sb, il, k0 + il, row0,
+                                                            pole_band, pole_end, iw_first, wx,
+                                                            pole_thr, acc, iw_count);
             }
         }
         if (SYNC == kSyncBlock) {
@@ -419,7 +443,11 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
                         S[(((warp * RNW + n) * RG + g) * NWC + w) * 2 + ri] = to_double(v);
                 }
     __syncthreads();
-    noflag_epilogue<BN, RG, NWC>(p, part, S, row0, band0, band_end, iw0, tile, row_tile);
+    if constexpr (LIST) {
+        near_epilogue<BN, NWC>(p, *near, S, band0, band_end, row_tile);
+    } else {
+        noflag_epilogue<BN, RG, NWC>(p, part, S, row0, band0, band_end, iw0, tile, row_tile);
+    }
     return true;
 }
 

@@ -185,7 +185,14 @@ typedef struct gpp_outputs {
 
 /* Device pointers in and out, asynchronous on `stream`.  Scratch memory comes
  * from a per-device workspace that the library grows on demand (the first
- * call at a larger size allocates; later calls do not). */
+ * call at a larger size allocates; later calls do not).
+ *
+ * Large calls with per-band frequencies (wx_stride > 0; the rule is on the
+ * sizes and the precision) sum the unoccupied (band, frequency) pairs whose
+ * wx lies away from wtilde through a series on the tensor cores, to the same
+ * precision, and the others term by term; where wtilde is spread so widely
+ * that this does not pay, all of them term by term.  A state gives the same
+ * bits through gpp_sigma, gpp_sigma_host and a batch. */
 gpp_status gpp_sigma(const gpp_problem *problem, const gpp_outputs *out, gpp_stream_t stream);
 
 /* Waits for `stream` (at most timeout_ms; < 0 waits forever) and reports
@@ -228,12 +235,12 @@ gpp_status gpp_context_last_trace(gpp_context *ctx, float *ms, int capacity, int
  * cudaMalloc's device-wide synchronisation mid-step.  It always runs the
  * per-term FP64 kernels and keeps their block partials in a fixed 8 MiB array
  * in the library's device image (resident on every GPU that loads the
- * library), so it allocates nothing.  With per-band wx (wx_stride > 0), or
- * fewer than 32 unoccupied bands, those are gpp_sigma's own kernels and the
- * results are bit-identical; with band-independent wx and 32 or more
- * unoccupied bands gpp_sigma sums the bands as a GEMM instead, and the two
- * agree to FP64 rounding (1e-12 relative), not bit for bit, the per-term
- * kernels being the slower of the two there.  The argument checks and grid
+ * library), so it allocates nothing.  Where gpp_sigma sums term by term too
+ * (small calls, or fewer than 32 unoccupied bands), those are its own kernels
+ * and the results are bit-identical; where it sums the bands as a GEMM (32 or
+ * more unoccupied bands, band-independent wx) or through the series (large
+ * calls, per-band wx) the two agree to FP64 rounding (1e-12 relative), not
+ * bit for bit, the per-term kernels being the slower of the two there.  The argument checks and grid
  * limits are gpp_sigma's.  FP64 only; achtemp and asxtemp only (acht_n1_loc
  * and achstemp must be NULL); problems needing more than 8 MiB of partials
  * (the production shape needs ~5 MiB) return GPP_ERR_UNSUPPORTED.  All calls
@@ -245,7 +252,9 @@ gpp_status gpp_sigma_static_scratch(const gpp_problem *problem, const gpp_output
 
 /* ------------------------------------------------------------------------
  * Batched states: many independent quasiparticle states (uneven sizes) in
- * one persistent launch over a work queue of (state, band tile, row tile).
+ * one persistent launch over a work queue of (state, band tile, row tile);
+ * states large enough for gpp_sigma's series run as calls of their own after
+ * it, on the same stream.
  * ------------------------------------------------------------------------ */
 /* One-shot: plans, runs and frees a batch on `stream`; returns when the
  * results are written.  All problems must share precision, nw and

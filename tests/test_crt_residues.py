@@ -1,7 +1,7 @@
 """The residue arithmetic of the tensor-core FP64 GEMM (gpp_crt.cuh), compiled
 for the host from the header the kernels use: the moduli are pairwise coprime
-and their product holds a 3M-form real or imaginary part over 512 products of
-53-bit integers; the float digits and residues of random and extreme integers
+and the products of each level's first moduli hold a 3M-form real or imaginary
+part over 512 products of the level's integers; the float digits and residues of random and extreme integers
 are exact and symmetric; the product sums' residues stay within the 2^23 that
 the drain's reduction takes; and the value rebuilt from the residues of
 re = P1 - P2 and im = P3 - P1 - P2 equals the exact 128-bit integer to its
@@ -34,16 +34,18 @@ static unsigned long long nx() {
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     return z ^ (z >> 31);
 }
-static long long draw(int kind) {
-    const long long top = 1ll << kCrtBits;
+static long long draw(int kind, int bits) {
+    const long long top = 1ll << bits;
     switch (kind) {
         case 0: return (long long)(nx() % (2 * (unsigned long long)top + 1)) - top;
         case 1: return nx() & 1 ? top : -top;
-        case 2: return (long long)(nx() % 2001) - 1000;
+        case 2: return ((long long)(nx() % 2001) - 1000) % (top + 1);
         default: return (long long)(nx() % 3) - 1;
     }
 }
-int main() {
+template <int L>
+static int check() {
+    constexpr int NM = kCrtLevel[L].n;
     int bad = 0;
     for (int trial = 0; trial < 400; ++trial) {
         const int K = trial % 4 == 3 ? 512 : 1 + (int)(nx() % 512), kind = trial % 4;
@@ -51,7 +53,7 @@ int main() {
         long long p[kCrtN][3] = {};
         for (int k = 0; k < K; ++k) {
             long long n[4];
-            for (int t = 0; t < 4; ++t) n[t] = draw(trial < 8 ? 1 : kind == 1 && k % 3 ? 0 : kind);
+            for (int t = 0; t < 4; ++t) n[t] = draw(trial < 8 ? 1 : kind == 1 && k % 3 ? 0 : kind, kCrtLevel[L].bits);
             re += (__int128)n[0] * n[2] - (__int128)n[1] * n[3];
             im += (__int128)n[0] * n[3] + (__int128)n[1] * n[2];
             float d[4][4];
@@ -60,7 +62,7 @@ int main() {
                 if ((long long)d[t][0] + 16384ll * (long long)d[t][1] + (1ll << 28) * (long long)d[t][2] +
                         (1ll << 42) * (long long)d[t][3] != n[t]) ++bad;
             }
-            for (int i = 0; i < kCrtN; ++i) {
+            for (int i = 0; i < NM; ++i) {
                 const CrtMod m = crt_mod(kCrtModuli[i]);
                 int r[6];
                 for (int t = 0; t < 4; ++t) {
@@ -81,7 +83,7 @@ int main() {
         }
         CrtSum sr, si;
         int rr[kCrtN + 1] = {}, ri[kCrtN + 1] = {};
-        for (int i = 0; i < kCrtN; ++i) {
+        for (int i = 0; i < NM; ++i) {
             const CrtMod m = crt_mod(kCrtModuli[i]);
             int u[3];
             for (int g = 0; g < 3; ++g) {
@@ -91,14 +93,14 @@ int main() {
             rr[i] = u[0] - u[1];
             ri[i] = u[2] - u[0] - u[1];
         }
-        for (int k = 0; k < kCrtGroups; ++k) {
-            sr.add<0>(rr[2 * k], rr[2 * k + 1], kCrtGroup[k]);
-            si.add<-128>(ri[2 * k], ri[2 * k + 1], kCrtGroup[k]);
+        for (int k = 0; k < (NM + 1) / 2; ++k) {
+            sr.add<0>(rr[2 * k], rr[2 * k + 1], kCrtGroup[L][k]);
+            si.add<-128>(ri[2 * k], ri[2 * k + 1], kCrtGroup[L][k]);
         }
         const CrtSum s[2] = {sr, si};
         const __int128 want[2] = {re, im};
         for (int t = 0; t < 2; ++t) {
-            const double v = crt_value(s[t], 0);
+            const double v = crt_value<L>(s[t], 0);
             const __int128 a = want[t] < 0 ? -want[t] : want[t];
             __int128 off = (__int128)v - want[t];
             if (off < 0) off = -off;
@@ -106,10 +108,14 @@ int main() {
                 if (bad++ < 5) printf("trial %d: %a, off by %a\n", trial, v, (double)off);
             }
             // The scale: 2^e is exact, also into the subnormal range.
-            if (crt_value(s[t], -200) != std::ldexp(v, -200)) ++bad;
-            if (crt_value(s[t], -1100) != std::ldexp(v, -1100) && std::fabs(v) > 1e30) ++bad;
+            if (crt_value<L>(s[t], -200) != std::ldexp(v, -200)) ++bad;
+            if (crt_value<L>(s[t], -1100) != std::ldexp(v, -1100) && std::fabs(v) > 1e30) ++bad;
         }
     }
+    return bad;
+}
+int main() {
+    const int bad = check<0>() + check<1>() + check<2>() + check<3>();
     printf("%d failures\n", bad);
     return bad ? 1 : 0;
 }
@@ -122,10 +128,11 @@ def test_moduli_are_coprime_and_their_product_is_large_enough():
     p = [int(v) for v in m.split(",")]
     assert len(p) == 15 and max(p) <= 256
     assert all(gcd(a, b) == 1 for i, a in enumerate(p) for b in p[:i])
-    product = 1
-    for v in p:
-        product *= v
-    assert 2 * 512 * 2 ** 106 < product // 2
+    for n, bits in re.findall(r"\{(\d+), (\d+), 0x[0-9A-F]{16}ull", text):
+        product = 1
+        for v in p[:int(n)]:
+            product *= v
+        assert 2 * 512 * 2 ** (2 * int(bits)) < product // 2
 
 
 def test_residues_rebuild_exact_product_sums(tmp_path):
