@@ -145,6 +145,7 @@ struct PrepOperand {
     int Lp, R;           // padded rows, rows per operand block
     __nv_bfloat16 *out;
     int *E;
+    const int *order;    // row l is order[l] of z (null: l)
 };
 
 // Exponents and residue planes of chunks [c0, c0 + nc): blocks [0, x blocks)
@@ -177,10 +178,11 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
     unsigned long long mx = 0;
     if (z.kfast) {  // a warp per row
         const int l = l0 + warp;
+        const int at = o.order && l < z.L ? o.order[l] : l;
 #pragma unroll 4
         for (int k = lane; k < Kc; k += 32) {
             const double2 v =
-                l < z.L && k < kn ? operand_at(z, l, kb + k) : make_double2(0.0, 0.0);
+                l < z.L && k < kn ? operand_at(z, at, kb + k) : make_double2(0.0, 0.0);
             stage[warp * pitch + k] = v;
             mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
         }
@@ -190,10 +192,11 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
         __syncthreads();
     } else {  // lanes along the 8 rows, 4 k per warp
         const int r = lane & 7, l = l0 + r;
+        const int at = o.order && l < z.L ? o.order[l] : l;
 #pragma unroll 4
         for (int k = warp * 4 + (lane >> 3); k < Kc; k += 32) {
             const double2 v =
-                l < z.L && k < kn ? operand_at(z, l, kb + k) : make_double2(0.0, 0.0);
+                l < z.L && k < kn ? operand_at(z, at, kb + k) : make_double2(0.0, 0.0);
             stage[r * pitch + k] = v;
             mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
         }
@@ -308,8 +311,10 @@ struct Walk {
 __global__ void __launch_bounds__(kThreads, 1)
 crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restrict__ SY, int Mp,
                 int Np, int KS, int nc, int mt0, int MT, int gq, unsigned char *__restrict__ res,
-                int Ms, int nmod, const int *go, int *err) {
+                int Ms, int nmod, const int *go, const int *rows, int *err) {
     if (go && !*go) return;
+    if (rows) MT = min(MT, (*rows + kTM - 1) / kTM);
+    if (MT <= 0) return;
     const int planes = 3 * nmod;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *sA = smem;
@@ -494,8 +499,10 @@ __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char
                                                              const int *EY, int row0, int rows,
                                                              int Ms, int N, int Mp, int Np, int nc,
                                                              int accumulate, double2 *Out,
-                                                             long long out_ld, const int *go) {
+                                                             long long out_ld, const int *go,
+                                                             const int *live) {
     if (go && !*go) return;
+    if (live) rows = min(rows, *live);
     constexpr int NM = kCrtLevel[L].n, PLANES = 3 * NM, GROUPS = (NM + 1) / 2;
     const unsigned quads = (N + 3) / 4;
     const long long n = (long long)rows * quads;
@@ -595,19 +602,19 @@ void launch_prep(const PrepOperand &px, const PrepOperand &py, int xblocks, int 
 
 }  // namespace
 
-cudaError_t crt_rows(const OzOperand &X, int Mp, int K, int Kc, int c0, int nc, int level, void *sx,
-                     int *ex, const int *go, cudaStream_t s) {
+cudaError_t crt_rows(const OzOperand &X, const int *order, int Mp, int K, int Kc, int c0, int nc,
+                     int level, void *sx, int *ex, const int *go, cudaStream_t s) {
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
-    const PrepOperand px{X, Mp, kTM, static_cast<__nv_bfloat16 *>(sx), ex};
+    const PrepOperand px{X, Mp, kTM, static_cast<__nv_bfloat16 *>(sx), ex, order};
     launch_prep(px, px, Mp / 8 * nc, 0, K, Kc, c0, nc, level, go, s);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0,
-                         int tiles, int level, unsigned char *res, int Ms, const int *go, int *err,
-                         cudaStream_t s) {
+                         int tiles, int level, unsigned char *res, int Ms, const int *go,
+                         const int *rows, int *err, cudaStream_t s) {
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
     const int nmod = kCrtLevel[level].n, ntiles = Np / kTN;
@@ -619,19 +626,20 @@ cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc,
                             std::min(ceil_div(grid, tiles), (int)((size_t(80) << 20) / plane)));
     crt_gemm_kernel<<<grid, kThreads, kSmem, s>>>(
         static_cast<const __nv_bfloat16 *>(sx), static_cast<const __nv_bfloat16 *>(sy), Mp, Np,
-        Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, err);
+        Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, rows, err);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t crt_combine(const unsigned char *res, const int *ex, const int *ey, int row0, int rows,
                         int Ms, int N, int Mp, int Np, int nc, int level, bool accumulate,
-                        double2 *Out, long long out_ld, const int *go, cudaStream_t s) {
+                        double2 *Out, long long out_ld, const int *go, const int *live,
+                        cudaStream_t s) {
     const long long want = ((long long)rows * ceil_div(N, 4) + 127) / 128;
     const int grid = (int)std::min<long long>(want, (long long)sm_count() * 32);
     auto launch = [&](auto kern) {
         kern<<<grid, 128, 0, s>>>(res, ex, ey, row0, rows, Ms, N, Mp, Np, nc, accumulate, Out, out_ld,
-                                  go);
+                                  go, live);
     };
     switch (level) {
         case 0: launch(crt_combine_kernel<0>); break;
@@ -668,7 +676,8 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                 Yn.z += (long long)n0 * (Y.kfast ? Y.ld : 1);
                 Yn.L = std::min(N - n0, g.Np);
                 const int Np = ceil_div(Yn.L, kTN) * kTN;
-                const PrepOperand px{X, g.Mp, kTM, b.sx, b.ex}, py{Yn, Np, kTN, b.sy, b.ey};
+                const PrepOperand px{X, g.Mp, kTM, b.sx, b.ex, nullptr},
+                    py{Yn, Np, kTN, b.sy, b.ey, nullptr};
                 // X's planes serve every pass over rows of Y.
                 launch_prep(px, py, n0 == 0 ? g.Mp / 8 * nc : 0, Np / 8 * nc, K, g.Kc, c0, nc, 0,
                             nullptr, s);
@@ -681,10 +690,10 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                     const int tiles = std::min(g.slab_tiles, mtiles - mt0);
                     const int row0 = mt0 * kTM, rows = std::min(M - row0, tiles * kTM);
                     e = crt_products(b.sx, b.sy, g.Mp, Np, g.Kc, nc, mt0, tiles, 0, b.res, Ms,
-                                     nullptr, err, s);
+                                     nullptr, nullptr, err, s);
                     if (e == cudaSuccess && rows > 0)
                         e = crt_combine(b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, 0,
-                                        c0 > zc0, Out + z * split_stride + n0, out_ld, nullptr, s);
+                                        c0 > zc0, Out + z * split_stride + n0, out_ld, nullptr, nullptr, s);
                     if (e != cudaSuccess) return e;
                 }
             }

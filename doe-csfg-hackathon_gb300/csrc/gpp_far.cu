@@ -16,12 +16,15 @@
 //
 //   sum_ig aqsn Q / (wx - wtilde) = sum_k b_k(wx) H_k,  H_k[n1][r] = sum_ig aqsn[n1][ig] P_k[r][ig],
 //
-// P_k = Q T_k(z): one complex product per k that every frequency of every band
+// P_k = Q T_k(z): one complex product per k that every frequency of a band
 // shares, instead of a division per (band, row, column, frequency).  |T_k| is
 // at most rho^k on the box (rho: its Bernstein ellipse); a pair is `far` when
 // |r| >= R rho, so the terms fall off by R and K = bits / log2 R of them reach
-// the working precision.  The products run as residues (gpp_crt.cu), each k at
-// the level of precision that R^-k leaves of the total's.
+// the working precision; a band whose wx all lie further off needs fewer, and
+// the bands are put in the order of what they need, so that the products of a
+// term stop at the bands that have it.  The products run as residues
+// (gpp_crt.cu), each k at the level of precision that R^-k leaves of the
+// total's.
 //
 // What the series does not cover is computed term by term:
 //  * near pairs (|r| < R rho, or a wx that is not finite): over every column,
@@ -35,9 +38,13 @@
 // here returns at once and the per-term kernel runs instead.  No host
 // synchronisation; nothing depends on the order in which blocks run.
 //
-// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 27 ms now (near
-// pairs 17, products 4.1, terms 2, combine 2); mixed, 128 bands x 819 x 16384 x
-// 32: 120 ms per term, 39 now (near 25, terms 7, products 4.3).
+// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 24 ms now (near
+// pairs 15, products 3.5, terms 2.6, combine 1.5); mixed, 128 bands x 819 x 16384
+// x 32: 120 ms per term, 35 now (near 23, terms 7, products 4.3); 512 bands x
+// 1638 x 32768 x 3, 1% strays: 210 per term, 140 now (near 55, products 30,
+// terms 26, strays 15, combine 12).  The near kernels run at 1.25 (FP64) and
+// 1.4 (mixed) of the per-term kernels' time per pair: an entry holds 1.8
+// frequencies on average where a tile there shares its columns among 3.
 #include <algorithm>
 #include <cmath>
 
@@ -50,6 +57,7 @@ namespace gpp {
 
 struct FarPlan {
     int active;
+    int next;            // the near kernel's tile counter
     int n_near;
     long long n_out;
     int lo, hi;          // the box's bins of Re(wtilde)
@@ -58,6 +66,7 @@ struct FarPlan {
     double z0, inv_h, h;
     double dfar;         // |wx - z0| of a far pair is at least this
     double log2_rho;
+    int bands_at[64];    // bands whose series has a term k
     unsigned long long count[512];
     unsigned im[512];    // bits of the largest |Im| (float, rounded up) in each bin
 };
@@ -71,7 +80,8 @@ struct Sizes {
     int bands, ng, nc, nw;
     bool mixed;
     double R;
-    int K;               // terms of the series
+    double bits;         // what the series is cut at
+    int K;               // its terms for a pair that is just far (at most 64)
     int Mp, ngp, nch, Kc;
     int gm, slab;        // series terms and chunks per pass
     int cap_near;
@@ -96,23 +106,30 @@ Sizes sizes(const Problem &p, int bands, bool mixed) {
     z.nc = p.nc;
     z.nw = p.nw;
     z.mixed = mixed;
-    z.R = mixed ? 3.0 : 2.5;
-    z.K = (int)std::ceil((mixed ? 50.0 : 55.0) / std::log2(z.R));
+    z.bits = mixed ? 50.0 : 55.0;
     z.Mp = ceil_div(bands, kCrtRowsX) * kCrtRowsX;
+    z.pairs = (long long)bands * p.nw;
+    // Per cell: a per-term pair takes 20 ps (FP64) or 2.6 ps (mixed); a term of
+    // the series 14 ps for its planes and 0.05 ps per padded band.
+    const double term = (14.0 + 0.05 * z.Mp) / (mixed ? 2.6 : 20.0);
+    // R balances the series' terms against the near pairs: where the terms are
+    // a small part of the call a low R leaves fewer pairs near.  GB300: FP64
+    // 512 x 409 x 8192 x 3, R = 2 / 2.25 / 2.5: 24.6 / 24.5 / 25.4 ms; mixed,
+    // R = 2.5 / 3 / 4: 163 / 155 / 152 ms for 512 x 1638 x 32768 x 3 and
+    // 64.6 / 64.3 / 68.0 ms for 128 x 819 x 16384 x 32.
+    z.R = !mixed ? 2.25 : 32 * term > 0.25 * z.pairs ? 4.0 : 3.0;
+    z.K = (int)std::ceil(z.bits / std::log2(z.R));
+    z.c0 = z.K * term;
     z.ngp = ceil_div(p.ng, 8) * 8;
     z.nch = std::max(1, ceil_div(p.nc, kCrtChunk));
     z.Kc = ceil_div(ceil_div(p.nc, z.nch), kCrtBlockK) * kCrtBlockK;
     const size_t per = (size_t)3 * kCrtN * z.ngp * (2 * (size_t)z.Kc + z.Mp);  // a term's, per chunk
     z.gm = (int)std::min<size_t>(z.K, std::max<size_t>(4, kPassBytes / (per * z.nch)));
     z.slab = (int)std::min<size_t>(z.nch, std::max<size_t>(1, kPassBytes / (per * z.gm)));
-    z.pairs = (long long)bands * p.nw;
     z.cap_near = (int)std::min<long long>(z.pairs / 2 + 1, 1 << 26);
     z.cap_out = (long long)p.ng * p.nc / 32 + 1;
     z.seg_len = std::max<long long>(2048, (z.cap_out + 511) / 512);
     z.segs = (int)((z.cap_out + z.seg_len - 1) / z.seg_len);
-    // Per cell: a per-term pair takes 20 ps (FP64) or 2.6 ps (mixed); a term of
-    // the series 14 ps for its planes and 0.07 ps per padded band.
-    z.c0 = z.K * (14.0 + 0.07 * z.Mp) / (mixed ? 2.6 : 20.0);
     return z;
 }
 
@@ -128,6 +145,7 @@ struct Buffers {
     double2 *near_part, *near_val, *out_part;
     double2 *state;    // P_(k-1), P_k between passes
     int *E0, *EX, *EY;
+    int *terms, *order;  // per band: its terms; the bands by their terms
     __nv_bfloat16 *sx, *sy;
     unsigned char *res;
     double2 *H;        // [bands][gm ngp]
@@ -155,6 +173,8 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     o.out_part = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.segs * z.pairs));
     o.state = reinterpret_cast<double2 *>(
         take(sizeof(double2) * 2 * (size_t)z.nch * z.ngp * z.Kc));
+    o.terms = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
+    o.order = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.E0 = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.ngp));
     o.EX = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.Mp));
     o.EY = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.slab * Np));
@@ -218,7 +238,7 @@ __global__ void __launch_bounds__(1024) far_range_kernel(Problem p, int b0, int 
             a = fmin(a, lo[w]);
             b = fmax(b, hi[w]);
         }
-        f->active = f->n_near = 0;
+        f->active = f->n_near = f->next = 0;
         f->n_out = 0;
         const double margin = 0.02 * (b - a) + 1e-3 * fmax(fabs(a), fabs(b));
         const double width = b - a + 2.0 * margin;
@@ -409,6 +429,53 @@ __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int 
         f->n_near = base;
         f->active = 1;
     }
+}
+
+// Terms each band's series needs (for the nearest of its far frequencies; 0
+// without one), and the bands by that number, the most first, in band order
+// where it is equal.  Past kOrderBands the bands keep their order and all
+// terms.
+constexpr int kOrderBands = 8192;
+__global__ void __launch_bounds__(256) far_need_kernel(Problem p, FarPlan *f, int b0, int bands,
+                                                       int K, double bits, int *terms) {
+    if (!f->active) return;
+    if (blockIdx.x == 0 && threadIdx.x < 64)
+        f->bands_at[threadIdx.x] = bands > kOrderBands && (int)threadIdx.x < K ? bands : 0;
+    const int n = blockIdx.x * 256 + threadIdx.x;
+    if (n >= bands) return;
+    double d = 1.0 / 0.0;
+    for (int w = 0; w < p.nw; ++w) {
+        const double x = p.wx[(size_t)(b0 + n) * p.wx_stride + w];
+        if (is_far(*f, x)) d = fmin(d, fabs(x - f->z0));
+    }
+    int k = 0;
+    if (d < 1e300) {
+        const double u = d * f->inv_h, lr = log2(u + sqrt((u - 1.0) * (u + 1.0))) - f->log2_rho;
+        k = min(K, (int)ceil(bits / lr));
+    }
+    terms[n] = bands > kOrderBands ? K : k;
+}
+__global__ void __launch_bounds__(256) far_order_kernel(FarPlan *f, int bands, const int *terms,
+                                                        int *order) {
+    if (!f->active) return;
+    __shared__ int tile[256];
+    const int n = blockIdx.x * 256 + threadIdx.x;
+    if (bands > kOrderBands) {
+        if (n < bands) order[n] = n;
+        return;
+    }
+    const int mine = n < bands ? terms[n] : 0;
+    int rank = 0;
+    for (int t0 = 0; t0 < bands; t0 += 256) {
+        tile[threadIdx.x] = t0 + (int)threadIdx.x < bands ? terms[t0 + threadIdx.x] : -1;
+        __syncthreads();
+        for (int i = 0; i < 256; ++i) rank += tile[i] > mine || (tile[i] == mine && t0 + i < n);
+        __syncthreads();
+    }
+    if (n < bands) order[rank] = n;
+    // Bands with a term k: those with more than k terms.
+    if (n < bands)
+        for (int k = 0; k < mine; ++k) atomicAdd(&f->bands_at[k], 1);
 }
 
 // Strays per row, their offsets, and their (row, column) list in order.
@@ -642,16 +709,21 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
     }
 }
 
-// S1[n][k0 + m] = sum_r c[n][r] H[n][m ngp + r].
-__global__ void __launch_bounds__(256) far_fold_kernel(const FarPlan *f, const double2 *C,
-                                                       const double2 *H, int ng, int ngp, int ld,
-                                                       int k0, int K, double2 *S1) {
+// S1[n][k0 + m] = sum_r c[n][r] H[.][m ngp + r] for the band n at place
+// blockIdx.x of the order; 0 for a band without the term.
+__global__ void __launch_bounds__(256) far_fold_kernel(const FarPlan *f, const int *order,
+                                                       const double2 *C, const double2 *H, int ng,
+                                                       int ngp, int ld, int k0, int K, double2 *S1) {
     if (!f->active) return;
     __shared__ double red[16], S[2];
-    const int n = blockIdx.x, m = blockIdx.y;
+    const int at = blockIdx.x, n = order[at], m = blockIdx.y;
     double v[2] = {0.0, 0.0};
+    if (at >= f->bands_at[k0 + m]) {
+        if (threadIdx.x == 0) S1[(size_t)n * K + k0 + m] = make_double2(0.0, 0.0);
+        return;
+    }
     for (int r = threadIdx.x; r < ng; r += 256) {
-        const double2 x = cmul(C[(size_t)n * ng + r], H[(size_t)n * ld + (size_t)m * ngp + r]);
+        const double2 x = cmul(C[(size_t)n * ng + r], H[(size_t)at * ld + (size_t)m * ngp + r]);
         v[0] += x.x;
         v[1] += x.y;
     }
@@ -669,7 +741,12 @@ __global__ void __launch_bounds__(128) far_near_fp64_kernel(Problem p, FarNear n
     const int count = *nr.count, tiles = (count + RN - 1) / RN, pairs = (p.ng + 1) / 2;
     const int nc = p.nc;
     constexpr int kRows = 16;  // row pairs in L2 while the entries stream past them
-    for (long long b = blockIdx.x; b < (long long)tiles * pairs; b += gridDim.x) {
+    __shared__ int item;
+    for (;;) {  // tiles differ in length: blocks take them from a counter
+        if (threadIdx.x == 0) item = atomicAdd(nr.next, 1);
+        __syncthreads();
+        const long long b = item;
+        if (b >= (long long)tiles * pairs) break;
         const long long per = (long long)kRows * tiles;
         const int g = (int)(b / per), in = (int)(b % per);
         const int here = min(kRows, pairs - g * kRows);
@@ -903,7 +980,8 @@ bool far_eligible(const Problem &p, int bands, bool mixed) {
     const double cells = (double)p.ng * p.nc;
     const double per_pair = mixed ? 2.6e-12 : 20e-12;
     return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > 3e-3 &&
-           z.pairs < (1 << 20) && cells < 2e9;
+           z.pairs < (1 << 20) && cells < 2e9 &&
+           (z.pairs / 8 + 1) * ((p.ng + 1) / 2) < (1 << 30);  // the near kernel's tile counter
 }
 
 size_t far_bytes(const Problem &p, int bands, bool mixed) {
@@ -928,7 +1006,9 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     far_scan_kernel<<<1, 1024, 0, s>>>(p.ng, b.plan, b.rows);
     far_list_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows, b.out);
     far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
-    count_launch(7);
+    far_need_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(p, b.plan, b0, bands, z.K, z.bits, b.terms);
+    far_order_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(b.plan, bands, b.terms, b.order);
+    count_launch(9);
     cudaError_t e = cudaGetLastError();
 
     // The series, a pass per group of terms of one level and slab of chunks.
@@ -944,7 +1024,7 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
             const int nc = std::min(z.slab, z.nch - c0);
             __nv_bfloat16 *sx = b.sx + (size_t)q * x_slab;
             int *ex = b.EX + (size_t)c0 * z.Mp;
-            if (l != level) e = crt_rows(X, z.Mp, p.nc, z.Kc, c0, nc, l, sx, ex, go, s);
+            if (l != level) e = crt_rows(X, b.order, z.Mp, p.nc, z.Kc, c0, nc, l, sx, ex, go, s);
             if (e != cudaSuccess) break;
             auto terms = [&](auto kern) {
                 kern<<<z.ngp / 8 * nc, 128, 0, s>>>(p, b.plan, z.ngp, c0, nc, z.Kc, Np, k0, gm,
@@ -957,27 +1037,28 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
                 default: terms(far_terms_kernel<3>); break;
             }
             count_launch();
+            const int *live = &b.plan->bands_at[k0];  // the most of the pass's terms
             e = crt_products(sx, b.sy, z.Mp, Np, z.Kc, nc, 0, z.Mp / kCrtRowsX, l, b.res, z.Mp, go,
-                             part.err, s);
+                             live, part.err, s);
             if (e == cudaSuccess)
                 e = crt_combine(b.res, ex, b.EY, 0, bands, z.Mp, rows, z.Mp, Np, nc, l, c0 > 0, b.H,
-                                rows, go, s);
+                                rows, go, live, s);
         }
         level = l;
         if (e != cudaSuccess) break;
-        far_fold_kernel<<<dim3(bands, gm), 256, 0, s>>>(b.plan, b.C, b.H, p.ng, z.ngp, rows, k0, z.K,
+        far_fold_kernel<<<dim3(bands, gm), 256, 0, s>>>(b.plan, b.order, b.C, b.H, p.ng, z.ngp, rows, k0, z.K,
                                                         b.S1);
         count_launch();
         k0 += gm;
     }
     if (e != cudaSuccess) return e;
 
-    const FarNear nr{b.near, &b.plan->n_near, go, b.C, b0, b.near_part};
+    const FarNear nr{b.near, &b.plan->n_near, go, b.C, b0, &b.plan->next, b.near_part};
     if (mixed) {
         e = launch_near_mixed(p, part, split_ws, nr, z.cap_near, s);
         if (e != cudaSuccess) return e;
     } else {
-        far_near_fp64_kernel<<<sms * 4, 128, 0, s>>>(p, nr);
+        far_near_fp64_kernel<<<sms * 2, 128, 0, s>>>(p, nr);
         count_launch();
     }
     far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, (p.ng + 1) / 2, b.near_val);

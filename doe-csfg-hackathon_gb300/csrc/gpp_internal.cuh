@@ -74,6 +74,7 @@ struct FarNear {
     const int *active;     // 0: nothing to do
     const double2 *coeff;  // [bands][ng]: 0.5 vcoul conj(aqsm) at the row's G'
     int b0;                // the band of coeff's first row
+    int *next;             // the next tile to take (zeroed beforehand)
     double2 *partial;
 };
 

@@ -360,16 +360,21 @@ cudaError_t launch_flag_mixed_t(const Problem &p, const Partials &part, const Sp
     return cudaGetLastError();
 }
 
-// The near pairs of gpp_far.cu, a list entry per warp: persistent blocks of 4 warps
-// over (row pair, 4 entries) tiles, in groups of kGroup row pairs that stay in
-// L2 while the entries stream past them.
+// The near pairs of gpp_far.cu, a list entry per warp: persistent blocks of 4
+// warps over (row pair, 4 entries) tiles, in groups of kGroup row pairs that
+// stay in L2 while the entries stream past them.
 __global__ void __launch_bounds__(kWarps * 32, 4)
 near_mixed_kernel(Problem p, Partials part, SplitPlanes s, FarNear near) {
     if (!*near.active) return;
     const int count = *near.count, tiles = (count + kWarps - 1) / kWarps, pairs = (p.ng + 1) / 2;
     const long long per = (long long)kGroup * tiles;
+    __shared__ int item;
     bool reinit = false;
-    for (long long b = blockIdx.x; b < (long long)tiles * pairs; b += gridDim.x) {
+    for (;;) {  // tiles differ in length: blocks take them from a counter
+        if (threadIdx.x == 0) item = atomicAdd(near.next, 1);
+        __syncthreads();
+        const long long b = item;
+        if (b >= (long long)tiles * pairs) break;
         const int g = (int)(b / per), in = (int)(b % per);
         const int here = min(kGroup, pairs - g * kGroup);
         if (!mixed_tile<1, 2, kNearFreq, kWarps, kNearCols, 2, kSyncBlock, true>(
@@ -389,6 +394,7 @@ cudaError_t launch_near_mixed(const Problem &p, const Partials &part, void *spli
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    prefer_max_shared(near_mixed_kernel);
     const long long most = (long long)ceil_div(cap, kWarps) * ((p.ng + 1) / 2);
     const int grid = (int)std::min<long long>(most, (long long)std::max(sms, 1) * 4);
     near_mixed_kernel<<<grid, kWarps * 32, smem, st>>>(p, part, planes(p, split_ws), near);

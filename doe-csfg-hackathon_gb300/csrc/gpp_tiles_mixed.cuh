@@ -246,7 +246,8 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
                                            int row_tile, int band_tile, int iw_chunk,
                                            long long tile, bool reinit,
                                            const FarNear *near = nullptr) {
-    static_assert(!LIST || (RNW == 1 && NWC == kNearFreq), "a warp takes one list entry");
+    static_assert(!LIST || (RNW == 1 && NWC == kNearFreq && kNearFreq == 3),
+                  "a warp takes one list entry");
     constexpr int BN = NWARP * RNW;            // bands per block
     constexpr int K = BN * RG * NWC * 2;       // doubles in the block result
     constexpr int STAGE = (2 * RG + BN) * KC;  // float4 per stage
@@ -380,9 +381,9 @@ __device__ __forceinline__ bool mixed_tile(const Problem &p, const Partials &par
             if (chunk_mask & pole_mask) {
 #pragma unroll kColUnroll
                 for (int il = lane; il < cnt; il += 32)
-                    mixed_column<RNW, NWC, KC, true, LIST>(p, st, sb, il, k0 + il, row0,
-                                                           pole_band, pole_end, iw_first, wx,
-                                                           pole_thr, acc, iw_count);
+                    mixed_column<RNW, NWC, KC, true, LIST>(p, st, sb, il, k0 + il, row0, pole_band,
+                                                           pole_end, iw_first, wx, pole_thr, acc,
+                                                           iw_count);
             } else {
 #pragma unroll kColUnroll
                 for (int il = lane; il < cnt; il += 32)

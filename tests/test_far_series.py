@@ -18,16 +18,18 @@ CSRC = os.path.join(REPO, "doe-csfg-hackathon_gb300", "csrc")
 
 def _constants():
     text = open(os.path.join(CSRC, "gpp_far.cu")).read()
-    mixed_r, fp64_r = map(float, re.search(r"z\.R = mixed \? ([\d.]+) : ([\d.]+);", text).groups())
-    mixed_b, fp64_b = map(float, re.search(r"\(mixed \? ([\d.]+) : ([\d.]+)\) / std::log2\(z\.R\)", text).groups())
-    return {"fp64": (fp64_r, fp64_b, 53), "mixed": (mixed_r, mixed_b, 48)}
+    fp64_r, high, low = map(float, re.search(
+        r"z\.R = !mixed \? ([\d.]+) : [^?]*\? ([\d.]+) : ([\d.]+);", text).groups())
+    mixed_b, fp64_b = map(float, re.search(r"z\.bits = mixed \? ([\d.]+) : ([\d.]+);", text).groups())
+    return {"fp64": (fp64_r, fp64_b, 53), "mixed": (low, mixed_b, 48), "mixed, high R": (high, mixed_b, 48)}
 
 
-@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed, high R"])
 @pytest.mark.parametrize("a,b,v", [(0.5, 2.0, 0.05), (-3.0, 1.0, 0.0), (0.2, 0.3, 0.4), (5.0, 60.0, 1.0)])
 def test_series_reaches_the_working_precision(precision, a, b, v):
     R, bits, want = _constants()[precision]
     K = math.ceil(bits / math.log2(R))
+    assert K <= 64  # the plan's table of terms
     z0, hw = 0.5 * (a + b), 0.5 * (b - a)
     h = max(hw + v, 1.02 * hw)
     corner = complex(hw / h, v / h)
