@@ -229,6 +229,13 @@ bool overlap_tensor_gemm() {
     return !(v && v[0] == '0');
 }
 
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 gpp_status side_stream(int dev, SideStream **out) {
     if (t_side.dev != dev) {
         int lo = 0, hi = 0;
@@ -349,9 +356,15 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     if (e == cudaSuccess && mixed)  // float-float planes of every band the call touches
         e = launch_split_bands(p, w + o_split, has_flag ? fb0 : nb0, has_noflag ? nb1 : fb1, s);
     SideStream *side = nullptr;
+    // Small calls: neither kernel's blocks fill the SMs, so the occupied bands
+    // run beside the unoccupied ones (16 bands, 2 occupied, 24 rows, 256
+    // columns, FP64: 88 us a call one after the other; 41 with this, the sums
+    // of a block folded together and one reduction launch).
+    const long long chunks = ceil_div(p.nw, ns.nwc);
+    const bool small = tiles_f * ceil_div(p.nw, fs.nwc) + tiles_n * chunks <= 2 * sm_count();
     const bool overlap =
         has_flag && has_noflag && !pieces &&
-        (gemm && tensor ? overlap_tensor_gemm() : mixed && overlap_occupied());
+        (gemm && tensor ? overlap_tensor_gemm() : small || (mixed && overlap_occupied()));
     // FP64 with the per-band output: the occupied-band kernel starts once the
     // tensor-core band sum's slicing passes are queued rather than with them
     // (measured 28.0 -> 26.5 ms per production call; without the per-band
@@ -455,23 +468,19 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     if (e == cudaSuccess && want_achs)
         e = launch_achstemp(p, reinterpret_cast<double2 *>(w + o_st), err, s);
 
-    // Fixed-order reduction of the block partials.
-    if (e == cudaSuccess && (o.ach || o.ach_re)) {
-        ReduceOut ro{o.ach, o.ach_re, o.ach_im, o.accumulate};
-        e = launch_reduce(part.ach, ach_seg, (int)ach_seg, p.nw, ro, s);
-    }
-    if (e == cudaSuccess && o.asx) {
-        ReduceOut ro{o.asx, nullptr, nullptr, o.accumulate};
-        e = launch_reduce(part.asx, tiles_f, (int)tiles_f, p.nw, ro, s);
-    }
-    if (e == cudaSuccess && want_n1 && b1 > b0) {
-        ReduceOut ro{o.n1 + b0, nullptr, nullptr, o.accumulate};
-        e = launch_reduce(part.n1 + (size_t)b0 * n1_seg, n1_seg, (int)n1_seg, b1 - b0, ro, s);
-    }
-    if (e == cudaSuccess && want_achs) {
-        ReduceOut ro{o.achs, o.achs_re, o.achs_im, o.accumulate};
-        e = launch_reduce(reinterpret_cast<double2 *>(w + o_st), achs_blocks, achs_blocks, 1, ro, s);
-    }
+    // Fixed-order reduction of the block partials, all outputs in one launch.
+    ReduceJobs jobs;
+    if (o.ach || o.ach_re)
+        jobs.add(part.ach, ach_seg, (int)ach_seg, p.nw, ReduceOut{o.ach, o.ach_re, o.ach_im, o.accumulate});
+    if (o.asx)
+        jobs.add(part.asx, tiles_f, (int)tiles_f, p.nw, ReduceOut{o.asx, nullptr, nullptr, o.accumulate});
+    if (want_n1 && b1 > b0)
+        jobs.add(part.n1 + (size_t)b0 * n1_seg, n1_seg, (int)n1_seg, b1 - b0,
+                 ReduceOut{o.n1 + b0, nullptr, nullptr, o.accumulate});
+    if (want_achs)
+        jobs.add(reinterpret_cast<double2 *>(w + o_st), achs_blocks, achs_blocks, 1,
+                 ReduceOut{o.achs, o.achs_re, o.achs_im, o.accumulate});
+    if (e == cudaSuccess) e = launch_reduce(jobs, s);
     cudaError_t e2 = cudaFreeAsync(ws, s);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync(workspace)");

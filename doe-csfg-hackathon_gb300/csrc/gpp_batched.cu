@@ -35,7 +35,7 @@ namespace {
 constexpr int kThreads = 128;  // every tile family runs 4 warps
 
 // Reduction job: dst[k] (=|+=) sum_t src[k*stride + t], k < nseg, t < len.
-struct ReduceJob {
+struct BatchReduce {
     const double2 *src;
     long long stride;
     int len, nseg;
@@ -45,7 +45,7 @@ struct ReduceJob {
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-batched_reduce_kernel(const ReduceJob *jobs, const int *seg_prefix, int njobs) {
+batched_reduce_kernel(const BatchReduce *jobs, const int *seg_prefix, int njobs) {
     __shared__ double red[(THREADS / 32) * 2];
     __shared__ double S[2];
     // Find the job of this block's segment (prefix sums of nseg).
@@ -54,7 +54,7 @@ batched_reduce_kernel(const ReduceJob *jobs, const int *seg_prefix, int njobs) {
         const int mid = (lo + hi + 1) / 2;
         if (seg_prefix[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
     }
-    const ReduceJob j = jobs[lo];
+    const BatchReduce j = jobs[lo];
     const int k = blockIdx.x - seg_prefix[lo];
     const double2 *seg = j.src + (long long)k * j.stride;
     double v[2] = {0.0, 0.0};
@@ -209,7 +209,7 @@ struct gpp_batch {
         std::vector<size_t> split_off;  // per state in the wave
     };
     std::vector<Wave> waves;
-    std::vector<ReduceJob> jobs;
+    std::vector<BatchReduce> jobs;
     std::vector<int> seg_prefix;
     int total_segs = 0;
     // Static term: per state, [partials] and a destination.
@@ -220,7 +220,7 @@ struct gpp_batch {
     Partials *d_parts = nullptr;
     SplitPlanes *d_splits = nullptr;
     BatchItem *d_items = nullptr;
-    ReduceJob *d_jobs = nullptr;
+    BatchReduce *d_jobs = nullptr;
     int *d_prefix = nullptr;
     int *d_heads = nullptr;
     char *d_split = nullptr;
@@ -414,7 +414,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
             b->jobs.push_back({nullptr, s.achs_blocks, s.achs_blocks, 1,
                                reinterpret_cast<double2 *>(outs[i].achstemp), 0});
     }
-    const size_t off_jobs = reserve(sizeof(ReduceJob) * b->jobs.size());
+    const size_t off_jobs = reserve(sizeof(BatchReduce) * b->jobs.size());
     const size_t off_prefix = reserve(sizeof(int) * (b->jobs.size() + 1));
     const size_t off_split = reserve(mixed ? max_wave : 0);
     b->dev_bytes = off;
@@ -427,7 +427,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     b->d_parts = reinterpret_cast<Partials *>(d + off_parts);
     b->d_splits = reinterpret_cast<SplitPlanes *>(d + off_splits);
     b->d_items = reinterpret_cast<BatchItem *>(d + off_items);
-    b->d_jobs = reinterpret_cast<ReduceJob *>(d + off_jobs);
+    b->d_jobs = reinterpret_cast<BatchReduce *>(d + off_jobs);
     b->d_prefix = reinterpret_cast<int *>(d + off_prefix);
     b->d_heads = reinterpret_cast<int *>(d + off_heads);
     b->d_split = d + off_split;
@@ -488,7 +488,7 @@ gpp_status upload_tables(gpp_batch *b, int *fault_word) {
         e = cudaMemcpy(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(),
                        cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !b->jobs.empty())
-        e = cudaMemcpy(b->d_jobs, b->jobs.data(), sizeof(ReduceJob) * b->jobs.size(),
+        e = cudaMemcpy(b->d_jobs, b->jobs.data(), sizeof(BatchReduce) * b->jobs.size(),
                        cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_prefix, b->seg_prefix.data(), sizeof(int) * b->seg_prefix.size(),

@@ -110,25 +110,28 @@ __global__ void __launch_bounds__(256) achstemp_kernel(Problem p, double2 *parti
     if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(S[0], S[1]);
 }
 
+// Block b sums segment b - (the segments of the jobs before it).
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS)
-reduce_kernel(const double2 *src, long long stride, int len, ReduceOut out) {
+__global__ void __launch_bounds__(THREADS) reduce_kernel(ReduceJobs jobs) {
     __shared__ double red[(THREADS / 32) * 2];
     __shared__ double S[2];
-    const double2 *seg = src + (long long)blockIdx.x * stride;
+    int s = blockIdx.x, j = 0;
+    while (s >= jobs.job[j].nseg) s -= jobs.job[j++].nseg;
+    const ReduceJob &r = jobs.job[j];
+    const double2 *seg = r.src + (long long)s * r.stride;
     double v[2] = {0.0, 0.0};
-    for (int t = threadIdx.x; t < len; t += THREADS) {
+    for (int t = threadIdx.x; t < r.len; t += THREADS) {
         const double2 x = seg[t];
         v[0] += x.x;
         v[1] += x.y;
     }
     block_reduce<2, THREADS>(v, red, S);
     if (threadIdx.x == 0) {
-        const int s = blockIdx.x;
+        const ReduceOut &out = r.out;
         if (out.c) {
-            double2 r = make_double2(S[0], S[1]);
-            if (out.accumulate) r = cadd(out.c[s], r);
-            out.c[s] = r;
+            double2 z = make_double2(S[0], S[1]);
+            if (out.accumulate) z = cadd(out.c[s], z);
+            out.c[s] = z;
         }
         if (out.re) out.re[s] += S[0];
         if (out.im) out.im[s] += S[1];
@@ -147,6 +150,13 @@ cudaError_t launch_noflag_t(const Problem &p, const Partials &part, int b0, int 
         p, part, b0, b1, r.begin, r.end - r.begin, row_tiles, band_tiles, skip);
     count_launch();
     return cudaGetLastError();
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
 }
 
 // Occupied bands in pairs when the frequencies are band-independent (the
@@ -196,7 +206,10 @@ cudaError_t launch_flag_t(const Problem &p, const Partials &part, RowTiles rt, i
     const int row_tiles = ceil_div(p.ng, RG);
     const RowTiles r = rt.clip(row_tiles);
     if (r.end <= r.begin) return cudaSuccess;
-    if (p.wx_stride == 0 && p.nv >= 2 && flag_multi_enabled())
+    // Pairs share the solver, but halve the blocks: with fewer pairs' blocks
+    // than SMs, one band per block (the same bits) uses more of the chip.
+    if (p.wx_stride == 0 && p.nv >= 2 && flag_multi_enabled() &&
+        (long long)(r.end - r.begin) * ceil_div(p.nv, 2) * ceil_div(p.nw, NWC) >= sm_count())
         return launch_flag_nb<RG, NWC, 2, THREADS>(p, part, r, row_tiles, blocks_per_sm, next, s);
     return launch_flag_nb<RG, NWC, 1, THREADS>(p, part, r, row_tiles, 0, nullptr, s);
 }
@@ -252,10 +265,11 @@ cudaError_t launch_achstemp(const Problem &p, double2 *partials, int *err, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(const double2 *src, long long stride, int len, int nseg, ReduceOut out,
-                          cudaStream_t s) {
-    if (nseg <= 0) return cudaSuccess;
-    reduce_kernel<512><<<nseg, 512, 0, s>>>(src, stride, len, out);
+cudaError_t launch_reduce(const ReduceJobs &jobs, cudaStream_t s) {
+    long long segs = 0;
+    for (int j = 0; j < jobs.n; ++j) segs += jobs.job[j].nseg;
+    if (segs <= 0) return cudaSuccess;
+    reduce_kernel<512><<<(unsigned)segs, 512, 0, s>>>(jobs);
     count_launch();
     return cudaGetLastError();
 }

@@ -144,16 +144,49 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Block-wide reduction of K doubles per thread (fixed shuffle tree within a
-// warp, fixed warp order across warps); the sums land in out[K] (shared).
+// Sums of K doubles over a warp, all together: at each of the five steps a
+// lane hands half of the values it still carries to its partner and adds the
+// partner's share of the other half, so that the sums take about K additions
+// and shuffles a lane instead of 5 K (a K = 48 tile's FP64 tree was 15,000
+// cycles of a block's FP64 pipe).  Lane l ends with the sums of the values
+// warp_fold_index<K>(l, j), j < (K + 31) / 32, in v[j] (an index of K: none).
+template <int K, int OFF>
+__device__ __forceinline__ void warp_fold_step(double *v) {
+    if constexpr (OFF > 0) {
+        constexpr int H = (K + 1) / 2;
+        const bool upper = threadIdx.x & OFF;
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const double a = v[i], b = i + H < K ? v[i + H] : 0.0;
+            const double give = upper ? a : b, keep = upper ? b : a;
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, OFF);
+        }
+        warp_fold_step<H, OFF / 2>(v);
+    }
+}
+template <int K, int OFF = 16>
+__device__ __forceinline__ int warp_fold_index(int lane, int j) {
+    if constexpr (OFF == 0) {
+        return j;
+    } else {
+        constexpr int H = (K + 1) / 2;
+        const int i = warp_fold_index<H, OFF / 2>(lane, j);
+        const int k = (lane & OFF) ? i + H : i;
+        return i < H && k < K ? k : K;
+    }
+}
+
+// Block-wide reduction of K doubles per thread (a fixed tree within a warp,
+// fixed warp order across warps); the sums land in out[K] (shared).
 template <int K, int THREADS>
 __device__ __forceinline__ void block_reduce(double (&v)[K], double *red, double *out) {
     constexpr int NWARP = THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    warp_fold_step<K, 16>(v);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double s = warp_sum(v[k]);
-        if (lane == 0) red[warp * K + k] = s;
+    for (int j = 0; j < (K + 31) / 32; ++j) {
+        const int k = warp_fold_index<K>(lane, j);
+        if (k < K) red[warp * K + k] = v[j];
     }
     __syncthreads();
     for (int k = threadIdx.x; k < K; k += THREADS) {

@@ -68,8 +68,21 @@ struct ReduceOut {
     double *im;
     int accumulate;  // for c: 1 adds into c[s], 0 overwrites
 };
-cudaError_t launch_reduce(const double2 *src, long long stride, int len, int nseg, ReduceOut out,
-                          cudaStream_t s);
+// Several such sums in one launch, their segments one after the other.
+struct ReduceJob {
+    const double2 *src;
+    long long stride;
+    int len, nseg;
+    ReduceOut out;
+};
+struct ReduceJobs {
+    ReduceJob job[4];
+    int n = 0;
+    void add(const double2 *src, long long stride, int len, int nseg, ReduceOut out) {
+        if (nseg > 0) job[n++] = ReduceJob{src, stride, len, nseg, out};
+    }
+};
+cudaError_t launch_reduce(const ReduceJobs &jobs, cudaStream_t s);
 
 // Host-to-device transfer by the SMs (host_pull_kernel): src_dev is the
 // device's address of device-accessible host memory; 16-byte aligned

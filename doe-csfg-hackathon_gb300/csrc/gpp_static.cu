@@ -141,12 +141,12 @@ extern "C" gpp_status gpp_sigma_static_scratch(const gpp_problem *problem, const
         e = launch_noflag_fp64(p, part, p.nv, p.nb, s);
     }
     if (e == cudaSuccess) {
-        ReduceOut ro{reinterpret_cast<double2 *>(out->achtemp), nullptr, nullptr, 0};
-        e = launch_reduce(part.ach, part.ach_seg, (int)part.ach_seg, p.nw, ro, s);
-    }
-    if (e == cudaSuccess) {
-        ReduceOut ro{reinterpret_cast<double2 *>(out->asxtemp), nullptr, nullptr, 0};
-        e = launch_reduce(part.asx, part.asx_seg, (int)part.asx_seg, p.nw, ro, s);
+        ReduceJobs jobs;
+        jobs.add(part.ach, part.ach_seg, (int)part.ach_seg, p.nw,
+                 ReduceOut{reinterpret_cast<double2 *>(out->achtemp), nullptr, nullptr, 0});
+        jobs.add(part.asx, part.asx_seg, (int)part.asx_seg, p.nw,
+                 ReduceOut{reinterpret_cast<double2 *>(out->asxtemp), nullptr, nullptr, 0});
+        e = launch_reduce(jobs, s);
     }
     if (e != cudaSuccess) return set_error(GPP_ERR_CUDA, cudaGetErrorString(e));
     return GPP_OK;

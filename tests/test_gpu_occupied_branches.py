@@ -73,3 +73,17 @@ def test_occupied_branches(nv, nc, ng, nw, one_row, semantics, precision, tol):
         assert np.all(np.isfinite(w))
         scale = np.max(np.abs(w))
         assert np.max(np.abs(got - w)) <= tol * scale, (key, got, w)
+
+
+@pytest.mark.parametrize("nv,ng", [(2, 304), (3, 400), (2, 60)])
+def test_band_pairs_give_the_per_band_bits_at_both_grid_sizes(nv, ng, monkeypatch):
+    """Pairs of occupied bands (enough blocks for the SMs) and one band per
+    block (fewer): the same bits as with pairs switched off."""
+    from gppsigma import ops
+    d = ops.DeviceInputs.from_host(_inputs(nv, 333, ng, 3, True, 11 * ng))
+    a = ops.sigma(d, "fp64")
+    ops.wait()
+    monkeypatch.setenv("GPP_FLAG_MULTI", "0")
+    b = ops.sigma(d, "fp64")
+    ops.wait()
+    assert torch.equal(a.asxtemp, b.asxtemp) and torch.equal(a.achtemp, b.achtemp)
