@@ -80,7 +80,7 @@ def test_band_pairs_give_the_per_band_bits_at_both_grid_sizes(nv, ng, monkeypatc
     """Pairs of occupied bands (enough blocks for the SMs) and one band per
     block (fewer): the same bits as with pairs switched off."""
     from gppsigma import ops
-    d = ops.DeviceInputs.from_host(_inputs(nv, 333, ng, 3, True, 11 * ng))
+    d = ops.DeviceInputs.from_host(_inputs(nv, 421, ng, 3, True, 11 * ng))
     a = ops.sigma(d, "fp64")
     ops.wait()
     monkeypatch.setenv("GPP_FLAG_MULTI", "0")
