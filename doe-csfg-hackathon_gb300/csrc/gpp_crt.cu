@@ -23,10 +23,9 @@
 // combination left 5e-15.
 //
 // GB300, 1638 x 32768 over 510 bands / 510 x 1638 over 32768 columns: prepare
-// 0.35 / 1.3 ms, products 2.04 / 2.45 ms (1.23 / 1.10 PFLOP/s), combine 1.0 /
+// 0.35 / 1.3 ms, products 1.42 / 1.75 ms (1.73 / 1.41 PFLOP/s), combine 1.0 /
 // 1.0 ms; the slices took 0.4 / 1.3, 4.6 / 5.4 and 1.3 / 1.4 ms.  The products
-// are bound by the bytes in flight: the 96 KB ring of Y blocks covers about
-// two thirds of the L2 latency at the rate the tensor cores take them.
+// are bound by the tensor pipe (91% of what a library GEMM reaches).
 //
 // crt_gemm_kernel keeps the core-matrix operand layout and the bulk-copy /
 // tcgen05.mma / TMEM pipeline of gpp_ozaki.cu and makes each block
@@ -54,12 +53,13 @@ constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli, at level 
 constexpr int kTM = 128, kTN = 256;     // tcgen05.mma M (rows of X) x N (rows of Y)
 constexpr int kTK = 64;                 // k per operand block
 constexpr int kKSMax = kKcMax / kTK;    // operand blocks per chunk
-constexpr int kStages = 3;              // ring of Y blocks
+constexpr int kStages = 3;              // ring of Y blocks (a pair of blocks: 6 half blocks each)
 constexpr unsigned kBytesA = kTM * kTK * 2, kBytesB = kTN * kTK * 2;  // 16 KB, 32 KB
-constexpr size_t kSmem = (size_t)kKSMax * kBytesA + (size_t)kStages * kBytesB + 256;
-constexpr int kThreads = 320;  // warp 0 loads, warp 1 issues the MMAs, warps 2-9 drain TMEM
+constexpr size_t kSmem = (size_t)kKSMax * kBytesA + (size_t)kStages * kBytesB + 512;
+constexpr int kDrain = 8;     // warps that drain TMEM (16: the same time)
+constexpr int kDrainCols = kTN / (kDrain / 4);
+constexpr int kThreads = 64 + 32 * kDrain;  // warp 0 loads, warp 1 issues the MMAs, the rest drain
 constexpr int kTmemCols = 2 * kTN;
-constexpr unsigned kIdesc = umma_idesc(kTM, kTN);
 
 __constant__ CrtGroup c_group[kCrtLevels][kCrtGroups] = {GPP_CRT_GROUPS};
 
@@ -241,13 +241,14 @@ __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOpe
     }
 }
 
-// The steps of one block: planes q in groups of `gq`, the (plane, row tile,
+// The steps of one block (or pair: a row tile is then two): planes q in groups of `gq`, the (plane, row tile,
 // column tile) steps of a group in order, each block a contiguous run of them
 // (rotated from group to group, so that the runs' rounding evens out).
 // Consecutive steps of a row tile share X's rows in shared memory, and the
 // blocks in flight work on a few planes, whose operands fit in L2.
 struct Walk {
     int Q, MT, NT, gq, grid;
+    unsigned unit;  // this block, or pair of blocks
     int g = 0;
     long long t = 0, end = 0;
     int q0 = 0, q = 0, mt = 0, nt = 0;
@@ -256,7 +257,7 @@ struct Walk {
         for (; g * gq < Q; ++g) {
             q0 = g * gq;
             const long long steps = (long long)min(gq, Q - q0) * MT * NT;
-            const long long j = (long long)((blockIdx.x + (unsigned)g * 61u) % (unsigned)grid);
+            const long long j = (long long)((unit + (unsigned)g * 61u) % (unsigned)grid);
             t = j * steps / grid;
             end = (j + 1) * steps / grid;
             if (t < end) return true;
@@ -301,13 +302,21 @@ struct Walk {
 // byte stored is the symmetric residue + 128, at res[(q Ms + row) Np + col].
 // Warp 0 (one thread) loads: X's blocks of a row tile into kKSMax resident
 // slots, each as soon as the MMAs of the previous run's last step released
-// it, and Y's blocks through a three-stage ring, all by 1-D bulk copies onto
-// mbarriers; warp 1 (one thread) issues four K = 16 tcgen05.mma per block into
-// one of two TMEM accumulators; warps 2-9 drain a finished accumulator (a
-// warp's 32 lanes x 128 columns), reduce the exact FP32 sums modulo p on the
-// FP32 pipe and store bytes, 32 at a time per thread.  Every wait is bounded;
-// a block that gives up records kErrPipelineTimeout, lets its copies and MMAs
-// finish and frees its TMEM.
+// it, and Y's blocks through a ring, all by 1-D bulk copies onto mbarriers;
+// warp 1 issues four K = 16 tcgen05.mma per block into one of two TMEM
+// accumulators; warps 2-9 drain a finished accumulator (a warp's 32 lanes x
+// 128 columns), reduce the exact FP32 sums modulo p on the FP32 pipe and store
+// bytes, 32 in one store per thread.  Warp 1 waits as a whole and one elected
+// lane issues, so that addresses and descriptors stay in uniform registers:
+// run by one thread, the loop's own latency (4 MMAs 280 cycles, the commits 130,
+// two waits 170) kept the tensor pipe at 53%; now 1073 -> 750 cycles a block.
+// CG = 2: a pair of blocks takes two row tiles (cta_group::2, M = 256); each
+// holds its own 128 rows of X and half of Y's rows, block 0 issues for both,
+// and block 1's warp 1 passes on to block 0's barriers what has landed in its
+// own shared memory.
+// Every wait is bounded; a block that gives up records kErrPipelineTimeout,
+// lets its copies and MMAs finish and frees its TMEM.
+template <int CG>
 __global__ void __launch_bounds__(kThreads, 1)
 crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restrict__ SY, int Mp,
                 int Np, int KS, int nc, int mt0, int MT, int gq, unsigned char *__restrict__ res,
@@ -315,13 +324,16 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
     if (go && !*go) return;
     if (rows) MT = min(MT, (*rows + kTM - 1) / kTM);
     if (MT <= 0) return;
+    constexpr int STAGES = kStages * CG;
+    constexpr unsigned BYTES_B = kBytesB / CG, IDESC = umma_idesc(kTM * CG, kTN);
+    const int rank = CG == 2 ? cluster_rank() : 0;
     const int planes = 3 * nmod;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *sA = smem;
     unsigned char *sB = smem + (size_t)kKSMax * kBytesA;
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(sB + (size_t)kStages * kBytesB);
-    unsigned long long *full = bars, *empty = full + kStages;
-    unsigned long long *afull = empty + kStages, *aempty = afull + kKSMax;
+    unsigned long long *full = bars, *empty = full + STAGES;
+    unsigned long long *afull = empty + STAGES, *aempty = afull + kKSMax;
     unsigned long long *accfull = aempty + kKSMax, *accempty = accfull + 2;
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(accempty + 2);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
@@ -332,40 +344,58 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
     const int ksteps = nc * KS;
     Walk w;
     w.Q = nc * planes;
-    w.MT = MT;
+    w.MT = (MT + CG - 1) / CG;
     w.NT = Np / kTN;
     w.gq = gq;
-    w.grid = gridDim.x;
+    w.grid = gridDim.x / CG;
+    w.unit = blockIdx.x / CG;
 
     if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            bar_init(&full[s], 1);
+        // Block 0 of a pair also waits for the other block's copies.
+        const int arrivals = CG == 2 && rank == 0 ? 2 : 1;
+        for (int s = 0; s < STAGES; ++s) {
+            bar_init(&full[s], arrivals);
             bar_init(&empty[s], 1);
         }
         for (int s = 0; s < kKSMax; ++s) {
-            bar_init(&afull[s], 1);
+            bar_init(&afull[s], arrivals);
             bar_init(&aempty[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
             bar_init(&accfull[a], 1);
-            bar_init(&accempty[a], 256);
+            bar_init(&accempty[a], kDrain * CG);
         }
         *abort_flag = 0;
         issued_a = issued_b = waited_a = waited_b = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_addr(tmem_slot)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                             smem_addr(tmem_slot)),
+                         "r"(kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                             smem_addr(tmem_slot)),
+                         "r"(kTmemCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (CG == 2) cluster_sync();  // both blocks' barriers are there
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
 
+    auto commit = [](unsigned long long *bar) {
+        if constexpr (CG == 2)
+            umma_commit_pair(bar);
+        else
+            umma_commit(bar);
+    };
     if (warp == 0) {
         if (lane == 0) {  // producer
             const size_t xplane = (size_t)Mp * ksteps * kTK, yplane = (size_t)Np * ksteps * kTK;
@@ -374,9 +404,10 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
             for (bool more = w.start(); ok && more; more = w.next()) {
                 const int c = w.q / planes, pl = w.q % planes;
                 const __nv_bfloat16 *a = SX + pl * xplane +
-                                         ((size_t)(mt0 + w.mt) * ksteps + (size_t)c * KS) * (kTM * kTK);
+                                         ((size_t)(mt0 + min(w.mt * CG + rank, MT - 1)) * ksteps + (size_t)c * KS) * (kTM * kTK);
                 const __nv_bfloat16 *b =
-                    SY + pl * yplane + ((size_t)w.nt * ksteps + (size_t)c * KS) * (kTN * kTK);
+                    SY + pl * yplane + ((size_t)w.nt * ksteps + (size_t)c * KS) * (kTN * kTK) +
+                    rank * (BYTES_B / sizeof(__nv_bfloat16));
                 if (w.first) ++run;
                 for (int s = 0; s < KS; ++s) {
                     if (w.first) {
@@ -385,63 +416,96 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
                         bulk_g2s(sA + (size_t)s * kBytesA, a + (size_t)s * (kTM * kTK), kBytesA, &afull[s]);
                         ++issued_a;
                     }
-                    const int st = nb % kStages;
-                    if (nb >= kStages && !bar_wait(&empty[st], (nb / kStages - 1) & 1, abort)) {
+                    const int st = nb % STAGES;
+                    if (nb >= STAGES && !bar_wait(&empty[st], (nb / STAGES - 1) & 1, abort)) {
                         ok = false;
                         break;
                     }
-                    bar_expect_tx(&full[st], kBytesB);
-                    bulk_g2s(sB + (size_t)st * kBytesB, b + (size_t)s * (kTN * kTK), kBytesB, &full[st]);
+                    bar_expect_tx(&full[st], BYTES_B);
+                    bulk_g2s(sB + (size_t)st * BYTES_B, b + (size_t)s * (kTN * kTK), BYTES_B, &full[st]);
                     ++nb;
                 }
             }
             issued_b = nb;
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer
-            int run = -1, nb = 0, G = 0;
+        if (lane == 0 && rank == 1) {  // tells block 0 what has landed here
+            int run = -1, nb = 0;
+            bool ok = true;
+            for (bool more = w.start(); ok && more; more = w.next()) {
+                if (w.first) ++run;
+                for (int s = 0; s < KS; ++s) {
+                    if (w.first) {
+                        if (!bar_wait(&afull[s], run & 1, abort)) { ok = false; break; }
+                        bar_arrive_leader(&afull[s]);
+                        ++waited_a;
+                    }
+                    const int st = nb % STAGES;
+                    if (!bar_wait(&full[st], (nb / STAGES) & 1, abort)) { ok = false; break; }
+                    bar_arrive_leader(&full[st]);
+                    ++nb;
+                }
+            }
+            waited_b = nb;
+        } else if (rank == 0) {  // MMA issuer: the warp waits, one lane issues
+            const bool one = elect_one();
+            const unsigned sa0 = smem_addr(sA), sb0 = smem_addr(sB);
+            int run = -1, nb = 0, st = 0, G = 0;
+            unsigned phase = 0;
             bool ok = true;
             for (bool more = w.start(); ok && more; more = w.next(), ++G) {
                 if (w.first) ++run;
                 const bool last = w.last();
                 const int acc = G & 1;
-                if (G >= 2 && !bar_wait(&accempty[acc], ((G >> 1) - 1) & 1, abort)) break;
+                if (G >= 2 && !__all_sync(~0u, bar_wait(&accempty[acc], ((G >> 1) - 1) & 1, abort))) break;
+                tc_fence_after();
                 for (int s = 0; s < KS; ++s) {
                     if (w.first) {
-                        if (!bar_wait(&afull[s], run & 1, abort)) { ok = false; break; }
-                        ++waited_a;
+                        ok = __all_sync(~0u, bar_wait(&afull[s], run & 1, abort));
+                        if (!ok) break;
+                        if (one) ++waited_a;
                     }
-                    const int st = nb % kStages;
-                    if (!bar_wait(&full[st], (nb / kStages) & 1, abort)) { ok = false; break; }
-                    tc_fence_after();
-                    const unsigned sa = smem_addr(sA + (size_t)s * kBytesA);
-                    const unsigned sb = smem_addr(sB + (size_t)st * kBytesB);
+                    ok = __all_sync(~0u, bar_wait(&full[st], phase, abort));
+                    if (!ok) break;
+                    const unsigned long long da = umma_desc(sa0 + (unsigned)s * kBytesA, 128, 1024),
+                                             db = umma_desc(sb0 + (unsigned)st * BYTES_B, 128, 1024);
+                    if (one) {
 #pragma unroll
-                    for (int k16 = 0; k16 < kTK / 16; ++k16)
-                        umma_bf16(tmem + acc * kTN, umma_desc(sa + k16 * 256, 128, 1024),
-                                  umma_desc(sb + k16 * 256, 128, 1024), kIdesc,
-                                  !(s == 0 && k16 == 0));
-                    umma_commit(&empty[st]);
-                    if (last) umma_commit(&aempty[s]);
+                        for (int k16 = 0; k16 < kTK / 16; ++k16) {  // 256 bytes on in both
+                            const unsigned add = !(s == 0 && k16 == 0);
+                            if constexpr (CG == 2)
+                                umma_bf16_pair(tmem + acc * kTN, da + k16 * 16, db + k16 * 16, IDESC, add);
+                            else
+                                umma_bf16(tmem + acc * kTN, da + k16 * 16, db + k16 * 16, IDESC, add);
+                        }
+                        commit(&empty[st]);
+                        if (last) commit(&aempty[s]);
+                        if (s == KS - 1) commit(&accfull[acc]);
+                    }
+                    __syncwarp();
                     ++nb;
+                    if (++st == STAGES) {
+                        st = 0;
+                        phase ^= 1;
+                    }
                 }
-                if (ok) umma_commit(&accfull[acc]);
             }
-            waited_b = nb;
+            if (one) waited_b = nb;
         }
-    } else {  // epilogue: TMEM lanes 32 (warp % 4) .., columns 128 ((warp - 2) / 4) ..
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+    } else {  // epilogue: TMEM lanes 32 (warp % 4) .., columns kDrainCols ((warp - 2) / 4) ..
+        const int quarter = warp & 3, group = (warp - 2) >> 2;
         int G = 0;
         for (bool more = w.start(); more; more = w.next(), ++G) {
             const int acc = G & 1;
             if (!bar_wait(&accfull[acc], (G >> 1) & 1, abort)) break;
             tc_fence_after();
             const CrtMod m = c_crt_mod[(w.q % planes) % nmod];
-            unsigned char *o = res + ((size_t)w.q * Ms + (size_t)w.mt * kTM + quarter * 32 + lane) * Np +
-                               (size_t)w.nt * kTN + half * 128;
-            const unsigned ta = tmem + ((unsigned)(quarter * 32) << 16) + acc * kTN + half * 128;
+            const int tile = w.mt * CG + rank;  // the pair's second may be past the end
+            unsigned char *o = res + ((size_t)w.q * Ms + (size_t)tile * kTM + quarter * 32 + lane) * Np +
+                               (size_t)w.nt * kTN + group * kDrainCols;
+            const unsigned ta = tmem + ((unsigned)(quarter * 32) << 16) + acc * kTN + group * kDrainCols;
 #pragma unroll 1
-            for (int cc = 0; cc < 128; cc += 32) {
+            for (int cc = 0; cc < kDrainCols; cc += 32) {
                 float v[32];
                 tmem_ld32(ta + cc, v);
                 unsigned word[8];
@@ -455,11 +519,20 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
                     const unsigned hi = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040);
                     word[j] = __byte_perm(lo, hi, 0x5410);
                 }
-                *reinterpret_cast<uint4 *>(o + cc) = make_uint4(word[0], word[1], word[2], word[3]);
-                *reinterpret_cast<uint4 *>(o + cc + 16) = make_uint4(word[4], word[5], word[6], word[7]);
+                if (tile < MT)  // 32 bytes per thread in one store
+                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + cc),
+                                 "r"(word[0]), "r"(word[1]), "r"(word[2]), "r"(word[3]), "r"(word[4]),
+                                 "r"(word[5]), "r"(word[6]), "r"(word[7])
+                                 : "memory");
             }
             tc_fence_before();
-            bar_arrive(&accempty[acc]);
+            __syncwarp();
+            if (lane == 0) {
+                if constexpr (CG == 2)
+                    bar_arrive_leader(&accempty[acc]);
+                else
+                    bar_arrive(&accempty[acc]);
+            }
         }
     }
 
@@ -473,19 +546,26 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
             }
         };
         for (int t = waited_b; t < issued_b; ++t)
-            settle(&full[t % kStages], (unsigned)((t / kStages) & 1));
+            settle(&full[t % STAGES], (unsigned)((t / STAGES) & 1));
         for (int t = waited_a; t < issued_a; ++t)
             settle(&afull[t % KS], (unsigned)((t / KS) & 1));
         if (waited_b > 0)
-            settle(&empty[(waited_b - 1) % kStages], (unsigned)(((waited_b - 1) / kStages) & 1));
+            settle(&empty[(waited_b - 1) % STAGES], (unsigned)(((waited_b - 1) / STAGES) & 1));
     }
     tc_fence_before();
     __syncthreads();
+    // Neither block goes while the other's MMAs or arrivals may reach it.
+    if constexpr (CG == 2) cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(kTmemCols)
-                     : "memory");
+        if constexpr (CG == 1)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                         "r"(kTmemCols)
+                         : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                         "r"(kTmemCols)
+                         : "memory");
     }
 }
 
@@ -580,13 +660,54 @@ int sm_count() {
     return sms > 0 ? sms : 132;
 }
 
+// Pairs of blocks (cta_group::2): each SM then reads half of Y's block for the
+// same products.  16384 columns, 510 bands, 1 / 3 / 5 / 7 / 13 row tiles:
+// single blocks 0.128 / 0.263 / 0.407 / 0.543 / 0.976 ms, pairs 0.138 / 0.240 /
+// 0.328 / 0.432 / 0.726 (an odd row tile leaves half of a pair idle).
+bool gemm_pairs(int tiles) { return tiles >= 2; }
+
+// A launch of `grid` blocks (cg 1) or pairs of blocks (cg 2, a cluster each).
+struct GemmLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute pair = {};
+    GemmLaunch(int cg, int grid, cudaStream_t s) {
+        cfg.gridDim = dim3(grid * cg);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = kSmem;
+        cfg.stream = s;
+        pair.id = cudaLaunchAttributeClusterDimension;
+        pair.val.clusterDim.x = 2;
+        pair.val.clusterDim.y = pair.val.clusterDim.z = 1;
+        cfg.attrs = &pair;
+        cfg.numAttrs = cg == 2 ? 1 : 0;
+    }
+    GemmLaunch(const GemmLaunch &) = delete;
+};
+
+// Pairs the device holds at once, one persistent pair each.
+int pair_count() {
+    static std::atomic<int> count[256] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    int n = count[dev & 255].load(std::memory_order_acquire);
+    if (n == 0) {
+        GemmLaunch l(2, std::max(1, sm_count() / 2), nullptr);
+        if (cudaOccupancyMaxActiveClusters(&n, crt_gemm_kernel<2>, &l.cfg) != cudaSuccess) return 0;
+        count[dev & 255].store(n, std::memory_order_release);
+    }
+    return n;
+}
+
 cudaError_t configure() {
     static std::atomic<bool> configured[256] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || configured[dev & 255].load(std::memory_order_acquire)) return e;
-    e = cudaFuncSetAttribute(crt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(crt_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(crt_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(crt_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double2) * 8 * (kKcMax + 1)));
@@ -618,15 +739,21 @@ cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc,
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
     const int nmod = kCrtLevel[level].n, ntiles = Np / kTN;
-    const int grid = (int)std::min<long long>(sm_count(), (long long)nc * 3 * nmod * tiles * ntiles);
+    const int cg = gemm_pairs(tiles) ? 2 : 1, units = ceil_div(tiles, cg);  // row tiles, or pairs
+    const int fit = cg == 2 ? pair_count() : sm_count();
+    if (fit <= 0) return cudaErrorUnknown;
+    const int grid = (int)std::min<long long>(fit, (long long)nc * 3 * nmod * units * ntiles);
     // Planes in flight: enough that every block has a step, with their
     // operands within about 80 MB of L2.
     const size_t plane = sizeof(__nv_bfloat16) * (size_t)Kc * (Mp + Np);
-    const int gq = std::max(ceil_div(grid, (long long)tiles * ntiles),
-                            std::min(ceil_div(grid, tiles), (int)((size_t(80) << 20) / plane)));
-    crt_gemm_kernel<<<grid, kThreads, kSmem, s>>>(
-        static_cast<const __nv_bfloat16 *>(sx), static_cast<const __nv_bfloat16 *>(sy), Mp, Np,
-        Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, rows, err);
+    const int gq = std::max(ceil_div(grid, (long long)units * ntiles),
+                            std::min(ceil_div(grid, units), (int)((size_t(80) << 20) / plane)));
+    const __nv_bfloat16 *x = static_cast<const __nv_bfloat16 *>(sx),
+                        *y = static_cast<const __nv_bfloat16 *>(sy);
+    GemmLaunch l(cg, grid, s);
+    e = cudaLaunchKernelEx(&l.cfg, cg == 2 ? crt_gemm_kernel<2> : crt_gemm_kernel<1>, x, y, Mp, Np,
+                           Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, rows, err);
+    if (e != cudaSuccess) return e;
     count_launch();
     return cudaGetLastError();
 }

@@ -31,6 +31,22 @@ __device__ __forceinline__ bool bar_try_wait(unsigned long long *bar, unsigned p
         : "memory");
     return ok != 0;
 }
+// Arrive on `bar` of block 0 of the cluster.
+__device__ __forceinline__ void bar_arrive_leader(unsigned long long *bar) {
+    asm volatile(
+        "{\n .reg .b32 r;\n mapa.shared::cluster.u32 r, %0, 0;\n"
+        " mbarrier.arrive.shared::cluster.b64 _, [r];\n}" ::"r"(smem_addr(bar))
+        : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+}
+__device__ __forceinline__ int cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
 // Bounded wait for phase `parity`: gives up after kWaitLimit polls, or as soon
 // as another thread of the block raised *abort (and then raises it itself).
 __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity,
@@ -79,6 +95,31 @@ __device__ __forceinline__ void umma_commit(unsigned long long *bar) {
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
             smem_addr(bar))
         : "memory");
+}
+// The same for a pair of blocks (cta_group::2): one thread of block 0 issues
+// for both, M = 256 (each block's 128 rows of A and of D) and N = 256 (each
+// block holds 128 rows of B); the commit arrives on `bar` in both blocks.
+__device__ __forceinline__ void umma_bf16_pair(unsigned tmem, unsigned long long a,
+                                               unsigned long long b, unsigned idesc,
+                                               unsigned accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(unsigned long long *bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+        "[%0], %1;" ::"r"(smem_addr(bar)),
+        "h"((unsigned short)3)
+        : "memory");
+}
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
 }
 __device__ __forceinline__ void tc_fence_before() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
