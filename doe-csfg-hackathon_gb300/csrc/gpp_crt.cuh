@@ -116,6 +116,27 @@ __host__ __device__ __forceinline__ void crt_digits_n(long long N, float (&d)[ND
     }
 }
 
+// The digits of rint(scale (h + l)) of two normalised float-float values, for
+// scale a power of two and scale |h + l| <= 2^53 (ND = 4), 2^41 (3) or 2^27 (2):
+// each digit is rounded from the remainder and taken off its high part exactly
+// (both are multiples of the smaller of the digit's weight and an ulp of h),
+// so the last remainder is exact but for what lies below the integers.  A
+// digit may pass its half range by two (2^41 + 2^29 below the top one).
+template <int ND>
+__host__ __device__ __forceinline__ void crt_digits_df2(const df2 &x, float scale, float2 (&d)[ND]) {
+    const float2 magic = f2(kCrtMagic, kCrtMagic);
+    float2 r = f2mul(x.h, f2(scale, scale));
+    const float2 l = f2mul(x.l, f2(scale, scale));
+#pragma unroll
+    for (int k = ND - 1; k > 0; --k) {
+        const float w = k == 3 ? 4398046511104.0f : k == 2 ? 268435456.0f : 16384.0f;  // 2^(14 k)
+        const float2 v = k == ND - 1 ? r : f2add(r, l);
+        d[k] = f2sub(f2fma(v, f2(1.0f / w, 1.0f / w), magic), magic);
+        r = f2fma(d[k], f2(-w, -w), r);
+    }
+    d[0] = f2sub(f2add(f2add(r, l), magic), magic);
+}
+
 // v - p rint(v / p) on both lanes for integers |v| <= 2^23: the quotient is
 // rounded once, from the product by a 1 / p whose relative error is at most
 // 2^-25, so it is off by under 1 / (2 p) before rounding and the result is

@@ -143,7 +143,7 @@ struct Buffers {
     double2 *C;        // [bands][ng]
     double2 *S1;       // [bands][K]
     double2 *near_part, *near_val, *out_part;
-    double2 *state;    // P_(k-1), P_k between passes
+    void *state;       // P_(k-1), P_k (mixed: and z) between passes
     int *E0, *EX, *EY;
     int *terms, *order;  // per band: its terms; the bands by their terms
     __nv_bfloat16 *sx, *sy;
@@ -171,8 +171,7 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     o.near_part = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near * rt));
     o.near_val = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near));
     o.out_part = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.segs * z.pairs));
-    o.state = reinterpret_cast<double2 *>(
-        take(sizeof(double2) * 2 * (size_t)z.nch * z.ngp * z.Kc));
+    o.state = take(sizeof(double2) * (z.mixed ? 3 : 2) * (size_t)z.nch * z.ngp * z.Kc);
     o.terms = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.order = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.E0 = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.ngp));
@@ -585,11 +584,17 @@ __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
 // exponent of term k is that of the chunk's largest |re|, |im| of Q, raised by
 // the bound rho^k of |T_k| and 1.  Columns outside the box are zero.
 constexpr int kTermK = 4;  // columns per thread
-template <int L>
+//
+// In mixed precision the recurrence runs in float-float (DF): FP64 kept its
+// pipe 62-76% busy with 4 instructions per term and column where the residues
+// take most of the issue slots.  Q is scaled by the chunk's exponent first, so
+// its range is FP64's; only the first pass reads the inputs, the next ones
+// find z with the last two terms in `state`.
+template <int L, bool DF>
 __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int c0,
                                                            int nc, int Kc, int Np, int k0, int gm,
                                                            int last, __nv_bfloat16 *out, int *EY,
-                                                           int *E0, double2 *state) {
+                                                           int *E0, void *state) {
     constexpr int NMOD = kCrtLevel[L].n, BITS = kCrtLevel[L].bits, ND = BITS > 41 ? 4 : BITS > 18 ? 3 : 2;
     if (!f->active) return;
     __shared__ unsigned long long red[4][8];
@@ -642,7 +647,85 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
 
     const int ksteps = nc * (Kc / kCrtBlockK);
     const size_t plane = (size_t)Np * ksteps * kCrtBlockK;
-    double2 *st = state + ((size_t)(c0 + c) * groups + grp) * (size_t)items * (2 * kTermK * 128);
+    if constexpr (DF) {
+        // Two pairs of columns per thread: z2, then P_(k-1) and P_k as df2.
+        constexpr int NP = kTermK / 2;
+        float4 *st = static_cast<float4 *>(state) + ((size_t)(c0 + c) * groups + grp) * (size_t)items * (NP * 6 * 128) + t;
+        auto load = [&](size_t at) {
+            const float4 v = st[at * 128];
+            return df2{f2(v.x, v.y), f2(v.z, v.w)};
+        };
+        auto store = [&](size_t at, const df2 &v) {
+            st[at * 128] = make_float4(v.h.x, v.h.y, v.l.x, v.l.y);
+        };
+        const bool finite = e0 != kExpZero && e0 != kExpNonFinite;
+        for (int i = 0; i < items; ++i) {
+            const int kg = kg0 + 8 * i;
+            df2 zr[NP], zi[NP], cr[NP], ci[NP], pr[NP], pi[NP];
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+                const size_t at6 = (size_t)(i * NP + h) * 6;
+                if (k0 > 0) {
+                    zr[h] = load(at6), zi[h] = load(at6 + 1);
+                    pr[h] = load(at6 + 2), pi[h] = load(at6 + 3);
+                    cr[h] = load(at6 + 4), ci[h] = load(at6 + 5);
+                    continue;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int ig = kb + kg * 8 + half * kTermK + 2 * h + j;
+                    double2 wt, z = make_double2(0.0, 0.0), q = z;
+                    if (at(ig, wt) && finite) {
+                        z = make_double2(2.0 * (wt.x - z0) * inv_h, 2.0 * wt.y * inv_h);
+                        q = cmul(wt, __ldg(erow + ig));
+                        q = make_double2(ldexp(q.x, -e0), ldexp(q.y, -e0));
+                    }
+                    df2_set_lane(zr[h], j, split_bits(z.x));
+                    df2_set_lane(zi[h], j, split_bits(z.y));
+                    df2_set_lane(cr[h], j, split_bits(q.x));
+                    df2_set_lane(ci[h], j, split_bits(q.y));
+                }
+                const df2 half_r = {f2mul(zr[h].h, f2(0.5f, 0.5f)), f2mul(zr[h].l, f2(0.5f, 0.5f))};
+                const df2 half_i = {f2mul(zi[h].h, f2(0.5f, 0.5f)), f2mul(zi[h].l, f2(0.5f, 0.5f))};
+                pr[h] = df2_norm(df2_sub(df2_mul(half_r, cr[h]), df2_mul(half_i, ci[h])));
+                pi[h] = df2_norm(df2_add(df2_mul(half_r, ci[h]), df2_mul(half_i, cr[h])));
+                if (!last) store(at6, zr[h]), store(at6 + 1, zi[h]);
+            }
+            const int ks = c * (Kc / kCrtBlockK) + i;
+#pragma unroll 1
+            for (int m = 0; m < gm; ++m) {
+                const float scale = ldexpf(1.0f, BITS - raise(k0 + m));
+                const int y = m * ngp + grp * 8;
+                __nv_bfloat16 *w = out + ((size_t)(y / kCrtRowsY) * ksteps + ks) * (kCrtRowsY * kCrtBlockK) +
+                                   (size_t)((y % kCrtRowsY) / 8) * 512 + kg0 * 64 + row * 8 + half * kTermK;
+                float2 dr[NP][ND], di[NP][ND];
+#pragma unroll
+                for (int h = 0; h < NP; ++h) {
+                    crt_digits_df2<ND>(cr[h], scale, dr[h]);
+                    crt_digits_df2<ND>(ci[h], scale, di[h]);
+                }
+                crt_store_residues<NP, ND>(dr, di, NMOD, w, plane);
+#pragma unroll
+                for (int h = 0; h < NP; ++h) {
+                    const df2 nr = df2_norm(df2_sub(df2_mul(zr[h], cr[h]),
+                                                    df2_add(df2_mul(zi[h], ci[h]), pr[h])));
+                    const df2 ni = df2_norm(df2_add(df2_mul(zr[h], ci[h]),
+                                                    df2_sub(df2_mul(zi[h], cr[h]), pi[h])));
+                    pr[h] = cr[h], pi[h] = ci[h];
+                    cr[h] = nr, ci[h] = ni;
+                }
+            }
+            if (last) continue;
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+                const size_t at6 = (size_t)(i * NP + h) * 6;
+                store(at6 + 2, pr[h]), store(at6 + 3, pi[h]);
+                store(at6 + 4, cr[h]), store(at6 + 5, ci[h]);
+            }
+        }
+        return;
+    } else {
+    double2 *st = static_cast<double2 *>(state) + ((size_t)(c0 + c) * groups + grp) * (size_t)items * (2 * kTermK * 128);
     for (int i = 0; i < items; ++i) {  // Kc is a multiple of 64: 8 k-cores per turn
         const int kg = kg0 + 8 * i;
         double2 cur[kTermK], prev[kTermK], z2[kTermK];
@@ -706,6 +789,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
                 st[((size_t)(i * kTermK + kk) * 2 + 1) * 128 + t] = cur[kk];
             }
         }
+    }
     }
 }
 
@@ -1031,10 +1115,10 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
                                                     k0 + gm >= z.K, b.sy, b.EY, b.E0, b.state);
             };
             switch (l) {
-                case 0: terms(far_terms_kernel<0>); break;
-                case 1: terms(far_terms_kernel<1>); break;
-                case 2: terms(far_terms_kernel<2>); break;
-                default: terms(far_terms_kernel<3>); break;
+                case 0: mixed ? terms(far_terms_kernel<0, true>) : terms(far_terms_kernel<0, false>); break;
+                case 1: mixed ? terms(far_terms_kernel<1, true>) : terms(far_terms_kernel<1, false>); break;
+                case 2: mixed ? terms(far_terms_kernel<2, true>) : terms(far_terms_kernel<2, false>); break;
+                default: mixed ? terms(far_terms_kernel<3, true>) : terms(far_terms_kernel<3, false>); break;
             }
             count_launch();
             const int *live = &b.plan->bands_at[k0];  // the most of the pass's terms
