@@ -285,12 +285,14 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const TileShape ns = mixed ? mixed_noflag_shape(p, variant) : fp64_noflag_shape(p);
     const bool want_n1 = o.n1 && p.nw >= 3 && p.ng > 0;
     const bool gemm = has_noflag && gemm_path(p.wx_stride, nb1 - nb0);
+    // One wx row, FP64: the occupied bands in the band sum's frequency pass.
+    const bool fused = gemm && has_flag && !mixed && !want_n1 && p.nv <= kRowsOccupiedMax;
     const long long rows_f = has_flag ? ceil_div(p.ng, fs.rg) : 0;
     const long long rows_n = has_noflag ? ceil_div(p.ng, ns.rg) : 0;
-    const long long tiles_f = has_flag ? rows_f * (fb1 - fb0) : 0;
+    const long long tiles_f = fused ? rows_f * gemm_row_parts(p) : has_flag ? rows_f * (fb1 - fb0) : 0;
     // The GEMM path writes one partial per row tile (all bands at once).
     const long long tiles_n =
-        !has_noflag ? 0 : gemm ? rows_n : rows_n * ceil_div(nb1 - nb0, ns.rn);
+        !has_noflag || fused ? 0 : gemm ? rows_n : rows_n * ceil_div(nb1 - nb0, ns.rn);
     st = check_grid_limits(p, has_flag ? fb1 - fb0 : 0, has_noflag ? nb1 - nb0 : 0, ns, gemm);
     if (st != GPP_OK) return st;
     if (has_flag && fb0 != 0)
@@ -363,7 +365,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const long long chunks = ceil_div(p.nw, ns.nwc);
     const bool small = tiles_f * ceil_div(p.nw, fs.nwc) + tiles_n * chunks <= 2 * sm_count();
     const bool overlap =
-        has_flag && has_noflag && !pieces &&
+        has_flag && has_noflag && !pieces && !fused &&
         (gemm && tensor ? overlap_tensor_gemm() : small || (mixed && overlap_occupied()));
     // FP64 with the per-band output: the occupied-band kernel starts once the
     // tensor-core band sum's slicing passes are queued rather than with them
@@ -391,13 +393,13 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
         if (e == cudaSuccess && mixed) e = launch_split_rows(p, w + o_split, rt, s);
         if (e == cudaSuccess && overlap && !late_fork)
             e = cudaEventRecord(side->fork, s);  // planes written
-        if (e == cudaSuccess && has_flag && !overlap) {
+        if (e == cudaSuccess && has_flag && !overlap && !fused) {
             part.ach_tile0 = 0;
             e = mixed ? launch_flag_mixed(p, part, w + o_split, s, rt)
                       : launch_flag_fp64(p, part, s, rt);
         }
         if (e == cudaSuccess && has_noflag) {
-            part.ach_tile0 = (int)tiles_f;
+            part.ach_tile0 = fused ? 0 : (int)tiles_f;
             if (k == 0 && t_timing && t_ev0) cudaEventRecord(t_ev0, s);
             if (gemm && mixed) {
                 st = GPP_OK;
@@ -424,7 +426,9 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
                 if (k == 0)
                     st = gemm_band_sum(p, part, w + o_gemm, nb0, nb1, s,
                                        late_fork ? side->fork : nullptr);
-                if (st == GPP_OK) st = gemm_rows(p, part, w + o_gemm, nb0, nb1, s, rt);
+                if (st == GPP_OK)
+                    st = fused ? gemm_rows_occupied(p, part, w + o_gemm, nb0, nb1, s, rt)
+                               : gemm_rows(p, part, w + o_gemm, nb0, nb1, s, rt);
                 if (st == GPP_OK && k == pc.n - 1) st = gemm_per_band(p, part, w + o_gemm, nb0, nb1, s);
                 if (st != GPP_OK) {
                     cudaFreeAsync(ws, s);

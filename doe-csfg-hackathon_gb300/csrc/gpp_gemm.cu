@@ -38,6 +38,7 @@
 #include "gpp_gemm.h"
 #include "gpp_gemm_mixed.h"
 #include "gpp_ozaki.h"
+#include "gpp_tiles_fp64.cuh"
 
 namespace gpp {
 
@@ -274,6 +275,116 @@ __global__ void __launch_bounds__(kThreads) gemm_epilogue_kernel(Problem p, Part
     }
 }
 
+// The frequency pass with the occupied bands in it: with one wx row their
+// solver (flag_term) depends on the row, the column and the frequency only, so
+// their band sum G_occ = sum c aqsn, formed here, takes its place beside G:
+// a branch-A term adds (G + G_occ) Q conj(wdiff) / |wdiff|^2 to achtemp and
+// G_occ Omega2 to asxtemp with one reciprocal for both; other branches add G's
+// term alone to achtemp and what flag_ssx gives to asxtemp.  One block per row
+// tile (rows 2j, 2j + 1), part of the columns and frequency chunk; the rows'
+// weights are in G, so both rows share the accumulators.
+// Bound by the FP64 pipe: 74 instructions per (row, column) at two bands and
+// three frequencies, where the occupied-band kernel takes 86 and
+// gemm_epilogue_kernel 45.
+constexpr int kOccThreads = 128;
+template <int NWC, int SEM>
+__global__ void __launch_bounds__(kOccThreads) gemm_occupied_kernel(Problem p, Partials part,
+                                                                    const double2 *G, int row_tile0,
+                                                                    int parts, int len) {
+    constexpr int K = NWC * 4;
+    __shared__ double red[(kOccThreads / 32) * K];
+    __shared__ double S[K];
+    __shared__ double2 C[kRowsOccupiedMax][2];
+    const int row_tile = row_tile0 + blockIdx.x / parts, at = blockIdx.x % parts;
+    const int iw0 = blockIdx.y * NWC, nc = p.nc, nv = p.nv;
+    for (int i = threadIdx.x; i < 2 * nv; i += kOccThreads) {
+        const int r = row_tile * 2 + (i & 1);
+        const int igp = r < p.ng ? resolve_igp(p, r, part.err) : -1;
+        double2 c = make_double2(0.0, 0.0);
+        if (igp >= 0) {
+            const double2 m = __ldg(p.aqsm + (size_t)(i >> 1) * nc + igp);
+            c = cscale(make_double2(0.5 * m.x, -0.5 * m.y), __ldg(p.vcoul + igp));
+        }
+        C[i >> 1][i & 1] = c;
+    }
+    FlagFreq f[NWC];
+    double bound = kFlagNoBound;
+    bool any_most = false;
+#pragma unroll
+    for (int w = 0; w < NWC; ++w) {
+        f[w] = flag_freq<SEM>(__ldg(p.wx + min(iw0 + w, p.nw - 1)));
+        bound = flag_bound(bound, f[w]);
+        any_most |= f[w].most;
+    }
+    double2 acc[NWC], y[NWC][1], all = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int w = 0; w < NWC; ++w) acc[w] = y[w][0] = make_double2(0.0, 0.0);
+    __syncthreads();
+    const int rows = min(2, p.ng - row_tile * 2);
+    const int end = min(nc, (at + 1) * len);
+    for (int ig = at * len + threadIdx.x; ig < end; ig += kOccThreads) {
+        double2 o[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll 2
+        for (int n = 0; n < nv; ++n) {
+            const double2 a = __ldg(p.aqsn + (size_t)n * nc + ig);
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                const double2 c = C[n][g];
+                o[g].x = fma(c.x, a.x, fma(-c.y, a.y, o[g].x));
+                o[g].y = fma(c.x, a.y, fma(c.y, a.x, o[g].y));
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            if (g >= rows) continue;
+            const size_t i = (size_t)(row_tile * 2 + g) * nc + ig;
+            const double2 wt = __ldg(p.wt + i), ie = __ldg(p.ieps + i), u = __ldg(G + i);
+            const double2 a[1] = {o[g]};
+            double2 A[1], Aw[1], B[1];
+            double wti2, awt2;
+            flag_products<1>(wt, ie, a, wti2, awt2, A, Aw, B);
+            const double2 Q = cmul_rn(wt, ie);
+            const double2 T = cmul_rn(make_double2(u.x + o[g].x, u.y + o[g].y), Q);
+            const double2 Tw = cscale_rn(T, wt.y);
+            // Inf and NaN compare above the bound.
+            const bool in_all = (unsigned long long)__double_as_longlong(awt2) <=
+                                (unsigned long long)__double_as_longlong(bound);
+            if (any_most && in_all) all = make_double2(all.x + B[0].x, all.y + B[0].y);
+#pragma unroll
+            for (int w = 0; w < NWC; ++w) {
+                const FlagSolve s = flag_solve(f[w], wt, wti2, awt2);
+                if (s.in_a) {
+                    flag_sch(s, T, Tw, acc[w]);
+                } else {
+                    const double2 U = cmul_rn(u, Q);
+                    flag_sch(s, U, cscale_rn(U, wt.y), acc[w]);
+                }
+                flag_ssx<1>(f[w], s, in_all, wt, wti2, awt2, A, Aw, B, y[w]);
+            }
+        }
+    }
+    double v[K];
+#pragma unroll
+    for (int w = 0; w < NWC; ++w) {
+        double2 t = y[w][0];
+        if (f[w].most) t = make_double2(t.x + all.x, t.y + all.y);
+        v[w * 4] = acc[w].x;
+        v[w * 4 + 1] = acc[w].y;
+        v[w * 4 + 2] = flag_ssx_scale(f[w].c, t.x);
+        v[w * 4 + 3] = flag_ssx_scale(f[w].c, t.y);
+    }
+    block_reduce<K, kOccThreads>(v, red, S);
+    const int w = threadIdx.x >> 1, asx = threadIdx.x & 1;
+    if (w < NWC && iw0 + w < p.nw) {
+        const double2 t = make_double2(S[w * 4 + 2 * asx], S[w * 4 + 2 * asx + 1]);
+        const long long slot = (long long)row_tile * parts + at;
+        if (asx)  // c has 0.5 vcoul; asxtemp takes occ vcoul
+            part.asx[(long long)(iw0 + w) * part.asx_seg + slot] = cscale(t, 2.0 * p.occ);
+        else
+            part.ach[(long long)(iw0 + w) * part.ach_seg + slot] = t;
+    }
+}
+
 // M_2[r][ig] = Q conj(wdiff) / |wdiff|^2 at iw = 2, rows [r0, r1).
 __global__ void __launch_bounds__(kThreads) gemm_m2_kernel(Problem p, int r0, int r1, double2 *M) {
     const size_t nc = (size_t)p.nc;
@@ -335,8 +446,33 @@ cudaError_t launch_epilogue_t(const Problem &p, const Partials &part, const doub
     return cudaGetLastError();
 }
 
+// Columns per part, a multiple of the block.
+int row_part_length(const Problem &p) {
+    return ceil_div(ceil_div(p.nc, gemm_row_parts(p)), kOccThreads) * kOccThreads;
+}
+
+template <int NWC>
+cudaError_t launch_occupied_t(const Problem &p, const Partials &part, const double2 *G, RowTiles r,
+                              cudaStream_t s) {
+    const int parts = gemm_row_parts(p), len = row_part_length(p);
+    dim3 grid((unsigned)((r.end - r.begin) * parts), (unsigned)ceil_div(p.nw, NWC));
+    if (p.semantics == kSemKerSeq)
+        gemm_occupied_kernel<NWC, kSemKerSeq><<<grid, kOccThreads, 0, s>>>(p, part, G, r.begin, parts, len);
+    else
+        gemm_occupied_kernel<NWC, kSemComplexSeq><<<grid, kOccThreads, 0, s>>>(p, part, G, r.begin, parts, len);
+    count_launch();
+    return cudaGetLastError();
+}
 
 }  // namespace
+
+// Parts of a row tile's columns: at least two (819 row tiles on 152 SMs: whole
+// rows leave a last round 40% full), more where few rows would leave SMs idle,
+// down to 1024 columns a part.
+int gemm_row_parts(const Problem &p) {
+    const int tiles = std::max(1, ceil_div(p.ng, 2));
+    return std::max(1, std::min(std::max(2, ceil_div(1216, tiles)), p.nc / 1024));
+}
 
 // Scratch of the tensor-core GEMMs: G's, then (reused) H's.
 size_t ozaki_scratch(const Problem &p, int bands, bool want_n1) {
@@ -423,6 +559,22 @@ gpp_status gemm_rows(const Problem &p, const Partials &part, void *ws, int b0, i
         default: e = launch_epilogue_t<8>(p, part, b.G, rt, s); break;
     }
     if (e != cudaSuccess) return cuda_fail(e, "gemm_epilogue_kernel");
+    return GPP_OK;
+}
+
+gpp_status gemm_rows_occupied(const Problem &p, const Partials &part, void *ws, int b0, int b1,
+                              cudaStream_t s, RowTiles rows) {
+    const RowTiles rt = rows.clip(ceil_div(p.ng, 2));
+    if (rt.end <= rt.begin || b1 <= b0) return GPP_OK;
+    const GemmBuffers b = carve(p, ws, b1 - b0, part.n1 != nullptr);
+    cudaError_t e;
+    switch (flag_nwc(p.nw)) {
+        case 1: e = launch_occupied_t<1>(p, part, b.G, rt, s); break;
+        case 2: e = launch_occupied_t<2>(p, part, b.G, rt, s); break;
+        case 3: e = launch_occupied_t<3>(p, part, b.G, rt, s); break;
+        default: e = launch_occupied_t<4>(p, part, b.G, rt, s); break;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "gemm_occupied_kernel");
     return GPP_OK;
 }
 

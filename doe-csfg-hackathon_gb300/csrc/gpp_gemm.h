@@ -32,6 +32,14 @@ gpp_status gemm_band_sum(const Problem &p, const Partials &part, void *ws, int b
                          cudaStream_t s, cudaEvent_t after_slices = nullptr);
 gpp_status gemm_rows(const Problem &p, const Partials &part, void *ws, int b0, int b1,
                      cudaStream_t s, RowTiles rows = RowTiles());
+// 2b. gemm_rows_occupied, in place of gemm_rows and the occupied-band kernel:
+//     the occupied bands [0, p.nv) in the same pass, no per-band output.  Each
+//     row tile leaves gemm_row_parts(p) achtemp and asxtemp partials (slot
+//     row tile * parts + part); part.ach_tile0 is 0.
+constexpr int kRowsOccupiedMax = 64;  // occupied bands it takes
+int gemm_row_parts(const Problem &p);
+gpp_status gemm_rows_occupied(const Problem &p, const Partials &part, void *ws, int b0, int b1,
+                              cudaStream_t s, RowTiles rows = RowTiles());
 // split_ws: the mixed path's split planes; M_2 is then formed in float-float
 // from them (mixed_m2_fp64) instead of in FP64.
 gpp_status gemm_per_band(const Problem &p, const Partials &part, void *ws, int b0, int b1,

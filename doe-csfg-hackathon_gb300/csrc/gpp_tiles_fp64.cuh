@@ -230,23 +230,31 @@ __device__ __forceinline__ double flag_ssx_scale(double c, double y) {
 // 16384, two bands, 3 frequencies: 2.3 ms, the pipe 87% busy.  Every rounding
 // is explicit, so a band gives the same bits alone and beside another one.
 // in_all: whether the sum over all columns holds this one.
+struct FlagSolve {
+    double wr, rden, delwr;  // Re(wdiff) (Im(wdiff) = -Im(wtilde)), 1 / |wdiff|^2, |delw|^2
+    bool in_a;
+};
+__device__ __forceinline__ FlagSolve flag_solve(const FlagFreq &f, double2 wt, double wti2,
+                                                double awt2) {
+    FlagSolve s;
+    s.wr = __dsub_rn(f.wx, wt.x);
+    const double d = __fma_rn(s.wr, s.wr, wti2);
+    s.rden = rcp_fp64(d);
+    s.delwr = __dmul_rn(awt2, s.rden);
+    s.in_a = pos_gt(d, kLimitTwo) && pos_lt(s.delwr, kLimitOne);
+    return s;
+}
+// acc += A conj(wdiff) / |wdiff|^2, with Aw = A Im(wtilde).
+__device__ __forceinline__ void flag_sch(const FlagSolve &s, double2 A, double2 Aw, double2 &acc) {
+    acc.x = __fma_rn(s.rden, __fma_rn(A.x, s.wr, -Aw.y), acc.x);
+    acc.y = __fma_rn(s.rden, __fma_rn(A.y, s.wr, Aw.x), acc.y);
+}
 template <int NB>
-__device__ __forceinline__ void flag_term(const FlagFreq &f, bool in_all, double2 wt, double wti2,
-                                          double awt2, const double2 (&A)[NB], const double2 (&Aw)[NB],
-                                          const double2 (&B)[NB], double2 (&acc_s)[NB],
-                                          double2 (&y)[NB]) {
-    const double wr = __dsub_rn(f.wx, wt.x);  // Re(wdiff); Im(wdiff) = -Im(wtilde)
-    const double rden = rcp_fp64(__fma_rn(wr, wr, wti2));
-    const double delwr = __dmul_rn(awt2, rden);
-    const bool in_a = pos_gt(__fma_rn(wr, wr, wti2), kLimitTwo) && pos_lt(delwr, kLimitOne);
-    if (in_a) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            acc_s[b].x = __fma_rn(rden, __fma_rn(A[b].x, wr, -Aw[b].y), acc_s[b].x);
-            acc_s[b].y = __fma_rn(rden, __fma_rn(A[b].y, wr, Aw[b].x), acc_s[b].y);
-        }
-    }
-    const bool inc = in_a && !(f.cut && pos_gt(awt2, __dmul_rn(4.0, f.c)));
+__device__ __forceinline__ void flag_ssx(const FlagFreq &f, const FlagSolve &s, bool in_all,
+                                         double2 wt, double wti2, double awt2,
+                                         const double2 (&A)[NB], const double2 (&Aw)[NB],
+                                         const double2 (&B)[NB], double2 (&y)[NB]) {
+    const bool inc = s.in_a && !(f.cut && pos_gt(awt2, __dmul_rn(4.0, f.c)));
     const bool base = f.most && in_all;
     if (inc != base) {  // a branch-A term to add, or one to take off the sum over all columns
 #pragma unroll
@@ -255,7 +263,7 @@ __device__ __forceinline__ void flag_term(const FlagFreq &f, bool in_all, double
             y[b].y = __dadd_rn(y[b].y, flip(B[b].y, base));
         }
     }
-    if (!in_a && pos_gt(delwr, kTo1)) {
+    if (!s.in_a && pos_gt(s.delwr, kTo1)) {
         const double sr = __dadd_rn(f.wx, wt.x);  // wx + wtilde = (sr, Im(wtilde))
         const double rs = rcp_fp64(__fma_rn(sr, sr, wti2));
         if (!(f.cut && pos_gt(__dmul_rn(awt2, rs), 64.0))) {
@@ -267,6 +275,19 @@ __device__ __forceinline__ void flag_term(const FlagFreq &f, bool in_all, double
             }
         }
     }
+}
+
+template <int NB>
+__device__ __forceinline__ void flag_term(const FlagFreq &f, bool in_all, double2 wt, double wti2,
+                                          double awt2, const double2 (&A)[NB], const double2 (&Aw)[NB],
+                                          const double2 (&B)[NB], double2 (&acc_s)[NB],
+                                          double2 (&y)[NB]) {
+    const FlagSolve s = flag_solve(f, wt, wti2, awt2);
+    if (s.in_a) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) flag_sch(s, A[b], Aw[b], acc_s[b]);
+    }
+    flag_ssx<NB>(f, s, in_all, wt, wti2, awt2, A, Aw, B, y);
 }
 
 // The products of one (row, column) that its frequencies share: A = aqsn Q,
