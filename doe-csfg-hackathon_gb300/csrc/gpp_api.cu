@@ -290,9 +290,10 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const long long rows_f = has_flag ? ceil_div(p.ng, fs.rg) : 0;
     const long long rows_n = has_noflag ? ceil_div(p.ng, ns.rg) : 0;
     const long long tiles_f = fused ? rows_f * gemm_row_parts(p) : has_flag ? rows_f * (fb1 - fb0) : 0;
-    // The GEMM path writes one partial per row tile (all bands at once).
+    // The GEMM path writes one partial (FP64: gemm_row_parts) per row tile, all bands
+    // at once.
     const long long tiles_n =
-        !has_noflag || fused ? 0 : gemm ? rows_n : rows_n * ceil_div(nb1 - nb0, ns.rn);
+        !has_noflag || fused ? 0 : gemm ? rows_n * (mixed ? 1 : gemm_row_parts(p)) : rows_n * ceil_div(nb1 - nb0, ns.rn);
     st = check_grid_limits(p, has_flag ? fb1 - fb0 : 0, has_noflag ? nb1 - nb0 : 0, ns, gemm);
     if (st != GPP_OK) return st;
     if (has_flag && fb0 != 0)

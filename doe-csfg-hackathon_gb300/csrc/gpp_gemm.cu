@@ -197,6 +197,11 @@ constexpr int kHSplits = 8;
 constexpr int kHSplitsTensor = 1;
 int h_splits() { return fp64_gemm_on_tensor_cores() ? kHSplitsTensor : kHSplits; }
 
+struct GemmBuffers {
+    double2 *C, *G, *M2, *H;
+    void *oz;  // tensor-core GEMM scratch
+};
+
 // c[k][r] for bands b0 + k (k < K) and rows [r0, r1); rows whose G' index
 // is invalid get 0 (their fault bit is set, as in the per-term epilogue).
 __global__ void __launch_bounds__(kThreads) gemm_coeff_kernel(Problem p, int b0, int K, int r0,
@@ -216,63 +221,61 @@ __global__ void __launch_bounds__(kThreads) gemm_coeff_kernel(Problem p, int b0,
     }
 }
 
-// One block per row tile (rows 2j, 2j+1): sum over ig of M_iw G for NWC
-// frequencies from iw0, written as the row tile's block partial.
-template <int NWC>
+// One block per row tile (rows 2j, 2j+1), part of the columns and frequency
+// chunk: sum over ig of M_iw G for NWC frequencies from iw0, the block's
+// partial.  G holds the rows' weights, so both rows share the accumulators.
+// With M, the chunk of iw = 2 also stores M_2 for the per-band output, from
+// the reciprocal at hand (a pass of its own took 1.5 ms at 1638 x 32768, of
+// 5.4 together).
+template <int NWC, bool M2>
 __global__ void __launch_bounds__(kThreads) gemm_epilogue_kernel(Problem p, Partials part,
-                                                                 const double2 *G,
-                                                                 int row_tile0) {
-    constexpr int RG = 2, K = RG * NWC * 2;
+                                                                 const double2 *G, int row_tile0,
+                                                                 int parts, int len, double2 *M) {
+    constexpr int K = NWC * 2;
     __shared__ double red[(kThreads / 32) * K];
     __shared__ double S[K];
-    const int row_tile = row_tile0 + blockIdx.x;
+    const int row_tile = row_tile0 + blockIdx.x / parts, at = blockIdx.x % parts;
     const int iw0 = blockIdx.y * NWC;
     const int nc = p.nc;
     double wx[NWC];
 #pragma unroll
     for (int w = 0; w < NWC; ++w) wx[w] = __ldg(p.wx + min(iw0 + w, p.nw - 1));
-    double2 acc[RG][NWC];
+    double2 acc[NWC];
 #pragma unroll
-    for (int g = 0; g < RG; ++g)
+    for (int w = 0; w < NWC; ++w) acc[w] = make_double2(0.0, 0.0);
+    const int rows = min(2, p.ng - row_tile * 2);
+    const int end = min(nc, (at + 1) * len);
+    for (int ig = at * len + threadIdx.x; ig < end; ig += kThreads) {
 #pragma unroll
-        for (int w = 0; w < NWC; ++w) acc[g][w] = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int g = 0; g < RG; ++g) {
-        const int r = row_tile * RG + g;
-        if (r >= p.ng) continue;
-        const double2 *grow = G + (size_t)r * nc;
-        const double2 *wrow = p.wt + (size_t)r * nc;
-        const double2 *erow = p.ieps + (size_t)r * nc;
-        for (int ig = threadIdx.x; ig < nc; ig += kThreads) {
-            const double2 wt = __ldg(wrow + ig);
-            const double2 A = cmul(__ldg(grow + ig), cmul(wt, __ldg(erow + ig)));
+        for (int g = 0; g < 2; ++g) {
+            if (g >= rows) continue;
+            const size_t i = (size_t)(row_tile * 2 + g) * nc + ig;
+            const double2 wt = __ldg(p.wt + i);
+            const double2 Q = cmul(wt, __ldg(p.ieps + i));
+            const double2 A = cmul(__ldg(G + i), Q);
             const double ayw = A.y * wt.y, axw = A.x * wt.y, wti2 = wt.y * wt.y;
 #pragma unroll
             for (int w = 0; w < NWC; ++w) {
                 const double wr = wx[w] - wt.x;        // Re(wdiff); Im(wdiff) = -Im(wtilde)
                 const double rr = rcp_fp64(fma(wr, wr, wti2));
-                acc[g][w].x = fma(rr, fma(A.x, wr, -ayw), acc[g][w].x);
-                acc[g][w].y = fma(rr, fma(A.y, wr, axw), acc[g][w].y);
+                acc[w].x = fma(rr, fma(A.x, wr, -ayw), acc[w].x);
+                acc[w].y = fma(rr, fma(A.y, wr, axw), acc[w].y);
+                if (M2 && w == 2 % NWC && iw0 + w == 2)
+                    M[i] = make_double2(rr * fma(Q.x, wr, -Q.y * wt.y), rr * fma(Q.y, wr, Q.x * wt.y));
             }
         }
     }
     double v[K];
 #pragma unroll
-    for (int g = 0; g < RG; ++g)
-#pragma unroll
-        for (int w = 0; w < NWC; ++w) {
-            v[(g * NWC + w) * 2] = acc[g][w].x;
-            v[(g * NWC + w) * 2 + 1] = acc[g][w].y;
-        }
+    for (int w = 0; w < NWC; ++w) {
+        v[w * 2] = acc[w].x;
+        v[w * 2 + 1] = acc[w].y;
+    }
     block_reduce<K, kThreads>(v, red, S);
     const int w = threadIdx.x;
-    if (w < NWC && iw0 + w < p.nw) {
-        double2 tot = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int g = 0; g < RG; ++g)
-            tot = cadd(tot, make_double2(S[(g * NWC + w) * 2], S[(g * NWC + w) * 2 + 1]));
-        part.ach[(long long)(iw0 + w) * part.ach_seg + part.ach_tile0 + row_tile] = tot;
-    }
+    if (w < NWC && iw0 + w < p.nw)
+        part.ach[(long long)(iw0 + w) * part.ach_seg + part.ach_tile0 + (long long)row_tile * parts + at] =
+            make_double2(S[w * 2], S[w * 2 + 1]);
 }
 
 // The frequency pass with the occupied bands in it: with one wx row their
@@ -385,22 +388,6 @@ __global__ void __launch_bounds__(kOccThreads) gemm_occupied_kernel(Problem p, P
     }
 }
 
-// M_2[r][ig] = Q conj(wdiff) / |wdiff|^2 at iw = 2, rows [r0, r1).
-__global__ void __launch_bounds__(kThreads) gemm_m2_kernel(Problem p, int r0, int r1, double2 *M) {
-    const size_t nc = (size_t)p.nc;
-    const size_t n = (size_t)(r1 - r0) * nc;
-    const double wx = __ldg(p.wx + 2);
-    for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * kThreads) {
-        const size_t at = (size_t)r0 * nc + i;
-        const double2 wt = __ldg(p.wt + at);
-        const double2 Q = cmul(wt, __ldg(p.ieps + at));
-        const double wr = wx - wt.x;
-        const double rr = rcp_fp64(fma(wr, wr, wt.y * wt.y));
-        M[at] = make_double2(rr * fma(Q.x, wr, -Q.y * wt.y), rr * fma(Q.y, wr, Q.x * wt.y));
-    }
-}
-
 // acht_n1_loc partials: band b0 + k, row tile j: sum over the tile's rows of
 // c[k][r] H[k][r], H being the sum of the per-band GEMM's k splits (added in
 // split order).
@@ -437,18 +424,22 @@ int grid_for(long long n) {
 
 int nwc_of(int nw) { return nw <= 4 ? nw : 8; }
 
-template <int NWC>
-cudaError_t launch_epilogue_t(const Problem &p, const Partials &part, const double2 *G, RowTiles r,
-                              cudaStream_t s) {
-    dim3 grid((unsigned)(r.end - r.begin), (unsigned)ceil_div(p.nw, NWC));
-    gemm_epilogue_kernel<NWC><<<grid, kThreads, 0, s>>>(p, part, G, r.begin);
-    count_launch();
-    return cudaGetLastError();
-}
-
 // Columns per part, a multiple of the block.
 int row_part_length(const Problem &p) {
     return ceil_div(ceil_div(p.nc, gemm_row_parts(p)), kOccThreads) * kOccThreads;
+}
+
+template <int NWC>
+cudaError_t launch_epilogue_t(const Problem &p, const Partials &part, const GemmBuffers &b, RowTiles r,
+                              cudaStream_t s) {
+    const int parts = gemm_row_parts(p), len = row_part_length(p);
+    dim3 grid((unsigned)((r.end - r.begin) * parts), (unsigned)ceil_div(p.nw, NWC));
+    if (b.M2)
+        gemm_epilogue_kernel<NWC, true><<<grid, kThreads, 0, s>>>(p, part, b.G, r.begin, parts, len, b.M2);
+    else
+        gemm_epilogue_kernel<NWC, false><<<grid, kThreads, 0, s>>>(p, part, b.G, r.begin, parts, len, nullptr);
+    count_launch();
+    return cudaGetLastError();
 }
 
 template <int NWC>
@@ -468,10 +459,10 @@ cudaError_t launch_occupied_t(const Problem &p, const Partials &part, const doub
 
 // Parts of a row tile's columns: at least two (819 row tiles on 152 SMs: whole
 // rows leave a last round 40% full), more where few rows would leave SMs idle,
-// down to 1024 columns a part.
+// down to 512 columns a part.
 int gemm_row_parts(const Problem &p) {
     const int tiles = std::max(1, ceil_div(p.ng, 2));
-    return std::max(1, std::min(std::max(2, ceil_div(1216, tiles)), p.nc / 1024));
+    return std::max(1, std::min(std::max(2, ceil_div(1216, tiles)), p.nc / 512));
 }
 
 // Scratch of the tensor-core GEMMs: G's, then (reused) H's.
@@ -491,11 +482,6 @@ size_t gemm_bytes(const Problem &p, int bands, bool want_n1) {
 }
 
 namespace {
-
-struct GemmBuffers {
-    double2 *C, *G, *M2, *H;
-    void *oz;  // tensor-core GEMM scratch
-};
 
 GemmBuffers carve(const Problem &p, void *ws, int K, bool want_n1) {
     const size_t ng = (size_t)p.ng, nc = (size_t)p.nc;
@@ -552,11 +538,11 @@ gpp_status gemm_rows(const Problem &p, const Partials &part, void *ws, int b0, i
     const GemmBuffers b = carve(p, ws, b1 - b0, part.n1 != nullptr);
     cudaError_t e;
     switch (nwc_of(p.nw)) {
-        case 1: e = launch_epilogue_t<1>(p, part, b.G, rt, s); break;
-        case 2: e = launch_epilogue_t<2>(p, part, b.G, rt, s); break;
-        case 3: e = launch_epilogue_t<3>(p, part, b.G, rt, s); break;
-        case 4: e = launch_epilogue_t<4>(p, part, b.G, rt, s); break;
-        default: e = launch_epilogue_t<8>(p, part, b.G, rt, s); break;
+        case 1: e = launch_epilogue_t<1>(p, part, b, rt, s); break;
+        case 2: e = launch_epilogue_t<2>(p, part, b, rt, s); break;
+        case 3: e = launch_epilogue_t<3>(p, part, b, rt, s); break;
+        case 4: e = launch_epilogue_t<4>(p, part, b, rt, s); break;
+        default: e = launch_epilogue_t<8>(p, part, b, rt, s); break;
     }
     if (e != cudaSuccess) return cuda_fail(e, "gemm_epilogue_kernel");
     return GPP_OK;
@@ -587,12 +573,7 @@ gpp_status gemm_per_band(const Problem &p, const Partials &part, void *ws, int b
     if (split_ws) {
         const gpp_status st = mixed_m2_fp64(p, split_ws, b0, b.M2, s);
         if (st != GPP_OK) return st;
-    } else {
-        gemm_m2_kernel<<<grid_for((long long)p.ng * p.nc), kThreads, 0, s>>>(p, 0, p.ng, b.M2);
-        count_launch();
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(e, "gemm_m2_kernel");
-    }
+    }  // FP64: gemm_rows has written M_2
     // H (K x ng) = aqsn M_2^T: X(k', ig) = aqsn[b0 + k'][ig], Y(r, ig) = M_2[r][ig],
     // the ncouls sum split up to h_splits() ways.
     int splits;

@@ -21,8 +21,9 @@ size_t gemm_bytes(const Problem &p, int bands, bool want_n1);
 // steps on stream s, each over every G' row so that the results do not
 // depend on how a caller splits the rows:
 //  1. gemm_band_sum: c and G = sum_n1 c aqsn (needs the band arrays only);
-//  2. gemm_rows: for row tiles `rows`, the achtemp partial of each row tile
-//     (slot part.ach_tile0 + row tile) -- needs those rows' wtilde/I_eps;
+//  2. gemm_rows: for row tiles `rows`, gemm_row_parts(p) achtemp partials of
+//     each row tile (slot part.ach_tile0 + row tile * parts + part) and, when
+//     part.n1 is set, M_2 for step 3 -- needs those rows' wtilde/I_eps;
 //  3. gemm_per_band: when part.n1 is set (nw >= 3), the per-band partials
 //     of acht_n1_loc -- needs every row.
 // `ws` holds gemm_bytes(p, b1 - b0, part.n1 != nullptr).
