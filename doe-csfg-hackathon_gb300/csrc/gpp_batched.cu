@@ -116,6 +116,7 @@ batched_flag_mixed_kernel(const Problem *probs, const Partials *parts, const Spl
     constexpr int KF = FRG * NWC * 4;
     __shared__ double red[(kThreads / 32) * KF];
     __shared__ double S[KF];
+    __shared__ float4 stage[kFlagStages * kFlagLoads * kThreads];
     __shared__ int s_item;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(head, 1);
@@ -129,10 +130,10 @@ batched_flag_mixed_kernel(const Problem *probs, const Partials *parts, const Spl
         const SplitPlanes sp = splits[bi.state];
         if (p.semantics == kSemKerSeq)
             flag_mixed_tile<FRG, NWC, kThreads, kSemKerSeq>(p, part, sp, bi.row_tile, bi.band_tile,
-                                                            bi.iw_chunk, bi.tile, red, S);
+                                                            bi.iw_chunk, bi.tile, red, S, stage);
         else
             flag_mixed_tile<FRG, NWC, kThreads, kSemComplexSeq>(
-                p, part, sp, bi.row_tile, bi.band_tile, bi.iw_chunk, bi.tile, red, S);
+                p, part, sp, bi.row_tile, bi.band_tile, bi.iw_chunk, bi.tile, red, S, stage);
         __syncthreads();
     }
 }

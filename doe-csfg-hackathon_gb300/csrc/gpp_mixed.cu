@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(THREADS, 3)
 flag_mixed_kernel(Problem p, Partials part, SplitPlanes s, int row_tile0, int count,
                   int row_tiles, int *next) {
     constexpr int K = RG * NWC * 4;
+    __shared__ float4 stage[kFlagStages * kFlagLoads * THREADS];
     __shared__ double red[(THREADS / 32) * K];
     __shared__ double S[K];
     __shared__ int item;
@@ -303,7 +304,7 @@ flag_mixed_kernel(Problem p, Partials part, SplitPlanes s, int row_tile0, int co
         for (int z = blockIdx.z; z < chunks; z += gridDim.z) {
             flag_mixed_tile<RG, NWC, THREADS, SEM>(p, part, s, row_tile, blockIdx.y, z,
                                                    (long long)blockIdx.y * row_tiles + row_tile,
-                                                   red, S);
+                                                   red, S, stage);
             __syncthreads();  // S read by the epilogue before the next chunk
         }
         return;
@@ -320,7 +321,7 @@ flag_mixed_kernel(Problem p, Partials part, SplitPlanes s, int row_tile0, int co
         const long long rest = it / count;
         const int band = (int)(rest % p.nv);
         flag_mixed_tile<RG, NWC, THREADS, SEM>(p, part, s, row_tile, band, (int)(rest / p.nv),
-                                               (long long)band * row_tiles + row_tile, red, S);
+                                               (long long)band * row_tiles + row_tile, red, S, stage);
         __syncthreads();  // S read by the epilogue, `item` by every thread, before reuse
     }
 }
