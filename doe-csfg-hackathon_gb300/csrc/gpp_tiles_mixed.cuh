@@ -598,8 +598,9 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
         const df2 qi = {f2(vqi.x, vqi.y), f2(vqi.z, vqi.w)};
         const df2 wti2 = df2_sqr(wti);
         const df2 awt2 = df2_add(df2_sqr(wtr), wti2);                  // |wtilde|^2
-        const df2 Ar = df2_sub(df2_mul(ar, qr), df2_mul(ai, qi));      // A = aqsn Q
-        const df2 Ai = df2_add(df2_mul(ar, qi), df2_mul(ai, qr));
+        // A = aqsn Q, normalised: its products drop l l.
+        const df2 Ar = df2_norm(df2_sub(df2_mul(ar, qr), df2_mul(ai, qi)));
+        const df2 Ai = df2_norm(df2_add(df2_mul(ar, qi), df2_mul(ai, qr)));
         const df2 Ai_wti = df2_mul(Ai, wti), Ar_wti = df2_mul(Ar, wti);
         const df2 Br = df2_sub(df2_mul(Ar, wtr), Ai_wti);              // aqsn Omega2 = A wtilde
         const df2 Bi = df2_add(df2_mul(Ai, wtr), Ar_wti);
