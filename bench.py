@@ -114,6 +114,18 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
+# With per-band frequencies a large call sums its unoccupied bands through the
+# series of gpp_far.cu: `kernel_ms` then covers these kernels together, and the
+# flops counted are those of the per-term sum they replace.
+SERIES_KERNELS = {
+    "mixed": "near_mixed_kernel, crt_gemm_kernel, far_terms_kernel, crt_combine_kernel, far_out_kernel",
+    "fp64": "far_near_fp64_kernel, crt_gemm_kernel, far_terms_kernel, crt_combine_kernel, far_out_kernel"}
+SERIES_NOTE = ("flops of the per-term sum over the time of the kernels that replace it (tensor-core "
+               "products of a series, and the per-term kernel where wx is near wtilde): a "
+               "fraction above 1 is work not done, not a rate; profiles/ncu_series_profile.txt "
+               "has each kernel's own")
+
+
 def profile_traffic(kernel: str, workload: str, precision: str):
     """DRAM bytes (read + write) per launch of `kernel` at `workload`, from the
     ncu launch-list summary committed in profiles/ (None when not captured)."""
@@ -337,7 +349,7 @@ def band_independent_leg(d, shape: W.Shape, steps: int) -> dict:
         legs[key]["achtemp_max_rel_err_vs_per_term_fp64"] = float(
             np.max(np.abs(g2 - w2) / np.where(w2 == 0, 1.0, np.abs(w2))))
     return {"wx": "band 0's frequencies for every band (the reference's wx_array[3])",
-            "band_sum": "tcgen05 tensor-core GEMM, operands cut into exact bf16 integer slices",
+            "band_sum": "tcgen05 tensor-core GEMM of exact residues (bf16 integers)",
             "steps": steps, **legs}
 
 
@@ -559,6 +571,7 @@ def main() -> int:
     clocks = ClockSampler(local)
     clocks.start()
     res, ms, kern_ms, launches = timed(precision, args.steps, args.warmup)
+    series = launches > 20 * args.steps  # a per-term call makes fewer than ten launches
     clk = clocks.stop()
 
     fp64_leg = None
@@ -598,7 +611,9 @@ def main() -> int:
             a64 = unocc_terms * (FLOPS_PER_TERM_BASE + FLOPS_PER_TRIPLE / shape.nw) / (k64ms * 1e-3)
             fp64_leg["roofline"] = {"bound": "fp64", "achieved": a64 * 1e-12, "peak": fp64_peak,
                                     "unit": "TFLOP/s", "frac": a64 * 1e-12 / fp64_peak,
-                                    "kernel": "noflag_fp64_kernel"}
+                                    "kernel": SERIES_KERNELS["fp64"] if series else "noflag_fp64_kernel"}
+            if series:
+                fp64_leg["roofline"]["note"] = SERIES_NOTE
 
     # End to end through the host-buffer C-ABI call: pinned host inputs
     # (which the library pulls with a kernel on the SMs, overlapped with the
@@ -635,14 +650,14 @@ def main() -> int:
     peak = fp32_peak if precision == "mixed" else fp64_peak
     achieved = flops / (kms * 1e-3) * 1e-12 if kms else None
     kname = "mixed_noflag_kernel" if precision == "mixed" else "noflag_fp64_kernel"
-    traffic = profile_traffic(kname, args.workload, precision)
+    traffic = None if series else profile_traffic(kname, args.workload, precision)
     pipe_file = "ncu_noflag_mixed_profile.txt" if precision == "mixed" else "ncu_noflag_fp64_profile.txt"
     # Pipe busy cycles: a packed f32x2 instruction occupies the FMA pipe for
     # two cycles, so instruction counts understate its load.
     pipe_metric = "sm__pipe_fma_cycles_active" if precision == "mixed" else "sm__inst_executed_pipe_fp64"
-    pipe_pct = profile_pipe(pipe_file, pipe_metric)
+    pipe_pct = None if series else profile_pipe(pipe_file, pipe_metric)
     issued = None
-    if precision == "mixed" and kms and fp32_peak:
+    if precision == "mixed" and kms and fp32_peak and not series:
         ops = mixed_fp32_ops_per_term(shape.nw if shape.nw <= 4 else 8)
         rate = ops * unocc_terms / (kms * 1e-3)  # FP32 operations per second
         issued = {"fp32_ops_per_term": ops, "achieved_tops": rate * 1e-12,
@@ -665,6 +680,10 @@ def main() -> int:
                 "fp64_fma_peak_tflops": fp64_peak, "fp32_fma_peak_tflops": fp32_peak}
     if issued:
         roofline["issued"] = issued
+    if series:
+        roofline["kernel"], roofline["note"] = SERIES_KERNELS[precision], SERIES_NOTE
+        for k in ("ncu_pipe_note", "traffic_note"):
+            roofline.pop(k)
 
     line = {"metric": METRIC, "value": job_terms / (ms * 1e-3), "unit": "terms/s",
             "n_gpus": ws, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,

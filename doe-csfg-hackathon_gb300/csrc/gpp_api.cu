@@ -369,9 +369,10 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
         has_flag && has_noflag && !pieces && !fused &&
         (gemm && tensor ? overlap_tensor_gemm() : small || (mixed && overlap_occupied()));
     // FP64 with the per-band output: the occupied-band kernel starts once the
-    // tensor-core band sum's slicing passes are queued rather than with them
-    // (measured 28.0 -> 26.5 ms per production call; without the per-band
-    // output it made calls queued back to back slower, 22.7 -> 25.7 ms).
+    // tensor-core band sum's operand pass is queued rather than with it (28.0
+    // -> 26.5 ms per production call when the GEMM took 4.6 ms; without the
+    // per-band output, now the fused pass, it made calls queued back to back
+    // slower, 22.7 -> 25.7 ms).
     const bool late_fork = overlap && gemm && tensor && !mixed && want_n1;
     RowPieces whole;
     whole.n = 1;

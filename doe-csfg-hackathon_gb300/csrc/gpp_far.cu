@@ -38,11 +38,11 @@
 // here returns at once and the per-term kernel runs instead.  No host
 // synchronisation; nothing depends on the order in which blocks run.
 //
-// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 24 ms now (near
-// pairs 15, products 3.5, terms 2.6, combine 1.5); mixed, 128 bands x 819 x 16384
-// x 32: 120 ms per term, 35 now (near 23, terms 7, products 4.3); 512 bands x
-// 1638 x 32768 x 3, 1% strays: 210 per term, 140 now (near 55, products 30,
-// terms 26, strays 15, combine 12).  The near kernels run at 1.25 (FP64) and
+// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 22 ms now (near
+// pairs 15, products 2.6, terms 2.7, combine 1.5); mixed, 128 bands x 819 x 16384
+// x 32: 120 ms per term, 34 now (near 23, terms 5.2, products 4.2); 512 bands x
+// 1638 x 32768 x 3, 1% strays: 210 per term, 122 now (near 57, products 23,
+// terms 19, strays 14, combine 13).  The near kernels run at 1.25 (FP64) and
 // 1.4 (mixed) of the per-term kernels' time per pair: an entry holds 1.8
 // frequencies on average where a tile there shares its columns among 3.
 #include <algorithm>
@@ -587,7 +587,7 @@ constexpr int kTermK = 4;  // columns per thread
 //
 // In mixed precision the recurrence runs in float-float (DF): FP64 kept its
 // pipe 62-76% busy with 4 instructions per term and column where the residues
-// take most of the issue slots.  Q is scaled by the chunk's exponent first, so
+// take most of the issue slots.  1638 x 32768, 25 terms: 26 -> 19 ms.  Q is scaled by the chunk's exponent first, so
 // its range is FP64's; only the first pass reads the inputs, the next ones
 // find z with the last two terms in `state`.
 template <int L, bool DF>

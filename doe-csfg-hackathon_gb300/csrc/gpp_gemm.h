@@ -9,8 +9,8 @@
 
 namespace gpp {
 
-// Whether this host thread's FP64 GEMMs run on the tensor cores (the Ozaki
-// split of gpp_ozaki.cu, the default) rather than on the FP64 pipe
+// Whether this host thread's FP64 GEMMs run on the tensor cores (by the
+// residues of gpp_crt.cu, the default) rather than on the FP64 pipe
 // (zgemm3m_kernel, gpp_set_gemm_path(2)).
 bool fp64_gemm_on_tensor_cores();
 
@@ -27,7 +27,7 @@ size_t gemm_bytes(const Problem &p, int bands, bool want_n1);
 //  3. gemm_per_band: when part.n1 is set (nw >= 3), the per-band partials
 //     of acht_n1_loc -- needs every row.
 // `ws` holds gemm_bytes(p, b1 - b0, part.n1 != nullptr).
-// after_slices: recorded on s once the tensor-core GEMM's slicing passes are
+// after_slices: recorded on s once the tensor-core GEMM's first operand pass is
 // queued (at the end of the call on the FP64-pipe path).
 gpp_status gemm_band_sum(const Problem &p, const Partials &part, void *ws, int b0, int b1,
                          cudaStream_t s, cudaEvent_t after_slices = nullptr);

@@ -149,8 +149,8 @@ int gpp_get_dropin_precision(void);
  * for every band the band sum factors out of the division:
  * achtemp[iw] = sum_{G',ig} M_iw G, G = sum_n1 c aqsn (one complex GEMM,
  * written in this library: in FP64 by default on the tensor cores, the
- * operands split into bf16 integer slices whose products the tensor cores
- * sum exactly (Ozaki scheme), with mode 2 as a 3M-form GEMM on the FP64
+ * operands taken as residues modulo small integers whose products the tensor
+ * cores sum exactly (Ozaki scheme II), with mode 2 as a 3M-form GEMM on the FP64
  * pipe; float-float on the FP32 pipes in mixed precision), several times
  * faster; the results agree with the per-term kernels to their rounding. */
 gpp_status gpp_set_gemm_path(int mode);
