@@ -1060,10 +1060,12 @@ bool far_eligible(const Problem &p, int bands, bool mixed) {
     if (p.wx_stride == 0 || bands < 32 || p.ng < 16 || p.nc < 512) return false;
     const Sizes z = sizes(p, bands, mixed);
     // The series and, say, a sixth of the pairs near must leave a gain, on a
-    // call long enough (3 ms of per-term work) for the fixed launches.
+    // call long enough for the fixed launches: 3 ms of per-term work, in FP64
+    // 2.2 (per term / series, ms, at estimates of 1.3, 1.7, 2.5 and 2.8 ms: 1.48
+    // / 1.81, 1.86 / 1.91, 2.97 / 2.26, 2.88 / 2.08).
     const double cells = (double)p.ng * p.nc;
     const double per_pair = mixed ? 2.6e-12 : 20e-12;
-    return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > 3e-3 &&
+    return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > (mixed ? 3e-3 : 2.2e-3) &&
            z.pairs < (1 << 20) && cells < 2e9 &&
            (z.pairs / 8 + 1) * ((p.ng + 1) / 2) < (1 << 30);  // the near kernel's tile counter
 }
