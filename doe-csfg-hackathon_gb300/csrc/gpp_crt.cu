@@ -4,20 +4,21 @@
 // 2025).
 //
 //  * Over a chunk of at most 512 k values every operand value x of a row is
-//    written as x = N 2^(e - 53), e the row's largest exponent in the chunk
-//    and N a 53-bit integer;
+//    written as x = N 2^(e - 57), e the row's largest exponent in the chunk
+//    and N a 57-bit integer (the slices of gpp_ozaki.cu hold 56 bits);
 //  * the product sum of such integers is an integer X, |X| < P / 2, fixed by
-//    its residues modulo 15 pairwise coprime integers p <= 256 of product
-//    P = 2^117.78 (gpp_crt.cuh): 15 products of 8-bit integers, each exact in
-//    bf16 with FP32 accumulation, where cutting the operands into slices
-//    (gpp_ozaki.cu) takes 36 products of slice pairs;
+//    its residues modulo 16 pairwise coprime integers p <= 256 of product
+//    P = 2^125.38 (gpp_crt.cuh): 16 products of 8-bit integers, each exact in
+//    bf16 with FP32 accumulation, where the slices take 36 products of slice
+//    pairs (15 integers would do for 53 bits, 6% faster, but what falls off
+//    below the chunk's largest value is then more than the slices lost);
 //  * complex products take the 3M form (P1 = sum xr yr, P2 = sum xi yi,
 //    P3 = sum (xr + xi)(yr + yi)); re = P1 - P2 and im = P3 - P1 - P2 are
 //    formed on the residues, exactly;
 //  * the combining pass turns the residues of re and im into 2^128 X / P and
-//    rounds X 2^(ex + ey - 106) to a double; chunks are added in FP64.
+//    rounds X 2^(ex + ey - 114) to a double; chunks are added in FP64.
 //
-// So the only roundings are those of the operands (to 53 bits of the chunk's
+// So the only roundings are those of the operands (to 57 bits of the chunk's
 // largest value), of each chunk's result and of the sum over chunks: at the
 // production shape the band sums are off by 1e-15 where the slices' float-float
 // combination left 5e-15.
@@ -49,7 +50,7 @@ namespace gpp {
 namespace {
 
 constexpr int kKcMax = 512;             // k values per chunk
-constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli, at level 0
+constexpr int kPlanes = 3 * kCrtN;      // (re, im, re + im) x moduli, at the wide level
 constexpr int kTM = 128, kTN = 256;     // tcgen05.mma M (rows of X) x N (rows of Y)
 constexpr int kTK = 64;                 // k per operand block
 constexpr int kKSMax = kKcMax / kTK;    // operand blocks per chunk
@@ -157,7 +158,7 @@ struct PrepOperand {
 // Layout of a plane, in memory order: row tile (R rows), k step (kTK), row
 // group of 8, k-core of 8, row, k -- the no-swizzle K-major core-matrix layout
 // of tcgen05.mma, one contiguous block per (row tile, k step).
-// Bound by its writes (90 bytes per complex value) and the FP32 pipe.
+// Bound by its writes (6 n bytes per complex value) and the FP32 pipe.
 __global__ void __launch_bounds__(256, 2) crt_prep_kernel(PrepOperand X, PrepOperand Y, int xblocks,
                                                           int K, int Kc, int c0, int nc, int nmod,
                                                           int bits, const int *go) {
@@ -570,9 +571,9 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
 }
 
 // Out (= or +=) the pass's chunks: a thread per row and 4 consecutive
-// columns reads the 45 residue words of a chunk, forms the residues of re and
+// columns reads the 3 n residue words of a chunk, forms the residues of re and
 // im for each column, their sum of fractions (integer multiply-adds) and
-// X 2^(ex + ey - 106), and adds it to the running FP64 result, chunk by chunk.
+// X 2^(ex + ey - 2 bits), and adds it to the running FP64 result, chunk by chunk.
 // Bound by integer issue.
 template <int L>
 __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char *res, const int *EX,
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char
                 u[q] = __ldg(reinterpret_cast<const unsigned *>(f + q * plane));
             const int ex = __ldg(EX + (size_t)c * Mp + row0 + r);
             const int4 ey = __ldg(reinterpret_cast<const int4 *>(EY + (size_t)c * Np + col0));
-            // Not unrolled: the residue words take 45 registers, and one column's
+            // Not unrolled: the residue words take up to 48 registers, and one column's
             // state at a time leaves room for five blocks per SM.
 #pragma unroll 1
             for (int j = 0; j < 4; ++j) {
@@ -772,7 +773,8 @@ cudaError_t crt_combine(const unsigned char *res, const int *ex, const int *ey, 
         case 0: launch(crt_combine_kernel<0>); break;
         case 1: launch(crt_combine_kernel<1>); break;
         case 2: launch(crt_combine_kernel<2>); break;
-        default: launch(crt_combine_kernel<3>); break;
+        case 3: launch(crt_combine_kernel<3>); break;
+        default: launch(crt_combine_kernel<kCrtWide>); break;
     }
     count_launch();
     return cudaGetLastError();
@@ -806,8 +808,8 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                 const PrepOperand px{X, g.Mp, kTM, b.sx, b.ex, nullptr},
                     py{Yn, Np, kTN, b.sy, b.ey, nullptr};
                 // X's planes serve every pass over rows of Y.
-                launch_prep(px, py, n0 == 0 ? g.Mp / 8 * nc : 0, Np / 8 * nc, K, g.Kc, c0, nc, 0,
-                            nullptr, s);
+                launch_prep(px, py, n0 == 0 ? g.Mp / 8 * nc : 0, Np / 8 * nc, K, g.Kc, c0, nc,
+                            kCrtWide, nullptr, s);
                 count_launch();
                 if (after_slices && z == 0 && c0 == 0 && n0 == 0) {
                     e = cudaEventRecord(after_slices, s);
@@ -816,10 +818,10 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
                 for (int mt0 = 0; mt0 < mtiles; mt0 += g.slab_tiles) {
                     const int tiles = std::min(g.slab_tiles, mtiles - mt0);
                     const int row0 = mt0 * kTM, rows = std::min(M - row0, tiles * kTM);
-                    e = crt_products(b.sx, b.sy, g.Mp, Np, g.Kc, nc, mt0, tiles, 0, b.res, Ms,
+                    e = crt_products(b.sx, b.sy, g.Mp, Np, g.Kc, nc, mt0, tiles, kCrtWide, b.res, Ms,
                                      nullptr, nullptr, err, s);
                     if (e == cudaSuccess && rows > 0)
-                        e = crt_combine(b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, 0,
+                        e = crt_combine(b.res, b.ex, b.ey, row0, rows, Ms, Yn.L, g.Mp, Np, nc, kCrtWide,
                                         c0 > zc0, Out + z * split_stride + n0, out_ld, nullptr, nullptr, s);
                     if (e != cudaSuccess) return e;
                 }

@@ -1,5 +1,5 @@
 // gpp_crt.cuh -- the residue arithmetic of gpp_crt.cu, host and device: a
-// fixed-point operand value as residues of 15 moduli, and an exact integer
+// fixed-point operand value as residues of up to 16 moduli, and an exact integer
 // from the residues of a product sum (Chinese remainder theorem).
 #pragma once
 
@@ -10,35 +10,41 @@
 
 namespace gpp {
 
-// The 15 largest pairwise coprime integers up to 256; their product is
-// P = 2^117.78.  Symmetric residues |r| <= p / 2 <= 128 are integers that
-// bf16 holds exactly, and a sum of 512 products of two of them is at most
-// 2^23, which FP32 accumulation adds exactly.
-constexpr int kCrtN = 15;
+// The 16 largest pairwise coprime integers up to 256 (GPP_CRT_MODULI and 193);
+// the product of the first 15 is 2^117.78, of all 2^125.38.  Symmetric
+// residues |r| <= p / 2 <= 128 are integers that bf16 holds exactly, and a sum
+// of 512 products of two of them is at most 2^23, which FP32 accumulation adds
+// exactly.
+constexpr int kCrtN = 16;
 #define GPP_CRT_MODULI \
     256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197
-constexpr int kCrtModuli[kCrtN] = {GPP_CRT_MODULI};
+constexpr int kCrtModuli[kCrtN] = {GPP_CRT_MODULI, 193};
 // Levels of precision: the first n moduli with operands of `bits` bits,
-// 2 512 2^(2 bits) < P / 2 for the product P of the n.  Level 0 is FP64's.
-constexpr int kCrtLevels = 4;
+// 2 512 2^(2 bits) < P / 2 for the product P of the n.  The last, wide one
+// stands for FP64 operands: four bits more than a double's 53 for what falls
+// off below a chunk's largest value.
+constexpr int kCrtLevels = 5, kCrtWide = 4, kCrtWideBits = 57;
 struct CrtLevel {
     int n, bits;
     unsigned long long pn;  // P = pn 2^pe, its top 64 bits rounded
     int pe;
     unsigned long long off_hi, off_lo;  // below
+    unsigned zero;  // what a zero's rounding can leave of the 2^128: below
 };
 constexpr CrtLevel kCrtLevel[kCrtLevels] = {
-    {15, 53, 0xDC47122BAA0C0C41ull, 54, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFFFFFECC9200ull},
-    {12, 41, 0xDF6327787D5133B8ull, 31, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFB6A7F4B9E00ull},
-    {9, 30, 0xAA977B6D2077B785ull, 8, 0xFFFFFFFFFFFFFFFCull, 0xFFA9A1B5A960FA00ull},
-    {6, 18, 0xE06F178117000000ull, -16, 0xFFFFFFFFFDB7FD11ull, 0x05004945E2C6AA00ull}};
+    {15, 53, 0xDC47122BAA0C0C41ull, 54, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFFFFFECC9200ull, 71000000u},
+    {12, 41, 0xDF6327787D5133B8ull, 31, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFB6A7F4B9E00ull, 71000000u},
+    {9, 30, 0xAA977B6D2077B785ull, 8, 0xFFFFFFFFFFFFFFFCull, 0xFFA9A1B5A960FA00ull, 71000000u},
+    {6, 18, 0xE06F178117000000ull, -16, 0xFFFFFFFFFDB7FD11ull, 0x05004945E2C6AA00ull, 71000000u},
+    {kCrtN, kCrtWideBits, 0xA61194B2EB33153Dull, 62, 0xFFFFFFFFFFFFFFFFull, 0xFFFFFFFFFE27E800ull, 82000000u}};
 
 // The residues of a pair of moduli (p, q) enter as t = r_p a + r_q b, with
 // a = w_p q mod p q, b = w_q p mod p q and w_p = (P / p)^-1 mod p: then
 // X / P = sum over the groups of t / (p q) (mod 1) for X = r mod every
 // modulus, formed with E = round(2^128 / (p q)), least significant word first.
 // A level's off is -512 sum (a + b) E mod 2^128: t is offset by 512 (a + b) to
-// be positive.
+// be positive.  Its zero is half a unit of each E times the largest residues,
+// sum 382 (a + b) / 2, rounded up.
 constexpr int kCrtGroups = 8;
 struct CrtGroup {
     unsigned a, b, E[4];
@@ -65,7 +71,15 @@ struct CrtGroup {
      {161u, 0u, {0xEF3B3FB8u, 0x313011E2u, 0xB3FB8744u, 0x011E2EF3u}}}, \
     {{42585u, 37376u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
      {13303u, 61479u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
-     {49646u, 45448u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}}
+     {49646u, 45448u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}}, \
+    {{8415u, 57344u, {0x01010101u, 0x01010101u, 0x01010101u, 0x00010101u}}, \
+     {48945u, 39721u, {0xA0B226C6u, 0x2BC9BD16u, 0x15BEAF4Eu, 0x00010832u}}, \
+     {32535u, 1235u, {0xD7954FBDu, 0xC9000119u, 0x954FBCA2u, 0x000119D7u}}, \
+     {42872u, 55209u, {0x317BC258u, 0x9B9BA76Cu, 0xEDD3DBC1u, 0x00012D46u}}, \
+     {6810u, 28625u, {0xD9951FDCu, 0x220C9DF6u, 0x89404322u, 0x000142BEu}}, \
+     {7378u, 15387u, {0x4AF518C9u, 0x79C54F61u, 0x7F7279BAu, 0x00015AB3u}}, \
+     {27462u, 9495u, {0xC98E25D0u, 0xC687FEF9u, 0xEA710C29u, 0x00018F8Fu}}, \
+     {24125u, 22852u, {0xF069AEDEu, 0x4809A44Eu, 0x073981F1u, 0x0001B943u}}}
 constexpr CrtGroup kCrtGroup[kCrtLevels][kCrtGroups] = {GPP_CRT_GROUPS};
 
 // 1.5 2^23: a float of magnitude below 2^22 added to it is rounded to an
@@ -88,7 +102,9 @@ __host__ __device__ constexpr CrtMod crt_mod(int p) {
 }
 
 // N = d0 + d1 2^14 + d2 2^28 + d3 2^42 with d0..d2 in [-8192, 8191] and
-// |d3| <= 2^11, as floats built from their bits (no conversion instruction).
+// |d3| <= 2^11 (2^15 for |N| up to 2^57: the sum of |d| times a residue's
+// constants stays below 2^23), as floats built from their bits (no conversion
+// instruction).
 __host__ __device__ __forceinline__ void crt_digits(long long N, float (&d)[4]) {
     constexpr long long kBalance = 8192ll * (1 + (1ll << 14) + (1ll << 28));
     const long long M = N + kBalance;
@@ -201,10 +217,10 @@ __device__ __noinline__
 inline
 #endif
 double crt_value_small(bool neg, unsigned w2, unsigned w1, unsigned w0, unsigned long long pn,
-                       int e) {
+                       unsigned zero, int e) {
     unsigned long long hi = ((unsigned long long)w2 << 32) | w1, lo = (unsigned long long)w0 << 32;
     int n = 32;
-    if (w2 == 0 && w1 == 0 && w0 < 71000000u) return 0.0;  // what a zero's rounding can leave
+    if (w2 == 0 && w1 == 0 && w0 < zero) return 0.0;
     while (!(hi >> 63)) {
         hi = (hi << 1) | (lo >> 63);
         lo <<= 1;
@@ -219,11 +235,11 @@ double crt_value_small(bool neg, unsigned w2, unsigned w1, unsigned w0, unsigned
 }
 
 // X 2^e as a double, X the integer of magnitude below P / 2 with the given
-// residues at level L (bounds for level 0, where they matter most): the sum is 2^128 X / P (mod 2^128) to within 2^26.1 (the rounding
-// of the E), X to within 2^17 (a sum of that size is taken as 0) where the
-// largest products are 2^106; the top 64 bits of the fraction times P, rounded
-// to nearest.  Integer operations only, but for results outside the normal
-// range.
+// residues at level L: the sum is 2^128 X / P (mod 2^128) to within 2^26.5, at
+// the wide level 2^26.7 (the rounding of the E), X to within 2^17 where the
+// largest products are 2^106, 2^24.1 where they are 2^114 (a sum of that size
+// is taken as 0); the top 64 bits of the fraction times P, rounded to nearest.
+// Integer operations only, but for results outside the normal range.
 template <int L>
 __host__ __device__ __forceinline__ double crt_value(const CrtSum &s, int e) {
     constexpr unsigned long long pn = kCrtLevel[L].pn, off_hi = kCrtLevel[L].off_hi,
@@ -241,7 +257,7 @@ __host__ __device__ __forceinline__ double crt_value(const CrtSum &s, int e) {
     const bool neg = (int)w3 < 0;
     const unsigned x = neg ? 0xFFFFFFFFu : 0u;  // one's complement: off by one unit of 2^-128
     const unsigned v3 = w3 ^ x, v2 = w2 ^ x, v1 = w1 ^ x, v0 = w0 ^ x;
-    if (v3 == 0) return crt_value_small(neg, v2, v1, v0, pn, e);
+    if (v3 == 0) return crt_value_small(neg, v2, v1, v0, pn, kCrtLevel[L].zero, e);
 #ifdef __CUDA_ARCH__
     const int z = __clz((int)v3);
     const unsigned long long hi =

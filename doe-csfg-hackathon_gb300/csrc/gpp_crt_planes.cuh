@@ -15,7 +15,7 @@ constexpr int kExpNonFinite = 1 << 20;  // of one that holds an Inf or a NaN
 static __constant__ CrtMod c_crt_mod[kCrtN] = {
     crt_mod(256), crt_mod(255), crt_mod(253), crt_mod(251), crt_mod(247),
     crt_mod(241), crt_mod(239), crt_mod(233), crt_mod(229), crt_mod(227),
-    crt_mod(223), crt_mod(217), crt_mod(211), crt_mod(199), crt_mod(197)};
+    crt_mod(223), crt_mod(217), crt_mod(211), crt_mod(199), crt_mod(197), crt_mod(193)};
 
 // The e of frexp for the nonzero magnitude with bits b (b < 2^e).
 __device__ __forceinline__ int crt_exponent(unsigned long long b) {

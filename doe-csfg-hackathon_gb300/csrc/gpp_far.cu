@@ -95,7 +95,7 @@ constexpr size_t kPassBytes = size_t(8) << 30;
 int level_of(const Sizes &z, int k) {
     const double need = (z.mixed ? 49.0 : 53.0) - k * std::log2(z.R);
     int l = 0;
-    while (l + 1 < kCrtLevels && kCrtLevel[l + 1].bits >= need) ++l;
+    while (l + 1 < kCrtWide && kCrtLevel[l + 1].bits >= need) ++l;
     return l;
 }
 
