@@ -138,6 +138,7 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 struct Buffers {
     FarPlan *plan;
     int4 *near;
+    int *place;        // [kNearFreq bands + 1]: a band's first entry of each length
     int *rows;         // [ng + 1]: strays before each row
     int2 *out;         // (row, column)
     double2 *C;        // [bands][ng]
@@ -164,6 +165,7 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     const int Np = ceil_div((long long)z.gm * z.ngp, kCrtRowsY) * kCrtRowsY;
     o.plan = reinterpret_cast<FarPlan *>(take(sizeof(FarPlan)));
     o.near = reinterpret_cast<int4 *>(take(sizeof(int4) * (size_t)z.cap_near));
+    o.place = reinterpret_cast<int *>(take(sizeof(int) * ((size_t)kNearFreq * z.bands + 1)));
     o.rows = reinterpret_cast<int *>(take(sizeof(int) * ((size_t)z.ng + 1)));
     o.out = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)z.cap_out));
     o.C = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.ng));
@@ -293,21 +295,18 @@ __device__ __forceinline__ Box box_of(float a, float b, float v) {
     return q;
 }
 
-// One block: chooses the box and lists the near pairs in order.  The cost of
-// a box is what it leaves to the per-term kernels, in pairs over all columns:
-// its near pairs (times w_near), and the strays' share of the far ones (times
-// w_out).
+// One block: chooses the box.  The cost of a box is what it leaves to the
+// per-term kernels, in pairs over all columns: its near pairs (times w_near),
+// and the strays' share of the far ones (times w_out).
 __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int bands, FarPlan *f,
-                                                         int4 *near, int cap_near, long long cap_out,
-                                                         float R, float c0, float w_near,
-                                                         float w_out) {
+                                                         long long cap_out, float R, float c0,
+                                                         float w_near, float w_out) {
     __shared__ unsigned long long pre[kBins + 1];
     __shared__ unsigned pairs_in[kBins];
     __shared__ unsigned ppre[kBins + 1];
     __shared__ float vb[kBins];
     __shared__ unsigned long long best[kBins / 32];
-    __shared__ int scan[kBins / 32];
-    __shared__ int base, outside;
+    __shared__ int outside;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const long long n = (long long)bands * p.nw;
     const long long cells = (long long)p.ng * p.nc;
@@ -359,11 +358,8 @@ __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int 
     for (int s = 16; s > 0; s >>= 1) mine = min(mine, __shfl_xor_sync(0xffffffffu, mine, s));
     if (lane == 0) best[warp] = mine;
     __syncthreads();
-    __shared__ int go;
     if (t == 0) {
         for (int i = 1; i < kBins / 32; ++i) mine = min(mine, best[i]);
-        go = 0;
-        base = 0;
         if (mine != ~0ull && __uint_as_float((unsigned)(mine >> 32)) + c0 < 0.9f * total) {
             const int lo = (int)((unsigned)mine / kBins), hi = (int)((unsigned)mine % kBins);
             float v = 0.f;
@@ -380,54 +376,108 @@ __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int 
             const double rho = (double)q.rho * 1.00001, r = (double)R * rho;
             f->log2_rho = log2(rho);
             f->dfar = f->h * 0.5 * (r + 1.0 / r);
-            go = 1;
+            f->active = 1;
         }
     }
-    __syncthreads();
-    if (!go) return;
-    // Near pairs: counted first, then listed in order.
-    int c = 0;
-    for (long long i = t; i < n; i += kBins) c += !is_far(*f, wx_at(i));
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (lane == 0) scan[warp] = c;
-    __syncthreads();
-    if (t == 0) {
-        int s = 0;
-        for (int i = 0; i < kBins / 32; ++i) s += scan[i];
-        if (s > cap_near || s * w_near + c0 >= 0.95f * total) go = 0;
+}
+
+// An entry of the near list covers up to kNearFreq consecutive near
+// frequencies of a band: every kNearFreq-th pair of a run of them starts one.
+// A warp walks band n's frequencies and calls found(start, iw, len) for each 32
+// of them, all lanes together: whether lane's frequency iw starts an entry, and
+// of which length.
+template <class Found>
+__device__ __forceinline__ void near_runs(const Problem &p, const FarPlan &f, int band, Found found) {
+    const int lane = threadIdx.x & 31;
+    const double *wx = p.wx + (size_t)band * p.wx_stride;
+    int carry = 0;  // the run that reaches the first of these 32
+    for (int w0 = 0; w0 < p.nw; w0 += 32) {
+        const int iw = w0 + lane;
+        const unsigned m = __ballot_sync(0xffffffffu, iw < p.nw && !is_far(f, wx[min(iw, p.nw - 1)]));
+        const unsigned gaps = ~m & ((1u << lane) - 1);
+        const int before = gaps ? lane - 32 + __clz(gaps) : lane + carry;
+        const bool start = ((m >> lane) & 1) && before % kNearFreq == 0;
+        int len = 1;
+        if (start)
+            while (len < kNearFreq && iw + len < p.nw && !is_far(f, wx[iw + len])) ++len;
+        found(start, iw, len);
+        carry = m == 0xffffffffu ? carry + 32 : __clz(~m);
     }
+}
+// Entries of each length per band: count[l bands + n], l = kNearFreq - length.
+__global__ void __launch_bounds__(256) far_near_count_kernel(Problem p, const FarPlan *f, int b0,
+                                                             int bands, int *count) {
+    if (!f->active) return;
+    const int n = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    if (n >= bands) return;
+    int c[kNearFreq] = {};
+    near_runs(p, *f, b0 + n, [&](bool start, int, int len) {
+#pragma unroll
+        for (int l = 0; l < kNearFreq; ++l)
+            c[l] += __popc(__ballot_sync(0xffffffffu, start && len == kNearFreq - l));
+    });
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int l = 0; l < kNearFreq; ++l) count[l * bands + n] = c[l];
+}
+// The counts become places, the longest entries first, so that the warps of a
+// block have equal work; the plan is dropped if too many pairs are near.
+__global__ void __launch_bounds__(1024) far_near_scan_kernel(FarPlan *f, int bands, int nw, int *count,
+                                                             int cap_near, float c0, float w_near) {
+    if (!f->active) return;
+    __shared__ int part[1024];
+    __shared__ unsigned long long pairs;
+    const int n = kNearFreq * bands, per = (n + 1023) / 1024;
+    const int a = threadIdx.x * per, b = min(n, a + per);
+    if (threadIdx.x == 0) pairs = 0;
     __syncthreads();
-    if (!go) return;
-    // An entry covers up to kNearFreq consecutive near frequencies of a band;
-    // the first pair of each such run of pairs writes it.  The longest entries
-    // come first, so that the warps of a block have equal work.
-    for (int want = kNearFreq; want >= 1; --want) {
-        for (long long i0 = 0; i0 < n; i0 += kBins) {
-            const long long i = i0 + t;
-            const int iw = (int)(i % p.nw);
-            int len = 0;
-            if (i < n && !is_far(*f, wx_at(i))) {
-                int before = 0;
-                while (before < iw && !is_far(*f, wx_at(i - before - 1))) ++before;
-                if (before % kNearFreq == 0)
-                    for (len = 1; len < kNearFreq && iw + len < p.nw && !is_far(*f, wx_at(i + len));) ++len;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, len == want);
-            if (lane == 0) scan[warp] = __popc(m);
-            __syncthreads();
-            int at = base + __popc(m & ((1u << lane) - 1));
-            for (int k = 0; k < warp; ++k) at += scan[k];
-            if (len == want) near[at] = make_int4(b0 + (int)(i / p.nw), iw, len, 0);
-            __syncthreads();
-            if (t == 0)
-                for (int k = 0; k < kBins / 32; ++k) base += scan[k];
-            __syncthreads();
+    int s = 0;
+    unsigned long long q = 0;
+    for (int i = a; i < b; ++i) {
+        s += count[i];
+        q += (unsigned long long)count[i] * (kNearFreq - i / bands);
+    }
+    part[threadIdx.x] = s;
+    if (q) atomicAdd(&pairs, q);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int acc = 0;
+        for (int i = 0; i < 1024; ++i) {
+            const int v = part[i];
+            part[i] = acc;
+            acc += v;
         }
+        const float total = (float)((long long)bands * nw);
+        if (pairs > (unsigned long long)cap_near || (float)pairs * w_near + c0 >= 0.95f * total)
+            f->active = 0;
+        f->n_near = acc;
+        count[n] = acc;
     }
-    if (t == 0) {
-        f->n_near = base;
-        f->active = 1;
+    __syncthreads();
+    s = part[threadIdx.x];
+    for (int i = a; i < b; ++i) {
+        const int v = count[i];
+        count[i] = s;
+        s += v;
     }
+}
+__global__ void __launch_bounds__(256) far_near_list_kernel(Problem p, const FarPlan *f, int b0,
+                                                            int bands, const int *place, int4 *near) {
+    if (!f->active) return;
+    const int n = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (n >= bands) return;
+    int at[kNearFreq];
+#pragma unroll
+    for (int l = 0; l < kNearFreq; ++l) at[l] = place[l * bands + n];
+    near_runs(p, *f, b0 + n, [&](bool start, int iw, int len) {
+#pragma unroll
+        for (int l = 0; l < kNearFreq; ++l) {
+            const bool mine = start && len == kNearFreq - l;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            if (mine) near[at[l] + __popc(m & ((1u << lane) - 1))] = make_int4(b0 + n, iw, len, 0);
+            at[l] += __popc(m);
+        }
+    });
 }
 
 // Terms each band's series needs (for the nearest of its far frequencies; 0
@@ -1007,7 +1057,8 @@ __device__ __forceinline__ double2 far_series(const FarPlan &f, double wx, const
 // block nw + n: band n's total at iw = 2.  Written into the first unoccupied
 // slot of the frequency, or the band's first row slot.
 __global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan *f, int b0, int bands,
-                                                        const int4 *near, const double2 *near_val,
+                                                        const int4 *near, const int *place,
+                                                        const double2 *near_val,
                                                         const double2 *out_part, long long seg_len,
                                                         const double2 *S1, int K, Partials part) {
     if (!f->active) return;
@@ -1031,12 +1082,15 @@ __global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan
             v[1] += x.y;
         }
     }
-    for (int e = threadIdx.x; e < f->n_near; e += 256) {
-        const int4 q = near[e];
-        const int w = iw - q.y;
-        if (w < 0 || w >= q.z || (band && q.x != b0 + n0)) continue;
-        v[0] += near_val[(size_t)e * kNearFreq + w].x;
-        v[1] += near_val[(size_t)e * kNearFreq + w].y;
+    for (int l = 0; l < (band ? kNearFreq : 1); ++l) {
+        const int e0 = band ? place[l * bands + n0] : 0, e1 = band ? place[l * bands + n0 + 1] : f->n_near;
+        for (int e = e0 + threadIdx.x; e < e1; e += 256) {
+            const int4 q = near[e];
+            const int w = iw - q.y;
+            if (w < 0 || w >= q.z) continue;
+            v[0] += near_val[(size_t)e * kNearFreq + w].x;
+            v[1] += near_val[(size_t)e * kNearFreq + w].y;
+        }
     }
     block_reduce<2, 256>(v, red, S);
     if (threadIdx.x == 0) {
@@ -1086,15 +1140,20 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     const int sms = sm_count();
     far_range_kernel<<<1, 1024, 0, s>>>(p, b0, bands, b.plan);
     far_hist_kernel<<<sms * 4, 256, 0, s>>>(p, b.plan);
-    far_plan_kernel<<<1, kBins, 0, s>>>(p, b0, bands, b.plan, b.near, z.cap_near, z.cap_out, (float)z.R,
-                                        (float)z.c0, 1.4f, mixed ? 16.f : 2.f);
+    const float w_near = 1.4f;
+    far_plan_kernel<<<1, kBins, 0, s>>>(p, b0, bands, b.plan, z.cap_out, (float)z.R, (float)z.c0,
+                                        w_near, mixed ? 16.f : 2.f);
+    const int band_warps = ceil_div(bands, 8);
+    far_near_count_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.place);
+    far_near_scan_kernel<<<1, 1024, 0, s>>>(b.plan, bands, p.nw, b.place, z.cap_near, (float)z.c0, w_near);
+    far_near_list_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.place, b.near);
     far_count_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows);
     far_scan_kernel<<<1, 1024, 0, s>>>(p.ng, b.plan, b.rows);
     far_list_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows, b.out);
     far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
     far_need_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(p, b.plan, b0, bands, z.K, z.bits, b.terms);
     far_order_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(b.plan, bands, b.terms, b.order);
-    count_launch(9);
+    count_launch(12);
     cudaError_t e = cudaGetLastError();
 
     // The series, a pass per group of terms of one level and slab of chunks.
@@ -1150,7 +1209,7 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, (p.ng + 1) / 2, b.near_val);
     far_out_kernel<<<dim3(z.segs, ceil_div(bands, kOutBands), ceil_div(p.nw, kOutFreq)), 128, 0, s>>>(
         p, b.plan, b.out, z.seg_len, b0, bands, b.C, b.out_part);
-    far_final_kernel<<<p.nw + (part.n1 ? bands : 0), 256, 0, s>>>(p, b.plan, b0, bands, b.near,
+    far_final_kernel<<<p.nw + (part.n1 ? bands : 0), 256, 0, s>>>(p, b.plan, b0, bands, b.near, b.place,
                                                                   b.near_val, b.out_part, z.seg_len,
                                                                   b.S1, z.K, part);
     count_launch(3);
