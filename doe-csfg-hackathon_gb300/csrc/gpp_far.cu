@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(256) far_coeff_kernel(Problem p, int b0, int b
     }
 }
 
-// round(x 2^(bits - e)) for bits <= 30 on 32-bit words, |x| < 2^e and x normal
-// or zero (a subnormal, far below any chunk that matters, counts as zero).
+// round(x 2^(bits - e)) for bits <= 30 on 32-bit words, e >= 0, |x| < 2^e (a
+// subnormal, then far below half a unit, counts as zero).
 __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
     const unsigned hi = __double2hiint(x), lo = __double2loint(x);
     const int E = (hi >> 20) & 0x7FF;
@@ -632,14 +632,16 @@ __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
 // resident warps) through the recurrence P_(k+1) = 2 z P_k - P_(k-1) (P_-1 =
 // z Q starts it) and leaves P_(k-1), P_k for the next pass in `state`.  The
 // exponent of term k is that of the chunk's largest |re|, |im| of Q, raised by
-// the bound rho^k of |T_k| and 1.  Columns outside the box are zero.
+// the bound rho^k of |T_k| and 1.  Q is scaled by the chunk's exponent first:
+// the terms of a chunk at either end of FP64's range keep their precision.
+// Columns outside the box are zero.
 constexpr int kTermK = 4;  // columns per thread
 //
 // In mixed precision the recurrence runs in float-float (DF): FP64 kept its
 // pipe 62-76% busy with 4 instructions per term and column where the residues
-// take most of the issue slots.  1638 x 32768, 25 terms: 26 -> 19 ms.  Q is scaled by the chunk's exponent first, so
-// its range is FP64's; only the first pass reads the inputs, the next ones
-// find z with the last two terms in `state`.
+// take most of the issue slots.  1638 x 32768, 25 terms: 26 -> 19 ms.  Only the
+// first pass reads the inputs, the next ones find z with the last two terms in
+// `state`.
 template <int L, bool DF>
 __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int c0,
                                                            int nc, int Kc, int Np, int k0, int gm,
@@ -690,6 +692,11 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
     }
     __syncthreads();
     const int e0 = exps[row];
+    // x 2^-e0 in two exact steps (what is lost below 2^-1022 of the largest
+    // value is far below the last bit).
+    const int h0 = max(-2000, min(e0, 2000)) / 2, h1 = max(-2000, min(e0, 2000)) - h0;
+    const double s0 = __hiloint2double((1023 - h0) << 20, 0), s1 = __hiloint2double((1023 - h1) << 20, 0);
+    auto scaled = [&](double2 q) { return make_double2(q.x * s0 * s1, q.y * s0 * s1); };
     const double log2_rho = f->log2_rho;
     auto raise = [&](int k) { return k == 0 ? 0 : 1 + (int)ceil(k * log2_rho); };
     if (half == 0)
@@ -728,7 +735,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
                     if (at(ig, wt) && finite) {
                         z = make_double2(2.0 * (wt.x - z0) * inv_h, 2.0 * wt.y * inv_h);
                         q = cmul(wt, __ldg(erow + ig));
-                        q = make_double2(ldexp(q.x, -e0), ldexp(q.y, -e0));
+                        q = scaled(q);
                     }
                     df2_set_lane(zr[h], j, split_bits(z.x));
                     df2_set_lane(zi[h], j, split_bits(z.y));
@@ -787,7 +794,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
             z2[kk] = in ? make_double2(2.0 * (wt.x - z0) * inv_h, 2.0 * wt.y * inv_h)
                         : make_double2(0.0, 0.0);
             if (k0 == 0) {
-                cur[kk] = in ? cmul(wt, __ldg(erow + ig)) : make_double2(0.0, 0.0);
+                cur[kk] = in ? scaled(cmul(wt, __ldg(erow + ig))) : make_double2(0.0, 0.0);
                 const double2 d = cmul(cur[kk], z2[kk]);
                 prev[kk] = make_double2(0.5 * d.x, 0.5 * d.y);
             } else {
@@ -798,7 +805,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
         const int ks = c * (Kc / kCrtBlockK) + i;
 #pragma unroll 1
         for (int m = 0; m < gm; ++m) {
-            const int e = e0 + raise(k0 + m);
+            const int e = raise(k0 + m);
             const int y = m * ngp + grp * 8;
             __nv_bfloat16 *w = out + ((size_t)(y / kCrtRowsY) * ksteps + ks) * (kCrtRowsY * kCrtBlockK) +
                                (size_t)((y % kCrtRowsY) / 8) * 512 + kg0 * 64 + row * 8 + half * kTermK;
