@@ -315,12 +315,14 @@ struct Walk {
 // holds its own 128 rows of X and half of Y's rows, block 0 issues for both,
 // and block 1's warp 1 passes on to block 0's barriers what has landed in its
 // own shared memory.
+// RAW: one plane of each operand, and the sums themselves as floats at
+// [(q Ms + row) Np + col] of the output.
 // Every wait is bounded; a block that gives up records kErrPipelineTimeout,
 // lets its copies and MMAs finish and frees its TMEM.
-template <int CG>
+template <int CG, bool RAW>
 __global__ void __launch_bounds__(kThreads, 1)
 crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__restrict__ SY, int Mp,
-                int Np, int KS, int nc, int mt0, int MT, int gq, unsigned char *__restrict__ res,
+                int Np, int KS, int nc, int mt0, int MT, int gq, void *__restrict__ res,
                 int Ms, int nmod, const int *go, const int *rows, int *err) {
     if (go && !*go) return;
     if (rows) MT = min(MT, (*rows + kTM - 1) / kTM);
@@ -328,7 +330,7 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
     constexpr int STAGES = kStages * CG;
     constexpr unsigned BYTES_B = kBytesB / CG, IDESC = umma_idesc(kTM * CG, kTN);
     const int rank = CG == 2 ? cluster_rank() : 0;
-    const int planes = 3 * nmod;
+    const int planes = RAW ? 1 : 3 * nmod;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *sA = smem;
     unsigned char *sB = smem + (size_t)kKSMax * kBytesA;
@@ -500,15 +502,23 @@ crt_gemm_kernel(const __nv_bfloat16 *__restrict__ SX, const __nv_bfloat16 *__res
             const int acc = G & 1;
             if (!bar_wait(&accfull[acc], (G >> 1) & 1, abort)) break;
             tc_fence_after();
-            const CrtMod m = c_crt_mod[(w.q % planes) % nmod];
+            const CrtMod m = RAW ? CrtMod{} : c_crt_mod[(w.q % planes) % nmod];
             const int tile = w.mt * CG + rank;  // the pair's second may be past the end
-            unsigned char *o = res + ((size_t)w.q * Ms + (size_t)tile * kTM + quarter * 32 + lane) * Np +
-                               (size_t)w.nt * kTN + group * kDrainCols;
+            const size_t at = ((size_t)w.q * Ms + (size_t)tile * kTM + quarter * 32 + lane) * Np +
+                              (size_t)w.nt * kTN + group * kDrainCols;
             const unsigned ta = tmem + ((unsigned)(quarter * 32) << 16) + acc * kTN + group * kDrainCols;
 #pragma unroll 1
             for (int cc = 0; cc < kDrainCols; cc += 32) {
                 float v[32];
                 tmem_ld32(ta + cc, v);
+                if constexpr (RAW) {
+                    float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(res) + at + cc);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (tile < MT) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    continue;
+                }
+                unsigned char *o = static_cast<unsigned char *>(res) + at;
                 unsigned word[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -693,7 +703,7 @@ int pair_count() {
     int n = count[dev & 255].load(std::memory_order_acquire);
     if (n == 0) {
         GemmLaunch l(2, std::max(1, sm_count() / 2), nullptr);
-        if (cudaOccupancyMaxActiveClusters(&n, crt_gemm_kernel<2>, &l.cfg) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveClusters(&n, crt_gemm_kernel<2, false>, &l.cfg) != cudaSuccess) return 0;
         count[dev & 255].store(n, std::memory_order_release);
     }
     return n;
@@ -704,11 +714,10 @@ cudaError_t configure() {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || configured[dev & 255].load(std::memory_order_acquire)) return e;
-    e = cudaFuncSetAttribute(crt_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(crt_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmem);
+    for (auto kern : {crt_gemm_kernel<1, false>, crt_gemm_kernel<2, false>, crt_gemm_kernel<1, true>,
+                      crt_gemm_kernel<2, true>})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(crt_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double2) * 8 * (kKcMax + 1)));
@@ -734,16 +743,18 @@ cudaError_t crt_rows(const OzOperand &X, const int *order, int Mp, int K, int Kc
     return cudaGetLastError();
 }
 
-cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0,
-                         int tiles, int level, unsigned char *res, int Ms, const int *go,
-                         const int *rows, int *err, cudaStream_t s) {
+namespace {
+template <bool RAW>
+cudaError_t products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0, int tiles,
+                     int nmod, void *res, int Ms, const int *go, const int *rows, int *err,
+                     cudaStream_t s) {
     cudaError_t e = configure();
     if (e != cudaSuccess) return e;
-    const int nmod = kCrtLevel[level].n, ntiles = Np / kTN;
+    const int planes = RAW ? 1 : 3 * nmod, ntiles = Np / kTN;
     const int cg = gemm_pairs(tiles) ? 2 : 1, units = ceil_div(tiles, cg);  // row tiles, or pairs
     const int fit = cg == 2 ? pair_count() : sm_count();
     if (fit <= 0) return cudaErrorUnknown;
-    const int grid = (int)std::min<long long>(fit, (long long)nc * 3 * nmod * units * ntiles);
+    const int grid = (int)std::min<long long>(fit, (long long)nc * planes * units * ntiles);
     // Planes in flight: enough that every block has a step, with their
     // operands within about 80 MB of L2.
     const size_t plane = sizeof(__nv_bfloat16) * (size_t)Kc * (Mp + Np);
@@ -752,11 +763,24 @@ cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc,
     const __nv_bfloat16 *x = static_cast<const __nv_bfloat16 *>(sx),
                         *y = static_cast<const __nv_bfloat16 *>(sy);
     GemmLaunch l(cg, grid, s);
-    e = cudaLaunchKernelEx(&l.cfg, cg == 2 ? crt_gemm_kernel<2> : crt_gemm_kernel<1>, x, y, Mp, Np,
-                           Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, rows, err);
+    e = cudaLaunchKernelEx(&l.cfg, cg == 2 ? crt_gemm_kernel<2, RAW> : crt_gemm_kernel<1, RAW>, x, y, Mp,
+                           Np, Kc / kTK, nc, mt0, tiles, gq, res, Ms, nmod, go, rows, err);
     if (e != cudaSuccess) return e;
     count_launch();
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0,
+                         int tiles, int level, unsigned char *res, int Ms, const int *go,
+                         const int *rows, int *err, cudaStream_t s) {
+    return products<false>(sx, sy, Mp, Np, Kc, nc, mt0, tiles, kCrtLevel[level].n, res, Ms, go, rows,
+                           err, s);
+}
+
+cudaError_t crt_sums(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, float *out,
+                     const int *go, int *err, cudaStream_t s) {
+    return products<true>(sx, sy, Mp, Np, Kc, nc, 0, Mp / kTM, 1, out, Mp, go, nullptr, err, s);
 }
 
 cudaError_t crt_combine(const unsigned char *res, const int *ex, const int *ey, int row0, int rows,

@@ -25,12 +25,16 @@ cudaError_t crt_zgemm(const OzOperand &X, const OzOperand &Y, int M, int N, int 
 //    rows each) with every row of Y: res [nc][3 n][Ms][Np] bytes.
 //  crt_combine: Out[row0 + m][n] = (+=) the sum over the chunks.
 // The last two stop at the first *rows (*live) rows of X, if given.
+//  crt_sums: out [nc][Mp][Np], the products of single bf16 planes of each
+//    operand (same blocks), summed in FP32 over each chunk.
 constexpr int kCrtRowsX = 128, kCrtRowsY = 256, kCrtChunk = 512, kCrtBlockK = 64;
 cudaError_t crt_rows(const OzOperand &X, const int *order, int Mp, int K, int Kc, int c0, int nc,
                      int level, void *sx, int *ex, const int *go, cudaStream_t s);
 cudaError_t crt_products(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, int mt0,
                          int tiles, int level, unsigned char *res, int Ms, const int *go,
                          const int *rows, int *err, cudaStream_t s);
+cudaError_t crt_sums(const void *sx, const void *sy, int Mp, int Np, int Kc, int nc, float *out,
+                     const int *go, int *err, cudaStream_t s);
 cudaError_t crt_combine(const unsigned char *res, const int *ex, const int *ey, int row0, int rows,
                         int Ms, int N, int Mp, int Np, int nc, int level, bool accumulate,
                         double2 *Out, long long out_ld, const int *go, const int *live,

@@ -29,8 +29,20 @@
 // What the series does not cover is computed term by term:
 //  * near pairs (|r| < R rho, or a wx that is not finite): over every column,
 //    in the call's precision;
+//  * bands whose terms a fixed point does not hold (below): as near pairs;
 //  * the columns whose wtilde lies outside the box (a few strays, such as
 //    wtilde next to another band's frequency), for the far pairs, in FP64.
+//
+// The products' operands are fixed point, 57 bits of a row's largest value in
+// each chunk of 512 columns, so their rounding is relative to max|aqsn| sum|Q| +
+// sum|aqsn| max|Q| of a chunk, where term by term it is relative to the sum of
+// |aqsn Q|.  The two differ where one factor is large just where the other is
+// small.  So both are summed for every band first (weighted as the rows are;
+// |aqsn| and |Q| in bf16, one product on the tensor cores), and a band whose
+// ratio of the two passes kSpread is computed term by term: up to there the
+// fixed point's rounding, ratio 2^-58 of the sum of |aqsn Q| at worst, is no more
+// than the per-term roundings.  Uniform data gives 5, a chunk over which both
+// factors fall by e^2 12.
 //
 // The box is chosen on the device from a histogram of Re(wtilde) against the
 // histogram of wx, by the cost of what it leaves over; where no box pays, or
@@ -75,6 +87,7 @@ namespace {
 
 constexpr int kBins = 512;
 constexpr int kNearTile = 4;  // entries per block of the FP64 near kernel
+constexpr double kSpread = 32.0;
 
 struct Sizes {
     int bands, ng, nc, nw;
@@ -92,8 +105,11 @@ struct Sizes {
 };
 
 constexpr size_t kPassBytes = size_t(8) << 30;
+// Term k counts R^-k; three bits more past the first, so that all of them
+// together round no worse than it does.
 int level_of(const Sizes &z, int k) {
-    const double need = (z.mixed ? 49.0 : 53.0) - k * std::log2(z.R);
+    const double need = (z.mixed ? 49.0 : 57.0) + (k > 0 ? 3.0 : 0.0) - k * std::log2(z.R);
+    if (need > kCrtLevel[0].bits) return kCrtWide;
     int l = 0;
     while (l + 1 < kCrtWide && kCrtLevel[l + 1].bits >= need) ++l;
     return l;
@@ -145,7 +161,9 @@ struct Buffers {
     double2 *S1;       // [bands][K]
     double2 *near_part, *near_val, *out_part;
     void *state;       // P_(k-1), P_k (mixed: and z) between passes
-    int *E0, *EX, *EY;
+    int *E0, *EA, *EX, *EY;
+    float *SQ, *SA;      // [chunks][rows], [chunks][Mp]: sums of |Q|, |aqsn| over the chunk's exponent
+    double2 *spread;     // per band: what the fixed point's rounding is relative to, and the sum of |aqsn Q|
     int *terms, *order;  // per band: its terms; the bands by their terms
     __nv_bfloat16 *sx, *sy;
     unsigned char *res;
@@ -177,6 +195,10 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     o.terms = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.order = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.E0 = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.ngp));
+    o.EA = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.Mp));
+    o.SQ = reinterpret_cast<float *>(take(sizeof(float) * (size_t)z.nch * z.ngp));
+    o.SA = reinterpret_cast<float *>(take(sizeof(float) * (size_t)z.nch * z.Mp));
+    o.spread = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands));
     o.EX = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.Mp));
     o.EY = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.slab * Np));
     o.sx = reinterpret_cast<__nv_bfloat16 *>(
@@ -203,6 +225,9 @@ __device__ __forceinline__ bool in_box(const FarPlan &f, double2 wt) {
     const int b = bin_of(f, wt);
     return b >= f.lo && b <= f.hi;
 }
+// Whether a band (its `spread`) is summed by the series at all, and a
+// frequency of such a band.
+__device__ __forceinline__ bool held(double2 spread) { return spread.x <= kSpread * spread.y; }
 __device__ __forceinline__ bool is_far(const FarPlan &f, double wx) {
     return is_finite(wx) && fabs(wx - f.z0) >= f.dfar;
 }
@@ -387,31 +412,32 @@ __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int 
 // of them, all lanes together: whether lane's frequency iw starts an entry, and
 // of which length.
 template <class Found>
-__device__ __forceinline__ void near_runs(const Problem &p, const FarPlan &f, int band, Found found) {
+__device__ __forceinline__ void near_runs(const Problem &p, const FarPlan &f, int band, bool far_band,
+                                          Found found) {
     const int lane = threadIdx.x & 31;
     const double *wx = p.wx + (size_t)band * p.wx_stride;
     int carry = 0;  // the run that reaches the first of these 32
     for (int w0 = 0; w0 < p.nw; w0 += 32) {
         const int iw = w0 + lane;
-        const unsigned m = __ballot_sync(0xffffffffu, iw < p.nw && !is_far(f, wx[min(iw, p.nw - 1)]));
+        const unsigned m = __ballot_sync(0xffffffffu, iw < p.nw && !(far_band && is_far(f, wx[min(iw, p.nw - 1)])));
         const unsigned gaps = ~m & ((1u << lane) - 1);
         const int before = gaps ? lane - 32 + __clz(gaps) : lane + carry;
         const bool start = ((m >> lane) & 1) && before % kNearFreq == 0;
         int len = 1;
         if (start)
-            while (len < kNearFreq && iw + len < p.nw && !is_far(f, wx[iw + len])) ++len;
+            while (len < kNearFreq && iw + len < p.nw && !(far_band && is_far(f, wx[iw + len]))) ++len;
         found(start, iw, len);
         carry = m == 0xffffffffu ? carry + 32 : __clz(~m);
     }
 }
 // Entries of each length per band: count[l bands + n], l = kNearFreq - length.
 __global__ void __launch_bounds__(256) far_near_count_kernel(Problem p, const FarPlan *f, int b0,
-                                                             int bands, int *count) {
+                                                             int bands, const double2 *spread, int *count) {
     if (!f->active) return;
     const int n = (blockIdx.x * 256 + threadIdx.x) >> 5;
     if (n >= bands) return;
     int c[kNearFreq] = {};
-    near_runs(p, *f, b0 + n, [&](bool start, int, int len) {
+    near_runs(p, *f, b0 + n, held(spread[n]), [&](bool start, int, int len) {
 #pragma unroll
         for (int l = 0; l < kNearFreq; ++l)
             c[l] += __popc(__ballot_sync(0xffffffffu, start && len == kNearFreq - l));
@@ -462,14 +488,15 @@ __global__ void __launch_bounds__(1024) far_near_scan_kernel(FarPlan *f, int ban
     }
 }
 __global__ void __launch_bounds__(256) far_near_list_kernel(Problem p, const FarPlan *f, int b0,
-                                                            int bands, const int *place, int4 *near) {
+                                                            int bands, const double2 *spread,
+                                                            const int *place, int4 *near) {
     if (!f->active) return;
     const int n = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (n >= bands) return;
     int at[kNearFreq];
 #pragma unroll
     for (int l = 0; l < kNearFreq; ++l) at[l] = place[l * bands + n];
-    near_runs(p, *f, b0 + n, [&](bool start, int iw, int len) {
+    near_runs(p, *f, b0 + n, held(spread[n]), [&](bool start, int iw, int len) {
 #pragma unroll
         for (int l = 0; l < kNearFreq; ++l) {
             const bool mine = start && len == kNearFreq - l;
@@ -486,14 +513,15 @@ __global__ void __launch_bounds__(256) far_near_list_kernel(Problem p, const Far
 // terms.
 constexpr int kOrderBands = 8192;
 __global__ void __launch_bounds__(256) far_need_kernel(Problem p, FarPlan *f, int b0, int bands,
-                                                       int K, double bits, int *terms) {
+                                                       int K, double bits, const double2 *spread,
+                                                       int *terms) {
     if (!f->active) return;
     if (blockIdx.x == 0 && threadIdx.x < 64)
         f->bands_at[threadIdx.x] = bands > kOrderBands && (int)threadIdx.x < K ? bands : 0;
     const int n = blockIdx.x * 256 + threadIdx.x;
     if (n >= bands) return;
     double d = 1.0 / 0.0;
-    for (int w = 0; w < p.nw; ++w) {
+    for (int w = 0; held(spread[n]) && w < p.nw; ++w) {
         const double x = p.wx[(size_t)(b0 + n) * p.wx_stride + w];
         if (is_far(*f, x)) d = fmin(d, fabs(x - f->z0));
     }
@@ -625,6 +653,113 @@ __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
     return (int)hi < 0 ? -(int)n : (int)n;
 }
 
+// What the spread of a band is formed from: for 8 rows x one chunk the exponent
+// E of the largest |re|, |im|, the magnitudes over 2^E in bf16 (core-matrix
+// blocks of R rows) and their sum S.  Y: rows of Q, 0 outside the box; else
+// rows of aqsn.  A thread per 8 consecutive columns of a row, which it reads
+// twice (from L1 and L2 the second time).
+template <bool Y>
+__global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan *f, int b0, int L, int Lp,
+                                                        int c0, int nc, int Kc, int *E, float *S,
+                                                        __nv_bfloat16 *out) {
+    constexpr int R = Y ? kCrtRowsY : kCrtRowsX;
+    if (!f->active) return;
+    __shared__ unsigned long long red[4][8];
+    __shared__ float sum[4][8];
+    __shared__ int exps[8];
+    const int groups = Lp / 8, l0 = blockIdx.x % groups * 8, c = blockIdx.x / groups;
+    const int t = threadIdx.x, row = t & 7, l = l0 + row, kb = (c0 + c) * Kc, end = min(p.nc, kb + Kc);
+    auto value = [&](int ig) {
+        if (l >= L || ig >= end) return make_double2(0.0, 0.0);
+        const size_t at = (size_t)((Y ? 0 : b0) + l) * p.nc + ig;
+        if constexpr (!Y) return __ldg(p.aqsn + at);
+        const double2 wt = __ldg(p.wt + at);
+        return in_box(*f, wt) ? cmul(wt, __ldg(p.ieps + at)) : make_double2(0.0, 0.0);
+    };
+    unsigned long long mx = 0;
+    for (int k = t >> 3; k < Kc / 8; k += 16)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double2 v = value(kb + k * 8 + j);
+            const unsigned long long a = (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
+            const unsigned long long b = (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
+            mx = max(mx, max(a, b));
+        }
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    if ((t & 24) == 0) red[t >> 5][row] = mx;
+    __syncthreads();
+    if (t < 8) {
+        for (int w = 1; w < 4; ++w) mx = max(mx, red[w][t]);
+        exps[t] = crt_exponent(mx);
+        E[(size_t)(c0 + c) * Lp + l0 + t] = exps[t];
+    }
+    __syncthreads();
+    const int e = exps[row], ksteps = nc * (Kc / kCrtBlockK);
+    __nv_bfloat16 *w0 = out + ((size_t)(l0 / R) * ksteps * (R / 8) + (size_t)(l0 % R) / 8) * 512 + row * 8;
+    // |x| 2^-e from the bits (top 20 of the mantissa); near FP64's lower end by FP64.
+    auto over = [&](double x) {
+        if (e < -1000) return fabsf((float)ldexp(x, -e));
+        const int hi = __double2hiint(x) & 0x7FFFFFFF, sh = (hi >> 20) - 1022 - e;
+        return sh < -60 ? 0.f : __int_as_float(((sh + 126) << 23) | ((hi & 0xFFFFF) << 3));
+    };
+    float total = 0.f;
+    for (int k = t >> 3; k < Kc / 8; k += 16) {
+        unsigned v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float m[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double2 x = value(kb + k * 8 + 2 * j + h);
+                const float a = over(x.x), b = over(x.y);
+                m[h] = e == kExpNonFinite || e == kExpZero ? 0.f : sqrtf(a * a + b * b);
+            }
+            const __nv_bfloat162 q = __floats2bfloat162_rn(m[0], m[1]);
+            total += __low2float(q) + __high2float(q);
+            v[j] = *reinterpret_cast<const unsigned *>(&q);
+        }
+        const int ks = c * (Kc / kCrtBlockK) + (k >> 3);
+        *reinterpret_cast<uint4 *>(w0 + (size_t)ks * (R / 8) * 512 + (k & 7) * 64) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    total += __shfl_xor_sync(0xffffffffu, total, 8);
+    total += __shfl_xor_sync(0xffffffffu, total, 16);
+    if ((t & 24) == 0) sum[t >> 5][row] = total;
+    __syncthreads();
+    if (t < 8) S[(size_t)(c0 + c) * Lp + l0 + t] = sum[0][t] + sum[1][t] + sum[2][t] + sum[3][t];
+}
+
+// spread[n] (+)= over the rows and chunks [c0, c0 + nc): |c| 2^(EA + E0) times
+// SA + SQ (the largest magnitudes count 1 each) and times V, the chunk's sum of
+// products.
+__global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const double2 *C, const int *EA,
+                                                         const int *E0, const float *SA, const float *SQ,
+                                                         const float *V, int ng, int ngp, int Mp, int Np,
+                                                         int c0, int nc, double2 *spread) {
+    if (!f->active) return;
+    __shared__ double red[16], S[2];
+    const int n = blockIdx.x;
+    double v[2] = {0.0, 0.0};
+    for (int r = threadIdx.x; r < ng; r += 256) {
+        const double2 z = C[(size_t)n * ng + r];
+        double a = 0.0, b = 0.0;
+        for (int c = 0; c < nc; ++c) {
+            const size_t x = (size_t)(c0 + c) * Mp + n, y = (size_t)(c0 + c) * ngp + r;
+            const double w = scalbn(1.0, EA[x] + E0[y]);
+            a = fma(w, (double)(SA[x] + SQ[y]), a);
+            b = fma(w, (double)V[((size_t)c * Mp + n) * Np + r], b);
+        }
+        const double m = sqrt(z.x * z.x + z.y * z.y);
+        v[0] = fma(m, a, v[0]);
+        v[1] = fma(m, b, v[1]);
+    }
+    block_reduce<2, 256>(v, red, S);
+    if (threadIdx.x == 0) {
+        const double2 old = c0 == 0 ? make_double2(0.0, 0.0) : spread[n];
+        spread[n] = make_double2(old.x + S[0], old.y + S[1]);
+    }
+}
+
 // Residue planes and exponents of P_k, k = k0 .. k0 + gm - 1, for 8 rows x one
 // chunk at level L: row r of term m is row m ngp + r of the product's Y
 // operand, in the core-matrix blocks of crt_prep_kernel.  A thread carries 4
@@ -646,10 +781,9 @@ template <int L, bool DF>
 __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int c0,
                                                            int nc, int Kc, int Np, int k0, int gm,
                                                            int last, __nv_bfloat16 *out, int *EY,
-                                                           int *E0, void *state) {
+                                                           const int *E0, void *state) {
     constexpr int NMOD = kCrtLevel[L].n, BITS = kCrtLevel[L].bits, ND = BITS > 41 ? 4 : BITS > 18 ? 3 : 2;
     if (!f->active) return;
-    __shared__ unsigned long long red[4][8];
     __shared__ int exps[8];
     const int groups = ngp / 8;
     const int grp = blockIdx.x % groups, c = blockIdx.x / groups;
@@ -663,33 +797,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
         wt = __ldg(wrow + ig);
         return in_box(*f, wt);
     };
-    if (k0 == 0) {
-        unsigned long long mx = 0;
-        for (int i = 0; i < items; ++i) {
-#pragma unroll
-            for (int kk = 0; kk < kTermK; ++kk) {
-                double2 wt;
-                const int ig = kb + (kg0 + 8 * i) * 8 + half * kTermK + kk;
-                if (!at(ig, wt)) continue;
-                const double2 q = cmul(wt, __ldg(erow + ig));
-                const unsigned long long a = (unsigned long long)__double_as_longlong(q.x) & 0x7FFFFFFFFFFFFFFFull;
-                const unsigned long long b = (unsigned long long)__double_as_longlong(q.y) & 0x7FFFFFFFFFFFFFFFull;
-                mx = max(mx, max(a, b));
-            }
-        }
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-        if ((t & 17) == 0) red[t >> 5][row] = mx;
-        __syncthreads();
-        if (t < 8) {
-            mx = red[0][t];
-            for (int w = 1; w < 4; ++w) mx = max(mx, red[w][t]);
-            exps[t] = crt_exponent(mx);
-            E0[(size_t)(c0 + c) * ngp + grp * 8 + t] = exps[t];
-        }
-    } else if (t < 8) {
-        exps[t] = E0[(size_t)(c0 + c) * ngp + grp * 8 + t];
-    }
+    if (t < 8) exps[t] = E0[(size_t)(c0 + c) * ngp + grp * 8 + t];
     __syncthreads();
     const int e0 = exps[row];
     // x 2^-e0 in two exact steps (what is lost below 2^-1022 of the largest
@@ -985,7 +1093,8 @@ __global__ void __launch_bounds__(256) far_near_sum_kernel(FarNear nr, int pairs
 constexpr int kOutBands = 4, kOutFreq = 4;
 __global__ void __launch_bounds__(128) far_out_kernel(Problem p, const FarPlan *f, const int2 *list,
                                                       long long seg_len, int b0, int bands,
-                                                      const double2 *C, double2 *part) {
+                                                      const double2 *C, const double2 *spread,
+                                                      double2 *part) {
     if (!f->active) return;
     constexpr int K = kOutBands * kOutFreq * 2;
     __shared__ double red[4 * K], S[K];
@@ -1002,7 +1111,7 @@ __global__ void __launch_bounds__(128) far_out_kernel(Problem p, const FarPlan *
         for (int w = 0; w < kOutFreq; ++w) {
             const int band = b0 + min(n0 + n, bands - 1);
             wx[n][w] = __ldg(p.wx + (size_t)band * p.wx_stride + min(w0 + w, p.nw - 1));
-            if (n0 + n < bands && w0 + w < p.nw && is_far(*f, wx[n][w])) far |= 1u << (n * kOutFreq + w);
+            if (n0 + n < bands && w0 + w < p.nw && held(spread[n0 + n]) && is_far(*f, wx[n][w])) far |= 1u << (n * kOutFreq + w);
         }
     any = far != 0;
     double2 acc[kOutBands][kOutFreq];
@@ -1067,7 +1176,8 @@ __global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan
                                                         const int4 *near, const int *place,
                                                         const double2 *near_val,
                                                         const double2 *out_part, long long seg_len,
-                                                        const double2 *S1, int K, Partials part) {
+                                                        const double2 *S1, int K, const double2 *spread,
+                                                        Partials part) {
     if (!f->active) return;
     __shared__ double red[16], S[2];
     const bool band = (int)blockIdx.x >= p.nw;
@@ -1077,7 +1187,7 @@ __global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan
     double v[2] = {0.0, 0.0};
     for (int n = n0 + (band ? 0 : (int)threadIdx.x); n < n1; n += 256) {
         const double wx = p.wx[(size_t)(b0 + n) * p.wx_stride + iw];
-        if (!is_far(*f, wx)) continue;
+        if (!held(spread[n]) || !is_far(*f, wx)) continue;
         if (!band || threadIdx.x == 0) {
             const double2 x = far_series(*f, wx, S1 + (size_t)n * K, K);
             v[0] += x.x;
@@ -1151,17 +1261,32 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     far_plan_kernel<<<1, kBins, 0, s>>>(p, b0, bands, b.plan, z.cap_out, (float)z.R, (float)z.c0,
                                         w_near, mixed ? 16.f : 2.f);
     const int band_warps = ceil_div(bands, 8);
-    far_near_count_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.place);
+    far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
+    count_launch(4);
+    // The spread of each band, a pass per slab of chunks that `sy` and `res` hold.
+    const int yp = ceil_div(z.ngp, kCrtRowsY) * kCrtRowsY, np = ceil_div((long long)z.gm * z.ngp, kCrtRowsY) * kCrtRowsY;
+    const int spread_slab = (int)std::min<long long>(z.nch, 3ll * kCrtN / 4 * z.slab * (np / yp));
+    cudaError_t e = cudaGetLastError();
+    for (int c0 = 0; c0 < z.nch && e == cudaSuccess; c0 += spread_slab) {
+        const int nc = std::min(spread_slab, z.nch - c0);
+        float *V = reinterpret_cast<float *>(b.res);
+        far_sizes_kernel<false><<<z.Mp / 8 * nc, 128, 0, s>>>(p, b.plan, b0, bands, z.Mp, c0, nc, z.Kc, b.EA, b.SA, b.sx);
+        far_sizes_kernel<true><<<z.ngp / 8 * nc, 128, 0, s>>>(p, b.plan, 0, p.ng, z.ngp, c0, nc, z.Kc, b.E0, b.SQ, b.sy);
+        e = crt_sums(b.sx, b.sy, z.Mp, yp, z.Kc, nc, V, go, part.err, s);
+        far_spread_kernel<<<bands, 256, 0, s>>>(b.plan, b.C, b.EA, b.E0, b.SA, b.SQ, V, p.ng, z.ngp, z.Mp, yp, c0, nc, b.spread);
+        count_launch(3);
+    }
+    if (e != cudaSuccess) return e;
+    far_near_count_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.spread, b.place);
     far_near_scan_kernel<<<1, 1024, 0, s>>>(b.plan, bands, p.nw, b.place, z.cap_near, (float)z.c0, w_near);
-    far_near_list_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.place, b.near);
+    far_near_list_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.spread, b.place, b.near);
     far_count_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows);
     far_scan_kernel<<<1, 1024, 0, s>>>(p.ng, b.plan, b.rows);
     far_list_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows, b.out);
-    far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
-    far_need_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(p, b.plan, b0, bands, z.K, z.bits, b.terms);
+    far_need_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(p, b.plan, b0, bands, z.K, z.bits, b.spread, b.terms);
     far_order_kernel<<<ceil_div(bands, 256), 256, 0, s>>>(b.plan, bands, b.terms, b.order);
-    count_launch(12);
-    cudaError_t e = cudaGetLastError();
+    count_launch(8);
+    e = cudaGetLastError();
 
     // The series, a pass per group of terms of one level and slab of chunks.
     const OzOperand X{p.aqsn + (size_t)b0 * p.nc, p.nc, true, bands};
@@ -1183,6 +1308,7 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
                                                     k0 + gm >= z.K, b.sy, b.EY, b.E0, b.state);
             };
             switch (l) {
+                case kCrtWide: terms(far_terms_kernel<kCrtWide, false>); break;
                 case 0: mixed ? terms(far_terms_kernel<0, true>) : terms(far_terms_kernel<0, false>); break;
                 case 1: mixed ? terms(far_terms_kernel<1, true>) : terms(far_terms_kernel<1, false>); break;
                 case 2: mixed ? terms(far_terms_kernel<2, true>) : terms(far_terms_kernel<2, false>); break;
@@ -1215,10 +1341,10 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     }
     far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, (p.ng + 1) / 2, b.near_val);
     far_out_kernel<<<dim3(z.segs, ceil_div(bands, kOutBands), ceil_div(p.nw, kOutFreq)), 128, 0, s>>>(
-        p, b.plan, b.out, z.seg_len, b0, bands, b.C, b.out_part);
+        p, b.plan, b.out, z.seg_len, b0, bands, b.C, b.spread, b.out_part);
     far_final_kernel<<<p.nw + (part.n1 ? bands : 0), 256, 0, s>>>(p, b.plan, b0, bands, b.near, b.place,
                                                                   b.near_val, b.out_part, z.seg_len,
-                                                                  b.S1, z.K, part);
+                                                                  b.S1, z.K, b.spread, part);
     count_launch(3);
     return cudaGetLastError();
 }
