@@ -59,6 +59,7 @@
 // frequencies on average where a tile there shares its columns among 3.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 #include "gpp_crt.h"
 #include "gpp_crt_planes.cuh"
@@ -96,15 +97,29 @@ struct Sizes {
     double bits;         // what the series is cut at
     int K;               // its terms for a pair that is just far (at most 64)
     int Mp, ngp, nch, Kc;
+    int gr;              // rows per group (a multiple of 8)
     int gm, slab;        // series terms and chunks per pass
-    int cap_near;
+    bool x_all;          // X's planes of every chunk at once
+    int cap_near, near_rows;  // entries, row pairs per pass of the near kernel
     long long cap_out, seg_len;
     int segs;
     long long pairs;
     double c0;           // cost of the series, in per-term pairs
 };
 
+// The scratch a call may take, apart from what has the size of an input or
+// less: the planes and residues of a pass (with H, the sums they give, at most
+// half as much again), the recurrence's state of a group of rows and X's planes
+// half each, the near partials a quarter, the strays' an eighth.  A larger
+// call runs in more passes.  GPP_SERIES_PASS_MB overrides it, for tests.
 constexpr size_t kPassBytes = size_t(8) << 30;
+size_t pass_bytes() {
+    const char *v = getenv("GPP_SERIES_PASS_MB");
+    const long long mb = v ? atoll(v) : 0;
+    return mb > 0 ? (size_t)mb << 20 : kPassBytes;
+}
+size_t x_planes(int Mp, int Kc) { return (size_t)6 * kCrtN * Mp * Kc; }  // a chunk's
+
 // Term k counts R^-k; three bits more past the first, so that all of them
 // together round no worse than it does.
 int level_of(const Sizes &z, int k) {
@@ -139,12 +154,24 @@ Sizes sizes(const Problem &p, int bands, bool mixed) {
     z.ngp = ceil_div(p.ng, 8) * 8;
     z.nch = std::max(1, ceil_div(p.nc, kCrtChunk));
     z.Kc = ceil_div(ceil_div(p.nc, z.nch), kCrtBlockK) * kCrtBlockK;
-    const size_t per = (size_t)3 * kCrtN * z.ngp * (2 * (size_t)z.Kc + z.Mp);  // a term's, per chunk
-    z.gm = (int)std::min<size_t>(z.K, std::max<size_t>(4, kPassBytes / (per * z.nch)));
-    z.slab = (int)std::min<size_t>(z.nch, std::max<size_t>(1, kPassBytes / (per * z.gm)));
+    const size_t budget = pass_bytes();
+    const size_t row_state = (size_t)(mixed ? 48 : 32) * z.nch * z.Kc;
+    // Rows a group holds: their state, and four terms' planes and sums of a chunk.
+    const size_t plane_rows = budget / (12 * (size_t)kCrtN * (2 * z.Kc + z.Mp)), sum_rows = budget / 2 / (64 * (size_t)bands);
+    const size_t most = std::min({budget / 2 / row_state, plane_rows, sum_rows, (size_t)z.ngp});
+    const int groups = ceil_div(z.ngp, (long long)std::max<size_t>(8, most / 8 * 8));
+    z.gr = ceil_div(ceil_div(z.ngp, groups), 8) * 8;
+    const size_t per = (size_t)3 * kCrtN * z.gr * (2 * (size_t)z.Kc + z.Mp);  // a term's, per chunk
+    z.gm = (int)std::min<size_t>(z.K, std::max<size_t>(4, budget / (per * z.nch)));
+    z.gm = (int)std::min<size_t>(z.gm, std::max<size_t>(1, budget / 2 / (16 * (size_t)bands * z.gr)));
+    z.slab = (int)std::min<size_t>(z.nch, std::max<size_t>(1, budget / (per * z.gm)));
+    z.x_all = x_planes(z.Mp, z.Kc) * z.nch <= budget / 2;
+    if (!z.x_all) z.slab = (int)std::min<size_t>(z.slab, std::max<size_t>(1, budget / 2 / x_planes(z.Mp, z.Kc)));
     z.cap_near = (int)std::min<long long>(z.pairs / 2 + 1, 1 << 26);
+    z.near_rows = (int)std::min<size_t>((p.ng + 1) / 2, std::max<size_t>(1, budget / 4 / (sizeof(double2) * kNearFreq * z.cap_near)));
     z.cap_out = (long long)p.ng * p.nc / 32 + 1;
-    z.seg_len = std::max<long long>(2048, (z.cap_out + 511) / 512);
+    const long long segs = std::max<long long>(1, std::min<long long>(512, (long long)(budget / 8 / (sizeof(double2) * z.pairs))));
+    z.seg_len = std::max<long long>(2048, (z.cap_out + segs - 1) / segs);
     z.segs = (int)((z.cap_out + z.seg_len - 1) / z.seg_len);
     return z;
 }
@@ -167,7 +194,7 @@ struct Buffers {
     int *terms, *order;  // per band: its terms; the bands by their terms
     __nv_bfloat16 *sx, *sy;
     unsigned char *res;
-    double2 *H;        // [bands][gm ngp]
+    double2 *H;        // [bands][gm rows of a group]
 };
 
 size_t carve(const Sizes &z, void *ws, Buffers *b) {
@@ -179,8 +206,7 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
         return q;
     };
     Buffers o;
-    const size_t rt = (size_t)(z.ng + 1) / 2;
-    const int Np = ceil_div((long long)z.gm * z.ngp, kCrtRowsY) * kCrtRowsY;
+    const int Np = ceil_div((long long)z.gm * z.gr, kCrtRowsY) * kCrtRowsY;
     o.plan = reinterpret_cast<FarPlan *>(take(sizeof(FarPlan)));
     o.near = reinterpret_cast<int4 *>(take(sizeof(int4) * (size_t)z.cap_near));
     o.place = reinterpret_cast<int *>(take(sizeof(int) * ((size_t)kNearFreq * z.bands + 1)));
@@ -188,10 +214,10 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     o.out = reinterpret_cast<int2 *>(take(sizeof(int2) * (size_t)z.cap_out));
     o.C = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.ng));
     o.S1 = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.K));
-    o.near_part = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near * rt));
+    o.near_part = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near * z.near_rows));
     o.near_val = reinterpret_cast<double2 *>(take(sizeof(double2) * kNearFreq * (size_t)z.cap_near));
     o.out_part = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.segs * z.pairs));
-    o.state = take(sizeof(double2) * (z.mixed ? 3 : 2) * (size_t)z.nch * z.ngp * z.Kc);
+    o.state = take(sizeof(double2) * (z.mixed ? 3 : 2) * (size_t)z.nch * z.gr * z.Kc);
     o.terms = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.order = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.bands));
     o.E0 = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.ngp));
@@ -202,11 +228,11 @@ size_t carve(const Sizes &z, void *ws, Buffers *b) {
     o.EX = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.nch * z.Mp));
     o.EY = reinterpret_cast<int *>(take(sizeof(int) * (size_t)z.slab * Np));
     o.sx = reinterpret_cast<__nv_bfloat16 *>(
-        take(sizeof(__nv_bfloat16) * 3 * kCrtN * (size_t)z.Mp * z.nch * z.Kc));
+        take(x_planes(z.Mp, z.Kc) * (z.x_all ? z.nch : z.slab)));
     o.sy = reinterpret_cast<__nv_bfloat16 *>(
         take(sizeof(__nv_bfloat16) * 3 * kCrtN * (size_t)Np * z.slab * z.Kc));
     o.res = reinterpret_cast<unsigned char *>(take((size_t)z.slab * 3 * kCrtN * z.Mp * Np));
-    o.H = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.gm * z.ngp));
+    o.H = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)z.bands * z.gm * z.gr));
     if (b) *b = o;
     return off;
 }
@@ -656,11 +682,12 @@ __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
 // What the spread of a band is formed from: for 8 rows x one chunk the exponent
 // E of the largest |re|, |im|, the magnitudes over 2^E in bf16 (core-matrix
 // blocks of R rows) and their sum S.  Y: rows of Q, 0 outside the box; else
-// rows of aqsn.  A thread per 8 consecutive columns of a row, which it reads
-// twice (from L1 and L2 the second time).
+// rows of aqsn, from row b0 on; E and S have a row of ld per chunk.  A thread
+// per 8 consecutive columns of a row, which it reads twice (from L1 and L2 the
+// second time).
 template <bool Y>
 __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan *f, int b0, int L, int Lp,
-                                                        int c0, int nc, int Kc, int *E, float *S,
+                                                        int ld, int c0, int nc, int Kc, int *E, float *S,
                                                         __nv_bfloat16 *out) {
     constexpr int R = Y ? kCrtRowsY : kCrtRowsX;
     if (!f->active) return;
@@ -671,7 +698,7 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
     const int t = threadIdx.x, row = t & 7, l = l0 + row, kb = (c0 + c) * Kc, end = min(p.nc, kb + Kc);
     auto value = [&](int ig) {
         if (l >= L || ig >= end) return make_double2(0.0, 0.0);
-        const size_t at = (size_t)((Y ? 0 : b0) + l) * p.nc + ig;
+        const size_t at = (size_t)(b0 + l) * p.nc + ig;
         if constexpr (!Y) return __ldg(p.aqsn + at);
         const double2 wt = __ldg(p.wt + at);
         return in_box(*f, wt) ? cmul(wt, __ldg(p.ieps + at)) : make_double2(0.0, 0.0);
@@ -692,7 +719,7 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
     if (t < 8) {
         for (int w = 1; w < 4; ++w) mx = max(mx, red[w][t]);
         exps[t] = crt_exponent(mx);
-        E[(size_t)(c0 + c) * Lp + l0 + t] = exps[t];
+        E[(size_t)(c0 + c) * ld + l0 + t] = exps[t];
     }
     __syncthreads();
     const int e = exps[row], ksteps = nc * (Kc / kCrtBlockK);
@@ -726,25 +753,26 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
     total += __shfl_xor_sync(0xffffffffu, total, 16);
     if ((t & 24) == 0) sum[t >> 5][row] = total;
     __syncthreads();
-    if (t < 8) S[(size_t)(c0 + c) * Lp + l0 + t] = sum[0][t] + sum[1][t] + sum[2][t] + sum[3][t];
+    if (t < 8) S[(size_t)(c0 + c) * ld + l0 + t] = sum[0][t] + sum[1][t] + sum[2][t] + sum[3][t];
 }
 
-// spread[n] (+)= over the rows and chunks [c0, c0 + nc): |c| 2^(EA + E0) times
+// spread[n] (+)= over the rows [r0, r0 + rows) and chunks [c0, c0 + nc): |c| 2^(EA + E0) times
 // SA + SQ (the largest magnitudes count 1 each) and times V, the chunk's sum of
 // products.
 __global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const double2 *C, const int *EA,
                                                          const int *E0, const float *SA, const float *SQ,
-                                                         const float *V, int ng, int ngp, int Mp, int Np,
-                                                         int c0, int nc, double2 *spread) {
+                                                         const float *V, int ng, int ngp, int r0, int rows,
+                                                         int Mp, int Np, int c0, int nc, int add,
+                                                         double2 *spread) {
     if (!f->active) return;
     __shared__ double red[16], S[2];
     const int n = blockIdx.x;
     double v[2] = {0.0, 0.0};
-    for (int r = threadIdx.x; r < ng; r += 256) {
-        const double2 z = C[(size_t)n * ng + r];
+    for (int r = threadIdx.x; r < rows; r += 256) {
+        const double2 z = C[(size_t)n * ng + r0 + r];
         double a = 0.0, b = 0.0;
         for (int c = 0; c < nc; ++c) {
-            const size_t x = (size_t)(c0 + c) * Mp + n, y = (size_t)(c0 + c) * ngp + r;
+            const size_t x = (size_t)(c0 + c) * Mp + n, y = (size_t)(c0 + c) * ngp + r0 + r;
             const double w = scalbn(1.0, EA[x] + E0[y]);
             a = fma(w, (double)(SA[x] + SQ[y]), a);
             b = fma(w, (double)V[((size_t)c * Mp + n) * Np + r], b);
@@ -755,14 +783,15 @@ __global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const
     }
     block_reduce<2, 256>(v, red, S);
     if (threadIdx.x == 0) {
-        const double2 old = c0 == 0 ? make_double2(0.0, 0.0) : spread[n];
+        const double2 old = add ? spread[n] : make_double2(0.0, 0.0);
         spread[n] = make_double2(old.x + S[0], old.y + S[1]);
     }
 }
 
 // Residue planes and exponents of P_k, k = k0 .. k0 + gm - 1, for 8 rows x one
-// chunk at level L: row r of term m is row m ngp + r of the product's Y
-// operand, in the core-matrix blocks of crt_prep_kernel.  A thread carries 4
+// chunk at level L, of the gr rows from r0 on: row r0 + l of term m is row
+// m gr + l of the product's Y operand, in the core-matrix blocks of
+// crt_prep_kernel.  A thread carries 4
 // consecutive columns of a row (half a core-matrix row; 8 would halve the
 // resident warps) through the recurrence P_(k+1) = 2 z P_k - P_(k-1) (P_-1 =
 // z Q starts it) and leaves P_(k-1), P_k for the next pass in `state`.  The
@@ -778,16 +807,16 @@ constexpr int kTermK = 4;  // columns per thread
 // first pass reads the inputs, the next ones find z with the last two terms in
 // `state`.
 template <int L, bool DF>
-__global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int c0,
+__global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int r0, int gr, int c0,
                                                            int nc, int Kc, int Np, int k0, int gm,
                                                            int last, __nv_bfloat16 *out, int *EY,
                                                            const int *E0, void *state) {
     constexpr int NMOD = kCrtLevel[L].n, BITS = kCrtLevel[L].bits, ND = BITS > 41 ? 4 : BITS > 18 ? 3 : 2;
     if (!f->active) return;
     __shared__ int exps[8];
-    const int groups = ngp / 8;
+    const int groups = gr / 8;
     const int grp = blockIdx.x % groups, c = blockIdx.x / groups;
-    const int t = threadIdx.x, half = t & 1, row = (t >> 1) & 7, kg0 = t >> 4, r = grp * 8 + row;
+    const int t = threadIdx.x, half = t & 1, row = (t >> 1) & 7, kg0 = t >> 4, l = grp * 8 + row, r = r0 + l;
     const int kb = (c0 + c) * Kc, items = (Kc + 63) / 64;
     const double2 *wrow = p.wt + (size_t)min(r, p.ng - 1) * p.nc;
     const double2 *erow = p.ieps + (size_t)min(r, p.ng - 1) * p.nc;
@@ -797,7 +826,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
         wt = __ldg(wrow + ig);
         return in_box(*f, wt);
     };
-    if (t < 8) exps[t] = E0[(size_t)(c0 + c) * ngp + grp * 8 + t];
+    if (t < 8) exps[t] = E0[(size_t)(c0 + c) * ngp + r0 + grp * 8 + t];
     __syncthreads();
     const int e0 = exps[row];
     // x 2^-e0 in two exact steps (what is lost below 2^-1022 of the largest
@@ -808,7 +837,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
     const double log2_rho = f->log2_rho;
     auto raise = [&](int k) { return k == 0 ? 0 : 1 + (int)ceil(k * log2_rho); };
     if (half == 0)
-        for (int m = kg0; m < gm; m += 8) EY[(size_t)c * Np + (size_t)m * ngp + r] = e0 + raise(k0 + m);
+        for (int m = kg0; m < gm; m += 8) EY[(size_t)c * Np + (size_t)m * gr + l] = e0 + raise(k0 + m);
 
     const int ksteps = nc * (Kc / kCrtBlockK);
     const size_t plane = (size_t)Np * ksteps * kCrtBlockK;
@@ -860,7 +889,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
 #pragma unroll 1
             for (int m = 0; m < gm; ++m) {
                 const float scale = ldexpf(1.0f, BITS - raise(k0 + m));
-                const int y = m * ngp + grp * 8;
+                const int y = m * gr + grp * 8;
                 __nv_bfloat16 *w = out + ((size_t)(y / kCrtRowsY) * ksteps + ks) * (kCrtRowsY * kCrtBlockK) +
                                    (size_t)((y % kCrtRowsY) / 8) * 512 + kg0 * 64 + row * 8 + half * kTermK;
                 float2 dr[NP][ND], di[NP][ND];
@@ -914,7 +943,7 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
 #pragma unroll 1
         for (int m = 0; m < gm; ++m) {
             const int e = raise(k0 + m);
-            const int y = m * ngp + grp * 8;
+            const int y = m * gr + grp * 8;
             __nv_bfloat16 *w = out + ((size_t)(y / kCrtRowsY) * ksteps + ks) * (kCrtRowsY * kCrtBlockK) +
                                (size_t)((y % kCrtRowsY) / 8) * 512 + kg0 * 64 + row * 8 + half * kTermK;
             float2 dr[kTermK / 2][ND], di[kTermK / 2][ND];
@@ -958,11 +987,12 @@ __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarP
     }
 }
 
-// S1[n][k0 + m] = sum_r c[n][r] H[.][m ngp + r] for the band n at place
-// blockIdx.x of the order; 0 for a band without the term.
+// S1[n][k0 + m] (+)= sum over l < rows of c[n][r0 + l] H[.][m gr + l] for the
+// band n at place blockIdx.x of the order; 0 for a band without the term.
 __global__ void __launch_bounds__(256) far_fold_kernel(const FarPlan *f, const int *order,
                                                        const double2 *C, const double2 *H, int ng,
-                                                       int ngp, int ld, int k0, int K, double2 *S1) {
+                                                       int r0, int rows, int gr, int ld, int k0, int K,
+                                                       double2 *S1) {
     if (!f->active) return;
     __shared__ double red[16], S[2];
     const int at = blockIdx.x, n = order[at], m = blockIdx.y;
@@ -971,13 +1001,16 @@ __global__ void __launch_bounds__(256) far_fold_kernel(const FarPlan *f, const i
         if (threadIdx.x == 0) S1[(size_t)n * K + k0 + m] = make_double2(0.0, 0.0);
         return;
     }
-    for (int r = threadIdx.x; r < ng; r += 256) {
-        const double2 x = cmul(C[(size_t)n * ng + r], H[(size_t)at * ld + (size_t)m * ngp + r]);
+    for (int l = threadIdx.x; l < rows; l += 256) {
+        const double2 x = cmul(C[(size_t)n * ng + r0 + l], H[(size_t)at * ld + (size_t)m * gr + l]);
         v[0] += x.x;
         v[1] += x.y;
     }
     block_reduce<2, 256>(v, red, S);
-    if (threadIdx.x == 0) S1[(size_t)n * K + k0 + m] = make_double2(S[0], S[1]);
+    if (threadIdx.x == 0) {
+        double2 *o = S1 + (size_t)n * K + k0 + m;
+        *o = r0 ? cadd(*o, make_double2(S[0], S[1])) : make_double2(S[0], S[1]);
+    }
 }
 
 // Near pairs in FP64: a block takes a row pair x kNearTile entries, threads
@@ -987,7 +1020,7 @@ __global__ void __launch_bounds__(128) far_near_fp64_kernel(Problem p, FarNear n
     constexpr int RN = kNearTile, NF = kNearFreq, K = RN * 2 * NF * 2;
     __shared__ double red[4 * K], S[K];
     if (!*nr.active) return;
-    const int count = *nr.count, tiles = (count + RN - 1) / RN, pairs = (p.ng + 1) / 2;
+    const int count = *nr.count, tiles = (count + RN - 1) / RN, pairs = nr.pairs;
     const int nc = p.nc;
     constexpr int kRows = 16;  // row pairs in L2 while the entries stream past them
     __shared__ int item;
@@ -999,7 +1032,7 @@ __global__ void __launch_bounds__(128) far_near_fp64_kernel(Problem p, FarNear n
         const long long per = (long long)kRows * tiles;
         const int g = (int)(b / per), in = (int)(b % per);
         const int here = min(kRows, pairs - g * kRows);
-        const int rp = g * kRows + in % here, e0 = in / here * RN;
+        const int rp = nr.pair0 + g * kRows + in % here, e0 = in / here * RN;
         const double2 *wr_[2], *er_[2], *nrow[RN];
         double wx[RN][NF];
         int len[RN];
@@ -1070,10 +1103,11 @@ __global__ void __launch_bounds__(128) far_near_fp64_kernel(Problem p, FarNear n
     }
 }
 
-// near_val[entry][frequency] = the sum over row pairs, a warp per sum.
-__global__ void __launch_bounds__(256) far_near_sum_kernel(FarNear nr, int pairs, double2 *val) {
+// near_val[entry][frequency] (+)= the sum over the pass's row pairs, a warp per
+// sum.
+__global__ void __launch_bounds__(256) far_near_sum_kernel(FarNear nr, double2 *val) {
     if (!*nr.active) return;
-    const int lane = threadIdx.x & 31, count = *nr.count * kNearFreq;
+    const int lane = threadIdx.x & 31, count = *nr.count * kNearFreq, pairs = nr.pairs;
     for (int e = (blockIdx.x * 256 + threadIdx.x) >> 5; e < count; e += (gridDim.x * 256) >> 5) {
         double x = 0.0, y = 0.0;
         for (int r = lane; r < pairs; r += 32) {
@@ -1083,7 +1117,7 @@ __global__ void __launch_bounds__(256) far_near_sum_kernel(FarNear nr, int pairs
         }
         x = warp_sum(x);
         y = warp_sum(y);
-        if (lane == 0) val[e] = make_double2(x, y);
+        if (lane == 0) val[e] = nr.pair0 ? cadd(val[e], make_double2(x, y)) : make_double2(x, y);
     }
 }
 
@@ -1237,7 +1271,7 @@ bool far_eligible(const Problem &p, int bands, bool mixed) {
     const double cells = (double)p.ng * p.nc;
     const double per_pair = mixed ? 2.6e-12 : 20e-12;
     return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > (mixed ? 3e-3 : 2.2e-3) &&
-           z.pairs < (1 << 20) && cells < 2e9 &&
+           x_planes(z.Mp, z.Kc) <= kPassBytes / 2 && z.pairs < (1 << 20) && cells < 2e9 &&
            (z.pairs / 8 + 1) * ((p.ng + 1) / 2) < (1 << 30);  // the near kernel's tile counter
 }
 
@@ -1263,18 +1297,26 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     const int band_warps = ceil_div(bands, 8);
     far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
     count_launch(4);
-    // The spread of each band, a pass per slab of chunks that `sy` and `res` hold.
-    const int yp = ceil_div(z.ngp, kCrtRowsY) * kCrtRowsY, np = ceil_div((long long)z.gm * z.ngp, kCrtRowsY) * kCrtRowsY;
+    // The spread of each band, a pass per group of rows and slab of chunks that
+    // `sx`, `sy` and `res` hold (an x plane is 1 of 3 kCrtN).
+    const int yp = ceil_div(z.gr, kCrtRowsY) * kCrtRowsY, np = ceil_div((long long)z.gm * z.gr, kCrtRowsY) * kCrtRowsY;
     const int spread_slab = (int)std::min<long long>(z.nch, 3ll * kCrtN / 4 * z.slab * (np / yp));
     cudaError_t e = cudaGetLastError();
-    for (int c0 = 0; c0 < z.nch && e == cudaSuccess; c0 += spread_slab) {
-        const int nc = std::min(spread_slab, z.nch - c0);
-        float *V = reinterpret_cast<float *>(b.res);
-        far_sizes_kernel<false><<<z.Mp / 8 * nc, 128, 0, s>>>(p, b.plan, b0, bands, z.Mp, c0, nc, z.Kc, b.EA, b.SA, b.sx);
-        far_sizes_kernel<true><<<z.ngp / 8 * nc, 128, 0, s>>>(p, b.plan, 0, p.ng, z.ngp, c0, nc, z.Kc, b.E0, b.SQ, b.sy);
-        e = crt_sums(b.sx, b.sy, z.Mp, yp, z.Kc, nc, V, go, part.err, s);
-        far_spread_kernel<<<bands, 256, 0, s>>>(b.plan, b.C, b.EA, b.E0, b.SA, b.SQ, V, p.ng, z.ngp, z.Mp, yp, c0, nc, b.spread);
-        count_launch(3);
+    for (int r0 = 0; r0 < z.ngp && e == cudaSuccess; r0 += z.gr) {
+        const int gr = std::min(z.gr, z.ngp - r0), rows = std::min(gr, p.ng - r0);
+        const int sxc = z.x_all ? z.nch : 3 * kCrtN * z.slab, slab = std::min(spread_slab, sxc);
+        for (int c0 = 0; c0 < z.nch && e == cudaSuccess; c0 += slab) {
+            const int nc = std::min(slab, z.nch - c0);
+            float *V = reinterpret_cast<float *>(b.res);
+            far_sizes_kernel<false><<<z.Mp / 8 * nc, 128, 0, s>>>(p, b.plan, b0, bands, z.Mp, z.Mp, c0, nc, z.Kc,
+                                                                  b.EA, b.SA, b.sx);
+            far_sizes_kernel<true><<<gr / 8 * nc, 128, 0, s>>>(p, b.plan, r0, rows, gr, z.ngp, c0, nc, z.Kc,
+                                                               b.E0 + r0, b.SQ + r0, b.sy);
+            e = crt_sums(b.sx, b.sy, z.Mp, yp, z.Kc, nc, V, go, part.err, s);
+            far_spread_kernel<<<bands, 256, 0, s>>>(b.plan, b.C, b.EA, b.E0, b.SA, b.SQ, V, p.ng, z.ngp, r0,
+                                                    rows, z.Mp, yp, c0, nc, r0 + c0 > 0, b.spread);
+            count_launch(3);
+        }
     }
     if (e != cudaSuccess) return e;
     far_near_count_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.spread, b.place);
@@ -1288,64 +1330,74 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     count_launch(8);
     e = cudaGetLastError();
 
-    // The series, a pass per group of terms of one level and slab of chunks.
+    // The series, a pass per group of rows, group of terms of one level and slab
+    // of chunks.
     const OzOperand X{p.aqsn + (size_t)b0 * p.nc, p.nc, true, bands};
-    const size_t x_slab = (size_t)3 * kCrtN * z.Mp * z.slab * z.Kc;  // elements, at level 0
+    const size_t x_slab = x_planes(z.Mp, z.Kc) / sizeof(__nv_bfloat16) * z.slab;
     int level = -1;
-    for (int k0 = 0; k0 < z.K && e == cudaSuccess;) {
-        const int l = level_of(z, k0);
-        int gm = 1;
-        while (gm < z.gm && k0 + gm < z.K && level_of(z, k0 + gm) == l) ++gm;
-        const int rows = gm * z.ngp, Np = ceil_div(rows, kCrtRowsY) * kCrtRowsY;
-        for (int c0 = 0, q = 0; c0 < z.nch && e == cudaSuccess; c0 += z.slab, ++q) {
-            const int nc = std::min(z.slab, z.nch - c0);
-            __nv_bfloat16 *sx = b.sx + (size_t)q * x_slab;
-            int *ex = b.EX + (size_t)c0 * z.Mp;
-            if (l != level) e = crt_rows(X, b.order, z.Mp, p.nc, z.Kc, c0, nc, l, sx, ex, go, s);
-            if (e != cudaSuccess) break;
-            auto terms = [&](auto kern) {
-                kern<<<z.ngp / 8 * nc, 128, 0, s>>>(p, b.plan, z.ngp, c0, nc, z.Kc, Np, k0, gm,
-                                                    k0 + gm >= z.K, b.sy, b.EY, b.E0, b.state);
-            };
-            switch (l) {
-                case kCrtWide: terms(far_terms_kernel<kCrtWide, false>); break;
-                case 0: mixed ? terms(far_terms_kernel<0, true>) : terms(far_terms_kernel<0, false>); break;
-                case 1: mixed ? terms(far_terms_kernel<1, true>) : terms(far_terms_kernel<1, false>); break;
-                case 2: mixed ? terms(far_terms_kernel<2, true>) : terms(far_terms_kernel<2, false>); break;
-                default: mixed ? terms(far_terms_kernel<3, true>) : terms(far_terms_kernel<3, false>); break;
+    for (int r0 = 0; r0 < z.ngp && e == cudaSuccess; r0 += z.gr) {
+        const int gr = std::min(z.gr, z.ngp - r0), rows = std::min(gr, p.ng - r0);
+        for (int k0 = 0; k0 < z.K && e == cudaSuccess;) {
+            const int l = level_of(z, k0);
+            int gm = 1;
+            while (gm < z.gm && k0 + gm < z.K && level_of(z, k0 + gm) == l) ++gm;
+            const int N = gm * gr, Np = ceil_div(N, kCrtRowsY) * kCrtRowsY;
+            for (int c0 = 0, q = 0; c0 < z.nch && e == cudaSuccess; c0 += z.slab, ++q) {
+                const int nc = std::min(z.slab, z.nch - c0);
+                __nv_bfloat16 *sx = b.sx + (z.x_all ? q * x_slab : 0);
+                int *ex = b.EX + (size_t)c0 * z.Mp;
+                if (!z.x_all || l != level)
+                    e = crt_rows(X, b.order, z.Mp, p.nc, z.Kc, c0, nc, l, sx, ex, go, s);
+                if (e != cudaSuccess) break;
+                auto terms = [&](auto kern) {
+                    kern<<<gr / 8 * nc, 128, 0, s>>>(p, b.plan, z.ngp, r0, gr, c0, nc, z.Kc, Np, k0, gm,
+                                                     k0 + gm >= z.K, b.sy, b.EY, b.E0, b.state);
+                };
+                switch (l) {
+                    case kCrtWide: terms(far_terms_kernel<kCrtWide, false>); break;
+                    case 0: mixed ? terms(far_terms_kernel<0, true>) : terms(far_terms_kernel<0, false>); break;
+                    case 1: mixed ? terms(far_terms_kernel<1, true>) : terms(far_terms_kernel<1, false>); break;
+                    case 2: mixed ? terms(far_terms_kernel<2, true>) : terms(far_terms_kernel<2, false>); break;
+                    default: mixed ? terms(far_terms_kernel<3, true>) : terms(far_terms_kernel<3, false>); break;
+                }
+                count_launch();
+                const int *live = &b.plan->bands_at[k0];  // the most of the pass's terms
+                e = crt_products(sx, b.sy, z.Mp, Np, z.Kc, nc, 0, z.Mp / kCrtRowsX, l, b.res, z.Mp, go,
+                                 live, part.err, s);
+                if (e == cudaSuccess)
+                    e = crt_combine(b.res, ex, b.EY, 0, bands, z.Mp, N, z.Mp, Np, nc, l, c0 > 0, b.H, N, go,
+                                    live, s);
             }
+            level = l;
+            if (e != cudaSuccess) break;
+            far_fold_kernel<<<dim3(bands, gm), 256, 0, s>>>(b.plan, b.order, b.C, b.H, p.ng, r0, rows, gr, N,
+                                                            k0, z.K, b.S1);
             count_launch();
-            const int *live = &b.plan->bands_at[k0];  // the most of the pass's terms
-            e = crt_products(sx, b.sy, z.Mp, Np, z.Kc, nc, 0, z.Mp / kCrtRowsX, l, b.res, z.Mp, go,
-                             live, part.err, s);
-            if (e == cudaSuccess)
-                e = crt_combine(b.res, ex, b.EY, 0, bands, z.Mp, rows, z.Mp, Np, nc, l, c0 > 0, b.H,
-                                rows, go, live, s);
+            k0 += gm;
         }
-        level = l;
-        if (e != cudaSuccess) break;
-        far_fold_kernel<<<dim3(bands, gm), 256, 0, s>>>(b.plan, b.order, b.C, b.H, p.ng, z.ngp, rows, k0, z.K,
-                                                        b.S1);
-        count_launch();
-        k0 += gm;
     }
     if (e != cudaSuccess) return e;
 
-    const FarNear nr{b.near, &b.plan->n_near, go, b.C, b0, &b.plan->next, b.near_part};
-    if (mixed) {
-        e = launch_near_mixed(p, part, split_ws, nr, z.cap_near, s);
-        if (e != cudaSuccess) return e;
-    } else {
-        far_near_fp64_kernel<<<sms * 2, 128, 0, s>>>(p, nr);
+    for (int p0 = 0; p0 < (p.ng + 1) / 2; p0 += z.near_rows) {
+        if (p0 > 0 && (e = cudaMemsetAsync(&b.plan->next, 0, sizeof(int), s)) != cudaSuccess) return e;
+        const FarNear nr{b.near, &b.plan->n_near, go, b.C, b0, p0, std::min(z.near_rows, (p.ng + 1) / 2 - p0),
+                         &b.plan->next, b.near_part};
+        if (mixed) {
+            e = launch_near_mixed(p, part, split_ws, nr, z.cap_near, s);
+            if (e != cudaSuccess) return e;
+        } else {
+            far_near_fp64_kernel<<<sms * 2, 128, 0, s>>>(p, nr);
+            count_launch();
+        }
+        far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, b.near_val);
         count_launch();
     }
-    far_near_sum_kernel<<<sms, 256, 0, s>>>(nr, (p.ng + 1) / 2, b.near_val);
     far_out_kernel<<<dim3(z.segs, ceil_div(bands, kOutBands), ceil_div(p.nw, kOutFreq)), 128, 0, s>>>(
         p, b.plan, b.out, z.seg_len, b0, bands, b.C, b.spread, b.out_part);
     far_final_kernel<<<p.nw + (part.n1 ? bands : 0), 256, 0, s>>>(p, b.plan, b0, bands, b.near, b.place,
                                                                   b.near_val, b.out_part, z.seg_len,
                                                                   b.S1, z.K, b.spread, part);
-    count_launch(3);
+    count_launch(2);
     return cudaGetLastError();
 }
 

@@ -66,7 +66,7 @@ struct Partials {
 // A list of entries -- a band and up to kNearFreq consecutive frequencies -- to
 // sum term by term over every column (the near pairs of gpp_far.cu): each
 // entry's weighted sums over a row pair go to partial[entry][frequency][row
-// pair].
+// pair - pair0].
 constexpr int kNearFreq = 3;
 struct FarNear {
     const int4 *list;      // (band, first frequency, frequencies, 0)
@@ -74,6 +74,7 @@ struct FarNear {
     const int *active;     // 0: nothing to do
     const double2 *coeff;  // [bands][ng]: 0.5 vcoul conj(aqsm) at the row's G'
     int b0;                // the band of coeff's first row
+    int pair0, pairs;      // the row pairs of this launch
     int *next;             // the next tile to take (zeroed beforehand)
     double2 *partial;
 };
@@ -250,7 +251,7 @@ __device__ __forceinline__ void near_epilogue(const Problem &p, const FarNear &n
     const double *s = S + (n * 2 * NF + w) * 2;
     double2 tot = cmul(c[2 * rp], make_double2(s[0], s[1]));
     if (2 * rp + 1 < p.ng) tot = cadd(tot, cmul(c[2 * rp + 1], make_double2(s[NF * 2], s[NF * 2 + 1])));
-    nr.partial[((size_t)e * kNearFreq + w) * ((p.ng + 1) / 2) + rp] = tot;
+    nr.partial[((size_t)e * kNearFreq + w) * nr.pairs + rp - nr.pair0] = tot;
 }
 
 }  // namespace gpp

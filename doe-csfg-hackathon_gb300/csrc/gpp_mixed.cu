@@ -367,7 +367,7 @@ cudaError_t launch_flag_mixed_t(const Problem &p, const Partials &part, const Sp
 __global__ void __launch_bounds__(kWarps * 32, 4)
 near_mixed_kernel(Problem p, Partials part, SplitPlanes s, FarNear near) {
     if (!*near.active) return;
-    const int count = *near.count, tiles = (count + kWarps - 1) / kWarps, pairs = (p.ng + 1) / 2;
+    const int count = *near.count, tiles = (count + kWarps - 1) / kWarps, pairs = near.pairs;
     const long long per = (long long)kGroup * tiles;
     __shared__ int item;
     bool reinit = false;
@@ -379,7 +379,7 @@ near_mixed_kernel(Problem p, Partials part, SplitPlanes s, FarNear near) {
         const int g = (int)(b / per), in = (int)(b % per);
         const int here = min(kGroup, pairs - g * kGroup);
         if (!mixed_tile<1, 2, kNearFreq, kWarps, kNearCols, 2, kSyncBlock, true>(
-                p, part, s, 0, count, g * kGroup + in % here, in / here, 0, 0, reinit, &near))
+                p, part, s, 0, count, near.pair0 + g * kGroup + in % here, in / here, 0, 0, reinit, &near))
             return;  // abandoned after a bounded wait; the fault bit is set
         reinit = true;
         __syncthreads();
@@ -396,7 +396,7 @@ cudaError_t launch_near_mixed(const Problem &p, const Partials &part, void *spli
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     prefer_max_shared(near_mixed_kernel);
-    const long long most = (long long)ceil_div(cap, kWarps) * ((p.ng + 1) / 2);
+    const long long most = (long long)ceil_div(cap, kWarps) * near.pairs;
     const int grid = (int)std::min<long long>(most, (long long)std::max(sms, 1) * 4);
     near_mixed_kernel<<<grid, kWarps * 32, smem, st>>>(p, part, planes(p, split_ws), near);
     count_launch();
