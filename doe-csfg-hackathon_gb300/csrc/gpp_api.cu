@@ -30,6 +30,7 @@ thread_local int t_gemm_path = -1;         // -1: automatic, 0: never, 1: whenev
 thread_local bool t_timing = false;
 thread_local cudaEvent_t t_ev0 = nullptr, t_ev1 = nullptr;
 thread_local bool t_timed = false;
+thread_local size_t t_scratch_limit = ~(size_t)0;  // gpp_selftest_scratch_limit
 }  // namespace
 
 void count_launch(int n) { t_launches += (unsigned long long)n; }
@@ -113,6 +114,7 @@ gpp_status workspace_alloc(void **ptr, size_t bytes, cudaStream_t s) {
     cudaMemPool_t pool = nullptr;
     gpp_status st = device_setup(&dev, &err, &pool);
     if (st != GPP_OK) return st;
+    if (bytes > t_scratch_limit) return cuda_fail(cudaErrorMemoryAllocation, "workspace (self-test)");
     GPP_CUDA_TRY(cudaMallocFromPoolAsync(ptr, bytes, pool, s), "cudaMallocFromPoolAsync(workspace)");
     return GPP_OK;
 }
@@ -267,8 +269,12 @@ struct RowPieces {
     cudaEvent_t started[kMaxRowPieces] = {};  // optional: compute stream passed ready[k]
 };
 
+// held: scratch of the caller's (a batch plan), used where it is large enough
+// (the variant in effect may have changed since), so that nothing is allocated;
+// the call then leaves no kernel timing.  need: only reports what it takes.
 gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutSpec &o,
-                     bool do_main, cudaStream_t s, const RowPieces *pieces = nullptr) {
+                     bool do_main, cudaStream_t s, const RowPieces *pieces = nullptr,
+                     Scratch held = Scratch(), size_t *need = nullptr) {
     int dev = 0;
     int *err = nullptr;
     gpp_status st = device_setup(&dev, &err);
@@ -324,9 +330,16 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const size_t o_far = off;
     const size_t ws_bytes = off > 0 ? off : 256;
 
-    void *ws = nullptr;
-    if (far) {
-        st = workspace_alloc(&ws, off + far_bytes(p, nb1 - nb0, mixed), s);
+    const size_t far_ws_bytes = ws_bytes + (far ? far_bytes(p, nb1 - nb0, mixed) : 0);
+    if (need) {
+        *need = far_ws_bytes;
+        return GPP_OK;
+    }
+    const bool timing = t_timing && !held.ptr;
+    if (held.bytes < far_ws_bytes) held = Scratch();
+    void *ws = held.ptr;
+    if (far && !ws) {
+        st = workspace_alloc(&ws, far_ws_bytes, s);
         if (st == GPP_ERR_OUT_OF_MEMORY) {  // the per-term kernel needs much less
             cudaGetLastError();
             far = false;
@@ -334,8 +347,9 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
             return st;
         }
     }
-    if (!far) st = workspace_alloc(&ws, ws_bytes, s);
+    if (!far && !ws) st = workspace_alloc(&ws, ws_bytes, s);
     if (st != GPP_OK) return st;
+    auto release = [&] { return held.ptr ? cudaSuccess : cudaFreeAsync(ws, s); };
     char *w = static_cast<char *>(ws);
 
     Partials part{};
@@ -382,7 +396,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     if (overlap) {
         st = side_stream(dev, &side);
         if (st != GPP_OK) {
-            cudaFreeAsync(ws, s);
+            release();
             return st;
         }
     }
@@ -402,7 +416,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
         }
         if (e == cudaSuccess && has_noflag) {
             part.ach_tile0 = fused ? 0 : (int)tiles_f;
-            if (k == 0 && t_timing && t_ev0) cudaEventRecord(t_ev0, s);
+            if (k == 0 && timing && t_ev0) cudaEventRecord(t_ev0, s);
             if (gemm && mixed) {
                 st = GPP_OK;
                 if (k == 0 && tensor) {
@@ -420,7 +434,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
                     st = tensor ? gemm_per_band(p, part, w + o_gemm64, nb0, nb1, s, w + o_split)
                                 : mixed_gemm_per_band(p, part, w + o_split, w + o_gemm, nb0, nb1, s);
                 if (st != GPP_OK) {
-                    cudaFreeAsync(ws, s);
+                    release();
                     return st;
                 }
             } else if (gemm) {
@@ -433,7 +447,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
                                : gemm_rows(p, part, w + o_gemm, nb0, nb1, s, rt);
                 if (st == GPP_OK && k == pc.n - 1) st = gemm_per_band(p, part, w + o_gemm, nb0, nb1, s);
                 if (st != GPP_OK) {
-                    cudaFreeAsync(ws, s);
+                    release();
                     return st;
                 }
             } else if (!far) {
@@ -448,7 +462,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
                                                     RowTiles(), active)
                               : launch_noflag_fp64(p, part, nb0, nb1, s, RowTiles(), active);
             }
-            if (k == pc.n - 1 && t_timing && t_ev1) {
+            if (k == pc.n - 1 && timing && t_ev1) {
                 cudaEventRecord(t_ev1, s);
                 t_timed = true;
             }
@@ -487,7 +501,7 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
         jobs.add(reinterpret_cast<double2 *>(w + o_st), achs_blocks, achs_blocks, 1,
                  ReduceOut{o.achs, o.achs_re, o.achs_im, o.accumulate});
     if (e == cudaSuccess) e = launch_reduce(jobs, s);
-    cudaError_t e2 = cudaFreeAsync(ws, s);
+    cudaError_t e2 = release();
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync(workspace)");
     return GPP_OK;
@@ -604,9 +618,10 @@ int gpp_get_dropin_precision(void) { return dropin_precision(); }
 }  // extern "C"
 
 namespace {
-// gpp_sigma, optionally over G' rows that reach the device in pieces.
+// gpp_sigma, optionally over G' rows that reach the device in pieces, or in
+// scratch of the caller's (held, need: run_sigma).
 gpp_status sigma_impl(const gpp_problem *problem, const gpp_outputs *out, cudaStream_t s,
-                      const RowPieces *pieces) {
+                      const RowPieces *pieces, Scratch held = Scratch(), size_t *need = nullptr) {
     gpp_status st = validate(problem);
     if (st != GPP_OK) return st;
     if (!out || !out->achtemp || !out->asxtemp)
@@ -620,6 +635,7 @@ gpp_status sigma_impl(const gpp_problem *problem, const gpp_outputs *out, cudaSt
     o.n1 = reinterpret_cast<double2 *>(out->acht_n1_loc);
     o.achs = reinterpret_cast<double2 *>(out->achstemp);
     o.accumulate = 0;
+    if (need) return run_sigma(p, 0, p.nb, problem->precision, o, true, s, nullptr, Scratch(), need);
     if (o.n1 && (p.nb == 0 || p.ng == 0)) {
         cudaError_t e = cudaMemsetAsync(o.n1, 0, sizeof(double2) * (size_t)p.nb, s);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(acht_n1_loc)");
@@ -628,9 +644,22 @@ gpp_status sigma_impl(const gpp_problem *problem, const gpp_outputs *out, cudaSt
         cudaError_t e = cudaMemsetAsync(o.achs, 0, sizeof(double2), s);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(achstemp)");
     }
-    return run_sigma(p, 0, p.nb, problem->precision, o, true, s, pieces);
+    return run_sigma(p, 0, p.nb, problem->precision, o, true, s, pieces, held);
 }
 }  // namespace
+
+namespace gpp {
+gpp_status sigma_scratch(const gpp_problem &problem, const gpp_outputs &out, size_t *bytes) {
+    const gpp_status st = sigma_impl(&problem, &out, nullptr, nullptr, Scratch(), bytes);
+    if (st == GPP_OK && *bytes > t_scratch_limit)
+        return cuda_fail(cudaErrorMemoryAllocation, "workspace (self-test)");
+    return st;
+}
+gpp_status sigma_in_scratch(const gpp_problem &problem, const gpp_outputs &out, Scratch scratch,
+                            cudaStream_t s) {
+    return sigma_impl(&problem, &out, s, nullptr, scratch);
+}
+}  // namespace gpp
 
 extern "C" {
 
@@ -1203,6 +1232,11 @@ gpp_status gpp_selftest_wait_timeout(int polls, gpp_stream_t stream) {
     if (st != GPP_OK) return st;
     cudaError_t e = launch_wait_selftest(err, polls, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "wait self-test launch");
+    return GPP_OK;
+}
+
+gpp_status gpp_selftest_scratch_limit(size_t bytes) {
+    t_scratch_limit = bytes > 0 ? bytes : ~(size_t)0;
     return GPP_OK;
 }
 

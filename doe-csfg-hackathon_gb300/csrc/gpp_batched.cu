@@ -199,7 +199,9 @@ struct gpp_batch {
     std::vector<SplitPlanes> splits;
     std::vector<BatchItem> items;
     // States whose unoccupied bands take the series of gpp_far.cu: each runs
-    // as its own gpp_sigma call on the stream (the same bits as alone).
+    // as its own gpp_sigma call on the stream (the same bits as alone), one
+    // after the other in the scratch of the largest (none in a one-shot batch:
+    // from the library's pool, per call).
     std::vector<char> direct;
     std::vector<gpp_problem> direct_problems;
     std::vector<gpp_outputs> direct_outs;
@@ -225,6 +227,7 @@ struct gpp_batch {
     int *d_prefix = nullptr;
     int *d_heads = nullptr;
     char *d_split = nullptr;
+    Scratch direct_scratch;
     std::vector<int> achs_blocks;
     std::vector<std::pair<double2 *, size_t>> n1_zero;
     int launches_per_run = 0;
@@ -238,8 +241,15 @@ struct gpp_batch {
 
 namespace {
 
+// How the states that are large enough for the series run.
+enum class Direct {
+    kHeld,    // in scratch of the plan's
+    kPool,    // in scratch from the pool, allocated in the run
+    kNone,    // term by term, in the batch's own launches
+};
+
 gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outputs *outs,
-                      int nstates, size_t split_budget) {
+                      int nstates, size_t split_budget, Direct how) {
     const int precision = problems[0].precision;
     const int nw = problems[0].nw;
     const int sem = problems[0].semantics;
@@ -292,7 +302,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
         int achs_blocks;
     };
     std::vector<StateGeom> g(nstates);
-    size_t off = 0;
+    size_t off = 0, direct_bytes = 0;
     auto reserve = [&](size_t bytes) { size_t o = off; off = align256(off + bytes); return o; };
     const size_t off_probs = reserve(sizeof(Problem) * nstates);
     const size_t off_parts = reserve(sizeof(Partials) * nstates);
@@ -318,9 +328,15 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
         p.semantics = q.semantics;
         b->probs.push_back(p);
         StateGeom &s = g[i];
-        const bool direct = p.ng > 0 && far_eligible(p, p.nb - p.nv, mixed);
+        const bool direct = how != Direct::kNone && p.ng > 0 && far_eligible(p, p.nb - p.nv, mixed);
         b->direct.push_back(direct);
         if (direct) {
+            size_t bytes = 0;
+            if (how == Direct::kHeld) {
+                const gpp_status st = sigma_scratch(q, outs[i], &bytes);
+                if (st != GPP_OK) return st;
+            }
+            direct_bytes = std::max(direct_bytes, bytes);
             b->direct_problems.push_back(q);
             b->direct_outs.push_back(outs[i]);
         }
@@ -418,6 +434,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     const size_t off_jobs = reserve(sizeof(BatchReduce) * b->jobs.size());
     const size_t off_prefix = reserve(sizeof(int) * (b->jobs.size() + 1));
     const size_t off_split = reserve(mixed ? max_wave : 0);
+    const size_t off_direct = reserve(direct_bytes);
     b->dev_bytes = off;
 
     cudaError_t e = cudaGetDevice(&b->device);
@@ -432,6 +449,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     b->d_prefix = reinterpret_cast<int *>(d + off_prefix);
     b->d_heads = reinterpret_cast<int *>(d + off_heads);
     b->d_split = d + off_split;
+    if (direct_bytes) b->direct_scratch = Scratch{d + off_direct, direct_bytes};
 
     // Per-state partial pointers (the fault word is filled in by
     // upload_tables), split planes and reduction sources.
@@ -628,8 +646,8 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
     b->launches_per_run = launches;
     if (e != cudaSuccess) return set_error(GPP_ERR_CUDA, cudaGetErrorString(e));
     for (size_t k = 0; k < b->direct_problems.size(); ++k) {
-        const gpp_status st = gpp_sigma(&b->direct_problems[k], &b->direct_outs[k],
-                                        reinterpret_cast<gpp_stream_t>(s));
+        const gpp_status st =
+            sigma_in_scratch(b->direct_problems[k], b->direct_outs[k], b->direct_scratch, s);
         if (st != GPP_OK) return st;
     }
     return GPP_OK;
@@ -647,15 +665,21 @@ extern "C" {
 
 int *gpp_internal_fault_word(void);
 
-gpp_status gpp_batch_create(gpp_batch **out, const gpp_problem *problems,
-                            const gpp_outputs *outs, int nstates) {
+static gpp_status create_batch(gpp_batch **out, const gpp_problem *problems, const gpp_outputs *outs,
+                               int nstates, Direct how) {
     if (!out || nstates <= 0 || !problems || !outs)
         return set_error(GPP_ERR_INVALID_ARGUMENT, "bad batch arguments");
     *out = nullptr;
     int *fault = gpp_internal_fault_word();
     if (!fault) return set_error(GPP_ERR_CUDA, "could not set up the device fault word");
     gpp_batch *b = new gpp_batch();
-    gpp_status st = plan_batch(b, problems, outs, nstates, default_split_budget());
+    gpp_status st = plan_batch(b, problems, outs, nstates, default_split_budget(), how);
+    if (st == GPP_ERR_OUT_OF_MEMORY) {
+        // No room for the series' scratch: every state term by term.
+        cudaGetLastError();
+        *b = gpp_batch();
+        st = plan_batch(b, problems, outs, nstates, default_split_budget(), Direct::kNone);
+    }
     if (st == GPP_OK) st = upload_tables(b, fault);
     if (st == GPP_OK) {
         cudaError_t e = prepare(b);
@@ -668,6 +692,11 @@ gpp_status gpp_batch_create(gpp_batch **out, const gpp_problem *problems,
     }
     *out = b;
     return GPP_OK;
+}
+
+gpp_status gpp_batch_create(gpp_batch **out, const gpp_problem *problems,
+                            const gpp_outputs *outs, int nstates) {
+    return create_batch(out, problems, outs, nstates, Direct::kHeld);
 }
 
 gpp_status gpp_batch_run(gpp_batch *b, gpp_stream_t stream) {
@@ -712,7 +741,7 @@ gpp_status gpp_sigma_batched(const gpp_problem *problems, const gpp_outputs *out
         return set_error(GPP_ERR_INVALID_ARGUMENT, "bad batch");
     if (nstates == 0) return GPP_OK;
     gpp_batch *b = nullptr;
-    gpp_status st = gpp_batch_create(&b, problems, outs, nstates);
+    gpp_status st = create_batch(&b, problems, outs, nstates, Direct::kPool);
     if (st != GPP_OK) return st;
     st = enqueue(b, reinterpret_cast<cudaStream_t>(stream));
     count_launch(b->launches_per_run);

@@ -168,4 +168,15 @@ inline void prefer_max_shared(Kernel *kernel) {
         cudaGetLastError();
 }
 
+// gpp_sigma in scratch that the caller holds (gpp_api.cu; a batch plan's): the
+// bytes it needs with the settings in effect, GPP_ERR_OUT_OF_MEMORY where the
+// self-test forbids them, and a run, which allocates only if it needs more now.
+struct Scratch {
+    void *ptr = nullptr;
+    size_t bytes = 0;
+};
+gpp_status sigma_scratch(const gpp_problem &problem, const gpp_outputs &out, size_t *bytes);
+gpp_status sigma_in_scratch(const gpp_problem &problem, const gpp_outputs &out, Scratch scratch,
+                            cudaStream_t s);
+
 }  // namespace gpp

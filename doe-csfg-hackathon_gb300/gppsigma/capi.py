@@ -72,6 +72,7 @@ _SIGS = {
                                      C.POINTER(C.c_float)]),
     "gpp_context_last_trace": (_i, [_vp, C.POINTER(C.c_float), _i, C.POINTER(_i)]),
     "gpp_selftest_wait_timeout": (_i, [_i, _vp]),
+    "gpp_selftest_scratch_limit": (_i, [C.c_size_t]),
     "gpp_set_dropin_precision": (_i, [_i]),
     "gpp_get_dropin_precision": (_i, []),
     "gpp_set_gemm_path": (_i, [_i]),

@@ -191,8 +191,10 @@ typedef struct gpp_outputs {
  * sizes and the precision) sum the unoccupied (band, frequency) pairs whose
  * wx lies away from wtilde through a series on the tensor cores, to the same
  * precision, and the others term by term; where wtilde is spread so widely
- * that this does not pay, all of them term by term.  A state gives the same
- * bits through gpp_sigma, gpp_sigma_host and a batch. */
+ * that this does not pay, all of them term by term; so are bands whose aqsn is
+ * large just where wtilde I_eps is small.  The series takes up to 24 GB of
+ * scratch; where that cannot be had the sum is term by term.  With it, a state
+ * gives the same bits through gpp_sigma, gpp_sigma_host and a batch. */
 gpp_status gpp_sigma(const gpp_problem *problem, const gpp_outputs *out, gpp_stream_t stream);
 
 /* Waits for `stream` (at most timeout_ms; < 0 waits forever) and reports
@@ -263,8 +265,10 @@ gpp_status gpp_sigma_batched(const gpp_problem *problems, const gpp_outputs *out
                              gpp_stream_t stream);
 
 /* Reusable plan: the work list, device tables and scratch are built once
- * (gpp_batch_create allocates; the arrays behind the problems' pointers may
- * change contents between runs but not move).  gpp_batch_run enqueues a run
+ * (gpp_batch_create allocates, the scratch of the largest state that takes the
+ * series among it, and plans all states term by term where that cannot be had;
+ * runs allocate nothing; the arrays behind the problems' pointers may change
+ * contents between runs but not move).  gpp_batch_run enqueues a run
  * on `stream`; on a stream other than the legacy/per-thread default the
  * first run is captured into a CUDA graph and later runs replay it.
  * gpp_batch_destroy waits for outstanding runs and frees the plan. */
@@ -321,6 +325,11 @@ gpp_status gpp_probe_fma_peaks(double *fp64_tflops, double *fp32_tflops);
  * word.  The next gpp_wait on that stream returns GPP_ERR_DEVICE_TIMEOUT
  * once; the context stays usable. */
 gpp_status gpp_selftest_wait_timeout(int polls, gpp_stream_t stream);
+
+/* No counterpart in the reference.  Failure-path self-test, per host thread:
+ * scratch of more than `bytes` bytes counts as not to be had, as if the device
+ * were out of memory (0 restores). */
+gpp_status gpp_selftest_scratch_limit(size_t bytes);
 
 #ifdef __cplusplus
 }
