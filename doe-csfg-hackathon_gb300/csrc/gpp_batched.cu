@@ -561,6 +561,7 @@ cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
         if (nf > 0) {
             batched_flag_mixed_kernel<NWCF, 2><<<std::min(nf, b->grid_flag), kThreads, 0, s>>>(
                 b->d_probs, b->d_parts, b->d_splits, b->d_items + w.i0, nf, heads);
+            count_launch();
             e = cudaGetLastError();
         }
         if (e == cudaSuccess && nu > 0) {
@@ -577,6 +578,7 @@ cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
                 batched_noflag_mixed_kernel<RG, NWC><<<std::min(nu, b->grid), kThreads, b->smem,
                                                        s>>>(
                     b->d_probs, b->d_parts, b->d_splits, b->d_items + w.i_mid, nu, heads + 1);
+            count_launch();
             e = cudaGetLastError();
         }
     } else {
@@ -585,6 +587,7 @@ cudaError_t launch_persistent(gpp_batch *b, int wave, cudaStream_t s) {
         if (n > 0) {
             batched_fp64_kernel<RN, 2, NWC, NWCF><<<std::min(n, b->grid), kThreads, 0, s>>>(
                 b->d_probs, b->d_parts, b->d_items + w.i0, n, heads);
+            count_launch();
             e = cudaGetLastError();
         }
     }
@@ -606,17 +609,14 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b->d_heads, 0, sizeof(int) * 2 * b->waves.size(), s);
     for (size_t k = 0; k < b->n1_zero.size() && e == cudaSuccess; ++k)
         e = cudaMemsetAsync(b->n1_zero[k].first, 0, b->n1_zero[k].second, s);
-    int launches = 0;
     const int nwc = b->nw <= 4 ? b->nw : 8;
     for (size_t wv = 0; wv < b->waves.size() && e == cudaSuccess; ++wv) {
         const auto &w = b->waves[wv];
         if (b->precision == GPP_PRECISION_MIXED)
             for (int i = w.s0; i < w.s1 && e == cudaSuccess; ++i) {
                 const Problem &p = b->probs[i];
-                if (p.nb > 0 && p.ng > 0 && !b->direct[i]) {
+                if (p.nb > 0 && p.ng > 0 && !b->direct[i])
                     e = launch_split(p, b->d_split + w.split_off[i - w.s0], 0, p.nb, s);
-                    launches += 2;
-                }
             }
         if (e != cudaSuccess) break;
         switch (nwc) {
@@ -629,21 +629,17 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
                                          : launch_persistent<8, 4>(b, (int)wv, s);
                 break;
         }
-        launches += 2;
     }
-    for (size_t k = 0; k < b->achs.size() && e == cudaSuccess; ++k) {
+    for (size_t k = 0; k < b->achs.size() && e == cudaSuccess; ++k)
         e = launch_achstemp(b->probs[b->achs[k].first], b->achs[k].second, b->err, s);
-        ++launches;
-    }
     if (e == cudaSuccess && b->total_segs > 0) {
         // Same tree width as the one-state reduction, so a state gives the
         // same bits alone or in a batch.
         batched_reduce_kernel<512><<<b->total_segs, 512, 0, s>>>(b->d_jobs, b->d_prefix,
                                                                  (int)b->jobs.size());
+        count_launch();
         e = cudaGetLastError();
-        ++launches;
     }
-    b->launches_per_run = launches;
     if (e != cudaSuccess) return set_error(GPP_ERR_CUDA, cudaGetErrorString(e));
     for (size_t k = 0; k < b->direct_problems.size(); ++k) {
         const gpp_status st =
@@ -703,15 +699,17 @@ gpp_status gpp_batch_run(gpp_batch *b, gpp_stream_t stream) {
     if (!b) return set_error(GPP_ERR_INVALID_ARGUMENT, "batch is NULL");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread) {
-        gpp_status st = enqueue(b, s);
-        count_launch(b->launches_per_run);
-        return st;
+        return enqueue(b, s);
     }
     if (!b->graph) {
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return set_error(GPP_ERR_CUDA, cudaGetErrorString(e));
+        // The capture's launches count when a run makes them.
+        const unsigned long long before = gpp_launch_count();
         gpp_status st = enqueue(b, s);
+        b->launches_per_run = (int)(gpp_launch_count() - before);
+        count_launch(-b->launches_per_run);
         e = cudaStreamEndCapture(s, &g);
         if (st != GPP_OK) {
             if (g) cudaGraphDestroy(g);
@@ -744,7 +742,6 @@ gpp_status gpp_sigma_batched(const gpp_problem *problems, const gpp_outputs *out
     gpp_status st = create_batch(&b, problems, outs, nstates, Direct::kPool);
     if (st != GPP_OK) return st;
     st = enqueue(b, reinterpret_cast<cudaStream_t>(stream));
-    count_launch(b->launches_per_run);
     cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream));
     gpp_batch_destroy(b);
     return st;
