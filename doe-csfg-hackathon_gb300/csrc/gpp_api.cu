@@ -107,6 +107,25 @@ gpp_status device_setup(int *dev_out, int **err_out, cudaMemPool_t *pool_out = n
     return GPP_OK;
 }
 
+// Whether s is being captured and `bytes` is more than the device has free or
+// keeps for graphs: the allocation would only fail when the graph is launched.
+bool capture_lacks(size_t bytes, int dev, cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (c != cudaStreamCaptureStatusActive) return false;
+    size_t free_b = 0, total_b = 0;
+    unsigned long long reserved = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+        cudaDeviceGetGraphMemAttribute(dev, cudaGraphMemAttrReservedMemCurrent, &reserved) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes > free_b + reserved;
+}
+
 // Stream-ordered workspace from the library's pool of the current device.
 gpp_status workspace_alloc(void **ptr, size_t bytes, cudaStream_t s) {
     int dev = 0;
@@ -114,7 +133,7 @@ gpp_status workspace_alloc(void **ptr, size_t bytes, cudaStream_t s) {
     cudaMemPool_t pool = nullptr;
     gpp_status st = device_setup(&dev, &err, &pool);
     if (st != GPP_OK) return st;
-    if (bytes > t_scratch_limit) return cuda_fail(cudaErrorMemoryAllocation, "workspace (self-test)");
+    if (bytes > t_scratch_limit || capture_lacks(bytes, dev, s)) return cuda_fail(cudaErrorMemoryAllocation, "workspace");
     GPP_CUDA_TRY(cudaMallocFromPoolAsync(ptr, bytes, pool, s), "cudaMallocFromPoolAsync(workspace)");
     return GPP_OK;
 }

@@ -122,3 +122,28 @@ def test_no_room_for_the_series():
     assert not np.array_equal(got[0][0], want[0][0])
     assert _close(got, want, 1e-12) and _close([alone], want[:1], 1e-12)
     assert all(np.array_equal(x, y) for x, y in zip(got[0], alone))
+
+
+def test_no_room_inside_a_capture():
+    """The same inside a caller's capture, where the allocation is only a node of
+    the graph: the captured call sums term by term."""
+    from gppsigma import ops
+    lib = capi.load()
+    d = ops.DeviceInputs.from_host(_inputs()[0])
+    out = ops.sigma(d, "fp64")
+    ops.wait()
+    want = out.achtemp.cpu().numpy()
+    capi.check(lib.gpp_selftest_scratch_limit(64 << 20), "limit")
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.sigma(d, "fp64", out=out)
+    finally:
+        capi.check(lib.gpp_selftest_scratch_limit(0), "limit")
+    for _ in range(2):
+        out.achtemp.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = out.achtemp.cpu().numpy()
+        assert not np.array_equal(got, want)
+        assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
