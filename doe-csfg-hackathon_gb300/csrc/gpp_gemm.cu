@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(kOccThreads) gemm_occupied_kernel(Problem p, P
         if (f[w].most) t = make_double2(t.x + all.x, t.y + all.y);
         v[w * 4] = acc[w].x;
         v[w * 4 + 1] = acc[w].y;
-        v[w * 4 + 2] = flag_ssx_scale(f[w].c, t.x);
-        v[w * 4 + 3] = flag_ssx_scale(f[w].c, t.y);
+        v[w * 4 + 2] = flag_ssx_scale(f[w], t.x);
+        v[w * 4 + 3] = flag_ssx_scale(f[w], t.y);
     }
     block_reduce<K, kOccThreads>(v, red, S);
     const int w = threadIdx.x >> 1, asx = threadIdx.x & 1;

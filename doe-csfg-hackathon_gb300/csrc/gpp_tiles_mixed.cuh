@@ -481,8 +481,9 @@ __device__ __forceinline__ df2 df2_mask(const df2 &a, bool x, bool y) {
 }
 
 // An occupied-band term near the pole, in FP64 from the original inputs,
-// split to float-float: aqsn*sch (sr, si) and its wx^2 aqsn*ssx, less its
-// share of the sum over all columns (xr, xi).  Out of line: inlined, its FP64
+// split to float-float: aqsn*sch (sr, si) and its wx^2 aqsn*ssx (aqsn*ssx where
+// the frequency is not plain), less its share of the sum over all columns (xr,
+// xi).  Out of line: inlined, its FP64
 // code took registers from the float-float term loop.
 struct FlagPole {
     df sr, si, xr, xi;
@@ -510,6 +511,7 @@ struct FlagFreqM {
     float clear;   // max(limittwo, (1e-3 wx)^2) with a margin above rounding
     float keep;    // |wtilde|^2 clearly below the cutoff (or no cutoff)
     bool most, cut;
+    bool plain;    // else every term goes through FP64, and clear is infinite
 };
 
 // One occupied-band tile in mixed precision: the row pair row_tile, one band,
@@ -520,7 +522,8 @@ struct FlagFreqM {
 // away from the pole takes one straight-line path of packed instructions;
 // any other term works out each lane's branch (df_gt: exact near the
 // thresholds) and zeroes the lanes a branch does not take.  Terms within
-// 1e-3 |wx| of the pole are computed in FP64 from the inputs.
+// 1e-3 |wx| of the pole, and all of a frequency that is not plain, are computed
+// in FP64 from the inputs.
 // ~78 packed instructions per frequency of a row pair and ~96 per column on
 // the straight-line path; three blocks of four warps an SM cannot hide a
 // column's five loads behind them (the FMA pipe 53% busy), so each thread
@@ -562,6 +565,8 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
         f[w].keep = d.cut ? 0.99998f * f[w].c4.h : __int_as_float(0x7F800000);
         f[w].most = d.most;
         f[w].cut = d.cut;
+        f[w].plain = d.plain;
+        if (!d.plain) f[w].clear = __int_as_float(0x7F800000);
         bound64 = flag_bound(bound64, d);
         any_most |= d.most;
     }
@@ -641,7 +646,7 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
                 const df dg = df2_lane(d, g), wg = df2_lane(delwr, g);
-                pole[g] = dg.h < thr;
+                pole[g] = dg.h < thr || !f[w].plain;
                 in_a[g] = !pole[g] && df_gt(dg, df{kLim2H, kLim2L}) && df_gt(df{kLim1H, kLim1L}, wg);
                 inc[g] = in_a[g] && !(f[w].cut && df_gt(df2_lane(awt2, g), f[w].c4));
                 in_b[g] = !pole[g] && !in_a[g] && df_gt(wg, df{kTo1H, kTo1L});
@@ -710,7 +715,7 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
     double v[K];
 #pragma unroll
     for (int w = 0; w < NWC; ++w) {
-        const double wx = __ldg(wxp + min(iw0 + w, p.nw - 1));
+        const FlagFreq d = flag_freq<SEM>(__ldg(wxp + min(iw0 + w, p.nw - 1)));
 #pragma unroll
         for (int g = 0; g < RG; ++g) {
             const int k = (g * NWC + w) * 4;
@@ -721,8 +726,8 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
             }
             v[k] = to_double(df2_lane(as_r[w], g));
             v[k + 1] = to_double(df2_lane(as_i[w], g));
-            v[k + 2] = flag_ssx_scale(wx * wx, tr);
-            v[k + 3] = flag_ssx_scale(wx * wx, ti);
+            v[k + 2] = flag_ssx_scale(d, tr);
+            v[k + 3] = flag_ssx_scale(d, ti);
         }
     }
     block_reduce<K, THREADS>(v, red, S);
