@@ -310,8 +310,10 @@ gpp_status run_sigma(const Problem &p, int b0, int b1, int precision, const OutS
     const TileShape ns = mixed ? mixed_noflag_shape(p, variant) : fp64_noflag_shape(p);
     const bool want_n1 = o.n1 && p.nw >= 3 && p.ng > 0;
     const bool gemm = has_noflag && gemm_path(p.wx_stride, nb1 - nb0);
-    // One wx row, FP64: the occupied bands in the band sum's frequency pass.
-    const bool fused = gemm && has_flag && !mixed && !want_n1 && p.nv <= kRowsOccupiedMax;
+    // One wx row, FP64: the occupied bands in the band sum's frequency pass
+    // (whose chunks of frequencies go along grid.y).
+    const bool fused = gemm && has_flag && !mixed && !want_n1 && p.nv <= kRowsOccupiedMax &&
+                       ceil_div(p.nw, flag_nwc(p.nw)) <= 65535;
     const long long rows_f = has_flag ? ceil_div(p.ng, fs.rg) : 0;
     const long long rows_n = has_noflag ? ceil_div(p.ng, ns.rg) : 0;
     const long long tiles_f = fused ? rows_f * gemm_row_parts(p) : has_flag ? rows_f * (fb1 - fb0) : 0;
