@@ -71,6 +71,8 @@ namespace gpp {
 struct FarPlan {
     int active;
     int next;            // the near kernel's tile counter
+    int planned;         // blocks of the plan that are done
+    unsigned long long best;  // the best box so far: its cost's bits, and bins
     int n_near;
     long long n_out;
     int lo, hi;          // the box's bins of Re(wtilde)
@@ -104,7 +106,9 @@ struct Sizes {
     long long cap_out, seg_len;
     int segs;
     long long pairs;
-    double c0;           // cost of the series, in per-term pairs
+    double c0;           // cost of the series at full occupancy, in per-term pairs
+    float c0_call;       // as the call's sizes leave it (planes, launches, grids that do not fill)
+    float near_least;    // near pairs that fill the near kernel's first round
 };
 
 // The scratch a call may take, apart from what has the size of an input or
@@ -152,8 +156,24 @@ Sizes sizes(const Problem &p, int bands, bool mixed) {
     z.K = (int)std::ceil(z.bits / std::log2(z.R));
     z.c0 = z.K * term;
     z.ngp = ceil_div(p.ng, 8) * 8;
+    z.near_least = mixed ? 0.f : 152.f * 4 * 1.8f / ceil_div(p.ng, 2);
     z.nch = std::max(1, ceil_div(p.nc, kCrtChunk));
     z.Kc = ceil_div(ceil_div(p.nc, z.nch), kCrtBlockK) * kCrtBlockK;
+    // The same in time (ps), from the kernels' own rates: terms 14 a term and cell
+    // from about 400 blocks on, the combination 0.018 a term, cell and band from
+    // 760, the products 0.0316 a term, cell and padded band or the bytes of their
+    // planes at 6 TB/s, X's planes 17 a level, band and column, the spread 30 a
+    // value, and 150 us of launches.  FP64, 192 x 33 x 25601 x 1: 3.9 ms of these
+    // and 1.8 of near pairs, which c0 put at 1.1 and 0.6 (per term 5.3); 420 x 17 x
+    // 7937 x 3: 2.3 + 1.1 where per term takes 4.0.
+    {
+        const double cells = (double)z.ngp * p.nc, kt = z.K * cells, x = (double)z.Mp * p.nc;
+        const double blocks = z.ngp / 8.0 * z.nch, quads = z.K / 5.0 * bands * z.ngp / 512;
+        const double t = 14 * kt * std::max(1.0, 400 / blocks) + 0.018 * bands * kt * std::max(1.0, 760 / quads) +
+                         std::max(0.0316 * z.Mp * kt, (64 * kt + 5 * 64 * x) / 6) + 5 * 17 * x +
+                         30 * (cells + x) + 1.5e8;
+        z.c0_call = (float)(t / ((mixed ? 2.6 : 20) * (double)p.ng * p.nc));
+    }
     const size_t budget = pass_bytes();
     const size_t row_state = (size_t)(mixed ? 48 : 32) * z.nch * z.Kc;
     // Rows a group holds: their state, and four terms' planes and sums of a chunk.
@@ -263,8 +283,8 @@ __device__ __forceinline__ bool is_far(const FarPlan &f, double wx) {
 __global__ void __launch_bounds__(1024) far_range_kernel(Problem p, int b0, int bands, FarPlan *f) {
     __shared__ double lo[32], hi[32];
     double a = 1.0 / 0.0, b = -1.0 / 0.0;
-    const long long n = (long long)bands * p.nw;
-    for (long long i = threadIdx.x; i < n; i += 1024) {
+    const unsigned n = (unsigned)bands * p.nw;  // below 2^20
+    for (unsigned i = threadIdx.x; i < n; i += 1024) {
         const double x = p.wx[(size_t)(b0 + i / p.nw) * p.wx_stride + i % p.nw];
         if (is_finite(x)) {
             a = fmin(a, x);
@@ -285,13 +305,18 @@ __global__ void __launch_bounds__(1024) far_range_kernel(Problem p, int b0, int 
         f->im[i] = 0;
     }
     __syncthreads();
+    if (threadIdx.x >= 32) return;
+    a = lo[threadIdx.x];
+    b = hi[threadIdx.x];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, s));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, s));
+    }
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 32; ++w) {
-            a = fmin(a, lo[w]);
-            b = fmax(b, hi[w]);
-        }
-        f->active = f->n_near = f->next = 0;
+        f->active = f->n_near = f->next = f->planned = 0;
         f->n_out = 0;
+        f->best = ~0ull;
         const double margin = 0.02 * (b - a) + 1e-3 * fmax(fabs(a), fabs(b));
         const double width = b - a + 2.0 * margin;
         // No finite wx, all zero, or a range past what the bins can divide: no bins.
@@ -346,90 +371,120 @@ __device__ __forceinline__ Box box_of(float a, float b, float v) {
     return q;
 }
 
-// One block: chooses the box.  The cost of a box is what it leaves to the
-// per-term kernels, in pairs over all columns: its near pairs (times w_near),
-// and the strays' share of the far ones (times w_out).
+// Chooses the box.  The cost of a box is what it leaves to the per-term
+// kernels, in pairs over all columns: its near pairs (times w_near), and the
+// strays' share of the far ones (times w_out).  A warp takes one first bin, its
+// lanes the last bins; the block that ends last takes the cheapest box of all
+// (the smallest key, whatever the order).  Where no box pays, this and the
+// launches that then return at once are what the series costs the call: with
+// one block for the choice, 64 us of 4.3 ms.
+constexpr int kPlanBlocks = kBins / 16;
 __global__ void __launch_bounds__(kBins) far_plan_kernel(Problem p, int b0, int bands, FarPlan *f,
                                                          long long cap_out, float R, float c0,
-                                                         float w_near, float w_out) {
-    __shared__ unsigned long long pre[kBins + 1];
-    __shared__ unsigned pairs_in[kBins];
-    __shared__ unsigned ppre[kBins + 1];
+                                                         float w_near, float near_least, float w_out) {
+    __shared__ unsigned long long pre[kBins + 1], warp_cells[kBins / 32];
+    __shared__ unsigned pairs_in[kBins], ppre[kBins + 1], warp_pairs[kBins / 32];
     __shared__ float vb[kBins];
-    __shared__ unsigned long long best[kBins / 32];
-    __shared__ int outside;
+    __shared__ int outside, last;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const long long n = (long long)bands * p.nw;
+    const unsigned n = (unsigned)bands * p.nw;
     const long long cells = (long long)p.ng * p.nc;
     if (t == 0) outside = 0;
     pairs_in[t] = 0;
     vb[t] = __uint_as_float(f->im[t]);
     __syncthreads();
-    auto wx_at = [&](long long i) {
-        return p.wx[(size_t)(b0 + i / p.nw) * p.wx_stride + i % p.nw];
-    };
-    for (long long i = t; i < n; i += kBins) {
-        const int b = bin_of(*f, make_double2(wx_at(i), 0.0));
+    for (unsigned i = t; i < n; i += kBins) {
+        const double x = p.wx[(size_t)(b0 + i / p.nw) * p.wx_stride + i % p.nw];
+        const int b = bin_of(*f, make_double2(x, 0.0));
         if (b >= 0)
             atomicAdd(&pairs_in[b], 1u);
         else
             atomicAdd(&outside, 1);  // not finite: always near
     }
     __syncthreads();
-    if (t == 0) {
-        pre[0] = 0;
-        ppre[0] = 0;
-        for (int i = 0; i < kBins; ++i) {
-            pre[i + 1] = pre[i] + f->count[i];
-            ppre[i + 1] = ppre[i] + pairs_in[i];
+    // Cells and pairs before each bin.
+    unsigned long long c = f->count[t];
+    unsigned q = pairs_in[t];
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const unsigned long long uc = __shfl_up_sync(0xffffffffu, c, s);
+        const unsigned uq = __shfl_up_sync(0xffffffffu, q, s);
+        if (lane >= s) {
+            c += uc;
+            q += uq;
         }
     }
+    if (lane == 31) {
+        warp_cells[warp] = c;
+        warp_pairs[warp] = q;
+    }
+    __syncthreads();
+    for (int k = 0; k < warp; ++k) {
+        c += warp_cells[k];
+        q += warp_pairs[k];
+    }
+    pre[t + 1] = c;
+    ppre[t + 1] = q;
+    if (t == 0) pre[0] = ppre[0] = 0;
     __syncthreads();
     const float w = (float)(1.0 / f->inv_w), total = (float)n, ncells = (float)cells;
+    const int lo = blockIdx.x * (kBins / 32) + warp;
     unsigned long long mine = ~0ull;
-    if (pre[t + 1] > pre[t] && f->inv_w > 0.0) {
-        float v = 0.f;
-        for (int j = t; j < kBins; ++j) {
-            v = fmaxf(v, vb[j]);
-            if (pre[j + 1] == pre[j]) continue;
-            const long long out = cells - (long long)(pre[j + 1] - pre[t]);
+    if (pre[lo + 1] > pre[lo] && f->inv_w > 0.0) {
+        float before = 0.f;  // the largest |Im| of the bins lo .. j0 - 1
+        for (int j0 = lo; j0 < kBins; j0 += 32) {
+            const int j = j0 + lane;
+            float v = j < kBins ? vb[j] : 0.f;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const float u = __shfl_up_sync(0xffffffffu, v, s);
+                if (lane >= s) v = fmaxf(v, u);
+            }
+            v = fmaxf(v, before);
+            before = __shfl_sync(0xffffffffu, v, 31);
+            if (j >= kBins || pre[j + 1] == pre[j]) continue;
+            const long long out = cells - (long long)(pre[j + 1] - pre[lo]);
             if (out > cap_out) continue;
-            const Box q = box_of(t * w, (j + 1) * w, v);
-            const float r = R * q.rho, d = q.h * 0.5f * (r + 1.f / r);
-            const int i0 = max(0, min(kBins, (int)floorf((q.z0 - d) / w)));
-            const int i1 = max(0, min(kBins, (int)floorf((q.z0 + d) / w) + 1));
+            const Box bx = box_of(lo * w, (j + 1) * w, v);
+            const float r = R * bx.rho, d = bx.h * 0.5f * (r + 1.f / r);
+            const int i0 = max(0, min(kBins, (int)floorf((bx.z0 - d) / w)));
+            const int i1 = max(0, min(kBins, (int)floorf((bx.z0 + d) / w) + 1));
             const float nr = (float)(ppre[i1] - ppre[i0]) + (float)outside;
-            const float cost = nr * w_near + (float)out / ncells * (total - nr) * w_out;
+            const float cost = (nr > 0.f ? fmaxf(nr, near_least) : 0.f) * w_near + (float)out / ncells * (total - nr) * w_out;
             const unsigned long long key =
-                ((unsigned long long)__float_as_uint(fmaxf(cost, 0.f)) << 32) | (unsigned)(t * kBins + j);
+                ((unsigned long long)__float_as_uint(fmaxf(cost, 0.f)) << 32) | (unsigned)(lo * kBins + j);
             if (key < mine) mine = key;
         }
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) mine = min(mine, __shfl_xor_sync(0xffffffffu, mine, s));
-    if (lane == 0) best[warp] = mine;
+    if (lane == 0 && mine != ~0ull) atomicMin(&f->best, mine);
+    __threadfence();
     __syncthreads();
-    if (t == 0) {
-        for (int i = 1; i < kBins / 32; ++i) mine = min(mine, best[i]);
-        if (mine != ~0ull && __uint_as_float((unsigned)(mine >> 32)) + c0 < 0.9f * total) {
-            const int lo = (int)((unsigned)mine / kBins), hi = (int)((unsigned)mine % kBins);
-            float v = 0.f;
-            for (int j = lo; j <= hi; ++j) v = fmaxf(v, vb[j]);
-            const Box q = box_of(lo * w, (hi + 1) * w, v);
-            f->lo = lo;
-            f->hi = hi;
-            f->n_out = cells - (long long)(pre[hi + 1] - pre[lo]);
-            // In double, with margins above the float rounding of the choice.
-            const double a = f->x0 + lo / f->inv_w, b = f->x0 + (hi + 1) / f->inv_w;
-            f->z0 = 0.5 * (a + b);
-            f->h = fmax((double)q.h, 0.5 * (b - a));
-            f->inv_h = 1.0 / f->h;
-            const double rho = (double)q.rho * 1.00001, r = (double)R * rho;
-            f->log2_rho = log2(rho);
-            f->dfar = f->h * 0.5 * (r + 1.0 / r);
-            f->active = 1;
-        }
-    }
+    if (t == 0) last = atomicAdd(&f->planned, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last || warp != 0) return;
+    __threadfence();
+    mine = *static_cast<volatile unsigned long long *>(&f->best);
+    if (mine == ~0ull || !(__uint_as_float((unsigned)(mine >> 32)) + c0 < 0.9f * total)) return;
+    const int a0 = (int)((unsigned)mine / kBins), a1 = (int)((unsigned)mine % kBins);
+    float v = 0.f;
+    for (int j = a0 + lane; j <= a1; j += 32) v = fmaxf(v, vb[j]);
+    v = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+    if (lane != 0) return;
+    const Box bx = box_of(a0 * w, (a1 + 1) * w, v);
+    f->lo = a0;
+    f->hi = a1;
+    f->n_out = cells - (long long)(pre[a1 + 1] - pre[a0]);
+    // In double, with margins above the float rounding of the choice.
+    const double a = f->x0 + a0 / f->inv_w, b = f->x0 + (a1 + 1) / f->inv_w;
+    f->z0 = 0.5 * (a + b);
+    f->h = fmax((double)bx.h, 0.5 * (b - a));
+    f->inv_h = 1.0 / f->h;
+    const double rho = (double)bx.rho * 1.00001, r = (double)R * rho;
+    f->log2_rho = log2(rho);
+    f->dfar = f->h * 0.5 * (r + 1.0 / r);
+    f->active = 1;
 }
 
 // An entry of the near list covers up to kNearFreq consecutive near
@@ -475,7 +530,8 @@ __global__ void __launch_bounds__(256) far_near_count_kernel(Problem p, const Fa
 // The counts become places, the longest entries first, so that the warps of a
 // block have equal work; the plan is dropped if too many pairs are near.
 __global__ void __launch_bounds__(1024) far_near_scan_kernel(FarPlan *f, int bands, int nw, int *count,
-                                                             int cap_near, float c0, float w_near) {
+                                                             int cap_near, float c0, float w_near,
+                                                             float near_least) {
     if (!f->active) return;
     __shared__ int part[1024];
     __shared__ unsigned long long pairs;
@@ -500,7 +556,7 @@ __global__ void __launch_bounds__(1024) far_near_scan_kernel(FarPlan *f, int ban
             acc += v;
         }
         const float total = (float)((long long)bands * nw);
-        if (pairs > (unsigned long long)cap_near || (float)pairs * w_near + c0 >= 0.95f * total)
+        if (pairs > (unsigned long long)cap_near || fmaxf((float)pairs, near_least) * w_near + c0 >= 0.95f * total)
             f->active = 0;
         f->n_near = acc;
         count[n] = acc;
@@ -1270,6 +1326,10 @@ bool far_eligible(const Problem &p, int bands, bool mixed) {
     // / 1.81, 1.86 / 1.91, 2.97 / 2.26, 2.88 / 2.08).
     const double cells = (double)p.ng * p.nc;
     const double per_pair = mixed ? 2.6e-12 : 20e-12;
+    // Calls whose sizes leave no gain do not plan (330 x 73 x 25601 x 2, mixed:
+    // 5.2 ms through the series, 3.9 per term); FP64's per-term pairs cost up to
+    // 1.6 of their 20 ps on such sizes, and the device decides.
+    if (z.c0_call > (mixed ? 0.8 : 1.5) * z.pairs) return false;
     return z.c0 + 0.25 * z.pairs < 0.8 * z.pairs && cells * z.pairs * per_pair > (mixed ? 3e-3 : 2.2e-3) &&
            x_planes(z.Mp, z.Kc) <= kPassBytes / 2 && z.pairs < (1 << 20) && cells < 2e9 &&
            (z.pairs / 8 + 1) * ((p.ng + 1) / 2) < (1 << 30);  // the near kernel's tile counter
@@ -1292,8 +1352,8 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     far_range_kernel<<<1, 1024, 0, s>>>(p, b0, bands, b.plan);
     far_hist_kernel<<<sms * 4, 256, 0, s>>>(p, b.plan);
     const float w_near = 1.4f;
-    far_plan_kernel<<<1, kBins, 0, s>>>(p, b0, bands, b.plan, z.cap_out, (float)z.R, (float)z.c0,
-                                        w_near, mixed ? 16.f : 2.f);
+    far_plan_kernel<<<kPlanBlocks, kBins, 0, s>>>(p, b0, bands, b.plan, z.cap_out, (float)z.R, z.c0_call,
+                                                  w_near, z.near_least, mixed ? 16.f : 2.f);
     const int band_warps = ceil_div(bands, 8);
     far_coeff_kernel<<<sms * 4, 256, 0, s>>>(p, b0, bands, b.C, b.plan, part.err);
     count_launch(4);
@@ -1320,7 +1380,8 @@ cudaError_t far_unoccupied(const Problem &p, const Partials &part, void *ws, voi
     }
     if (e != cudaSuccess) return e;
     far_near_count_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.spread, b.place);
-    far_near_scan_kernel<<<1, 1024, 0, s>>>(b.plan, bands, p.nw, b.place, z.cap_near, (float)z.c0, w_near);
+    far_near_scan_kernel<<<1, 1024, 0, s>>>(b.plan, bands, p.nw, b.place, z.cap_near, z.c0_call, w_near,
+                                             z.near_least);
     far_near_list_kernel<<<band_warps, 256, 0, s>>>(p, b.plan, b0, bands, b.spread, b.place, b.near);
     far_count_kernel<<<p.ng, 256, 0, s>>>(p, b.plan, b.rows);
     far_scan_kernel<<<1, 1024, 0, s>>>(p.ng, b.plan, b.rows);
