@@ -114,16 +114,23 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-# With per-band frequencies a large call sums its unoccupied bands through the
-# series of gpp_far.cu: `kernel_ms` then covers these kernels together, and the
-# flops counted are those of the per-term sum they replace.
+# With per-band frequencies a large call may sum its unoccupied bands through
+# the series of gpp_far.cu: `kernel_ms` then covers these kernels together, and
+# the per-term flops they replace say nothing of a rate: they are given as such,
+# without a fraction of a peak.
 SERIES_KERNELS = {
     "mixed": "near_mixed_kernel, crt_gemm_kernel, far_terms_kernel, crt_combine_kernel, far_out_kernel",
     "fp64": "far_near_fp64_kernel, crt_gemm_kernel, far_terms_kernel, crt_combine_kernel, far_out_kernel"}
-SERIES_NOTE = ("flops of the per-term sum over the time of the kernels that replace it (tensor-core "
-               "products of a series, and the per-term kernel where wx is near wtilde): a "
-               "fraction above 1 is work not done, not a rate; profiles/ncu_series_profile.txt "
-               "has each kernel's own")
+SERIES_NOTE = ("per_term_equivalent: flops of the per-term sum over the time of the kernels that "
+               "replace it (tensor-core products of a series, and the per-term kernel where wx is "
+               "near wtilde), not a rate of theirs; profiles/ncu_series_profile.txt has each "
+               "kernel's own")
+
+
+def series_roofline(bound: str, equivalent: float | None, peak: float, precision: str) -> dict:
+    """The roofline entry of a run that took the series."""
+    return {"bound": bound, "achieved": None, "peak": peak, "unit": "TFLOP/s", "frac": None,
+            "per_term_equivalent": equivalent, "kernel": SERIES_KERNELS[precision], "note": SERIES_NOTE}
 
 
 def profile_traffic(kernel: str, workload: str, precision: str):
@@ -551,6 +558,20 @@ def main() -> int:
         ms = gdist.max_over_ranks(e0.elapsed_time(e1) / steps, dist, "cuda")
         return out, ms, kern_ms, launches
 
+    def series_ran(precision: str, out, launches: int, steps: int) -> bool:
+        """Whether the device took the series: the launches are made either way,
+        but with the series' scratch refused the call is the per-term kernels',
+        whose bits differ."""
+        if launches <= 20 * steps:  # a per-term call makes fewer than ten
+            return False
+        capi.check(lib.gpp_selftest_scratch_limit(int(2e9 * input_gb) + (64 << 20)), "scratch limit")
+        try:
+            per_term = ops.sigma(d, precision)
+            ops.wait()
+        finally:
+            capi.check(lib.gpp_selftest_scratch_limit(0), "scratch limit")
+        return not torch.equal(per_term.achtemp, out.achtemp)
+
     fp64_peak, fp32_peak = 0.0, 0.0
     if rank == 0:
         import ctypes as C
@@ -571,13 +592,14 @@ def main() -> int:
     clocks = ClockSampler(local)
     clocks.start()
     res, ms, kern_ms, launches = timed(precision, args.steps, args.warmup)
-    series = launches > 20 * args.steps  # a per-term call makes fewer than ten launches
     clk = clocks.stop()
+    series = series_ran(precision, res, launches, args.steps)
 
     fp64_leg = None
     mixed_vs_oracle = None
     if precision == "mixed":
-        r64, ms64, k64, _ = timed("fp64", args.fp64_steps, args.fp64_warmup)
+        r64, ms64, k64, launches64 = timed("fp64", args.fp64_steps, args.fp64_warmup)
+        series64 = series_ran("fp64", r64, launches64, args.fp64_steps)
         a, b = res.achtemp.cpu().numpy(), r64.achtemp.cpu().numpy()
         x, y = res.asxtemp.cpu().numpy(), r64.asxtemp.cpu().numpy()
 
@@ -609,11 +631,9 @@ def main() -> int:
         if k64ms and fp64_peak:
             # The FP64 kernel against the measured FP64 FMA rate (algorithmic flops).
             a64 = unocc_terms * (FLOPS_PER_TERM_BASE + FLOPS_PER_TRIPLE / shape.nw) / (k64ms * 1e-3)
-            fp64_leg["roofline"] = {"bound": "fp64", "achieved": a64 * 1e-12, "peak": fp64_peak,
-                                    "unit": "TFLOP/s", "frac": a64 * 1e-12 / fp64_peak,
-                                    "kernel": SERIES_KERNELS["fp64"] if series else "noflag_fp64_kernel"}
-            if series:
-                fp64_leg["roofline"]["note"] = SERIES_NOTE
+            fp64_leg["roofline"] = series_roofline("fp64", a64 * 1e-12, fp64_peak, "fp64") if series64 else {
+                "bound": "fp64", "achieved": a64 * 1e-12, "peak": fp64_peak, "unit": "TFLOP/s",
+                "frac": a64 * 1e-12 / fp64_peak, "kernel": "noflag_fp64_kernel"}
 
     # End to end through the host-buffer C-ABI call: pinned host inputs
     # (which the library pulls with a kernel on the SMs, overlapped with the
@@ -681,9 +701,9 @@ def main() -> int:
     if issued:
         roofline["issued"] = issued
     if series:
-        roofline["kernel"], roofline["note"] = SERIES_KERNELS[precision], SERIES_NOTE
         for k in ("ncu_pipe_note", "traffic_note"):
             roofline.pop(k)
+        roofline.update(series_roofline(roofline["bound"], achieved, peak, precision))
 
     line = {"metric": METRIC, "value": job_terms / (ms * 1e-3), "unit": "terms/s",
             "n_gpus": ws, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,

@@ -40,9 +40,12 @@
 // small.  So both are summed for every band first (weighted as the rows are;
 // |aqsn| and |Q| in bf16, one product on the tensor cores), and a band whose
 // ratio of the two passes kSpread is computed term by term: up to there the
-// fixed point's rounding, ratio 2^-58 of the sum of |aqsn Q| at worst, is no more
-// than the per-term roundings.  Uniform data gives 5, a chunk over which both
-// factors fall by e^2 12.
+// fixed point's rounding, about ratio 2^-57 of a term (all of the series' terms
+// together), is no more than a term's in the per-term sums with their
+// accumulation over the columns (2^-51).  Measured without the limit, 62 x 17 x
+// 5003, FP64, at ratios of 3 to 87: 2.4e-16 of the band totals at all of them,
+// per term 2.9e-16.  Uniform data gives 3 to 5, a chunk over which both factors
+// fall by e^2 12.
 //
 // The box is chosen on the device from a histogram of Re(wtilde) against the
 // histogram of wx, by the cost of what it leaves over; where no box pays, or
@@ -90,7 +93,7 @@ namespace {
 
 constexpr int kBins = 512;
 constexpr int kNearTile = 4;  // entries per block of the FP64 near kernel
-constexpr double kSpread = 32.0;
+constexpr double kSpread = 64.0;
 
 struct Sizes {
     int bands, ng, nc, nw;
@@ -847,21 +850,20 @@ __global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const
 // Residue planes and exponents of P_k, k = k0 .. k0 + gm - 1, for 8 rows x one
 // chunk at level L, of the gr rows from r0 on: row r0 + l of term m is row
 // m gr + l of the product's Y operand, in the core-matrix blocks of
-// crt_prep_kernel.  A thread carries 4
-// consecutive columns of a row (half a core-matrix row; 8 would halve the
-// resident warps) through the recurrence P_(k+1) = 2 z P_k - P_(k-1) (P_-1 =
-// z Q starts it) and leaves P_(k-1), P_k for the next pass in `state`.  The
-// exponent of term k is that of the chunk's largest |re|, |im| of Q, raised by
-// the bound rho^k of |T_k| and 1.  Q is scaled by the chunk's exponent first:
-// the terms of a chunk at either end of FP64's range keep their precision.
-// Columns outside the box are zero.
-constexpr int kTermK = 4;  // columns per thread
+// crt_prep_kernel.  A thread carries 4 consecutive columns of a row (half a
+// core-matrix row; 8 would halve the resident warps) through the recurrence
+// P_(k+1) = 2 z P_k - P_(k-1) (P_-1 = z Q starts it) and leaves P_(k-1), P_k for
+// the next pass in `state`.  The exponent of term k is that of the chunk's
+// largest |re|, |im| of Q, raised by the bound rho^k of |T_k| and 1.  Q is scaled
+// by the chunk's exponent first: the terms of a chunk at either end of FP64's
+// range keep their precision.  Columns outside the box are zero.
 //
 // In mixed precision the recurrence runs in float-float (DF): FP64 kept its
 // pipe 62-76% busy with 4 instructions per term and column where the residues
 // take most of the issue slots.  1638 x 32768, 25 terms: 26 -> 19 ms.  Only the
 // first pass reads the inputs, the next ones find z with the last two terms in
 // `state`.
+constexpr int kTermK = 4;  // columns per thread
 template <int L, bool DF>
 __global__ void __launch_bounds__(128, 4) far_terms_kernel(Problem p, const FarPlan *f, int ngp, int r0, int gr, int c0,
                                                            int nc, int Kc, int Np, int k0, int gm,
