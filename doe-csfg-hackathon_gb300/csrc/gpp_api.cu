@@ -149,8 +149,6 @@ struct OutSpec {
     int accumulate = 0;
 };
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-
 // Pipeline variant of the mixed kernel per (device, frequency chunk): chosen
 // by gpp_autotune or gpp_set_variant, else the compiled-in default.  A
 // thread-local override lets the autotuner time each variant.
@@ -248,13 +246,6 @@ bool overlap_occupied() {
 bool overlap_tensor_gemm() {
     const char *v = getenv("GPP_OVERLAP_TENSOR_GEMM");
     return !(v && v[0] == '0');
-}
-
-int sm_count() {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
 }
 
 gpp_status side_stream(int dev, SideStream **out) {

@@ -106,8 +106,6 @@ Geometry geometry(int M, int N, int K, int splits) {
     return g;
 }
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-
 struct Buffers {
     __nv_bfloat16 *sx, *sy;  // [kPlanes][rows][slab k], core-matrix blocks
     int *ex, *ey;            // [slab chunks][rows]
@@ -662,13 +660,6 @@ __global__ void __launch_bounds__(128, 5) crt_combine_kernel(const unsigned char
         for (int j = 0; j < 4; ++j)
             if (col0 + j < N) out[j] = acc[j];
     }
-}
-
-int sm_count() {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 132;
 }
 
 // Pairs of blocks (cta_group::2): each SM then reads half of Y's block for the

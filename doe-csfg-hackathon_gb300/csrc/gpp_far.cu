@@ -199,8 +199,6 @@ Sizes sizes(const Problem &p, int bands, bool mixed) {
     return z;
 }
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-
 struct Buffers {
     FarPlan *plan;
     int4 *near;
@@ -1308,13 +1306,6 @@ __global__ void __launch_bounds__(256) far_final_kernel(Problem p, const FarPlan
         else
             part.ach[(long long)iw * part.ach_seg + part.ach_tile0] = make_double2(S[0], S[1]);
     }
-}
-
-int sm_count() {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 132;
 }
 
 }  // namespace

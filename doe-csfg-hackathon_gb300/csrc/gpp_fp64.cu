@@ -152,13 +152,6 @@ cudaError_t launch_noflag_t(const Problem &p, const Partials &part, int b0, int 
     return cudaGetLastError();
 }
 
-int sm_count() {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Occupied bands in pairs when the frequencies are band-independent (the
 // solver once per pair; the same bits).  GPP_FLAG_MULTI=0 keeps one band per
 // block, read on every call.

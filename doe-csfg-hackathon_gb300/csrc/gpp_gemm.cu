@@ -46,8 +46,6 @@ gpp_status set_error(gpp_status s, const char *msg);
 
 namespace {
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-
 gpp_status cuda_fail(cudaError_t e, const char *what) {
     char buf[256];
     snprintf(buf, sizeof(buf), "%s: %s", what, cudaGetErrorString(e));

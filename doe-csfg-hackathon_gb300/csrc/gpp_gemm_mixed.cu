@@ -44,7 +44,6 @@ constexpr int kGMinBlocks = 3;
 constexpr int kHBands = 64;    // H: bands per block
 constexpr int kHMinBlocks = 5;
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 int row_pairs(const Problem &p) { return (p.ng + 1) / 2; }
 
 gpp_status cuda_fail(cudaError_t e, const char *what) {

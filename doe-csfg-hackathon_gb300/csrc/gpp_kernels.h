@@ -21,6 +21,14 @@ TileShape fp64_noflag_shape(const Problem &p);
 TileShape flag_shape(const Problem &p);
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
+// SMs of the current device (GB300's where the runtime does not say).
+inline int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 152;
+}
 
 // A range of row tiles [begin, end).  Every kernel family tiles G' rows in
 // pairs (RG = 2), so a row-pair range means the same rows to all of them;

@@ -123,8 +123,6 @@ Geometry geometry(int M, int N, int K, int splits) {
     return g;
 }
 
-size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
-
 struct Buffers {
     __nv_bfloat16 *sx, *sy;
     int *ex, *ey, *exmax, *eymax;

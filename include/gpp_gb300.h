@@ -286,7 +286,10 @@ gpp_status gpp_batch_destroy(gpp_batch *batch);
  * fastest for problems with the same frequency chunk on the current device,
  * and writes the choice to the file named by the GPP_TUNE_CACHE environment
  * variable, if set (read back on first use).  gpp_set_variant overrides the
- * choice (-1 restores the default); gpp_tuned_variant reports it.
+ * choice (-1 restores the default); gpp_tuned_variant reports it.  Calls that
+ * take the series have a tile of one shape for the pairs they sum term by term;
+ * the variant is that of the calls that do not, and of those whose state the
+ * device finds not to pay.
  * ------------------------------------------------------------------------ */
 gpp_status gpp_autotune(const gpp_problem *problem, int max_bands, gpp_stream_t stream,
                         int *best_variant);
