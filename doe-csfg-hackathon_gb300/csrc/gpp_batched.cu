@@ -335,6 +335,8 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
             if (how == Direct::kHeld) {
                 const gpp_status st = sigma_scratch(q, outs[i], &bytes);
                 if (st != GPP_OK) return st;
+                if (bytes > split_budget)
+                    return set_error(GPP_ERR_OUT_OF_MEMORY, "a state's scratch is more than the batch's share of the device's memory");
             }
             direct_bytes = std::max(direct_bytes, bytes);
             b->direct_problems.push_back(q);
@@ -433,8 +435,8 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     }
     const size_t off_jobs = reserve(sizeof(BatchReduce) * b->jobs.size());
     const size_t off_prefix = reserve(sizeof(int) * (b->jobs.size() + 1));
-    const size_t off_split = reserve(mixed ? max_wave : 0);
-    const size_t off_direct = reserve(direct_bytes);
+    // The states with scratch of their own run after the waves: one region.
+    const size_t off_split = reserve(std::max(mixed ? max_wave : 0, direct_bytes));
     b->dev_bytes = off;
 
     cudaError_t e = cudaGetDevice(&b->device);
@@ -449,7 +451,7 @@ gpp_status plan_batch(gpp_batch *b, const gpp_problem *problems, const gpp_outpu
     b->d_prefix = reinterpret_cast<int *>(d + off_prefix);
     b->d_heads = reinterpret_cast<int *>(d + off_heads);
     b->d_split = d + off_split;
-    if (direct_bytes) b->direct_scratch = Scratch{d + off_direct, direct_bytes};
+    if (direct_bytes) b->direct_scratch = Scratch{d + off_split, direct_bytes};
 
     // Per-state partial pointers (the fault word is filled in by
     // upload_tables), split planes and reduction sources.
@@ -649,6 +651,7 @@ gpp_status enqueue(gpp_batch *b, cudaStream_t s) {
     return GPP_OK;
 }
 
+// What a plan takes for split planes, and for the series' scratch, at most.
 size_t default_split_budget() {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return (size_t)16 << 30;

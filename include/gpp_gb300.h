@@ -266,7 +266,8 @@ gpp_status gpp_sigma_batched(const gpp_problem *problems, const gpp_outputs *out
 
 /* Reusable plan: the work list, device tables and scratch are built once
  * (gpp_batch_create allocates, the scratch of the largest state that takes the
- * series among it, and plans all states term by term where that cannot be had;
+ * series among it, and plans all states term by term where that cannot be had
+ * or is more than a quarter of the free memory and 1 GB;
  * runs allocate nothing; the arrays behind the problems' pointers may change
  * contents between runs but not move).  gpp_batch_run enqueues a run
  * on `stream`; on a stream other than the legacy/per-thread default the

@@ -147,3 +147,22 @@ def test_no_room_inside_a_capture():
         got = out.achtemp.cpu().numpy()
         assert not np.array_equal(got, want)
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+def test_planes_and_scratch_share_their_memory():
+    """A plan's split planes and the scratch of its states that take the series
+    are one region, used one after the other: a plan of two such states and a
+    small one, run several times, gives every state the bits it has alone."""
+    from gppsigma import ops
+    inputs = [W.make_inputs(W.Shape(64, 2, 20003, 40, 32, dw=0.25), 3),
+              W.make_inputs(W.Shape(40, 2, 3000, 30, 32), 5),
+              W.make_inputs(W.Shape(66, 1, 19001, 42, 32, dw=0.25), 4)]
+    plan, stream = _Plan(inputs, "mixed"), torch.cuda.Stream()
+    runs = [plan.run(stream) for _ in range(3)]
+    plan.close()
+    for k, inp in enumerate(inputs):
+        r = ops.sigma(ops.DeviceInputs.from_host(inp), "mixed", acht_n1=True)
+        ops.wait()
+        want = [r.achtemp.cpu().numpy(), r.asxtemp.cpu().numpy(), r.acht_n1_loc.cpu().numpy()]
+        for got in runs:
+            assert all(np.array_equal(x, y) for x, y in zip(got[k], want))
