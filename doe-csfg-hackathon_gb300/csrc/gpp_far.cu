@@ -740,8 +740,10 @@ __device__ __forceinline__ int fixed_point32(double x, int e, int bits) {
 // E of the largest |re|, |im|, the magnitudes over 2^E in bf16 (core-matrix
 // blocks of R rows) and their sum S.  Y: rows of Q, 0 outside the box; else
 // rows of aqsn, from row b0 on; E and S have a row of ld per chunk.  A thread
-// per 8 consecutive columns of a row, which it reads twice (from L1 and L2 the
-// second time).
+// per 8 consecutive columns of a row, which it reads twice (from L2 the second
+// time): Q in FP64 for its exponent and the box, then the magnitudes in float,
+// |Q| as |wtilde| |I_eps| (1638 x 32768: 1.3 ms, bound by the first; 2.2 with
+// both in FP64).
 template <bool Y>
 __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan *f, int b0, int L, int Lp,
                                                         int ld, int c0, int nc, int Kc, int *E, float *S,
@@ -753,18 +755,21 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
     __shared__ int exps[8];
     const int groups = Lp / 8, l0 = blockIdx.x % groups * 8, c = blockIdx.x / groups;
     const int t = threadIdx.x, row = t & 7, l = l0 + row, kb = (c0 + c) * Kc, end = min(p.nc, kb + Kc);
-    auto value = [&](int ig) {
-        if (l >= L || ig >= end) return make_double2(0.0, 0.0);
-        const size_t at = (size_t)(b0 + l) * p.nc + ig;
-        if constexpr (!Y) return __ldg(p.aqsn + at);
-        const double2 wt = __ldg(p.wt + at);
-        return in_box(*f, wt) ? cmul(wt, __ldg(p.ieps + at)) : make_double2(0.0, 0.0);
-    };
+    const double2 *at = (Y ? p.wt : p.aqsn) + (size_t)(b0 + l) * p.nc, *ie = p.ieps + (size_t)(b0 + l) * p.nc;
     unsigned long long mx = 0;
+    unsigned in = 0;  // the columns that count, in the order of the loops (at most 4 x 8)
+    int bit = 0;
     for (int k = t >> 3; k < Kc / 8; k += 16)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const double2 v = value(kb + k * 8 + j);
+        for (int j = 0; j < 8; ++j, ++bit) {
+            const int ig = kb + k * 8 + j;
+            if (l >= L || ig >= end) continue;
+            double2 v = __ldg(at + ig);
+            if constexpr (Y) {
+                if (!in_box(*f, v)) continue;
+                v = cmul(v, __ldg(ie + ig));
+            }
+            in |= 1u << bit;
             const unsigned long long a = (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
             const unsigned long long b = (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
             mx = max(mx, max(a, b));
@@ -781,12 +786,25 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
     __syncthreads();
     const int e = exps[row], ksteps = nc * (Kc / kCrtBlockK);
     __nv_bfloat16 *w0 = out + ((size_t)(l0 / R) * ksteps * (R / 8) + (size_t)(l0 % R) / 8) * 512 + row * 8;
-    // |x| 2^-e from the bits (top 20 of the mantissa); near FP64's lower end by FP64.
-    auto over = [&](double x) {
-        if (e < -1000) return fabsf((float)ldexp(x, -e));
-        const int hi = __double2hiint(x) & 0x7FFFFFFF, sh = (hi >> 20) - 1022 - e;
-        return sh < -60 ? 0.f : __int_as_float(((sh + 126) << 23) | ((hi & 0xFFFFF) << 3));
+    // |z| 2^-e2, each part from its bits (the top 20 of the mantissa), between
+    // 2^-120 and 2^120.  wtilde is taken over the box's exponent eb, I_eps over
+    // 2^(e - eb); near FP64's lower end by FP64.
+    const int eb = Y ? ilogb(fabs(f->z0) + f->h) + 2 : 0;
+    auto over = [&](double2 z, int e2) {
+        float m[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double x = h ? z.y : z.x;
+            const int hi = __double2hiint(x) & 0x7FFFFFFF, sh = min((hi >> 20) - 1022 - e2, 120);
+            m[h] = e2 < -900 ? (float)fmin(fabs(ldexp(x, -e2)), 0x1p120)
+                   : sh < -120 ? 0.f
+                               : __int_as_float(((sh + 126) << 23) | ((hi & 0xFFFFF) << 3));
+        }
+        // Within 4% of the magnitude (a square would leave float's range).
+        return fmaxf(0.96f * fmaxf(m[0], m[1]) + 0.4f * fminf(m[0], m[1]), fmaxf(m[0], m[1]));
     };
+    if (e == kExpNonFinite || e == kExpZero) in = 0;
+    bit = 0;
     float total = 0.f;
     for (int k = t >> 3; k < Kc / 8; k += 16) {
         unsigned v[4];
@@ -795,9 +813,14 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
             float m[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const double2 x = value(kb + k * 8 + 2 * j + h);
-                const float a = over(x.x), b = over(x.y);
-                m[h] = e == kExpNonFinite || e == kExpZero ? 0.f : sqrtf(a * a + b * b);
+                m[h] = 0.f;
+                const int ig = kb + k * 8 + 2 * j + h;
+                if ((in >> bit++) & 1) {
+                    if constexpr (Y)
+                        m[h] = over(__ldg(at + ig), eb) * over(__ldg(ie + ig), e - eb);
+                    else
+                        m[h] = over(__ldg(at + ig), e);
+                }
             }
             const __nv_bfloat162 q = __floats2bfloat162_rn(m[0], m[1]);
             total += __low2float(q) + __high2float(q);
@@ -815,7 +838,8 @@ __global__ void __launch_bounds__(128) far_sizes_kernel(Problem p, const FarPlan
 
 // spread[n] (+)= over the rows [r0, r0 + rows) and chunks [c0, c0 + nc): |c| 2^(EA + E0) times
 // SA + SQ (the largest magnitudes count 1 each) and times V, the chunk's sum of
-// products.
+// products.  A row's chunks are summed in float over its largest E0 and the
+// band's largest EA (512 x 1638 x 64 chunks: 0.26 ms, 1.0 in FP64).
 __global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const double2 *C, const int *EA,
                                                          const int *E0, const float *SA, const float *SQ,
                                                          const float *V, int ng, int ngp, int r0, int rows,
@@ -824,19 +848,25 @@ __global__ void __launch_bounds__(256) far_spread_kernel(const FarPlan *f, const
     if (!f->active) return;
     __shared__ double red[16], S[2];
     const int n = blockIdx.x;
+    int ea = kExpZero;
+    for (int c = 0; c < nc; ++c) ea = max(ea, EA[(size_t)(c0 + c) * Mp + n]);
     double v[2] = {0.0, 0.0};
     for (int r = threadIdx.x; r < rows; r += 256) {
-        const double2 z = C[(size_t)n * ng + r0 + r];
-        double a = 0.0, b = 0.0;
+        const int *e0 = E0 + (size_t)c0 * ngp + r0 + r;
+        int er = kExpZero;
+        for (int c = 0; c < nc; ++c) er = max(er, e0[(size_t)c * ngp]);
+        float a = 0.f, b = 0.f;
         for (int c = 0; c < nc; ++c) {
-            const size_t x = (size_t)(c0 + c) * Mp + n, y = (size_t)(c0 + c) * ngp + r0 + r;
-            const double w = scalbn(1.0, EA[x] + E0[y]);
-            a = fma(w, (double)(SA[x] + SQ[y]), a);
-            b = fma(w, (double)V[((size_t)c * Mp + n) * Np + r], b);
+            const size_t x = (size_t)(c0 + c) * Mp + n, y = (size_t)c * ngp;
+            const int ex = EA[x] - ea + e0[y] - er;  // at most 0
+            const float w = ex < -126 ? 0.f : __int_as_float((127 + ex) << 23);
+            a = fmaf(w, SA[x] + SQ[(size_t)c0 * ngp + r0 + r + y], a);
+            b = fmaf(w, V[((size_t)c * Mp + n) * Np + r], b);
         }
-        const double m = sqrt(z.x * z.x + z.y * z.y);
-        v[0] = fma(m, a, v[0]);
-        v[1] = fma(m, b, v[1]);
+        const double2 z = C[(size_t)n * ng + r0 + r];
+        const double m = scalbn(sqrt(z.x * z.x + z.y * z.y), ea + er);
+        v[0] = fma(m, (double)a, v[0]);
+        v[1] = fma(m, (double)b, v[1]);
     }
     block_reduce<2, 256>(v, red, S);
     if (threadIdx.x == 0) {
