@@ -24,9 +24,9 @@
 // combination left 5e-15.
 //
 // GB300, 1638 x 32768 over 510 bands / 510 x 1638 over 32768 columns: prepare
-// 0.35 / 1.3 ms, products 1.42 / 1.75 ms (1.73 / 1.41 PFLOP/s), combine 1.0 /
-// 1.0 ms; the slices took 0.4 / 1.3, 4.6 / 5.4 and 1.3 / 1.4 ms.  The products
-// are bound by the tensor pipe (91% of what a library GEMM reaches).
+// 0.36 / 1.4 ms, products 1.54 / 1.87 ms (1.71 / 1.41 PFLOP/s), combine 1.0 /
+// 1.1 ms; the slices took 0.4 / 1.3, 4.6 / 5.4 and 1.3 / 1.4 ms.  The products
+// are bound by the tensor pipe (90% of what a library GEMM reaches).
 //
 // crt_gemm_kernel keeps the core-matrix operand layout and the bulk-copy /
 // tcgen05.mma / TMEM pipeline of gpp_ozaki.cu and makes each block

@@ -53,13 +53,13 @@
 // here returns at once and the per-term kernel runs instead.  No host
 // synchronisation; nothing depends on the order in which blocks run.
 //
-// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 22 ms now (near
-// pairs 15, products 2.6, terms 2.7, combine 1.5); mixed, 128 bands x 819 x 16384
-// x 32: 120 ms per term, 34 now (near 23, terms 5.2, products 4.2); 512 bands x
-// 1638 x 32768 x 3, 1% strays: 210 per term, 122 now (near 57, products 23,
-// terms 19, strays 14, combine 13).  The near kernels run at 1.25 (FP64) and
-// 1.4 (mixed) of the per-term kernels' time per pair: an entry holds 1.8
-// frequencies on average where a tile there shares its columns among 3.
+// GB300, FP64, 512 bands x 409 x 8192 x 3: 102.9 ms per term, 23-25 now (near
+// pairs 15, products 3.2, terms 3.0, combine 1.6); mixed, 128 bands x 819 x 16384
+// x 32: 120 ms per term, 36 now (near 23, terms 5.5, products 4.6); 512 bands x
+// 1638 x 32768 x 3, 1% strays: 210 per term, 129 now (near 57, products 24,
+// terms 19, strays 14, combine 13, spread 1.7).  The near kernels run at 1.25
+// (FP64) and 1.4 (mixed) of the per-term kernels' time per pair: an entry holds
+// 1.8 frequencies on average where a tile there shares its columns among 3.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -1345,8 +1345,10 @@ bool far_eligible(const Problem &p, int bands, bool mixed) {
     const Sizes z = sizes(p, bands, mixed);
     // The series and, say, a sixth of the pairs near must leave a gain, on a
     // call long enough for the fixed launches: 3 ms of per-term work, in FP64
-    // 2.2 (per term / series, ms, at estimates of 1.3, 1.7, 2.5 and 2.8 ms: 1.48
-    // / 1.81, 1.86 / 1.91, 2.97 / 2.26, 2.88 / 2.08).
+    // 2.2 (per term / series, ms: FP64 at estimates of 2.5 and 2.6 ms 2.88 / 2.47
+    // and 2.66 / 2.24, before the bands' spread was formed 1.86 / 1.91 at 1.7; mixed at
+    // 3.0, 3.0 and 3.3 ms 3.17 / 3.02, 2.93 / 2.28 and 3.39 / 3.03).  A chunk of X's
+    // planes has to fit the scratch (87,000 bands), and with it the grids do.
     const double cells = (double)p.ng * p.nc;
     const double per_pair = mixed ? 2.6e-12 : 20e-12;
     // Calls whose sizes leave no gain do not plan (330 x 73 x 25601 x 2, mixed:

@@ -655,7 +655,7 @@ int grid_for(long long n) {
 
 }  // namespace
 
-// The products take the residues of gpp_crt.cu: 45 real products instead of
+// The products take the residues of gpp_crt.cu: 48 real products instead of
 // 108 (measured, slices against residues: 4.5 and 2.2 ms for 1638 x 32768 over
 // 64 k, 0.30 and 0.03 ms for 40 x 800), and no size was found where slices
 // were faster.  GPP_TENSOR_GEMM=slices in the environment (read on every
