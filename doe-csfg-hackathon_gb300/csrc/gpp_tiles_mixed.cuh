@@ -481,9 +481,8 @@ __device__ __forceinline__ df2 df2_mask(const df2 &a, bool x, bool y) {
 }
 
 // An occupied-band term near the pole, in FP64 from the original inputs,
-// split to float-float: aqsn*sch (sr, si) and its wx^2 aqsn*ssx (aqsn*ssx where
-// the frequency is not plain), less its share of the sum over all columns (xr,
-// xi).  Out of line: inlined, its FP64
+// split to float-float: aqsn*sch (sr, si) and its wx^2 aqsn*ssx, less its
+// share of the sum over all columns (xr, xi).  Out of line: inlined, its FP64
 // code took registers from the float-float term loop.
 struct FlagPole {
     df sr, si, xr, xi;
@@ -511,8 +510,16 @@ struct FlagFreqM {
     float clear;   // max(limittwo, (1e-3 wx)^2) with a margin above rounding
     float keep;    // |wtilde|^2 clearly below the cutoff (or no cutoff)
     bool most, cut;
-    bool plain;    // else every term goes through FP64, and clear is infinite
 };
+
+// A tile with a frequency that is not plain (FlagFreq): in FP64 as a whole, since
+// 1/wx^2 takes its terms out of float's range.  Out of line, for the rare call.
+template <int RG, int NWC, int THREADS, int SEM>
+static __device__ __noinline__ void flag_wide_tile(const Problem &p, const Partials &part, int row_tile,
+                                                   int band, int iw_chunk, double *red, double *S) {
+    flag_fp64_tile<RG, NWC, 1, THREADS, SEM>(p, part, row_tile, band, iw_chunk, (p.ng + RG - 1) / RG,
+                                             red, S);
+}
 
 // One occupied-band tile in mixed precision: the row pair row_tile, one band,
 // frequencies iw_chunk*NWC..; reads the float-float split planes (bands
@@ -522,8 +529,7 @@ struct FlagFreqM {
 // away from the pole takes one straight-line path of packed instructions;
 // any other term works out each lane's branch (df_gt: exact near the
 // thresholds) and zeroes the lanes a branch does not take.  Terms within
-// 1e-3 |wx| of the pole, and all of a frequency that is not plain, are computed
-// in FP64 from the inputs.
+// 1e-3 |wx| of the pole are computed in FP64 from the inputs.
 // ~78 packed instructions per frequency of a row pair and ~96 per column on
 // the straight-line path; three blocks of four warps an SM cannot hide a
 // column's five loads behind them (the FMA pipe 53% busy), so each thread
@@ -555,7 +561,7 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
     const double *wxp = p.wx + (size_t)band * p.wx_stride;
     FlagFreqM f[NWC];
     double bound64 = kFlagNoBound;
-    bool any_most = false;
+    bool any_most = false, all_plain = true;
 #pragma unroll
     for (int w = 0; w < NWC; ++w) {
         const FlagFreq d = flag_freq<SEM>(__ldg(wxp + min(iw0 + w, p.nw - 1)));
@@ -565,10 +571,13 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
         f[w].keep = d.cut ? 0.99998f * f[w].c4.h : __int_as_float(0x7F800000);
         f[w].most = d.most;
         f[w].cut = d.cut;
-        f[w].plain = d.plain;
-        if (!d.plain) f[w].clear = __int_as_float(0x7F800000);
+        all_plain &= d.plain;
         bound64 = flag_bound(bound64, d);
         any_most |= d.most;
+    }
+    if (!all_plain) {
+        flag_wide_tile<RG, NWC, THREADS, SEM>(p, part, row_tile, band, iw_chunk, red, S);
+        return;
     }
     const float bound = (float)fmin(bound64, 3e38);
     const df2 z = {f2(0.f, 0.f), f2(0.f, 0.f)};
@@ -646,7 +655,7 @@ __device__ __forceinline__ void flag_mixed_tile(const Problem &p, const Partials
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
                 const df dg = df2_lane(d, g), wg = df2_lane(delwr, g);
-                pole[g] = dg.h < thr || !f[w].plain;
+                pole[g] = dg.h < thr;
                 in_a[g] = !pole[g] && df_gt(dg, df{kLim2H, kLim2L}) && df_gt(df{kLim1H, kLim1L}, wg);
                 inc[g] = in_a[g] && !(f[w].cut && df_gt(df2_lane(awt2, g), f[w].c4));
                 in_b[g] = !pole[g] && !in_a[g] && df_gt(wg, df{kTo1H, kTo1L});

@@ -50,3 +50,25 @@ def test_branch_b_at_any_frequency(precision, tol, semantics, one_row, acht_n1):
     if not one_row:  # sch: the unoccupied bands' frequencies are ordinary
         ach = r.achtemp.cpu().numpy()
         assert np.max(np.abs(ach - want["achtemp"])) <= tol * np.max(np.abs(want["achtemp"]))
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-8)])
+@pytest.mark.parametrize("one_row", [True, False])
+def test_branch_a_far_past_the_range_of_float(precision, tol, one_row):
+    """wx of 1e-20 with |wtilde| above 0.5 (branch A): ssx is 1e40 times Omega2, past
+    float's range; wx of 1e17, where it is 1e-34 of it."""
+    import oracle_py
+    from gppsigma import ops
+    wx = [1e-20, -1e-20, 2.0, 1e17]
+    inp = W.make_inputs(W.Shape(40, 3, 300, 13, len(wx)), 3)
+    if one_row:
+        inp.wx_array = np.array([wx])
+    else:
+        inp.wx_array[:3] = wx
+    want = oracle_py.run(inp, "kerseq", nthreads=4)
+    r = ops.sigma(ops.DeviceInputs.from_host(inp), precision, "kerseq")
+    ops.wait()
+    got = r.asxtemp.cpu().numpy()
+    assert np.all(np.isfinite(want["asxtemp"])) and abs(want["asxtemp"][0]) > 1e38
+    for w in range(len(wx)):
+        assert abs(got[w] - want["asxtemp"][w]) <= tol * abs(want["asxtemp"][w]), wx[w]
